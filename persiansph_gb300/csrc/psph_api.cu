@@ -476,6 +476,7 @@ void derive_class_options(const std::vector<PClass>& classes, bool mixed, bool d
   if (o.eos_cls < 0) o.eos_cls = 0;
   // two materials: a wall takes its density from its partner's EOS pair by pair
   if (mixed) o.uniform_eos = 0;
+  double m_u = 0.0, wall_u = 1.0;  // the free particles' mass, the walls' FPMassC
   // pair constants that are the same for every class: the FP32C fluid pair
   // loop takes them from the launch parameters (the same FP32 values the class
   // table holds, so the results are identical)
@@ -494,6 +495,8 @@ void derive_class_options(const std::vector<PClass>& classes, bool mixed, bool d
     o.beta32 = (float)C0.beta;
     o.m_free32 = (float)std::max(m_free, 0.0);
     o.fpm_wall32 = (float)std::max(fpm_wall, 0.0);
+    m_u = m_free;
+    wall_u = fpm_wall;
   }
   o.uniform_mu = !dyn_mu;
   o.mu_u = 0.0;
@@ -508,6 +511,40 @@ void derive_class_options(const std::vector<PClass>& classes, bool mixed, bool d
     if (!(o.mu_u > 0.0)) o.uniform_mu = 0;
   }
   o.inv_h = 1.0 / classes[0].h;
+  // (W(r) / W(TIInitDist))^TIn: not finite with TIInitDist outside the support or TIn < 0
+  {
+    double tid = 0.0, h = classes[0].h;
+    bool odd = false;
+    for (const PClass& C : classes) {
+      tid = std::max(tid, C.tid);
+      h = std::min(h, C.h);
+      odd = odd || !(C.tin >= 0.0) || !(C.tid >= 0.0);
+    }
+    o.ti_always = odd || !(tid < 0.99 * (o.kt == PSPH_QUINTIC_SPLINE ? 3.0 : 2.0) * h);
+  }
+  // the FP64 fluid pair kernel's SPEC form (psph_forces.cu)
+  o.spec64 = o.vis_eq == PSPH_MORRIS && o.grad_type == PSPH_SQUARED_DENSITY && o.uniform_h && o.uniform_av &&
+             o.uniform_mass && o.uniform_mu && o.uniform_eos && !o.any_ti && !o.need_sr && !mixed;
+  {
+    const PClass& C0 = classes[0];
+    const double cw = o.kt == 0 ? (o.dim == 2 ? Kern<2, 0>::cw() : Kern<3, 0>::cw())
+                    : o.kt == 1 ? (o.dim == 2 ? Kern<2, 1>::cw() : Kern<3, 1>::cw())
+                                : (o.dim == 2 ? Kern<2, 2>::cw() : Kern<3, 2>::cw());
+    const double ih2 = o.inv_h * o.inv_h;
+    const double cwh = cw * (o.dim == 2 ? ih2 : ih2 * o.inv_h);
+    o.spec.h = C0.h;
+    o.spec.inv_h = o.inv_h;
+    o.spec.cwh_m = cwh * m_u;
+    o.spec.cwg_m = cwh * ih2 * m_u;
+    o.spec.eps2 = 0.01 * C0.h * C0.h;
+    o.spec.neg_alpha_h = -C0.alpha * C0.h;
+    o.spec.beta_h = C0.beta * C0.h;
+    o.spec.mu2 = 2.0 * o.mu_u;
+    o.spec.wall_scale = wall_u;  // a wall's mass is FPMassC times its partner's
+    o.spec.wall_scaled = wall_u >= 0.0 && wall_u != 1.0;
+    o.spec.av_beta = C0.beta != 0.0;
+    o.spec.av = C0.alpha != 0.0 || C0.beta != 0.0;
+  }
 }
 
 psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
@@ -920,11 +957,13 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
   if (o.couple_soil && o.swi != 2 && (st = dalloc(c, &S.satcheck, N))) return st;
   if (o.couple_solid && ((st = dalloc(c, &S.fsi_p, N)) || (st = dalloc(c, &S.fsi_nsv, N)))) return st;
   if ((st = dalloc(c, &S.nl, (size_t)o.nl_cap * nl_stride_of(c->ncap)))) return st;
+  if (!o.fp32 && (st = dalloc(c, &S.pair_info, N))) return st;
   // FP64 fluids without strain-rate sums, XSPH or solids: each pair evaluated once
   o.fp64_half = !o.fp32 && !o.has_solid && !o.need_sr && o.xsph == 0.0;
   if (o.fp64_half) {
     const size_t slots = (size_t)o.nl_cap * nl_stride_of(c->ncap);
-    if ((st = dalloc(c, &S.half4, slots)) || (st = dalloc(c, &S.half2, slots)) ||
+    if ((st = dalloc(c, &S.half4, slots)) || (st = dalloc(c, &S.half_zw, slots)) ||
+        (o.any_shepard && (st = dalloc(c, &S.half_sd, slots))) ||
         (st = dalloc(c, &S.half_stamp, slots)))
       return st;
   }
@@ -2075,6 +2114,10 @@ psph_status patch_impl(psph_ctx* c, const psph_particles* p) {
     CUDA_TRY(c, cudaMemcpyAsync(c->d_cls, c->classes.data(), c->classes.size() * sizeof(PClass),
                                 cudaMemcpyHostToDevice, s));
     launch_class_constants(c->d_cls, (int)c->classes.size(), o.dim, s);
+    // constants the pair kernel takes from the launch may no longer be shared
+    c->opt.spec64 = o1.spec64;
+    c->opt.ti_always = o1.ti_always;
+    c->opt.spec = o1.spec;
     c->opt.nclasses = (int)c->classes.size();
     int* dnext = reinterpret_cast<int*>(c->dl_buf);
     CUDA_TRY(c, cudaMemcpyAsync(dnext, next.data(), (size_t)m * sizeof(int), cudaMemcpyHostToDevice, s));

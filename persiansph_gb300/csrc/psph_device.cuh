@@ -58,8 +58,10 @@ struct Scratch {
   // FP64 once-per-pair form: a partner's terms of a pair, in the partner's own
   // list slot (nl_index layout): (a, dDensity) and (ZWab, SumDen)
   double4_32a* half4;
-  double2* half2;
+  double* half_zw;
+  double* half_sd;       // (on Shepard steps)
   int* half_stamp;       // instance step + 1 when the slot was written this step
+  int* pair_info;        // FP64 form: class | free << 16 | list in use << 17 (kInfo* of psph_forces.cu)
   double* zwab;
   double* s_acc;         // SWIType 1: Particle::S, the surface-erosion velocity derivative
   uint8_t* satcheck;     // fluid-soil: Particle::SatCheck of this step
@@ -86,12 +88,25 @@ struct Scratch {
   double* nut;           // eddy viscosity from the network; -1 = use Smagorinsky
 };
 
+// Pair constants of the FP64 fluid kernel's SPEC form (Options::spec64).
+struct Spec64 {
+  double h, inv_h;
+  double cwh_m, cwg_m;      // kernel normalisations cw / h^dim and cw / h^(dim+2), times a free particle's mass
+  double eps2;              // 0.01 h^2, the artificial viscosity's regularisation
+  double neg_alpha_h, beta_h;  // artificial viscosity, -alpha h and beta h
+  double mu2;               // twice the viscosity
+  double wall_scale;        // a wall's mass as its partner sees it over a free particle's
+  int av, av_beta;          // alpha or beta non-zero; beta non-zero
+  int wall_scaled;          // wall_scale is not 1
+};
+
 struct Options {
   int dim, kt, vis_eq, grad_type, scheme, wallp_physical;
   int fp32;           // PSPH_FP32C pair arithmetic
   int has_solid;      // any Material 2/3
   int any_av;         // any alpha/beta != 0
   int any_ti;         // any TI > 0
+  int ti_always;      // a tensile-instability power that may not be finite: evaluated for every pair
   int need_sr;        // strain rate needed (fluid T0>0 or LES)
   int any_shepard;
   int uniform_eos;    // all free particles of the material share one EOS class
@@ -116,6 +131,8 @@ struct Options {
   int uniform_av;     // every class has the same artificial-viscosity alpha and beta (alpha32, beta32)
   int uniform_mass;   // every free class has one mass (m_free32), every fixed class one FPMassC (fpm_wall32)
   float alpha32, beta32, m_free32, fpm_wall32;
+  int spec64;         // the FP64 fluid pair kernel's SPEC form applies, with these constants
+  Spec64 spec;
   double mu_u;        // that viscosity
   double inv_h;       // 1/h when uniform
   int nl_cap;         // neighbour-list capacity per particle

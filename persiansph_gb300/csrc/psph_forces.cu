@@ -132,21 +132,53 @@ PSPH_D void tensile_tir(const double* S, double TI, double rho, double* TIR) {
 }
 constexpr int kQN = 16;  // queued FP64 pair evaluations per lane between flushes
 
+// Lanes of a particle: kernels whose work is one particle's neighbour list give
+// each particle a group of 2^lg consecutive lanes of a warp.
+struct LaneGroup {
+  int sub, base;       // lane within the group, the group's first lane of the warp
+  unsigned bits;       // the group's lanes, counted from its first
+  PSPH_D explicit LaneGroup(int lg) {
+    const int lane = threadIdx.x & 31, L = 1 << lg;
+    sub = lane & (L - 1);
+    base = lane - sub;
+    bits = (L == 32) ? 0xffffffffu : ((1u << L) - 1u);
+  }
+};
+constexpr int kMinLanesLog2 = 2;  // the smallest lanes_log2
+// Sum over a group's lanes, in every lane (a fixed order: the butterfly's).
+PSPH_D double group_sum(double x, int lg) {
+  for (int o = 1; o < (1 << lg); o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+// What the pair loops need to know of a partner, in one word (pair_info, written
+// by prepare_wall_kernel): its class, whether it is free, whether its list is in use,
+// whether its tensile-instability stress is non-zero.
+constexpr int kInfoCls = 0xffff, kInfoFree = 1 << 16, kInfoList = 1 << 17, kInfoTir = 1 << 18;
+
+// kInfoTir of particle w, from its tensile-instability stress
+PSPH_D int tir_bit(const DevView& v, const Persist& P, int w) {
+  if (!v.o.any_ti || !P.tir) return 0;
+  const double* T = P.tir + 9 * (size_t)w;
+  long long b = 0;
+#pragma unroll
+  for (int e = 0; e < 9; ++e) b |= __double_as_longlong(T[e]);
+  return (b << 1) ? kInfoTir : 0;
+}
+
 // ---------------------------------------------------------------------------
 // Per-particle preparation and wall interpolation
 // ---------------------------------------------------------------------------
+// The wall interpolation of particles first .. first + (kFT >> lg) - 1 (those
+// that are fixed), 2^lg lanes each; every thread of the block calls it.
 template <int DIM, int KT>
-__global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v) {
-  const StepScalars* sc = v.sc;
-  if (sc->all_stop) return;
-  const Persist& P = cur_persist(v);
-  const int n = sc->n;
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int first, int n, double (*sums)[14]) {
+  const LaneGroup G(lg);
   const Options& o = v.o;
   const PClass* __restrict__ CT = v.cls;
+  int w = first + (threadIdx.x >> lg);
   const int winst = (w < n) ? CT[P.cls[w]].inst : 0;
   const GridDev& g = grid_of(v, winst);
-  const bool run = (w < n) && !v.inst[winst].stop;
   bool wall = false;
   int mat = 0;
   double sk = 0.0, p = 0.0, n0 = 0.0, n1 = 0.0, n2 = 0.0;
@@ -157,25 +189,17 @@ __global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v) {
   int ow = 0, cell = -1;
   double hw = 0.0;
   bool noslip = false;
-  if (run) {
+  if (w < n && !v.inst[winst].stop && !CT[P.cls[w]].is_free) {
     const PClass& Cw = CT[P.cls[w]];
-    if (Cw.is_free) {
-      const double rho = P.X4[w].w;
-      const double inv = 1.0 / rho;
-      const double pr = P.V4[w].w;
-      v.S.D4[w] = make_double4_32a(inv, pr * inv * inv, sound_speed(Cw.pres_eq, Cw.cs, rho, Cw.rho0), rho);
-      if (o.has_solid && Cw.material > 1 && Cw.ti > 0.0)
-        tensile_tir<DIM>(P.sigma + 9 * (size_t)w, Cw.ti, rho, P.tir + 9 * (size_t)w);
-    } else {
-      wall = true;
-      mat = Cw.material;
-      xw = P.X4[w];
-      ow = P.orig[w];
-      cell = v.S.cellid[w];
-      hw = Cw.h;
-      noslip = Cw.no_slip;
-    }
+    wall = true;
+    mat = Cw.material;
+    xw = P.X4[w];
+    ow = P.orig[w];
+    cell = v.S.cellid[w];
+    hw = Cw.h;
+    noslip = Cw.no_slip;
   }
+  if (__syncthreads_or(wall) == 0) return;
   // Wall interpolation (FSMPairs only: free partners of the same material).
   const bool any_periodic = g.periodic[0] | g.periodic[1] | g.periodic[2];
   const double gx = o.gravity[0], gy = o.gravity[1], gz = o.gravity[2];
@@ -201,7 +225,7 @@ __global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v) {
       x0 = xf.x - xw.x; x1 = xf.y - xw.y; x2 = xf.z - xw.z;
       if (any_periodic) periodic_fix(g, x0, x1, x2, hb, cf, cw);
     }
-    const double r = sqrt(x0 * x0 + x1 * x1 + x2 * x2);
+    const double r = sqrt_newton(x0 * x0 + x1 * x1 + x2 * x2);
     const double inv_hb = o.uniform_h ? o.inv_h : 1.0 / hb;
     const double q = r * inv_hb;
     const double ih2 = inv_hb * inv_hb;
@@ -216,39 +240,54 @@ __global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v) {
     }
     if (noslip) { n0 += vf.x * K; n1 += vf.y * K; n2 += vf.z * K; }
   };
-  const int cnt = (wall && cell >= 0) ? v.S.nl_count[w] : 0;
-  if (cnt >= 0) {  // the neighbour list, 4 entries per 16-byte load
-    const int4* __restrict__ nl4 = reinterpret_cast<const int4*>(v.S.nl) + nl_slot(w);
-    const size_t N = (size_t)v.nl_stride;
-    const int nch = (cnt + 3) >> 2;
-    for (int ch = 0; ch < nch; ++ch) {
-      const int4 qe = nl4[(size_t)ch * N];
-      const int rem = cnt - 4 * ch;
-      visit(qe.x & kIndexMask, qe.x >> kCodeShift);
-      if (rem > 1) visit(qe.y & kIndexMask, qe.y >> kCodeShift);
-      if (rem > 2) visit(qe.z & kIndexMask, qe.z >> kCodeShift);
-      if (rem > 3) visit(qe.w & kIndexMask, qe.w >> kCodeShift);
-    }
-  } else {  // list overflow: scan the cells
-    NbrSource<DIM> src;
-    src.init(v, g, w, true, 1.004f);
-    while (true) {
+  const int cnt = (wall && cell >= 0) ? v.S.nl_count[w] : 0;  // -1: overflowed, the first lane scans the cells
+  NbrSource<DIM> src;
+  src.init(v, g, w, cnt < 0, 1.004f);
+  for (int k = G.sub;; k += 1 << lg) {
+    if (cnt >= 0) {
+      if (k >= cnt) break;
+      const int e = v.S.nl[nl_index(v.nl_stride, w, k)];
+      visit(e & kIndexMask, e >> kCodeShift);
+    } else {
+      if (G.sub != 0) break;
       int code;
       const int f = src.next(v, &code);
       if (f < 0) break;
       visit(f, code);
     }
   }
-  if (!wall) return;
+  sk = group_sum(sk, lg);
+  p = group_sum(p, lg);
+  n0 = group_sum(n0, lg);
+  n1 = group_sum(n1, lg);
+  n2 = group_sum(n2, lg);
+  if (o.has_solid) {
+#pragma unroll
+    for (int e = 0; e < 9; ++e) sig[e] = group_sum(sig[e], lg);
+  }
+  // the rest is per wall: one thread each, so that the FP64 divisions and the
+  // inverse EOS run with full warps
+  if (wall && G.sub == 0) {
+    double* f = sums[threadIdx.x >> lg];
+    f[0] = sk; f[1] = p; f[2] = n0; f[3] = n1; f[4] = n2;
+    if (o.has_solid) {
+#pragma unroll
+      for (int e = 0; e < 9; ++e) f[5 + e] = sig[e];
+    }
+  }
+  __syncthreads();  // (the next batch's barrier at its start keeps its sums off these)
+  w = first + threadIdx.x;
+  if ((int)threadIdx.x >= (kFT >> lg) || w >= n) return;
   const PClass& Cw = CT[P.cls[w]];
+  if (Cw.is_free || v.inst[Cw.inst].stop) return;
+  mat = Cw.material;
+  noslip = Cw.no_slip;
+  xw = P.X4[w];
+  const double* f = sums[threadIdx.x];
+  sk = f[0]; p = f[1]; n0 = f[2]; n1 = f[3]; n2 = f[4];
   const PClass& Ce = CT[o.eos_cls];
   if (sk != 0.0) {
     if (mat < 3) p = p / sk;
-    if (mat > 1) {
-      const double s = 1.0 / sk;
-#pragma unroll
-      for (int e = 0; e < 9; ++e) sig[e] = sig[e] * s;
-    }
     if (noslip) { n0 = n0 / sk; n1 = n1 / sk; n2 = n2 / sk; }
   } else {
     p = 0.0; n0 = n1 = n2 = 0.0;
@@ -259,6 +298,9 @@ __global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v) {
   v.S.sumkernel[w] = sk;
   v.S.nsv4[w] = make_double4_32a(n0, n1, n2, 0.0);
   if (o.has_solid) {
+    const double is = (sk != 0.0 && mat > 1) ? 1.0 / sk : 1.0;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) sig[e] = f[5 + e] * is;
     double* sw = P.sigma + 9 * (size_t)w;
 #pragma unroll
     for (int e = 0; e < 9; ++e) sw[e] = sig[e];
@@ -267,7 +309,10 @@ __global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v) {
 #pragma unroll
       for (int e = 0; e < 9; ++e) tw[e] = 0.0;
     }
-    if (sk != 0.0 && mat > 1 && Cw.ti > 0.0) tensile_tir<DIM>(sig, Cw.ti, xw.w, P.tir + 9 * (size_t)w);
+    if (sk != 0.0 && mat > 1 && Cw.ti > 0.0) {
+      tensile_tir<DIM>(sig, Cw.ti, xw.w, P.tir + 9 * (size_t)w);
+      if (v.S.pair_info) v.S.pair_info[w] = (v.S.pair_info[w] & ~kInfoTir) | tir_bit(v, P, w);
+    }
   }
   // density, 1/density, p/density^2 and sound speed the partners see (Source/Interaction.cpp:41-61)
   double rw = xw.w, cwv = 0.0;
@@ -277,6 +322,42 @@ __global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v) {
   }
   const double inv = 1.0 / rw;
   v.S.D4[w] = make_double4_32a(inv, p * inv * inv, cwv, rw);
+}
+
+template <int DIM, int KT>
+__global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v, int lg, int per_block) {
+  __shared__ double sums[kFT >> kMinLanesLog2][14];  // per wall: kernel, pressure, velocity (3), stress (9) sums
+  const StepScalars* sc = v.sc;
+  if (sc->all_stop) return;
+  const Persist& P = cur_persist(v);
+  const int n = sc->n;
+  const Options& o = v.o;
+  const PClass* __restrict__ CT = v.cls;
+  // every particle of the block's range, one thread each: what partners see of
+  // the free ones
+  const int first = blockIdx.x * per_block;
+  const int q = first + threadIdx.x;
+  bool wall_q = false;
+  if ((int)threadIdx.x < per_block && q < n && !v.inst[CT[P.cls[q]].inst].stop) {
+    const int cls = P.cls[q];
+    const PClass& C = CT[cls];
+    wall_q = !C.is_free;
+    if (C.is_free) {
+      const double rho = P.X4[q].w;
+      const double inv = 1.0 / rho;
+      const double pr = P.V4[q].w;
+      v.S.D4[q] = make_double4_32a(inv, pr * inv * inv, sound_speed(C.pres_eq, C.cs, rho, C.rho0), rho);
+      if (o.has_solid && C.material > 1 && C.ti > 0.0)
+        tensile_tir<DIM>(P.sigma + 9 * (size_t)q, C.ti, rho, P.tir + 9 * (size_t)q);
+    }
+    // (the FP32C pair kernels have copies of their own)
+    if (v.S.pair_info)
+      v.S.pair_info[q] = cls | (C.is_free ? kInfoFree : 0) |
+                         (v.S.cellid[q] >= 0 && v.S.nl_count[q] >= 0 ? kInfoList : 0) | tir_bit(v, P, q);
+  }
+  if (__syncthreads_or(wall_q) == 0) return;
+  // the fixed ones, 2^lg lanes each, as many at a time as the block's threads serve
+  for (int at = 0; at < per_block; at += kFT >> lg) wall_interpolation<DIM, KT>(v, P, lg, first + at, n, sums);
 }
 
 // ---------------------------------------------------------------------------
@@ -294,6 +375,11 @@ __global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v) {
 // in the gather form. forces_fluid_fold_kernel (pass B) then adds the
 // partners' terms in list order. Both sums keep a fixed order: no atomics,
 // deterministic results.
+//
+// Measured per step (pass A + pass B; 2D dam break of 86k particles / 3D of 177k
+// / the 920-particle channel): 422 / 1635 / 280 us with one lane per particle
+// and every constant read per pair, 232 / 788 / 49 us with lane groups and SPEC;
+// pass A keeps the FP64 pipe 79 % busy (177k particles).
 // ---------------------------------------------------------------------------
 // Which side of a shared pair evaluates it: by the parity of i + j the lower or
 // the higher index, so each particle evaluates about half of its shared pairs
@@ -315,20 +401,42 @@ PSPH_D int partner_slot(const DevView& v, int j, int code, int i) {
   return -1;
 }
 
-template <int DIM, int KT, bool HALF>
-__global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v) {
+// LastComputeAcceleration's time-step bound sqrt_h_a sqrt(h / |a|) of one
+// particle's (a, dDensity), which must be finite.
+PSPH_D double dt_bound(const DevView& v, const double* a, double h) {
+  if (!(isfinite(a[0]) && isfinite(a[1]) && isfinite(a[2]) && isfinite(a[3]))) atomicOr(&v.sc->status, ST_NONFINITE);
+  const double an = sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]);
+  const double cand = v.o.sqrt_h_a * sqrt(h / an);
+  return (cand < DBL_MAX) ? cand : DBL_MAX;  // NaN never compares less, as in the reference
+}
+
+// SPEC: Morris viscosity, squared-density gradient, one h, one EOS and pair
+// constants (artificial viscosity, masses, viscosity) the same for every class,
+// without tensile instability, strain rates, XSPH or a second material (the dam
+// breaks and the channel): those constants come from the launch parameters and
+// the terms that vanish are not compiled. The FP64 pipe (2 lanes per SM per
+// clock) bounds this kernel, so what counts is FP64 instructions per pair.
+//
+// A particle's list is walked by 2^lg lanes (LaneGroup): each round reads 2^lg
+// entries, drops those the partner evaluates, and queues the rest in shared
+// memory across the group, so that every lane then evaluates the same number of
+// pairs to within one.
+template <int DIM, int KT, bool HALF, bool SPEC>
+__global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v, int lg) {
   __shared__ double red[kFT / 32];
   __shared__ unsigned long long cred[kFT / 32];
-  __shared__ int qbuf[kQN][kFT];
+  __shared__ int qbuf[(kQN + 1) * kFT];  // a group's queue: 17 * 2^lg words (the odd stride keeps groups off each other's banks)
+  __shared__ double fin[kFT >> kMinLanesLog2][4];  // a particle's summed acceleration and density rate, for the epilogue
   const StepScalars* sc = v.sc;
   if (sc->all_stop) return;
   const Persist& P = cur_persist(v);
   const int n = sc->n;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int tid = threadIdx.x;
+  const LaneGroup G(lg);
+  const int L = 1 << lg;
+  const int i = (blockIdx.x * kFT + tid) >> lg;
   const Options& o = v.o;
   const PClass* __restrict__ CT = v.cls;
-  double dtc = DBL_MAX;
   unsigned long long npair2 = 0;
   bool active = false;
   int cell = -1, ci_cls = 0;
@@ -338,12 +446,13 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v) {
     const bool run = !v.inst[CT[ci_cls].inst].stop && (!o.mixed || CT[ci_cls].material == 1);
     active = run && CT[ci_cls].is_free;
     cell = v.S.cellid[i];
-    if (run && !active) {
+    if (run && !active && G.sub == 0) {
       if (!o.a_from_hook) v.S.A4[i] = make_double4_32a(o.gravity[0], o.gravity[1], o.gravity[2], 0.0);
       v.S.zwab[i] = 1.0;
       if (v.S.s_acc) v.S.s_acc[i] = 0.0;
     }
   }
+  if (__syncthreads_or(active) == 0) return;  // a block of walls
   const PClass& Ci = CT[ci_cls];
   const GridDev& g = grid_of(v, Ci.inst);
   const InstState& Is = v.inst[Ci.inst];
@@ -354,77 +463,150 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v) {
   const double mi = Ci.mass, hi = Ci.h;
   const double mui = o.dyn_mu ? (active ? P.mu[i] : 0.0) : Ci.mu0;
   const bool shep = Ci.shepard && (Is.shepard_counter == o.shepard_step);
-  const bool sr_self = (Ci.t0 > 0.0 || Ci.les);
-  double ax = o.gravity[0] + o.body_force[0], ay = o.gravity[1] + o.body_force[1],
-         az = o.gravity[2] + o.body_force[2];
+  const bool sr_self = !SPEC && (Ci.t0 > 0.0 || Ci.les);
+  double ax = 0.0, ay = 0.0, az = 0.0;
   double drho = 0.0, zw = 0.0, sd = 0.0, xs0 = 0.0, xs1 = 0.0, xs2 = 0.0;
-  if (o.a_from_hook && active) {  // StartAcceleration's values as a GeneralBefore hook left them
-    const double4_32a a0 = v.S.A4[i];
-    ax = a0.x + o.body_force[0];
-    ay = a0.y + o.body_force[1];
-    az = a0.z + o.body_force[2];
-    drho = a0.w;
-  }
   double sr0 = 0.0, sr1 = 0.0, sr2 = 0.0, sr4 = 0.0, sr5 = 0.0, sr8 = 0.0;
   double w01 = 0.0, w02 = 0.0, w12 = 0.0;  // antisymmetric counterpart of the strain-rate sums (closure)
   double ss = 0.0;  // SWIType 1: the surface-erosion velocity derivative S
-  const bool want_s = v.S.s_acc != nullptr;
+  const bool want_s = !SPEC && v.S.s_acc != nullptr;
   int nnb = 0;
-  const bool closure = o.closure && Ci.les;
+  const bool closure = !SPEC && o.closure && Ci.les;
   const bool any_periodic = g.periodic[0] | g.periodic[1] | g.periodic[2];
   CellCoord cci = decode(g, cell >= 0 ? cell : 0);
-  NbrSource<DIM> src;
-  src.init(v, g, i, active && cell >= 0, 1.004f);
   bool more = active && cell >= 0;
-  // once-per-pair form: i's list is in use (not overflowed)
-  const bool own_list = HALF && active && cell >= 0 && v.S.nl_count[i] >= 0;
-  const int shep_pair = o.shepard_step;  // the counter is per instance: partners share it
+  const int cnt = more ? v.S.nl_count[i] : 0;  // -1: overflowed, the group's first lane scans the cells
+  NbrSource<DIM> src;
+  src.init(v, g, i, more && cnt < 0, 1.004f);
+  const bool own_list = HALF && more && cnt >= 0;
   // a partner slot written this step carries the instance's step number + 1
   const int stamp = (int)(Is.steps & 0x3fffffff) + 1;
+  const unsigned full = 0xffffffffu;
+  int* const queue = qbuf + (tid >> lg) * (L * (kQN + 1));
+  int next = 0;  // the list's entries read so far
+  const int qcap = (kQN - 1) * L;
+  more = more && cnt != 0;
   while (true) {
     int qn = 0;
-    while (more && qn < kQN) {
-      int code;
-      const int j = src.next(v, &code);
-      if (j < 0) {
-        more = false;
-        break;
+    while (true) {  // queue the group's next pairs
+      const bool want = more && qn <= qcap;
+      if (!__any_sync(full, want)) break;
+      int e = -1;
+      if (want) {
+        if (cnt >= 0) {
+          if (next + G.sub < cnt) e = v.S.nl[nl_index(v.nl_stride, i, next + G.sub)];
+          next += L;
+          more = next < cnt;
+        } else if (G.sub == 0) {
+          int code;
+          const int j = src.next(v, &code);
+          if (j < 0) more = false;
+          else e = j | (code << kCodeShift);
+        }
       }
-      // once-per-pair form: a shared pair the partner evaluates is left out of
-      // the queue, so the lanes' queues hold only work
-      if (HALF && own_list && !evaluates_pair(i, j) && v.S.nl_count[j] >= 0 && CT[P.cls[j]].is_free) continue;
-      qbuf[qn++][tid] = HALF ? (j | (code << kCodeShift)) : j;
+      more = __shfl_sync(full, more, G.base);
+      bool keep = e >= 0;
+      if (HALF && keep && own_list) {
+        // a shared pair (both free, both lists in use) is evaluated by one side
+        const int j = e & kIndexMask;
+        const int both = kInfoFree | kInfoList;
+        if ((v.S.pair_info[j] & both) == both) {
+          keep = evaluates_pair(i, j);
+          e |= (int)0x80000000;  // the partner takes its terms
+        }
+      }
+      const unsigned kept = (__ballot_sync(full, keep) >> G.base) & G.bits;
+      if (keep) queue[qn + __popc(kept & ((1u << G.sub) - 1u))] = e;
+      qn += __popc(kept);
     }
-    const int qmax = __reduce_max_sync(0xffffffffu, qn);
-    for (int k = 0; k < qmax; ++k) {
-      if (k >= qn) continue;
-      const int qe = qbuf[k][tid];
-      const int j = HALF ? (qe & kIndexMask) : qe;
+    __syncwarp();
+    for (int k = G.sub; k < qn; k += L) {
+      const int qe = queue[k];
+      const int j = qe & kIndexMask;
+      const bool share = HALF && qe < 0;
       const double4_32a xj = P.X4[j];
-      const PClass& Cj = CT[P.cls[j]];
-      if (!HALF && o.mixed && Cj.material != 1) continue;  // soil or solid partners: the coupling kernel
-      // shared pair: both free, both lists in use; evaluates_pair picks the
-      // side (the queue holds only those this side evaluates)
-      const bool share = own_list && Cj.is_free && v.S.nl_count[j] >= 0;
-      const double hb = (hi + Cj.h) / 2;
+      const int infoj = v.S.pair_info[j];
+      const bool fj = infoj & kInfoFree;
+      const PClass& Cj = CT[SPEC ? 0 : (infoj & kInfoCls)];
+      if (!HALF && !SPEC && o.mixed && Cj.material != 1) continue;  // soil or solid partners: the coupling kernel
+      const double hb = SPEC ? o.spec.h : (hi + Cj.h) / 2;
       double x0 = xi.x - xj.x, x1 = xi.y - xj.y, x2 = xi.z - xj.z;
       if (any_periodic) periodic_fix(g, x0, x1, x2, hb, cci, decode(g, v.S.cellid[j]));
       const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
-      const double inv_hb = o.uniform_h ? o.inv_h : 1.0 / hb;
+      const double inv_hb = SPEC ? o.spec.inv_h : (o.uniform_h ? o.inv_h : 1.0 / hb);
       double rij, inv_r = 0.0;
-      if (KT == 1 && o.vis_eq <= 1) {
-        rij = sqrt(r2);
+      if (KT == 1 && (SPEC || o.vis_eq <= 1)) {
+        rij = sqrt_newton(r2);
       } else {
-        inv_r = (r2 > 0.0) ? rsqrt(r2) : 0.0;
+        inv_r = rsqrt_newton(r2);
         rij = r2 * inv_r;
       }
       const double q = rij * inv_hb;
-      if (q > g.cellfac) continue;
-      const bool fj = Cj.is_free;
+      if (above(q, g.cellfac)) continue;
       npair2 += fj ? 1ull : 2ull;
-      ++nnb;
       const double4_32a vj = P.V4[j];
       const double4_32a dj4 = v.S.D4[j];
+      const double v0 = vi.x - vj.x, v1 = vi.y - vj.y, v2 = vi.z - vj.z;
+      const double vx = v0 * x0 + v1 * x1 + v2 * x2;
+      if (SPEC) {
+        // kernel and gradient times a free partner's mass
+        double GKm = Kern<DIM, KT>::GK(q, hb * inv_r, o.spec.cwg_m);
+        double Km = Kern<DIM, KT>::W(q, o.spec.cwh_m);
+        const double inv_j = dj4.x;
+        double PI = 0.0;
+        if (o.spec.av && negative(vx)) {
+          // (-a c MU + b MU^2) / rho_ij with MU = h v.x / D; without b one factor D less
+          const double D = r2 + o.spec.eps2, c2 = ci_snd + dj4.z, d2 = di + dj4.w;
+          if (!o.spec.av_beta) {
+            PI = (vx * o.spec.neg_alpha_h) * c2 * rcp_newton(D * d2);
+          } else {
+            const double t = o.spec.h * vx;
+            PI = vx * (0.5 * (o.spec.neg_alpha_h * c2) * D + o.spec.beta_h * t) * rcp_newton(D * D * (0.5 * d2));
+          }
+        }
+        double vab0 = v0, vab1 = v1, vab2 = v2;
+        double c = 0.0;
+        if (fj) {
+          c = o.spec.mu2 * inv_i;
+        } else {  // a wall: its mass, and its no-slip velocity, or no viscous term between two that slip
+          if (o.spec.wall_scaled) {
+            GKm *= o.spec.wall_scale;
+            Km *= o.spec.wall_scale;
+          }
+          if (Ci.no_slip || CT[infoj & kInfoCls].no_slip) {
+            const double4_32a ns = v.S.nsv4[j];
+            vab0 = vi.x - (2.0 * vj.x - ns.x);
+            vab1 = vi.y - (2.0 * vj.y - ns.y);
+            vab2 = vi.z - (2.0 * vj.z - ns.z);
+            c = o.spec.mu2 * inv_i;
+          }
+        }
+        c = c * inv_j * GKm;
+        const double s = -(Pi + dj4.y + PI) * GKm;
+        const double fx = s * x0 + c * vab0, fy = s * x1 + c * vab1, fz = DIM == 3 ? s * x2 + c * vab2 : 0.0;
+        ax += fx;
+        ay += fy;
+        if (DIM == 3) az += fz;
+        const double gv = GKm * vx;
+        drho += inv_j * gv;  // times rho_i at the end
+        zw += Km * inv_j;
+        if (shep) sd += Km;
+        if (HALF && share) {
+          npair2 += 1ull;  // the partner's half of the count
+          const int slot = partner_slot(v, j, (qe >> kCodeShift) & 31, i);
+          if (slot < 0) {
+            atomicOr(&v.sc->status, ST_LIST_MISMATCH);
+          } else {
+            const size_t e = nl_index(v.nl_stride, j, slot);
+            v.S.half4[e] = make_double4_32a(-fx, -fy, -fz, inv_i * gv);
+            v.S.half_zw[e] = Km * inv_i;
+            if (o.any_shepard && Is.shepard_counter == o.shepard_step) v.S.half_sd[e] = Km;
+            v.S.half_stamp[e] = stamp;  // written this step
+          }
+        }
+        continue;
+      }
+      ++nnb;
       double dj, inv_j, Pj, cj_snd;
       const double mj = fj ? Cj.mass : Cj.fpmassc * mi;
       const double pj = vj.w;
@@ -442,15 +624,13 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v) {
       const double inv_q = hb * inv_r;
       const double GK = Kern<DIM, KT>::GK(q, inv_q, cwg);
       const double K = Kern<DIM, KT>::W(q, cwh);
-      const double v0 = vi.x - vj.x, v1 = vi.y - vj.y, v2 = vi.z - vj.z;
-      const double vx = v0 * x0 + v1 * x1 + v2 * x2;
       double PI = 0.0;
       const double Alpha = (Ci.alpha + Cj.alpha) / 2.0, Beta = (Ci.beta + Cj.beta) / 2.0;
       if ((Alpha != 0.0 || Beta != 0.0) && vx < 0) {
         // (-a c MU + b MU^2) / rho_ij with MU = h v.x / D, as one division
         const double D = r2 + 0.01 * hb * hb;
         const double t = hb * vx;
-        PI = t * (-Alpha * 0.5 * (ci_snd + cj_snd) * D + Beta * t) / (D * D * (0.5 * (di + dj)));
+        PI = t * (-Alpha * 0.5 * (ci_snd + cj_snd) * D + Beta * t) * rcp_newton(D * D * (0.5 * (di + dj)));
       }
       double TI = 0.0;
       if (Ci.ti > 0.0 || Cj.ti > 0.0) {
@@ -520,7 +700,7 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v) {
       ax += mj * (s * x0 + VI0);
       ay += mj * (s * x1 + VI1);
       if (DIM == 3) az += mj * (s * x2 + VI2);
-      drho += mj * di * inv_j * (GK * vx);
+      drho += mj * inv_j * (GK * vx);  // times rho_i at the end
       zw += mj * inv_j * K;
       if (shep) sd += mj * K;
       if (!HALF && want_s) ss = ss + mj / dj * vab0 * x1 * -GK;  // Source/Interaction.cpp:154
@@ -529,53 +709,96 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v) {
         // a_j -= m_i F, dDensity_j += m_i (rho_j / rho_i) v.GK x, ZWab_j += m_i / rho_i W,
         // SumDen_j += m_i W (Source/Interaction.cpp:139-145, :170-177)
         npair2 += 1ull;  // the partner's half of the count
-        const int slot = partner_slot(v, j, qe >> kCodeShift, i);
+        const int slot = partner_slot(v, j, (qe >> kCodeShift) & 31, i);
         if (slot < 0) {
           atomicOr(&v.sc->status, ST_LIST_MISMATCH);
         } else {
           const size_t e = nl_index(v.nl_stride, j, slot);
           const double fx = mi * (s * x0 + VI0), fy = mi * (s * x1 + VI1), fz = DIM == 3 ? mi * (s * x2 + VI2) : 0.0;
-          v.S.half4[e] = make_double4_32a(-fx, -fy, -fz, mi * dj * inv_i * (GK * vx));
-          const bool shep_j = Cj.shepard && (Is.shepard_counter == shep_pair);
-          v.S.half2[e] = make_double2(mi * inv_i * K, shep_j ? mi * K : 0.0);
+          v.S.half4[e] = make_double4_32a(-fx, -fy, -fz, mi * inv_i * (GK * vx));
+          v.S.half_zw[e] = mi * inv_i * K;
+          if (o.any_shepard && Is.shepard_counter == o.shepard_step) v.S.half_sd[e] = mi * K;
           v.S.half_stamp[e] = stamp;  // written this step
         }
       }
     }
-    if (!__any_sync(0xffffffffu, more)) break;
+    __syncwarp();  // the queue is read before it is filled again
+    if (!__any_sync(full, more)) break;
   }
-  if (HALF) {  // own terms; pass B adds the partners', then the dt bound
-    if (active) {
-      v.S.A4[i] = make_double4_32a(ax, ay, az, drho);
-      v.S.zwab[i] = zw;
-      if (o.any_shepard) v.S.sumden[i] = sd;
-    }
-    block_dt_and_pairs<kFT>(v, Ci.inst, false, dtc, npair2, red, cred);
-    return;
-  }
-  if (active) {
+  // the group's lanes together
+  ax = group_sum(ax, lg);
+  ay = group_sum(ay, lg);
+  if (DIM == 3) az = group_sum(az, lg);
+  drho = group_sum(drho, lg);
+  zw = group_sum(zw, lg);
+  if (o.any_shepard) sd = group_sum(sd, lg);
+  if (active && G.sub == 0) {
+    double4_32a a0 = make_double4_32a(o.gravity[0], o.gravity[1], o.gravity[2], 0.0);
+    if (o.a_from_hook) a0 = v.S.A4[i];  // StartAcceleration's values as a GeneralBefore hook left them
+    ax += a0.x + o.body_force[0];
+    ay += a0.y + o.body_force[1];
+    az += a0.z + o.body_force[2];
+    drho = a0.w + di * drho;
     v.S.A4[i] = make_double4_32a(ax, ay, az, drho);
     v.S.zwab[i] = zw;
     if (o.any_shepard) v.S.sumden[i] = sd;
-    if (want_s) v.S.s_acc[i] = ss;
-    if (o.xsph != 0.0) v.S.vxsph4[i] = make_double4_32a(xs0, xs1, xs2, 0.0);
+  }
+  double dtc = DBL_MAX;
+  if (HALF) {  // own terms; pass B adds the partners', then the dt bound
+    block_dt_and_pairs<kFT>(v, Ci.inst, false, dtc, npair2, red, cred);
+    return;
+  }
+  if (!SPEC) {
+    if (want_s) {
+      ss = group_sum(ss, lg);
+      if (active && G.sub == 0) v.S.s_acc[i] = ss;
+    }
+    if (o.xsph != 0.0) {
+      xs0 = group_sum(xs0, lg);
+      xs1 = group_sum(xs1, lg);
+      xs2 = group_sum(xs2, lg);
+      if (active && G.sub == 0) v.S.vxsph4[i] = make_double4_32a(xs0, xs1, xs2, 0.0);
+    }
     if (o.need_sr) {
-      double* out = v.S.strain_rate + 9 * (size_t)i;
-      out[0] = sr0; out[1] = sr1; out[2] = sr2;
-      out[3] = sr1; out[4] = sr4; out[5] = sr5;
-      out[6] = sr2; out[7] = sr5; out[8] = sr8;
+      double* const sums[6] = {&sr0, &sr1, &sr2, &sr4, &sr5, &sr8};
+#pragma unroll
+      for (int k = 0; k < 6; ++k) *sums[k] = group_sum(*sums[k], lg);
+      if (active && G.sub == 0) {
+        double* out = v.S.strain_rate + 9 * (size_t)i;
+        out[0] = sr0; out[1] = sr1; out[2] = sr2;
+        out[3] = sr1; out[4] = sr4; out[5] = sr5;
+        out[6] = sr2; out[7] = sr5; out[8] = sr8;
+      }
     }
-    if (closure) {
-      v.S.cvort[i] = (float)sqrt(w01 * w01 + w02 * w02 + w12 * w12);
-      v.S.cnnb[i] = (float)nnb;
+    if (o.closure) {
+      w01 = group_sum(w01, lg);
+      w02 = group_sum(w02, lg);
+      w12 = group_sum(w12, lg);
+      for (int k = 1; k < L; k <<= 1) nnb += __shfl_xor_sync(full, nnb, k);
+      if (active && closure && G.sub == 0) {
+        v.S.cvort[i] = (float)sqrt(w01 * w01 + w02 * w02 + w12 * w12);
+        v.S.cnnb[i] = (float)nnb;
+      }
     }
-    if (!(isfinite(ax) && isfinite(ay) && isfinite(az) && isfinite(drho))) atomicOr(&v.sc->status, ST_NONFINITE);
-    const double an = sqrt(ax * ax + ay * ay + az * az);
-    const double cand = o.sqrt_h_a * sqrt(hi / an);
-    if (cand < dtc) dtc = cand;  // NaN never compares less, as in the reference
+  }
+  // the finiteness check and the dt bound of the block's particles, one thread
+  // each (the FP64 pipe takes as long for one active lane as for 32)
+  if (G.sub == 0) {
+    double* f = fin[tid >> lg];
+    f[0] = ax; f[1] = ay; f[2] = az; f[3] = drho;
+  }
+  __syncthreads();
+  const int p = blockIdx.x * (kFT >> lg) + tid;
+  bool act = tid < (kFT >> lg) && p < n;
+  int inst = Ci.inst;
+  if (act) {
+    const PClass& C = CT[P.cls[p]];
+    inst = C.inst;
+    act = C.is_free && !v.inst[inst].stop && (!o.mixed || C.material == 1);
+    if (act) dtc = dt_bound(v, fin[tid], C.h);
   }
   // two materials: the dt bound waits for the coupling kernel's terms
-  block_dt_and_pairs<kFT>(v, Ci.inst, active && !o.mixed, dtc, npair2, red, cred);
+  block_dt_and_pairs<kFT>(v, inst, act && !o.mixed, dtc, npair2, red, cred);
 }
 
 // Pass B of the once-per-pair form: adds, in list order, the terms the
@@ -583,15 +806,19 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v) {
 // stamp is this step's; a slot of a pair outside the support, or of a partner
 // that evaluated its own side, keeps an older stamp), then the dt bound and
 // the finiteness check of the gather form.
-template <int DIM>
-__global__ void __launch_bounds__(kFT) forces_fluid_fold_kernel(DevView v) {
+__global__ void __launch_bounds__(kFT) forces_fluid_fold_kernel(DevView v, int lg) {
+  __shared__ int qbuf[(kQN + 1) * kFT];
   __shared__ double red[kFT / 32];
   __shared__ unsigned long long cred[kFT / 32];
+  __shared__ double fin[kFT >> kMinLanesLog2][4];
   const StepScalars* sc = v.sc;
   if (sc->all_stop) return;
   const Persist& P = cur_persist(v);
   const int n = sc->n;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int tid = threadIdx.x;
+  const LaneGroup G(lg);
+  const int L = 1 << lg;
+  const int i = (blockIdx.x * kFT + tid) >> lg;
   const Options& o = v.o;
   const PClass* __restrict__ CT = v.cls;
   bool active = false;
@@ -601,61 +828,109 @@ __global__ void __launch_bounds__(kFT) forces_fluid_fold_kernel(DevView v) {
     active = !v.inst[CT[ci_cls].inst].stop && CT[ci_cls].is_free;
     cell = v.S.cellid[i];
   }
+  if (__syncthreads_or(active) == 0) return;  // a block of walls
   const PClass& Ci = CT[ci_cls];
-  double dtc = DBL_MAX;
-  if (active) {
-    const int stamp = (int)(v.inst[Ci.inst].steps & 0x3fffffff) + 1;
-    double4_32a a = v.S.A4[i];
-    double zw = v.S.zwab[i], sd = o.any_shepard ? v.S.sumden[i] : 0.0;
-    const int cnt = cell >= 0 ? v.S.nl_count[i] : -1;
-    const int4* __restrict__ nl4 = reinterpret_cast<const int4*>(v.S.nl) + nl_slot(i);
-    const size_t N = (size_t)v.nl_stride;
-    for (int c = 0; 4 * c < cnt; ++c) {  // one 16-byte chunk of 4 entries per load
-      const int4 q = nl4[(size_t)c * N];
-      const int ent[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (4 * c + e >= cnt || evaluates_pair(i, ent[e] & kIndexMask)) continue;
-        const size_t sl = nl_index(v.nl_stride, i, 4 * c + e);
-        if (v.S.half_stamp[sl] != stamp) continue;
-        const double4_32a t = v.S.half4[sl];
-        const double2 u = v.S.half2[sl];
-        a.x += t.x;
-        a.y += t.y;
-        a.z += t.z;
-        a.w += t.w;
-        zw += u.x;
-        sd += u.y;
+  double4_32a a = make_double4_32a(0, 0, 0, 0);
+  double zw = 0.0, sd = 0.0;
+  const bool shep = Ci.shepard && v.inst[Ci.inst].shepard_counter == o.shepard_step;
+  const int stamp = (int)(v.inst[Ci.inst].steps & 0x3fffffff) + 1;
+  const int cnt = (active && cell >= 0) ? v.S.nl_count[i] : 0;
+  const unsigned full = 0xffffffffu;
+  int* const queue = qbuf + (tid >> lg) * (L * (kQN + 1));
+  const int qcap = (kQN - 1) * L;
+  int next = 0;
+  bool more = cnt > 0;
+  while (__any_sync(full, more)) {
+    int qn = 0;
+    while (true) {  // queue the entries whose slot was written this step (as the pair kernel queues its pairs)
+      const bool want = more && qn <= qcap;
+      if (!__any_sync(full, want)) break;
+      const int k = next + G.sub;
+      bool keep = want && k < cnt;
+      if (keep) {
+        const size_t sl = nl_index(v.nl_stride, i, k);
+        keep = !evaluates_pair(i, v.S.nl[sl] & kIndexMask) && v.S.half_stamp[sl] == stamp;
       }
+      if (want) {
+        next += L;
+        more = next < cnt;
+      }
+      const unsigned kept = (__ballot_sync(full, keep) >> G.base) & G.bits;
+      if (keep) queue[qn + __popc(kept & ((1u << G.sub) - 1u))] = k;
+      qn += __popc(kept);
     }
-    v.S.A4[i] = a;
-    v.S.zwab[i] = zw;
-    if (o.any_shepard) v.S.sumden[i] = sd;
-    if (!(isfinite(a.x) && isfinite(a.y) && isfinite(a.z) && isfinite(a.w))) atomicOr(&v.sc->status, ST_NONFINITE);
-    const double an = sqrt(a.x * a.x + a.y * a.y + a.z * a.z);
-    const double cand = o.sqrt_h_a * sqrt(Ci.h / an);
-    if (cand < dtc) dtc = cand;  // NaN never compares less, as in the reference
+    __syncwarp();
+    for (int k = G.sub; k < qn; k += L) {
+      const size_t sl = nl_index(v.nl_stride, i, queue[k]);
+      const double4_32a t = v.S.half4[sl];
+      a.x += t.x;
+      a.y += t.y;
+      a.z += t.z;
+      a.w += t.w;
+      zw += v.S.half_zw[sl];
+      if (shep) sd += v.S.half_sd[sl];
+    }
+    __syncwarp();
   }
-  block_dt_and_pairs<kFT>(v, Ci.inst, active, dtc, 0ull, red, cred);
+  a.x = group_sum(a.x, lg);
+  a.y = group_sum(a.y, lg);
+  a.z = group_sum(a.z, lg);
+  a.w = group_sum(a.w, lg);
+  zw = group_sum(zw, lg);
+  if (o.any_shepard) sd = group_sum(sd, lg);
+  if (active && G.sub == 0) {
+    const double4_32a own = v.S.A4[i];
+    a.x += own.x;
+    a.y += own.y;
+    a.z += own.z;
+    a.w = own.w + P.X4[i].w * a.w;
+    v.S.A4[i] = a;
+    v.S.zwab[i] += zw;
+    if (shep) v.S.sumden[i] += sd;
+    double* f = fin[tid >> lg];
+    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+  }
+  __syncthreads();
+  // as the gather form's epilogue: one thread per particle
+  double dtc = DBL_MAX;
+  const int p = blockIdx.x * (kFT >> lg) + tid;
+  bool act = tid < (kFT >> lg) && p < n;
+  int inst = Ci.inst;
+  if (act) {
+    const PClass& C = CT[P.cls[p]];
+    inst = C.inst;
+    act = C.is_free && !v.inst[inst].stop;
+    if (act) dtc = dt_bound(v, fin[tid], C.h);
+  }
+  block_dt_and_pairs<kFT>(v, inst, act, dtc, 0ull, red, cred);
 }
 
 // ---------------------------------------------------------------------------
 // Soil / solid pair force (CalcForce2233) from the side of free particle i
 // ---------------------------------------------------------------------------
+// A particle's list is walked by 2^lg lanes (LaneGroup). The FP64 pipe bounds
+// it, so what every pair shares is taken out of the loop (the kernel
+// normalisations with one h, the own stress over density squared, the density
+// factor of the rate), the strain and rotation rates are sums of the nine
+// products a_r x_c, and the tensile-instability power is evaluated only where
+// one of the two particles carries a tensile stress (kInfoTir: elsewhere it
+// multiplies a zero; Options::ti_always: parameters under which the power is not
+// finite).
 template <int DIM, int KT>
-__global__ void __launch_bounds__(kFT) forces_solid_kernel(DevView v) {
+__global__ void __launch_bounds__(kFT) forces_solid_kernel(DevView v, int lg) {
   __shared__ double red[kFT / 32];
   __shared__ unsigned long long cred[kFT / 32];
-  __shared__ int qbuf[kQN][kFT];
+  __shared__ double fin[kFT >> kMinLanesLog2][4];  // a particle's summed acceleration and density rate
   const StepScalars* sc = v.sc;
   if (sc->all_stop) return;
   const Persist& P = cur_persist(v);
   const int n = sc->n;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int tid = threadIdx.x;
+  const LaneGroup G(lg);
+  const int L = 1 << lg;
+  const int i = (blockIdx.x * kFT + tid) >> lg;
   const Options& o = v.o;
   const PClass* __restrict__ CT = v.cls;
-  double dtc = DBL_MAX;
   unsigned long long npair2 = 0;
   bool active = false;
   int cell = -1, ci_cls = 0;
@@ -665,12 +940,13 @@ __global__ void __launch_bounds__(kFT) forces_solid_kernel(DevView v) {
     const bool run = !v.inst[CT[ci_cls].inst].stop && (!o.mixed || CT[ci_cls].material != 1);
     active = run && CT[ci_cls].is_free;
     cell = v.S.cellid[i];
-    if (run && !active) {
+    if (run && !active && G.sub == 0) {
       if (!o.a_from_hook) v.S.A4[i] = make_double4_32a(o.gravity[0], o.gravity[1], o.gravity[2], 0.0);
       v.S.zwab[i] = 1.0;
       if (v.S.s_acc) v.S.s_acc[i] = 0.0;
     }
   }
+  if (__syncthreads_or(active) == 0) return;  // a block of walls
   const PClass& Ci = CT[ci_cls];
   const GridDev& g = grid_of(v, Ci.inst);
   const InstState& Is = v.inst[Ci.inst];
@@ -682,168 +958,191 @@ __global__ void __launch_bounds__(kFT) forces_solid_kernel(DevView v) {
   const double4_32a di4 = v.S.D4[is];
   const double di = xi.w, inv_i = di4.x, mi = Ci.mass, hi = Ci.h;
   const bool shep = Ci.shepard && (Is.shepard_counter == o.shepard_step);
-  const double* __restrict__ Si = P.sigma + 9 * (size_t)is;
   const double* __restrict__ Ti = P.tir + 9 * (size_t)is;
-  double ax = o.gravity[0] + o.body_force[0], ay = o.gravity[1] + o.body_force[1],
-         az = o.gravity[2] + o.body_force[2];
-  double drho = 0.0, zw = 0.0, sd = 0.0, xs0 = 0.0, xs1 = 0.0, xs2 = 0.0;
-  if (o.a_from_hook && active) {  // StartAcceleration's values as a GeneralBefore hook left them
-    const double4_32a a0 = v.S.A4[i];
-    ax = a0.x + o.body_force[0];
-    ay = a0.y + o.body_force[1];
-    az = a0.z + o.body_force[2];
-    drho = a0.w;
+  double Si[9];  // the own stress, over density squared for the squared-density gradient
+  {
+    const double* __restrict__ S = P.sigma + 9 * (size_t)is;
+    const double c = (o.grad_type == 0) ? inv_i * inv_i : 1.0;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) Si[e] = S[e] * c;
   }
-  double sr[6] = {0, 0, 0, 0, 0, 0}, rr[3] = {0, 0, 0};  // sr: 00 01 02 11 12 22; rr: 01 02 12
+  double ax = 0.0, ay = 0.0, az = 0.0;
+  double drho = 0.0, zw = 0.0, sd = 0.0, xs0 = 0.0, xs1 = 0.0, xs2 = 0.0;
+  double m[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // sums of a_r x_c, a = -1/2 GK (m_j / rho_j) vab
   const bool any_periodic = g.periodic[0] | g.periodic[1] | g.periodic[2];
   const double I22 = (DIM == 2) ? 0.0 : 1.0;  // Domain::I (Source/Domain.cpp:1665)
   CellCoord cci = decode(g, cell >= 0 ? cell : 0);
+  const bool uniform_h = o.uniform_h;
+  const double ih_u = o.inv_h, cwh_u = Kern<DIM, KT>::cw() * (DIM == 2 ? ih_u * ih_u : ih_u * ih_u * ih_u);
+  const double cwg_u = cwh_u * (ih_u * ih_u);
+  const int cnt = (active && cell >= 0) ? v.S.nl_count[i] : 0;  // -1: overflowed, the first lane scans the cells
+  const int tir_i = active ? v.S.pair_info[i] : 0;
   NbrSource<DIM> src;
-  src.init(v, g, i, active && cell >= 0, 1.004f);
-  bool more = active && cell >= 0;
-  while (true) {
-    int qn = 0;
-    while (more && qn < kQN) {
+  src.init(v, g, i, cnt < 0, 1.004f);
+  for (int k = G.sub;; k += L) {
+    int j;
+    if (cnt >= 0) {
+      if (k >= cnt) break;
+      j = v.S.nl[nl_index(v.nl_stride, i, k)] & kIndexMask;
+    } else {
+      if (G.sub != 0) break;
       int code;
-      const int j = src.next(v, &code);
-      if (j < 0) {
-        more = false;
-        break;
-      }
-      qbuf[qn++][tid] = j;
+      j = src.next(v, &code);
+      if (j < 0) break;
     }
-    const int qmax = __reduce_max_sync(0xffffffffu, qn);
-    for (int k = 0; k < qmax; ++k) {
-      if (k >= qn) continue;
-      const int j = qbuf[k][tid];
-      const double4_32a xj = P.X4[j];
-      const PClass& Cj = CT[P.cls[j]];
-      if (o.mixed && Cj.material != Ci.material) continue;  // fluid partners: the coupling kernel
-      const double hb = (hi + Cj.h) / 2;
-      double x0 = xi.x - xj.x, x1 = xi.y - xj.y, x2 = xi.z - xj.z;
-      if (any_periodic) periodic_fix(g, x0, x1, x2, hb, cci, decode(g, v.S.cellid[j]));
-      const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
-      const double inv_hb = o.uniform_h ? o.inv_h : 1.0 / hb;
-      const double inv_r = (r2 > 0.0) ? rsqrt(r2) : 0.0;
-      const double q = r2 * inv_r * inv_hb;
-      if (q > g.cellfac) continue;
-      const bool fj = Cj.is_free;
-      npair2 += fj ? 1ull : 2ull;
-      const double4_32a vj = P.V4[j];
-      const bool soil = (Ci.material * Cj.material == 9);
-      double dj, inv_j, cj_snd = 0.0;
-      double mj;
-      if (fj) {
+    const double4_32a xj = P.X4[j];
+    const PClass& Cj = CT[P.cls[j]];
+    if (o.mixed && Cj.material != Ci.material) continue;  // fluid partners: the coupling kernel
+    const double hb = uniform_h ? hi : (hi + Cj.h) / 2;
+    double x0 = xi.x - xj.x, x1 = xi.y - xj.y, x2 = xi.z - xj.z;
+    if (any_periodic) periodic_fix(g, x0, x1, x2, hb, cci, decode(g, v.S.cellid[j]));
+    const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
+    const double inv_hb = uniform_h ? ih_u : 1.0 / hb;
+    const double inv_r = rsqrt_newton(r2);
+    const double q = r2 * inv_r * inv_hb;
+    if (above(q, g.cellfac)) continue;
+    const bool fj = Cj.is_free;
+    npair2 += fj ? 1ull : 2ull;
+    const double4_32a vj = P.V4[j];
+    const bool soil = (Ci.material * Cj.material == 9);
+    double dj, inv_j, cj_snd = 0.0;
+    double mj;
+    if (fj) {
+      const double4_32a dj4 = v.S.D4[j];
+      dj = xj.w; inv_j = dj4.x; cj_snd = dj4.z; mj = Cj.mass;
+    } else if (soil) {  // soil walls take the partner's density (Source/Interaction.cpp:201-205)
+      dj = di; inv_j = inv_i; mj = Cj.fpmassc * mi;
+    } else {
+      if (o.uniform_eos) {
         const double4_32a dj4 = v.S.D4[j];
-        dj = xj.w; inv_j = dj4.x; cj_snd = dj4.z; mj = Cj.mass;
-      } else if (soil) {  // soil walls take the partner's density (Source/Interaction.cpp:201-205)
-        dj = di; inv_j = inv_i; mj = Cj.fpmassc * mi;
+        dj = dj4.w; inv_j = dj4.x; cj_snd = dj4.z;
       } else {
-        if (o.uniform_eos) {
-          const double4_32a dj4 = v.S.D4[j];
-          dj = dj4.w; inv_j = dj4.x; cj_snd = dj4.z;
-        } else {
-          dj = density_solid(Ci.pres_eq, Ci.cs, Ci.p0, vj.w, Ci.rho0);
-          inv_j = 1.0 / dj;
-          cj_snd = sound_speed(Ci.pres_eq, Ci.cs, dj, Ci.rho0);
-        }
-        mj = Cj.fpmassc * mi;
+        dj = density_solid(Ci.pres_eq, Ci.cs, Ci.p0, vj.w, Ci.rho0);
+        inv_j = 1.0 / dj;
+        cj_snd = sound_speed(Ci.pres_eq, Ci.cs, dj, Ci.rho0);
       }
-      const double ih2 = inv_hb * inv_hb;
-      const double cwh = Kern<DIM, KT>::cw() * (DIM == 2 ? ih2 : ih2 * inv_hb);
-      const double cwg = cwh * ih2;
-      const double GK = Kern<DIM, KT>::GK(q, hb * inv_r, cwg);
-      const double K = Kern<DIM, KT>::W(q, cwh);
-      const double v0 = vi.x - vj.x, v1 = vi.y - vj.y, v2 = vi.z - vj.z;
-      const double vx = v0 * x0 + v1 * x1 + v2 * x2;
-      double PIs = 0.0;  // PIij = PIs * I
-      const double Alpha = (Ci.alpha + Cj.alpha) / 2.0, Beta = (Ci.beta + Cj.beta) / 2.0;
-      if ((Alpha != 0.0 || Beta != 0.0) && vx < 0) {
-        const double Cij = soil ? 0.5 * (Ci.cs + Cj.cs) : 0.5 * (di4.z + cj_snd);
-        const double D = r2 + 0.01 * hb * hb;
-        const double t = hb * vx;
-        PIs = t * (Alpha * Cij * D + Beta * t) / (D * D * (0.5 * (di + dj)));
-      }
-      double TIs = 0.0;
-      const bool ti = (Ci.ti > 0.0 || Cj.ti > 0.0);
-      if (ti) {
-        const double Wd = Kern<DIM, KT>::W((Ci.tid + Cj.tid) / (2.0 * hb), cwh);
-        TIs = pow(K / Wd, (Ci.tin + Cj.tin) / 2.0);
-      }
-      double vab0, vab1, vab2;
-      if (fj) { vab0 = v0; vab1 = v1; vab2 = v2; }
-      else if (Ci.no_slip || Cj.no_slip) {
-        const double4_32a ns = v.S.nsv4[j];
-        vab0 = vi.x - (2.0 * vj.x - ns.x);
-        vab1 = vi.y - (2.0 * vj.y - ns.y);
-        vab2 = vi.z - (2.0 * vj.z - ns.z);
-      } else {
-        const double4_32a vbj = (o.scheme == PSPH_MVERLET) ? P.H4[j] : P.H4b[j];
-        vab0 = vi.x - vbj.x; vab1 = vi.y - vbj.y; vab2 = vi.z - vbj.z;
-      }
-      const double* __restrict__ Sj = P.sigma + 9 * (size_t)j;
-      const double* __restrict__ Tj = P.tir + 9 * (size_t)j;
-      double M[9];
-      if (o.grad_type == 0) {
-        const double ci2 = inv_i * inv_i, cj2 = inv_j * inv_j;
-#pragma unroll
-        for (int e = 0; e < 9; ++e) M[e] = Si[e] * ci2 + Sj[e] * cj2;
-      } else {
-        const double c = inv_i * inv_j;
-#pragma unroll
-        for (int e = 0; e < 9; ++e) M[e] = (Si[e] + Sj[e]) * c;
-      }
-      M[0] += PIs; M[4] += PIs; M[8] += PIs * I22;
-      if (ti) {
-#pragma unroll
-        for (int e = 0; e < 9; ++e) M[e] += (Ti[e] + Tj[e]) * TIs;
-      }
-      const double g0 = GK * x0, g1 = GK * x1, g2 = GK * x2;
-      ax += mj * (g0 * M[0] + g1 * M[3] + g2 * M[6]);
-      ay += mj * (g0 * M[1] + g1 * M[4] + g2 * M[7]);
-      if (DIM == 3) az += mj * (g0 * M[2] + g1 * M[5] + g2 * M[8]);
-      drho += mj * di * inv_j * (v0 * g0 + v1 * g1 + v2 * g2);
-      const double md = mj * inv_j;
-      zw += md * K;
-      const double c2 = -0.5 * GK * md;
-      sr[0] += c2 * (2.0 * vab0 * x0);
-      sr[1] += c2 * (vab0 * x1 + vab1 * x0);
-      sr[2] += c2 * (vab0 * x2 + vab2 * x0);
-      sr[3] += c2 * (2.0 * vab1 * x1);
-      sr[4] += c2 * (vab1 * x2 + vab2 * x1);
-      sr[5] += c2 * (2.0 * vab2 * x2);
-      rr[0] += c2 * (vab0 * x1 - vab1 * x0);
-      rr[1] += c2 * (vab0 * x2 - vab2 * x0);
-      rr[2] += c2 * (vab1 * x2 - vab2 * x1);
-      if (o.xsph != 0.0 && fj) {
-        const double s = o.xsph * mj / (0.5 * (di + dj)) * K;
-        xs0 -= s * v0; xs1 -= s * v1; xs2 -= s * v2;
-      }
-      if (shep) sd += mj * K;
-      if (want_s) ss = ss + mj / dj * vab0 * x1 * -GK;  // Source/Interaction.cpp:347
+      mj = Cj.fpmassc * mi;
     }
-    if (!__any_sync(0xffffffffu, more)) break;
+    double cwh = cwh_u, cwg = cwg_u;
+    if (!uniform_h) {
+      const double ih2 = inv_hb * inv_hb;
+      cwh = Kern<DIM, KT>::cw() * (DIM == 2 ? ih2 : ih2 * inv_hb);
+      cwg = cwh * ih2;
+    }
+    const double GK = Kern<DIM, KT>::GK(q, hb * inv_r, cwg);
+    const double K = Kern<DIM, KT>::W(q, cwh);
+    const double v0 = vi.x - vj.x, v1 = vi.y - vj.y, v2 = vi.z - vj.z;
+    const double vx = v0 * x0 + v1 * x1 + v2 * x2;
+    double PIs = 0.0;  // PIij = PIs * I
+    if (o.any_av && negative(vx)) {
+      const double Alpha = o.uniform_av ? Ci.alpha : (Ci.alpha + Cj.alpha) / 2.0;
+      const double Beta = o.uniform_av ? Ci.beta : (Ci.beta + Cj.beta) / 2.0;
+      const double Cij = soil ? 0.5 * (Ci.cs + Cj.cs) : 0.5 * (di4.z + cj_snd);
+      const double D = r2 + 0.01 * hb * hb;
+      const double t = hb * vx;
+      PIs = t * (Alpha * Cij * D + Beta * t) * rcp_newton(D * D * (0.5 * (di + dj)));
+    }
+    double vab0, vab1, vab2;
+    if (fj) { vab0 = v0; vab1 = v1; vab2 = v2; }
+    else if (Ci.no_slip || Cj.no_slip) {
+      const double4_32a ns = v.S.nsv4[j];
+      vab0 = vi.x - (2.0 * vj.x - ns.x);
+      vab1 = vi.y - (2.0 * vj.y - ns.y);
+      vab2 = vi.z - (2.0 * vj.z - ns.z);
+    } else {
+      const double4_32a vbj = (o.scheme == PSPH_MVERLET) ? P.H4[j] : P.H4b[j];
+      vab0 = vi.x - vbj.x; vab1 = vi.y - vbj.y; vab2 = vi.z - vbj.z;
+    }
+    const double* __restrict__ Sj = P.sigma + 9 * (size_t)j;
+    double M[9];
+    if (o.grad_type == 0) {
+      const double cj2 = inv_j * inv_j;
+#pragma unroll
+      for (int e = 0; e < 9; ++e) M[e] = Sj[e] * cj2 + Si[e];
+    } else {
+      const double c = inv_i * inv_j;
+#pragma unroll
+      for (int e = 0; e < 9; ++e) M[e] = (Si[e] + Sj[e]) * c;
+    }
+    M[0] += PIs; M[4] += PIs; M[8] += PIs * I22;
+    if (o.any_ti && (Ci.ti > 0.0 || Cj.ti > 0.0) && (o.ti_always || ((tir_i | v.S.pair_info[j]) & kInfoTir))) {
+      const double Wd = Kern<DIM, KT>::W((Ci.tid + Cj.tid) / (2.0 * hb), cwh);
+      const double TIs = pow(K / Wd, (Ci.tin + Cj.tin) / 2.0);
+      const double* __restrict__ Tj = P.tir + 9 * (size_t)j;
+#pragma unroll
+      for (int e = 0; e < 9; ++e) M[e] += (Ti[e] + Tj[e]) * TIs;
+    }
+    const double GKm = GK * mj;
+    const double g0 = GKm * x0, g1 = GKm * x1, g2 = GKm * x2;
+    ax += g0 * M[0] + g1 * M[3] + g2 * M[6];
+    ay += g0 * M[1] + g1 * M[4] + g2 * M[7];
+    if (DIM == 3) az += g0 * M[2] + g1 * M[5] + g2 * M[8];
+    drho += inv_j * (GKm * vx);  // times rho_i at the end
+    zw += mj * inv_j * K;
+    const double c2 = -0.5 * (GKm * inv_j);
+    const double a0 = c2 * vab0, a1 = c2 * vab1, a2 = c2 * vab2;
+    m[0] += a0 * x0; m[1] += a0 * x1; m[2] += a0 * x2;
+    m[3] += a1 * x0; m[4] += a1 * x1; m[5] += a1 * x2;
+    m[6] += a2 * x0; m[7] += a2 * x1; m[8] += a2 * x2;
+    if (o.xsph != 0.0 && fj) {
+      const double s = o.xsph * mj / (0.5 * (di + dj)) * K;
+      xs0 -= s * v0; xs1 -= s * v1; xs2 -= s * v2;
+    }
+    if (shep) sd += mj * K;
+    if (want_s) ss = ss + mj / dj * vab0 * x1 * -GK;  // Source/Interaction.cpp:347
   }
-  if (active) {
+  ax = group_sum(ax, lg);
+  ay = group_sum(ay, lg);
+  if (DIM == 3) az = group_sum(az, lg);
+  drho = group_sum(drho, lg);
+  zw = group_sum(zw, lg);
+#pragma unroll
+  for (int e = 0; e < 9; ++e) m[e] = group_sum(m[e], lg);
+  if (o.any_shepard) sd = group_sum(sd, lg);
+  if (want_s) ss = group_sum(ss, lg);
+  if (o.xsph != 0.0) {
+    xs0 = group_sum(xs0, lg);
+    xs1 = group_sum(xs1, lg);
+    xs2 = group_sum(xs2, lg);
+  }
+  if (active && G.sub == 0) {
+    double4_32a a0 = make_double4_32a(o.gravity[0], o.gravity[1], o.gravity[2], 0.0);
+    if (o.a_from_hook) a0 = v.S.A4[i];  // StartAcceleration's values as a GeneralBefore hook left them
+    ax += a0.x + o.body_force[0];
+    ay += a0.y + o.body_force[1];
+    az += a0.z + o.body_force[2];
+    drho = a0.w + di * drho;
     v.S.A4[i] = make_double4_32a(ax, ay, az, drho);
     v.S.zwab[i] = zw;
     if (o.any_shepard) v.S.sumden[i] = sd;
     if (want_s) v.S.s_acc[i] = ss;
     if (o.xsph != 0.0) v.S.vxsph4[i] = make_double4_32a(xs0, xs1, xs2, 0.0);
     double* out = v.S.strain_rate + 9 * (size_t)i;
-    out[0] = sr[0]; out[1] = sr[1]; out[2] = sr[2];
-    out[3] = sr[1]; out[4] = sr[3]; out[5] = sr[4];
-    out[6] = sr[2]; out[7] = sr[4]; out[8] = sr[5];
+    const double s01 = m[1] + m[3], s02 = m[2] + m[6], s12 = m[5] + m[7];
+    out[0] = 2.0 * m[0]; out[1] = s01; out[2] = s02;
+    out[3] = s01; out[4] = 2.0 * m[4]; out[5] = s12;
+    out[6] = s02; out[7] = s12; out[8] = 2.0 * m[8];
     double* ro = v.S.rotation_rate + 9 * (size_t)i;
-    ro[0] = 0.0; ro[1] = rr[0]; ro[2] = rr[1];
-    ro[3] = -rr[0]; ro[4] = 0.0; ro[5] = rr[2];
-    ro[6] = -rr[1]; ro[7] = -rr[2]; ro[8] = 0.0;
-    if (!(isfinite(ax) && isfinite(ay) && isfinite(az) && isfinite(drho))) atomicOr(&v.sc->status, ST_NONFINITE);
-    const double an = sqrt(ax * ax + ay * ay + az * az);
-    const double cand = o.sqrt_h_a * sqrt(hi / an);
-    if (cand < dtc) dtc = cand;
+    const double r01 = m[1] - m[3], r02 = m[2] - m[6], r12 = m[5] - m[7];
+    ro[0] = 0.0; ro[1] = r01; ro[2] = r02;
+    ro[3] = -r01; ro[4] = 0.0; ro[5] = r12;
+    ro[6] = -r02; ro[7] = -r12; ro[8] = 0.0;
+    double* f = fin[tid >> lg];
+    f[0] = ax; f[1] = ay; f[2] = az; f[3] = drho;
   }
-  block_dt_and_pairs<kFT>(v, Ci.inst, active && !o.mixed, dtc, npair2, red, cred);
+  __syncthreads();
+  // the finiteness check and the dt bound, one thread per particle
+  double dtc = DBL_MAX;
+  const int p = blockIdx.x * (kFT >> lg) + tid;
+  bool act = tid < (kFT >> lg) && p < n;
+  int inst = Ci.inst;
+  if (act) {
+    const PClass& C = CT[P.cls[p]];
+    inst = C.inst;
+    act = C.is_free && !v.inst[inst].stop && (!o.mixed || C.material != 1);
+    if (act) dtc = dt_bound(v, fin[tid], C.h);
+  }
+  block_dt_and_pairs<kFT>(v, inst, act && !o.mixed, dtc, npair2, red, cred);
 }
 
 // Per-instance step control, one block looping over the instances.
@@ -1326,53 +1625,51 @@ __global__ void __launch_bounds__(kFT) fsi_kernel(DevView v) {
 
 inline int nblk(int n, int bt) { return n <= 0 ? 1 : (n + bt - 1) / bt; }
 
+// Lanes per particle (as a power of two) of a kernel that walks lists: 4, and 8
+// for the quintic spline, whose support of 3h lists more than twice as many
+// neighbours (a 2D dam break of 86k particles, cubic spline: 285 / 260 / 256 /
+// 344 us for 1 / 2 / 4 / 8 lanes; the 920-particle quintic channel: 222 / 121 /
+// 72 / 49 us). The order of a particle's sum follows from it, so it depends on
+// nothing that differs between an ensemble and its instances run alone.
+int lanes_log2(int kt) { return kt == PSPH_QUINTIC_SPLINE ? 3 : 2; }
+
 template <int DIM>
 void prepare_dispatch(const DevView& v, cudaStream_t st) {
-  const int nb = nblk(v.ncap, kFT);
+  const int lg = lanes_log2(v.o.kt);
+  // particles per block: as many as its lanes serve at once, so that the walls
+  // spread over the chip; large soil domains, mostly free particles with a
+  // tensile-instability test each, one per thread (ten columns, 1.0M particles:
+  // 371 us against 268; the 177k-particle dam break, half of it walls: 187
+  // against 273)
+  const int per = (v.o.has_solid && v.ncap >= kFT * 1024) ? kFT : kFT >> lg;
+  const int nb = nblk(v.ncap, per);
   switch (v.o.kt) {
-    case 0: prepare_wall_kernel<DIM, 0><<<nb, kFT, 0, st>>>(v); break;
-    case 1: prepare_wall_kernel<DIM, 1><<<nb, kFT, 0, st>>>(v); break;
-    default: prepare_wall_kernel<DIM, 2><<<nb, kFT, 0, st>>>(v); break;
+    case 0: prepare_wall_kernel<DIM, 0><<<nb, kFT, 0, st>>>(v, lg, per); break;
+    case 1: prepare_wall_kernel<DIM, 1><<<nb, kFT, 0, st>>>(v, lg, per); break;
+    default: prepare_wall_kernel<DIM, 2><<<nb, kFT, 0, st>>>(v, lg, per); break;
   }
 }
 
-template <int DIM>
-void forces_dispatch(const DevView& v, cudaStream_t st) {
-  const int nb = nblk(v.ncap, kFT);
-  if (v.o.has_solid) {
-    if (v.o.mixed) {  // fluid-soil: the fluid's pairs, then the soil's (each kernel keeps to its material)
-      switch (v.o.kt) {
-        case 0: forces_fluid_kernel<DIM, 0, false><<<nb, kFT, 0, st>>>(v); break;
-        case 1: forces_fluid_kernel<DIM, 1, false><<<nb, kFT, 0, st>>>(v); break;
-        default: forces_fluid_kernel<DIM, 2, false><<<nb, kFT, 0, st>>>(v); break;
-      }
-    }
-    switch (v.o.kt) {
-      case 0: forces_solid_kernel<DIM, 0><<<nb, kFT, 0, st>>>(v); break;
-      case 1: forces_solid_kernel<DIM, 1><<<nb, kFT, 0, st>>>(v); break;
-      default: forces_solid_kernel<DIM, 2><<<nb, kFT, 0, st>>>(v); break;
-    }
-  } else if (v.o.fp64_half) {  // each pair once: pass A, then the partners' terms
-    switch (v.o.kt) {
-      case 0:
-        forces_fluid_kernel<DIM, 0, true><<<nb, kFT, 0, st>>>(v);
-        forces_fluid_fold_kernel<DIM><<<nb, kFT, 0, st>>>(v);
-        break;
-      case 1:
-        forces_fluid_kernel<DIM, 1, true><<<nb, kFT, 0, st>>>(v);
-        forces_fluid_fold_kernel<DIM><<<nb, kFT, 0, st>>>(v);
-        break;
-      default:
-        forces_fluid_kernel<DIM, 2, true><<<nb, kFT, 0, st>>>(v);
-        forces_fluid_fold_kernel<DIM><<<nb, kFT, 0, st>>>(v);
-        break;
-    }
+template <int DIM, int KT>
+void fluid_forces(const DevView& v, cudaStream_t st) {
+  const int lg = lanes_log2(v.o.kt);
+  const int nb = nblk(v.ncap, kFT >> lg);
+  if (v.o.fp64_half) {  // each pair once: pass A, then the partners' terms
+    if (v.o.spec64) forces_fluid_kernel<DIM, KT, true, true><<<nb, kFT, 0, st>>>(v, lg);
+    else forces_fluid_kernel<DIM, KT, true, false><<<nb, kFT, 0, st>>>(v, lg);
+    forces_fluid_fold_kernel<<<nb, kFT, 0, st>>>(v, lg);
   } else {
-    switch (v.o.kt) {
-      case 0: forces_fluid_kernel<DIM, 0, false><<<nb, kFT, 0, st>>>(v); break;
-      case 1: forces_fluid_kernel<DIM, 1, false><<<nb, kFT, 0, st>>>(v); break;
-      default: forces_fluid_kernel<DIM, 2, false><<<nb, kFT, 0, st>>>(v); break;
-    }
+    forces_fluid_kernel<DIM, KT, false, false><<<nb, kFT, 0, st>>>(v, lg);
+  }
+}
+
+template <int DIM, int KT>
+void forces_dispatch(const DevView& v, cudaStream_t st) {
+  // fluid-soil: the fluid's pairs, then the soil's (each kernel keeps to its material)
+  if (!v.o.has_solid || v.o.mixed) fluid_forces<DIM, KT>(v, st);
+  if (v.o.has_solid) {
+    const int lg = lanes_log2(v.o.kt);
+    forces_solid_kernel<DIM, KT><<<nblk(v.ncap, kFT >> lg), kFT, 0, st>>>(v, lg);
   }
 }
 
@@ -1386,11 +1683,6 @@ void launch_prepare(const DevView& v, cudaStream_t st) {
 }
 
 void launch_wall(const DevView&, cudaStream_t) {}  // fused into launch_prepare
-
-void launch_forces(const DevView& v, cudaStream_t st) {
-  if (v.o.dim == 2) forces_dispatch<2>(v, st);
-  else forces_dispatch<3>(v, st);
-}
 
 void launch_saturation(const DevView& v, cudaStream_t st) {
   const int nb = nblk(v.ncap, kFT);
@@ -1424,6 +1716,15 @@ template <int DIM, int KT>
 struct FsiLaunch {
   static void run(const DevView& v, int nb, cudaStream_t st) { fsi_kernel<DIM, KT><<<nb, kFT, 0, st>>>(v); }
 };
+
+template <int DIM, int KT>
+struct ForcesLaunch {
+  static void run(const DevView& v, int, cudaStream_t st) { forces_dispatch<DIM, KT>(v, st); }
+};
+
+void launch_forces(const DevView& v, cudaStream_t st) {
+  by_dim_kernel<ForcesLaunch>(v, st);
+}
 
 void launch_coupling(const DevView& v, cudaStream_t st) { by_dim_kernel<CouplingLaunch>(v, st); }
 
