@@ -109,6 +109,7 @@ struct psph_ctx {
   int in_hook = 0;                      // PSPH_HOOK_* while a hook runs
   bool hook_set_a = false;              // the GeneralBefore hook patched accelerations or density rates
   bool hook_set_x = false;              // ... or positions (the FP32 cell offsets follow)
+  bool hook_freed = false;              // ... or made fixed particles free (or the reverse)
   std::map<std::string, int> class_index;  // class record -> index (classes added as particles are recycled)
 };
 
@@ -943,7 +944,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
   }
   Scratch& S = c->S;
   const size_t NC = (size_t)c->total_cells;
-  const size_t NB = NC * kMaxXsub;  // sort bins at the finest x-slab split
+  const size_t NB = 2 * NC * kMaxXsub;  // sort bins at the finest x-slab split, free and fixed apart
   if ((st = dalloc(c, &S.key, N)) || (st = dalloc(c, &S.count, NB + 2)) || (st = dalloc(c, &S.start, NC + 3)) ||
       (st = dalloc(c, &S.sstart, NB + 3)) ||
       (st = dalloc(c, &S.tmp_perm, N)) || (st = dalloc(c, &S.perm, N)) || (st = dalloc(c, &S.cellid, N)) ||
@@ -1510,9 +1511,14 @@ psph_status split_steps(psph_ctx* c, int64_t nsteps, long long* launched, bool o
       const int n = c->h_sc->n;
       const double* gv = c->opt.gravity;
       start_accel_kernel<<<n > 0 ? (n + 255) / 256 : 1, 256, 0, s>>>(c->S.A4, c->d_sc, gv[0], gv[1], gv[2]);
-      c->hook_set_a = c->hook_set_x = false;
+      c->hook_set_a = c->hook_set_x = c->hook_freed = false;
       if ((st = run_hook(c, PSPH_HOOK_BEFORE))) return st;
       c->opt.a_from_hook = c->hook_set_a ? 1 : 0;
+      if (c->hook_freed) {  // a fixed particle's list leaves out the fixed ones: list again with them
+        DevView v = view(c);
+        v.o.list_all = 1;
+        launch_nlist(v, s);
+      }
       if (c->hook_set_x) offsets32_kernel<<<n > 0 ? (n + 255) / 256 : 1, 256, 0, s>>>(view(c));
     }
     {
@@ -2071,6 +2077,7 @@ psph_status patch_impl(psph_ctx* c, const psph_particles* p) {
         c->classes.push_back(C);
         c->class_index.emplace(key, id);
       }
+      if (c->classes[(size_t)id].is_free != c->classes[(size_t)cur[(size_t)r]].is_free) c->hook_freed = true;
       last_in = cur[(size_t)r];
       last_out = id;
       last_rec = C;

@@ -30,7 +30,7 @@ struct Scratch {
   int* key;        // cell key per particle (pre-sort order)
   int* count;      // ncells + 2 counters
   int* start;      // ncells + 3 exclusive prefix: cell c's particles are [start[c], start[c+1])
-  int* sstart;     // ncells * xsub + 3 exclusive prefix over the x-slabs of the cells (xsub > 1)
+  int* sstart;     // 2 ncells * xsub + 3 exclusive prefix over the x-slabs of the cells, free and fixed apart
   int* tmp_perm;
   int* perm;
   int* cellid;     // cell of each sorted particle (orphan/dead: -1)
@@ -136,6 +136,7 @@ struct Options {
   double mu_u;        // that viscosity
   double inv_h;       // 1/h when uniform
   int nl_cap;         // neighbour-list capacity per particle
+  int list_all;       // fixed particles' lists hold fixed candidates too (a hook may have freed some of them)
   int pair_block;     // threads per block of the FP32C pair kernels (psph_autotune)
   int xsub;           // x-slabs per cell in the sort (1, 2 or 4; psph_autotune)
   int nlist_stage;    // staged candidates per block of the neighbour scan (0 = global; psph_autotune)

@@ -94,7 +94,9 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
     return;
   }
   const Persist& P = cur_persist(v);
-  const GridDev& g = grid_of(v, v.cls[P.cls[i]].inst);
+  const PClass& C = v.cls[P.cls[i]];
+  const GridDev& g = grid_of(v, C.inst);
+  const bool fixed = !C.is_free && !v.o.list_all;  // its list holds free particles only (it has no other pairs)
   const float3 cs = cell_size_f(g);
   const float4 oi = v.S.OFF32[i];
   const float cf = (float)g.cellfac;
@@ -109,7 +111,7 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
   const bool cull = UNIFORM_H && inner;
   const float thr_cull = thr_u * 1.0001f;
   const int xs = v.o.xsub;
-  const int* __restrict__ sstart = xs > 1 ? v.S.sstart : v.S.start;
+  const int* __restrict__ sstart = v.S.sstart;  // two bins per slab: its free, then its fixed particles
   const float inv_sw = (float)xs / cs.x;  // 1 / slab width
   const int zlo = (DIM == 3) ? -1 : 0, zhi = (DIM == 3) ? 1 : 0;
   for (int dz = zlo; dz <= zhi; ++dz) {
@@ -138,8 +140,10 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
         else if (x < 0 || x >= g.nc[0]) continue;
         const int s0 = max(slo - dx * xs, 0), s1 = min(shi - dx * xs, xs - 1);
         if (s0 > s1) continue;
-        int lo = sstart[(base + x) * xs + s0];
-        const int hi = sstart[(base + x) * xs + s1 + 1];
+        for (int sl = s0; sl <= s1; sl += fixed ? 1 : xs) {  // a free particle's slabs in one range
+        const int bin = 2 * ((base + x) * xs + sl);
+        int lo = sstart[bin];
+        const int hi = sstart[fixed ? bin + 1 : 2 * ((base + x) * xs + s1 + 1)];
         const int tag = ((dx + 1) + cyz) << kCodeShift;
         // i's position relative to this cell's origin: x_i - x_j = a - off_j
         // (one rounding away from rel_pos's form, which the pair kernels
@@ -175,6 +179,7 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
           w.flush(k0, cap, N);
         }
         for (; j < hi; ++j) one(j);
+        }
       }
     }
   }
@@ -251,7 +256,14 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
     return;
   }
   const Persist& P = cur_persist(v);
-  const GridDev& g = grid_of(v, v.cls[P.cls[ia]].inst);
+  const PClass& C = v.cls[P.cls[ia]];
+  const GridDev& g = grid_of(v, C.inst);
+  // a fixed particle lists free candidates only: two fixed ones scan the free
+  // half of each slab, a free and a fixed one scan both, the fixed one with a
+  // threshold nothing meets in the fixed half
+  const bool fixed_a = !C.is_free && !v.o.list_all;
+  const bool fixed_b = pair ? !v.cls[P.cls[ib]].is_free && !v.o.list_all : fixed_a;
+  const bool fixed = fixed_a && fixed_b, mixed = fixed_a != fixed_b;
   const float3 cs = cell_size_f(g);
   // particle b far away when it is not paired: its tests always fail
   constexpr float kFar = 1e18f;
@@ -270,7 +282,7 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
                     (DIM == 2 || (c.z > 0 && c.z < g.nc[2] - 1));
   const float thr_cull = thr * 1.0001f;
   const int xs = v.o.xsub;
-  const int* __restrict__ sstart = xs > 1 ? v.S.sstart : v.S.start;
+  const int* __restrict__ sstart = v.S.sstart;  // two bins per slab: its free, then its fixed particles
   const float inv_sw = (float)xs / cs.x;
   const int zlo = (DIM == 3) ? -1 : 0, zhi = (DIM == 3) ? 1 : 0;
   for (int dz = zlo; dz <= zhi; ++dz) {
@@ -306,8 +318,13 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
         else if (x < 0 || x >= g.nc[0]) continue;
         const int s0 = max(slo - dx * xs, 0), s1 = min(shi - dx * xs, xs - 1);
         if (s0 > s1) continue;
-        int lo = sstart[(base + x) * xs + s0];
-        const int hi = sstart[(base + x) * xs + s1 + 1];
+        const int bin0 = 2 * ((base + x) * xs + s0), bin1 = 2 * ((base + x) * xs + s1 + 1);
+        const int step = fixed ? 2 : (mixed ? 1 : bin1 - bin0);  // two free ones: the slabs in one range
+        for (int bin = bin0; bin < bin1; bin += step) {
+        int lo = sstart[bin];
+        const int hi = sstart[fixed ? bin + 1 : bin + step];
+        const bool second = mixed && (bin & 1);
+        const float thra = (second && fixed_a) ? -1.f : thr, thrb = (second && fixed_b) ? -1.f : thr;
         const int tag = ((dx + 1) + cyz) << kCodeShift;
         const float cx = -(float)dx * cs.x;
         const float axa = oa.x + cx, aya = oa.y + cy, aza = oa.z + cz;
@@ -327,8 +344,8 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
             const float2 ez = __ffma2_rn(make_float2(oj.z, oj.z), M1, AZ);
             d2 = __ffma2_rn(ez, ez, d2);
           }
-          ina = d2.x <= thr;
-          inb = d2.y <= thr;
+          ina = d2.x <= thra;
+          inb = d2.y <= thrb;
         };
         auto one = [&](int j, bool ena, bool enb) {
           bool ina, inb;
@@ -370,6 +387,7 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
           wb.flush(kb, cap, N);
         }
         for (; j < hi; ++j) one(j, true, true);
+        }
       }
     }
   }

@@ -2,20 +2,27 @@
 // Source/Domain.cpp:662-806, and the per-step pair arrays of MainNeighbourSearch).
 //
 //   bin      cell key per particle, exactly ListGenerate's floor/clamp rule;
-//            each cell is split into xsub slabs along x (the key counts
-//            slabs: cell * xsub + slab), so the particles of a cell lie in
-//            x-slab order and the neighbour-list walk can skip slabs out of
-//            reach; key = nbins (= ncells * xsub) for a particle that
-//            ListGenerate would drop into a periodic ghost column (it then
-//            sits in no list), nbins+1 for one that CheckParticleLeave removed.
-//   scan     exclusive prefix of the per-cell counts (3-phase, block-level).
-//   scatter  atomic slot inside its cell's segment.
-//   rank     deterministic order inside each slab: by original index, so the
-//            sorted state depends only on positions, never on atomic timing.
-//   starts   per-cell segment starts (start[c] = slab start of c's first slab)
-//            for everything that walks whole cells, and the particles the
-//            neighbour-list scan handles one per lane.
-//   reorder  gathers every persistent field into the new order (HBM-bound).
+//            each cell is split into xsub slabs along x and each slab into its
+//            free and its fixed particles (the key counts them: (cell * xsub +
+//            slab) * 2 + fixed), so the particles of a cell lie in x-slab order,
+//            free ones first: the neighbour-list walk can skip slabs out of
+//            reach, a fixed particle's walk the fixed ones (it has no pairs with
+//            them), and warps hold fewer particles of both kinds;
+//            key = nbins (= 2 xsub ncells) for a particle that ListGenerate
+//            would drop into a periodic ghost column (it then sits in no list),
+//            nbins+1 for one that CheckParticleLeave removed. The counting
+//            atomic's old value is the particle's slot inside its segment.
+//   scan     exclusive prefix of the counts (block scans, then each block adds
+//            the totals before it and clears the counts for the next sort).
+//   scatter  into the slots.
+//   reorder  deterministic order inside each segment: by original index, so the
+//            sorted state depends only on positions, never on atomic timing;
+//            each particle's fields move to that place (HBM-bound).
+//   starts   per-cell segment starts (start[c] = start of c's first slab) for
+//            everything that walks whole cells, the particles the neighbour-list
+//            scan handles one per lane, and the new counts and buffer.
+// Six launches (eleven with separate clearing, scan of totals, ranking and
+// finish kernels): 57 -> 44 us for 86k particles, where launches are what counts.
 #include <cstdio>
 
 #include "psph_device.cuh"
@@ -27,18 +34,20 @@ namespace {
 constexpr int kBT = 256;
 
 __global__ void bin_kernel(DevView v, const uint8_t* __restrict__ alive, int* __restrict__ key,
-                           int* __restrict__ count, StepScalars* sc, int dim, int xsub) {
+                           int* __restrict__ count, int* __restrict__ slot_of, StepScalars* sc, int dim, int xsub) {
   if (sc->all_stop || !sc->rebuild) return;
   const Persist& P = cur_persist(v);
   const int n = sc->n;
-  const int nbins = v.total_cells * xsub;
+  const int nbins = 2 * v.total_cells * xsub;
+  if (blockIdx.x == 0 && threadIdx.x == 0) sc->nl_rest = 0;  // cell_starts_kernel counts them
   const int orphan_key = nbins, dead_key = nbins + 1;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     int k;
     if (!alive[i]) {
       k = dead_key;
     } else {
-      const GridDev& g = grid_of(v, v.cls[P.cls[i]].inst);
+      const PClass& C = v.cls[P.cls[i]];
+      const GridDev& g = grid_of(v, C.inst);
       const double4_32a x = P.X4[i];
       const double xs[3] = {x.x, x.y, x.z};
       int c[3] = {0, 0, 0};
@@ -78,28 +87,37 @@ __global__ void bin_kernel(DevView v, const uint8_t* __restrict__ alive, int* __
           const float ox = d2f_bits(a0) - (float)c[0] * g.cell_size32[0];
           slab = min(max((int)floorf(ox * (float)xsub * g.inv_cell_size32[0]), 0), xsub - 1);
         }
-        k = (g.cell_base + (c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0]) * xsub + slab;
+        k = 2 * ((g.cell_base + (c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0]) * xsub + slab) + (C.is_free ? 0 : 1);
       }
     }
     key[i] = k;
     // one atomic per distinct cell of the warp: consecutive particles (sorted
     // by the previous step) mostly share their cell
     const unsigned peers = __match_any_sync(__activemask(), k);
-    if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&count[k], __popc(peers));
+    const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(&count[k], __popc(peers));
+    base = __shfl_sync(peers, base, leader);
+    slot_of[i] = base + __popc(peers & ((1u << lane) - 1u));
   }
 }
 
 // Phase 1: in-block exclusive scan of `in` (len entries), block totals to sums.
-__global__ void scan_blocks(const int* __restrict__ in, int* __restrict__ out, int* __restrict__ sums, int len,
-                            const StepScalars* sc) {
+// A thread takes kScanPer consecutive entries, a block kScanBlock: few enough
+// totals that phase 2 needs no scan of them in between.
+constexpr int kScanPer = 8, kScanBlock = 1024 * kScanPer;
+__global__ void __launch_bounds__(1024) scan_blocks(const int* __restrict__ in, int* __restrict__ out,
+                                                    int* __restrict__ sums, int len, const StepScalars* sc) {
   if (sc && (sc->all_stop || !sc->rebuild)) return;  // the cell sort's scan, on a step without a rebuild
   __shared__ int warp_tot[32];
-  const int base = blockIdx.x * 1024;
-  const int t = threadIdx.x;
-  const int i = base + t;
-  int v = (i < len) ? in[i] : 0;
-  const int lane = t & 31, w = t >> 5;
-  int incl = v;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int first = blockIdx.x * kScanBlock + t * kScanPer;
+  int v[kScanPer], own = 0;
+#pragma unroll
+  for (int e = 0; e < kScanPer; ++e) v[e] = (first + e < len) ? in[first + e] : 0;
+#pragma unroll
+  for (int e = 0; e < kScanPer; ++e) own += v[e];
+  int incl = own;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     int y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -119,126 +137,92 @@ __global__ void scan_blocks(const int* __restrict__ in, int* __restrict__ out, i
     if (lane == 31) sums[blockIdx.x] = si;
   }
   __syncthreads();
-  if (i < len) out[i] = incl - v + warp_tot[w];
+  int at = incl - own + warp_tot[w];
+#pragma unroll
+  for (int e = 0; e < kScanPer; ++e) {
+    if (first + e < len) out[first + e] = at;
+    at += v[e];
+  }
 }
 
-// Phase 2: one block scans the block totals (exclusive), writes the grand total.
-__global__ void scan_sums(int* __restrict__ sums, int nb, int* __restrict__ total_out, const StepScalars* sc) {
+// Phase 2: every block adds the totals of the blocks before it; the last one
+// writes the grand total. clear (if given): entries set to zero behind the scan.
+__global__ void __launch_bounds__(1024) scan_add(int* __restrict__ out, const int* __restrict__ sums, int len,
+                                                 int* __restrict__ clear, const StepScalars* sc) {
   if (sc && (sc->all_stop || !sc->rebuild)) return;
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = 0;
+  __shared__ int part[32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  int before = 0;
+  for (int b = t; b < (int)blockIdx.x; b += 1024) before += sums[b];
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 0) part[w] = before;
   __syncthreads();
-  for (int base = 0; base < nb; base += 1024) {
-    const int t = threadIdx.x, i = base + t;
-    int v = (i < nb) ? sums[i] : 0;
-    const int lane = t & 31, w = t >> 5;
-    __shared__ int wt[32];
-    int incl = v;
+  before = __reduce_add_sync(0xffffffffu, part[lane]);
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
+  for (int e = 0; e < kScanPer; ++e) {
+    const int i = blockIdx.x * kScanBlock + e * 1024 + t;
+    if (i < len) {
+      out[i] += before;
+      if (clear) clear[i] = 0;
     }
-    if (lane == 31) wt[w] = incl;
-    __syncthreads();
-    if (w == 0) {
-      int s = wt[lane], si = s;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, si, o);
-        if (lane >= o) si += y;
-      }
-      wt[lane] = si - s;
-    }
-    __syncthreads();
-    int excl = incl - v + wt[w] + carry;
-    if (i < nb) sums[i] = excl;
-    __syncthreads();
-    if (t == 1023) carry = excl + v;
-    __syncthreads();
   }
-  if (threadIdx.x == 0) *total_out = carry;
+  if (blockIdx.x == gridDim.x - 1 && t == 0) out[len] = before + sums[blockIdx.x];
 }
 
-__global__ void scan_add(int* __restrict__ out, const int* __restrict__ sums, int len, const StepScalars* sc) {
-  if (sc && (sc->all_stop || !sc->rebuild)) return;
-  const int i = blockIdx.x * 1024 + threadIdx.x;
-  if (i < len) out[i] += sums[blockIdx.x];
-}
+inline int scan_blocks_for(int len) { return len > kScanBlock ? (len - 1) / kScanBlock + 1 : 1; }
 
-__global__ void scatter_kernel(const int* __restrict__ key, const int* __restrict__ start, int* __restrict__ fill,
-                               int* __restrict__ tmp_perm, const StepScalars* sc) {
+__global__ void scatter_kernel(const int* __restrict__ key, const int* __restrict__ start,
+                               const int* __restrict__ slot_of, int* __restrict__ tmp_perm, const StepScalars* sc) {
   if (sc->all_stop || !sc->rebuild) return;
   const int n = sc->n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int k = key[i];
-    // warp-aggregated slot claim (the order inside a cell is fixed by rank_kernel)
-    const unsigned peers = __match_any_sync(__activemask(), k);
-    const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(&fill[k], __popc(peers));
-    base = __shfl_sync(peers, base, leader);
-    tmp_perm[start[k] + base + __popc(peers & ((1u << lane) - 1u))] = i;
-  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    tmp_perm[start[key[i]] + slot_of[i]] = i;
 }
 
-__global__ void rank_kernel(const int* __restrict__ key, const int* __restrict__ start,
-                            const int* __restrict__ tmp_perm, DevView v, int* __restrict__ perm,
-                            const StepScalars* sc, int ncells) {
-  if (sc->all_stop || !sc->rebuild) return;
-  const int* __restrict__ orig = cur_persist(v).orig;
-  const int n = sc->n;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-    const int i = tmp_perm[s];
-    const int k = key[i];
-    if (k <= ncells) {
-      const int lo = start[k], hi = start[k + 1];
-      const int mine = orig[i];
-      int r = 0;
-      for (int t = lo; t < hi; ++t) r += (orig[tmp_perm[t]] < mine);
-      perm[lo + r] = i;
-    } else {
-      perm[s] = i;
-    }
-  }
-}
-
-__global__ void reorder_kernel(DevView v, const int* __restrict__ perm, const int* __restrict__ key,
-                               const int* __restrict__ start, int* __restrict__ cellid, uint8_t* __restrict__ alive,
-                               const StepScalars* sc, int nbins, int xsub, int has_solid, int dyn_mu) {
+// One thread per scattered particle i: its place s is its segment's start plus
+// the number of the segment's particles with a smaller original index; then its
+// fields move there. perm[s] = i serves the solids' tensors.
+__global__ void reorder_kernel(DevView v, const int* __restrict__ tmp_perm, int* __restrict__ perm,
+                               const int* __restrict__ key, const int* __restrict__ start, int* __restrict__ cellid,
+                               uint8_t* __restrict__ alive, const StepScalars* sc, int nbins, int xsub, int dyn_mu) {
   if (sc->all_stop || !sc->rebuild) return;
   const Persist& src = cur_persist(v);
   const Persist& dst = next_persist(v);
-  const int n_new = start[nbins + 1];
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_new; s += gridDim.x * blockDim.x) {
-    const int i = perm[s];
+  const int n_new = start[nbins + 1];  // the removed particles' segment comes last
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n_new; q += gridDim.x * blockDim.x) {
+    const int i = tmp_perm[q];
+    const int k = key[i];
+    const int lo = start[k], hi = start[k + 1];
+    const int mine = src.orig[i];
+    int s = lo;
+    for (int t = lo; t < hi; ++t) s += src.orig[tmp_perm[t]] < mine;
+    perm[s] = i;
     dst.X4[s] = src.X4[i];
     dst.V4[s] = src.V4[i];
     dst.H4[s] = src.H4[i];
     if (src.H4b) dst.H4b[s] = src.H4b[i];
-    dst.cls[s] = src.cls[i];
+    const int cls = src.cls[i];
+    dst.cls[s] = cls;
     {
       // FP32 offset from the cell origin (absolute position outside any cell)
       const double4_32a xs = src.X4[i];
-      const int kk = key[i];
-      const float h = (float)v.cls[src.cls[i]].h;
-      if (kk < nbins) {
-        const GridDev& g = grid_of(v, v.cls[src.cls[i]].inst);
-        const int lk = kk / xsub - g.cell_base;
+      const float h = d2f_rn(v.cls[cls].h);
+      if (k < nbins) {
+        const GridDev& g = grid_of(v, v.cls[cls].inst);
+        const int lk = k / (2 * xsub) - g.cell_base;
         const int cx = lk % g.nc[0], t = lk / g.nc[0], cy = t % g.nc[1], cz = t / g.nc[1];
-        v.S.OFF32[s] = make_float4((float)(xs.x - (g.blpf[0] + cx * g.cell_size[0])),
-                                   (float)(xs.y - (g.blpf[1] + cy * g.cell_size[1])),
-                                   (float)(v.o.dim == 3 ? xs.z - (g.blpf[2] + cz * g.cell_size[2]) : 0.0), h);
+        v.S.OFF32[s] = make_float4(d2f_rn(xs.x - (g.blpf[0] + cx * g.cell_size[0])),
+                                   d2f_rn(xs.y - (g.blpf[1] + cy * g.cell_size[1])),
+                                   v.o.dim == 3 ? d2f_rn(xs.z - (g.blpf[2] + cz * g.cell_size[2])) : 0.f, h);
       } else {
-        v.S.OFF32[s] = make_float4((float)xs.x, (float)xs.y, (float)xs.z, h);
+        v.S.OFF32[s] = make_float4(d2f_rn(xs.x), d2f_rn(xs.y), d2f_rn(xs.z), h);
       }
       if (v.o.skin > 0.f)  // displacements are measured from here (FP32, truncated)
         v.S.OFFREF[s] = make_float4(d2f_bits(xs.x), d2f_bits(xs.y), d2f_bits(xs.z), 0.f);
     }
-    dst.orig[s] = src.orig[i];
+    dst.orig[s] = mine;
     if (src.io) dst.io[s] = src.io[i];
-    const int k = key[i];
-    cellid[s] = (k < nbins) ? k / xsub : -1;
+    cellid[s] = (k < nbins) ? k / (2 * xsub) : -1;
     alive[s] = 1;
     if (dyn_mu) dst.mu[s] = src.mu[i];
   }
@@ -278,33 +262,29 @@ __global__ void reorder_tensors_kernel(DevView v, const int* __restrict__ perm, 
   }
 }
 
-__global__ void finish_sort_kernel(const int* __restrict__ start, StepScalars* sc, int nbins) {
-  if (sc->all_stop || !sc->rebuild) return;
-  sc->n_cells = start[nbins];
-  sc->n = start[nbins + 1];
-  sc->buf ^= 1;
-  sc->nl_rest = 0;
-}
-
-// Per-cell segment starts from the slab starts (split cells): start[c] =
-// sstart[c * xsub] for c <= ncells, and the orphan / dead / total boundaries
-// after them. Also lists the particles the two-per-lane neighbour-list scan
-// leaves to a lane of their own: lanes take sorted particles 2t and 2t+1
-// together when they share a cell, so the odd particles left are exactly the
-// cells' first particles at odd indices (into rest, at most cap of them).
+// Per-cell segment starts from the bin starts: start[c] = sstart[c * 2 xsub] for
+// c <= ncells, and the orphan / dead / total boundaries after them; the sorted
+// state's counts and buffer. Also lists the particles the two-per-lane
+// neighbour-list scan leaves to a lane of their own: lanes take sorted particles
+// 2t and 2t+1 together when they share a cell, so the odd particles left are
+// exactly the cells' first particles at odd indices (into rest, at most cap).
 __global__ void cell_starts_kernel(const int* __restrict__ sstart, int* __restrict__ start, int ncells, int xsub,
                                    StepScalars* sc, int* __restrict__ rest, int cap) {
   if (sc->all_stop || !sc->rebuild) return;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (xsub > 1) {
-    if (c <= ncells) start[c] = sstart[(size_t)c * xsub];
-    else if (c <= ncells + 2) start[c] = sstart[(size_t)ncells * xsub + (c - ncells)];
+  const size_t per = 2 * (size_t)xsub, nbins = per * ncells;
+  if (c <= ncells) start[c] = sstart[c * per];
+  else if (c <= ncells + 2) start[c] = sstart[nbins + (c - ncells)];
+  if (c == 0) {
+    sc->n_cells = sstart[nbins];
+    sc->n = sstart[nbins + 1];
+    sc->buf ^= 1;
   }
   bool odd_first = false;
   int s0 = 0;
   if (c < ncells) {
-    s0 = sstart[(size_t)c * xsub];
-    odd_first = (s0 & 1) && sstart[(size_t)(c + 1) * xsub] > s0;
+    s0 = sstart[c * per];
+    odd_first = (s0 & 1) && sstart[(c + 1) * per] > s0;
   }
   const unsigned want = __ballot_sync(0xffffffffu, odd_first);  // every lane of the grid gets here
   if (odd_first) {  // one atomic per warp
@@ -385,23 +365,20 @@ void launch_sort(const DevView& v, cudaStream_t st) {
   const Scratch& S = v.S;
   const int ncells = v.total_cells;
   const int xsub = v.o.xsub;
-  const int nbins = ncells * xsub;
+  const int nbins = 2 * ncells * xsub;
   const int len = nbins + 2;
-  int* sstart = xsub > 1 ? S.sstart : S.start;  // one slab per cell: the slab starts are the cell starts
-  cudaMemsetAsync(S.count, 0, sizeof(int) * (size_t)len, st);
-  bin_kernel<<<grid_for(v.ncap), kBT, 0, st>>>(v, v.alive, S.key, S.count, v.sc, v.o.dim, xsub);
-  const int nb = (len + 1023) / 1024;
-  scan_blocks<<<nb, 1024, 0, st>>>(S.count, sstart, S.block_sums, len, v.sc);
-  scan_sums<<<1, 1024, 0, st>>>(S.block_sums, nb, sstart + len, v.sc);
-  scan_add<<<nb, 1024, 0, st>>>(sstart, S.block_sums, len, v.sc);
-  cudaMemsetAsync(S.count, 0, sizeof(int) * (size_t)len, st);
-  scatter_kernel<<<grid_for(v.ncap), kBT, 0, st>>>(S.key, sstart, S.count, S.tmp_perm, v.sc);
-  rank_kernel<<<grid_for(v.ncap), kBT, 0, st>>>(S.key, sstart, S.tmp_perm, v, S.perm, v.sc, nbins);
-  reorder_kernel<<<grid_for(v.ncap), kBT, 0, st>>>(v, S.perm, S.key, sstart, S.cellid, v.alive, v.sc, nbins, xsub,
-                                                    v.o.has_solid, v.o.dyn_mu);
-  if (v.o.has_solid) reorder_tensors_kernel<<<grid_for(v.ncap), kBT, 0, st>>>(v, S.perm, sstart, v.sc, nbins);
-  finish_sort_kernel<<<1, 1, 0, st>>>(sstart, v.sc, nbins);
-  cell_starts_kernel<<<grid_for(ncells + 3), kBT, 0, st>>>(sstart, S.start, ncells, xsub, v.sc, S.tmp_perm, v.ncap);
+  const int gp = grid_for(v.ncap);
+  // S.count is zero here (allocated so, and cleared behind every scan); S.perm
+  // holds the slots until the reorder writes the permutation
+  bin_kernel<<<gp, kBT, 0, st>>>(v, v.alive, S.key, S.count, S.perm, v.sc, v.o.dim, xsub);
+  const int nb = scan_blocks_for(len);
+  scan_blocks<<<nb, 1024, 0, st>>>(S.count, S.sstart, S.block_sums, len, v.sc);
+  scan_add<<<nb, 1024, 0, st>>>(S.sstart, S.block_sums, len, S.count, v.sc);
+  scatter_kernel<<<gp, kBT, 0, st>>>(S.key, S.sstart, S.perm, S.tmp_perm, v.sc);
+  reorder_kernel<<<gp, kBT, 0, st>>>(v, S.tmp_perm, S.perm, S.key, S.sstart, S.cellid, v.alive, v.sc, nbins, xsub,
+                                     v.o.dyn_mu);
+  if (v.o.has_solid) reorder_tensors_kernel<<<gp, kBT, 0, st>>>(v, S.perm, S.sstart, v.sc, nbins);
+  cell_starts_kernel<<<grid_for(ncells + 3), kBT, 0, st>>>(S.sstart, S.start, ncells, xsub, v.sc, S.tmp_perm, v.ncap);
 }
 
 }  // namespace psph
@@ -412,10 +389,9 @@ namespace psph {
 // block_sums (>= ceil(len/1024) entries) as scratch. Used by the pair export
 // that takes its scratch from caller-owned or static device memory.
 void launch_exclusive_scan(const int* in, int* out, int len, int* block_sums, cudaStream_t st) {
-  const int nb = (len + 1023) / 1024 > 0 ? (len + 1023) / 1024 : 1;
+  const int nb = scan_blocks_for(len);
   scan_blocks<<<nb, 1024, 0, st>>>(in, out, block_sums, len, nullptr);
-  scan_sums<<<1, 1024, 0, st>>>(block_sums, nb, out + len, nullptr);
-  scan_add<<<nb, 1024, 0, st>>>(out, block_sums, len, nullptr);
+  scan_add<<<nb, 1024, 0, st>>>(out, block_sums, len, nullptr, nullptr);
 }
 
 }  // namespace psph
