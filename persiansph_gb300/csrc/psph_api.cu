@@ -543,8 +543,37 @@ void derive_class_options(const std::vector<PClass>& classes, bool mixed, bool d
     o.spec.mu2 = 2.0 * o.mu_u;
     o.spec.wall_scale = wall_u;  // a wall's mass is FPMassC times its partner's
     o.spec.wall_scaled = wall_u >= 0.0 && wall_u != 1.0;
-    o.spec.av_beta = C0.beta != 0.0;
     o.spec.av = C0.alpha != 0.0 || C0.beta != 0.0;
+    o.spec.av_beta = C0.beta != 0.0;
+    // the FP32C fluid kernel's: flags shared by every free and every fixed class too
+    int ff = -1, fw = -1;
+    bool one = true;
+    for (const PClass& C : classes) {
+      const int f = (C.no_slip ? CF_NOSLIP : 0) | (C.les ? CF_LES : 0) | (C.t0 > 0.0 ? CF_T0 : 0);
+      int& ref = C.is_free ? ff : fw;
+      if (ref < 0) ref = f;
+      else if (f != ref) one = false;
+    }
+    if (ff < 0) ff = 0;
+    if (fw < 0) fw = 0;
+    o.spec32 = o.fp32 && o.vis_eq == PSPH_MORRIS && o.grad_type == PSPH_SQUARED_DENSITY && o.uniform_h &&
+               o.uniform_av && o.uniform_mass && (o.uniform_mu || dyn_mu) && !o.any_ti && o.xsph == 0.0 &&
+               !o.has_solid && one;
+    Spec32& f = o.spec32c;
+    f.h = (float)C0.h;
+    f.m_free = o.m_free32;
+    f.m_wall = o.fpm_wall32 * o.m_free32;
+    f.wall_scale = o.fpm_wall32;
+    f.eps2 = (float)o.spec.eps2;
+    f.neg_alpha_h = (float)o.spec.neg_alpha_h;
+    f.beta_h2 = (float)(C0.beta * C0.h * C0.h);
+    f.far2 = (float)(100.0 * C0.h * C0.h);
+    const int self = ff & (CF_T0 | CF_LES);
+    f.sr_free = (self && ((ff & CF_T0) || (ff & CF_LES))) ? -1.f : 0.f;
+    f.sr_wall = (self && ((ff | fw) & CF_NOSLIP) && (((ff | fw) & CF_T0) || (ff & fw & CF_LES))) ? -1.f : 0.f;
+    f.av = o.spec.av;
+    f.wall_scaled = o.spec.wall_scaled;
+    f.wall_visc = ((ff | fw) & CF_NOSLIP) != 0;
   }
 }
 
@@ -975,6 +1004,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
     if ((st = dalloc(c, &S.V32, N)) || (st = dalloc(c, &S.D32, N)) || (st = dalloc(c, &S.NSV32, N)) ||
         (st = dalloc(c, &S.V32LO, N)))
       return st;
+    if (o.spec32 && (st = dalloc(c, &S.PX32, N))) return st;
     if (dyn_mu && (st = dalloc(c, &S.MU32, N))) return st;
     if (o.need_sr && !o.has_solid &&  // FP32 ShearRate and strain-rate sums of the fluid kernel
         ((st = dalloc(c, &S.cshear, N)) || (st = dalloc(c, &S.sr32, 6 * N))))

@@ -43,13 +43,14 @@ struct Scratch {
   int* nl;           // per-step neighbour lists, entry k of particle i at nl[k*ncap + i]:
                      // index | cell-offset code << 26
   int* nl_count;     // list length, or -1 when it exceeded the capacity (scan instead)
+  float4* PX32;      // FP32C form, Options::spec32: (position - cell origin, +-1/density), negative for a fixed one
   float4* V32;       // FP32C form: (v, pressure)
   float4* D32;       // FP32C form: (1/density, pressure/density^2, sound speed, density)
   float4* SIG32;     // FP32C solids: symmetric Sigma, 2 per particle (00 01 02 11 | 12 22 - -)
   float4* TIR32;     // FP32C solids with TI: symmetric TIR, same layout
   float4* VB32;      // FP32C solids: wall history velocity (MVerlet vb / leapfrog vb)
   float4* V32LO;     // FP32C: v - (float)v, the low-order part of the velocity (fluids: .w = the
-                     // particle's class index as int bits, loaded with it by the pair kernel)
+                     // particle's class index and flags as int bits, or the sound speed (spec32))
   float* MU32;       // FP32C, per-particle viscosity (LES / Bingham): FP32 copy of Persist::mu
   float4* NSV32;     // FP32C: wall no-slip velocity in FP32
   double4_32a* D4;   // seen by partners: (1/density, pressure/density^2, sound speed, density);
@@ -100,6 +101,14 @@ struct Spec64 {
   int wall_scaled;          // wall_scale is not 1
 };
 
+// The same for the FP32C fluid kernel's constant-parameter form (Options::spec32).
+struct Spec32 {
+  float h, m_free, m_wall, wall_scale, eps2, neg_alpha_h, beta_h2;  // m_wall: a wall's mass as its partner sees it
+  float far2;               // a squared distance outside the support
+  float sr_free, sr_wall;   // -1 where a strain rate is summed over free / fixed neighbours, else 0
+  int av, wall_scaled, wall_visc;  // wall_visc: a viscous term with walls (one side is no-slip)
+};
+
 struct Options {
   int dim, kt, vis_eq, grad_type, scheme, wallp_physical;
   int fp32;           // PSPH_FP32C pair arithmetic
@@ -133,6 +142,8 @@ struct Options {
   float alpha32, beta32, m_free32, fpm_wall32;
   int spec64;         // the FP64 fluid pair kernel's SPEC form applies, with these constants
   Spec64 spec;
+  int spec32;         // the FP32C fluid pair kernel's
+  Spec32 spec32c;
   double mu_u;        // that viscosity
   double inv_h;       // 1/h when uniform
   int nl_cap;         // neighbour-list capacity per particle

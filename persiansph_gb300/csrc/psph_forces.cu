@@ -130,6 +130,7 @@ PSPH_D void tensile_tir(const double* S, double TI, double rho, double* TIR) {
       for (int c = 0; c < 3; ++c) TIR[3 * r + c] = Q[3 * r + 0] * val[0] * Q[3 * c + 0] + Q[3 * r + 1] * val[1] * Q[3 * c + 1] + Q[3 * r + 2] * val[2] * Q[3 * c + 2];
   }
 }
+constexpr int kShared = 1 << 30;  // (queue words) the partner takes the pair's terms
 constexpr int kQN = 16;  // queued FP64 pair evaluations per lane between flushes
 
 // Lanes of a particle: kernels whose work is one particle's neighbour list give
@@ -247,7 +248,7 @@ PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int f
     if (cnt >= 0) {
       if (k >= cnt) break;
       const int e = v.S.nl[nl_index(v.nl_stride, w, k)];
-      visit(e & kIndexMask, e >> kCodeShift);
+      visit(e & kIndexMask, entry_code(e));
     } else {
       if (G.sub != 0) break;
       int code;
@@ -389,7 +390,7 @@ PSPH_D bool evaluates_pair(int i, int j) { return ((i ^ j) & 1) ? (i < j) : (i >
 
 // i's slot in j's list: the entry (mirror code, i) of j's ascending list, or -1
 PSPH_D int partner_slot(const DevView& v, int j, int code, int i) {
-  const unsigned key = ((unsigned)(26 - code) << kCodeShift) | (unsigned)i;
+  const unsigned key = ((unsigned)(kCodeMirror - code) << kCodeShift) | (unsigned)i;
   int lo = 0, hi = v.S.nl_count[j] - 1;
   while (lo <= hi) {
     const int mid = (lo + hi) >> 1;
@@ -491,28 +492,29 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v, int lg) {
     while (true) {  // queue the group's next pairs
       const bool want = more && qn <= qcap;
       if (!__any_sync(full, want)) break;
+      // a queue word: the entry's place in the list, with a mark when the partner
+      // takes its terms, or the neighbour's index where there is no list
       int e = -1;
       if (want) {
         if (cnt >= 0) {
-          if (next + G.sub < cnt) e = v.S.nl[nl_index(v.nl_stride, i, next + G.sub)];
+          if (next + G.sub < cnt) e = next + G.sub;
           next += L;
           more = next < cnt;
         } else if (G.sub == 0) {
           int code;
-          const int j = src.next(v, &code);
-          if (j < 0) more = false;
-          else e = j | (code << kCodeShift);
+          e = src.next(v, &code);
+          if (e < 0) more = false;
         }
       }
       more = __shfl_sync(full, more, G.base);
       bool keep = e >= 0;
       if (HALF && keep && own_list) {
         // a shared pair (both free, both lists in use) is evaluated by one side
-        const int j = e & kIndexMask;
+        const int j = v.S.nl[nl_index(v.nl_stride, i, e)] & kIndexMask;
         const int both = kInfoFree | kInfoList;
         if ((v.S.pair_info[j] & both) == both) {
           keep = evaluates_pair(i, j);
-          e |= (int)0x80000000;  // the partner takes its terms
+          e |= kShared;
         }
       }
       const unsigned kept = (__ballot_sync(full, keep) >> G.base) & G.bits;
@@ -522,8 +524,9 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v, int lg) {
     __syncwarp();
     for (int k = G.sub; k < qn; k += L) {
       const int qe = queue[k];
-      const int j = qe & kIndexMask;
-      const bool share = HALF && qe < 0;
+      const bool share = HALF && own_list && (qe & kShared);
+      const int entry = cnt >= 0 ? v.S.nl[nl_index(v.nl_stride, i, qe & ~kShared)] : qe;
+      const int j = entry & kIndexMask;
       const double4_32a xj = P.X4[j];
       const int infoj = v.S.pair_info[j];
       const bool fj = infoj & kInfoFree;
@@ -593,7 +596,7 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v, int lg) {
         if (shep) sd += Km;
         if (HALF && share) {
           npair2 += 1ull;  // the partner's half of the count
-          const int slot = partner_slot(v, j, (qe >> kCodeShift) & 31, i);
+          const int slot = partner_slot(v, j, entry_code(entry), i);
           if (slot < 0) {
             atomicOr(&v.sc->status, ST_LIST_MISMATCH);
           } else {
@@ -709,7 +712,7 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v, int lg) {
         // a_j -= m_i F, dDensity_j += m_i (rho_j / rho_i) v.GK x, ZWab_j += m_i / rho_i W,
         // SumDen_j += m_i W (Source/Interaction.cpp:139-145, :170-177)
         npair2 += 1ull;  // the partner's half of the count
-        const int slot = partner_slot(v, j, (qe >> kCodeShift) & 31, i);
+        const int slot = partner_slot(v, j, entry_code(entry), i);
         if (slot < 0) {
           atomicOr(&v.sc->status, ST_LIST_MISMATCH);
         } else {

@@ -156,14 +156,20 @@ __global__ void __launch_bounds__(kFT32) copies32_kernel(DevView v) {
   // to ~2^-48 of |v|; the class index and its flags ride along in .w (class |
   // flags << 16: one load per pair, and no class-table load when the pair
   // constants are uniform)
-  v.S.V32LO[w] = make_float4(lx, ly, lz, __int_as_float(P.cls[w] | (C.flags << 16)));
+  float lw = __int_as_float(P.cls[w] | (C.flags << 16));
   if (C.flags & CF_FREE) {
     const float rho = d2f_rn(P.X4[w].w);
     const float inv = 1.f / rho;
     const float ratio = rho / C.rho0;
     const float c = (C.pres_eq == 1) ? C.cs * ratio * ratio * ratio : C.cs;
     v.S.D32[w] = make_float4(inv, p * inv * inv, c, rho);
+    if (v.o.spec32) {  // the constant-parameter pair kernel's record (the walls' comes with their pressure)
+      const float4 x = v.S.OFF32[w];
+      v.S.PX32[w] = make_float4(x.x, x.y, x.z, inv);
+      lw = c;
+    }
   }
+  v.S.V32LO[w] = make_float4(lx, ly, lz, lw);
   // FP32 copy of a per-particle viscosity: the pair loop then converts nothing
   // (a double-to-float conversion runs on the FP64 pipe, 1/64 of the FP32 rate)
   if (v.o.dyn_mu) v.S.MU32[w] = d2f_rn(P.mu[w]);
@@ -238,10 +244,10 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
     for (int c = 0; c < nch; ++c) {
       const int4 q = nl4[(size_t)c * N];
       const int rem = cnt - 4 * c;
-      visit(q.x & kIndexMask, q.x >> kCodeShift);
-      if (rem > 1) visit(q.y & kIndexMask, q.y >> kCodeShift);
-      if (rem > 2) visit(q.z & kIndexMask, q.z >> kCodeShift);
-      if (rem > 3) visit(q.w & kIndexMask, q.w >> kCodeShift);
+      visit(q.x & kIndexMask, entry_code(q.x));
+      if (rem > 1) visit(q.y & kIndexMask, entry_code(q.y));
+      if (rem > 2) visit(q.z & kIndexMask, entry_code(q.z));
+      if (rem > 3) visit(q.w & kIndexMask, entry_code(q.w));
     }
   } else {  // list overflow: scan the cells
     NbrSource<DIM> src;
@@ -279,29 +285,23 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
     cwv = (Ce.pres_eq == 1) ? Ce.cs * ratio * ratio * ratio : Ce.cs;
   }
   const float inv = 1.f / rw;
-  v.S.D32[w] = make_float4(inv, p * inv * inv, cwv, rw);
+  if (o.spec32) {
+    v.S.PX32[w] = make_float4(oi.x, oi.y, oi.z, -inv);
+    v.S.V32LO[w].w = cwv;
+  } else {
+    v.S.D32[w] = make_float4(inv, p * inv * inv, cwv, rw);
+  }
 }
 
 // ---------------------------------------------------------------------------
 // Fluid pair force, FP32 with compensated sums, over the neighbour lists
 // ---------------------------------------------------------------------------
-// FL selects a compile-time specialisation: 0 = every option read at run time;
-// 1, 2 and 3 = Morris viscosity, squared-density gradient, no tensile-instability
-// term, no XSPH, one h, and pair constants (artificial viscosity, masses) the
-// same for every class, taken from the launch parameters instead of the class
-// table (the dam-break configuration): without (1) or with (2) the strain-rate
-// sums of the LES / Bingham options, or with them and the learned closure's
-// vorticity (3). The list walk is a counted
-// loop so that the next neighbour's loads can be issued before this one's
-// arithmetic; each pair issues all of its neighbour loads before the support
-// test (ld_early).
-// Register caps measured on the 6.7M-particle dam break (64 to 112 swept): the
-// strain-rate flavours run best at 96 (20 warps/SM), the plain one at 80, the
-// general one at 128.
-template <int DIM, int KT, int FL>
-__global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_kernel(DevView v) {
-  constexpr bool SPEC = FL != 0;
-  constexpr bool CLOSURE = FL == 3;
+// Every option read at run time (forces_spec32_kernel serves the usual ones).
+// The list walk is a counted loop so that the next neighbour's loads can be
+// issued before this one's arithmetic; each pair issues all of its neighbour
+// loads before the support test (ld_early).
+template <int DIM, int KT>
+__global__ void __maxnreg__(128) forces_fluid32_kernel(DevView v) {
   __shared__ unsigned long long cred[32];
   const StepScalars* sc = v.sc;
   if (sc->all_stop) return;
@@ -338,13 +338,13 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
   const int fi = Ci.flags;
   const bool shep = (fi & CF_SHEPARD) && (Is.shepard_counter == o.shepard_step);
   const bool sr_self = fi & (CF_T0 | CF_LES);
-  const bool use_sr = SPEC ? (FL >= 2) : (bool)o.need_sr;
-  const bool xsph_on = SPEC ? false : o.xsph != 0.0;
+  const bool use_sr = o.need_sr;
+  const bool xsph_on = o.xsph != 0.0;
   const float xsph = o.xsph32;
   const float3 cs = cell_size_f(g);
   const float mu_u = o.mu_u32;
   const bool uniform_mu = o.uniform_mu, dyn_mu = o.dyn_mu;
-  const int vis_eq = SPEC ? 0 : o.vis_eq, grad_type = SPEC ? 0 : o.grad_type;
+  const int vis_eq = o.vis_eq, grad_type = o.grad_type;
   Kahan ax, ay, az, dr;
   float zw = 0.f, sd = 0.f, xs0 = 0.f, xs1 = 0.f, xs2 = 0.f;
   // strain-rate sums as sums of products a_r x_c (a = c2 vab): diagonal
@@ -353,9 +353,8 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
   // apart (m01, m10, ...)
   float m00 = 0.f, m11 = 0.f, m22 = 0.f, m01 = 0.f, m02 = 0.f, m12 = 0.f, m10 = 0.f, m20 = 0.f, m21 = 0.f;
   int nnb = 0;
-  const bool closure = SPEC ? (CLOSURE && (fi & CF_LES)) : (o.closure && (fi & CF_LES));
-  // the closure flavour always keeps the antisymmetric sums apart
-  const bool split_sr = SPEC ? CLOSURE : closure;
+  const bool closure = o.closure && (fi & CF_LES);
+  const bool split_sr = closure;
   const float cf2 = g.cellfac2_32;
   const bool uniform_h = o.uniform_h;
   const float ih_u = o.inv_h32;
@@ -368,11 +367,11 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
     const int clsj = wj & 0xffff;
     float x0, x1, x2;
     rel_pos<DIM>(cs, oi, oj, code, x0, x1, x2);
-    const float hb = SPEC ? hi : 0.5f * (hi + oj.w);  // one h: (h + h) / 2 = h exactly
+    const float hb = 0.5f * (hi + oj.w);
     const float r2 = x0 * x0 + x1 * x1 + x2 * x2;
     // the list's own support test (exact in FP32; lists with a skin hold more)
     if (r2 > cf2 * hb * hb) return;
-    const PClass32& Cj = CT[SPEC ? 0 : clsj];
+    const PClass32& Cj = CT[clsj];
     const int fjf = wj >> 16;
     const bool fj = fjf & CF_FREE;
     npair2 += fj ? 1u : 2u;
@@ -388,20 +387,20 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
     const float GK = KernF<DIM, KT>::GK(q, inv_q, cwg);
     const float K = KernF<DIM, KT>::W(q, cwh);
     const float dj = dj4.w, inv_j = dj4.x, Pj = dj4.y, cj_snd = dj4.z, pj = vj.w;
-    const float mj = SPEC ? (fj ? o.m_free32 : o.fpm_wall32 * mi) : (fj ? Cj.mass : Cj.fpmassc * mi);
+    const float mj = fj ? Cj.mass : Cj.fpmassc * mi;
     const float v0 = (vi.x - vj.x) + (vil.x - vjl.x), v1 = (vi.y - vj.y) + (vil.y - vjl.y),
                 v2 = (vi.z - vj.z) + (vil.z - vjl.z);
     const float vx = v0 * x0 + v1 * x1 + v2 * x2;
     float PI = 0.f;
-    const float Alpha = SPEC ? o.alpha32 : 0.5f * (Ci.alpha + Cj.alpha);
-    const float Beta = SPEC ? o.beta32 : 0.5f * (Ci.beta + Cj.beta);
+    const float Alpha = 0.5f * (Ci.alpha + Cj.alpha);
+    const float Beta = 0.5f * (Ci.beta + Cj.beta);
     if ((Alpha != 0.f || Beta != 0.f) && vx < 0.f) {
       const float D = r2 + 0.01f * hb * hb;
       const float t = hb * vx;
       PI = __fdividef(t * (-Alpha * 0.5f * (ci_snd + cj_snd) * D + Beta * t), D * D * (0.5f * (di + dj)));
     }
     float TI = 0.f;
-    if (!SPEC && ((fi | fjf) & CF_TI)) {
+    if ((fi | fjf) & CF_TI) {
       float Ri = 0.f, Rj = 0.f;
       if ((pi + pj) < 0.f) {
         if (pi < 0.f) Ri = -pi * inv_i * inv_i;
@@ -417,7 +416,7 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
         vab0 = v0; vab1 = v1; vab2 = v2;
         if (uniform_mu) Mu = mu_u;
         else {
-          const float muj = dyn_mu ? v.S.MU32[j] : (SPEC ? Ci.mu0 : Cj.mu0);
+          const float muj = dyn_mu ? v.S.MU32[j] : Cj.mu0;
           Mu = __fdividef(2.f * mui * muj, mui + muj);
         }
       } else {
@@ -483,23 +482,13 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
     const int4* __restrict__ nl4 = reinterpret_cast<const int4*>(v.S.nl) + nl_slot(i);
     const size_t N = (size_t)v.nl_stride;
     const int nch = (cnt + 3) >> 2;
-    // the strain-rate flavour loads the next chunk one chunk ahead (measured:
-    // it helps there and costs the plain flavour a little)
-    constexpr bool kAhead = FL >= 2;
-    int4 qn = (kAhead && nch > 0) ? nl4[0] : make_int4(0, 0, 0, 0);
     for (int c = 0; c < nch; ++c) {  // one 16-byte chunk of 4 entries per load
-      int4 q;
-      if (kAhead) {
-        q = qn;
-        if (c + 1 < nch) qn = nl4[(size_t)(c + 1) * N];
-      } else {
-        q = nl4[(size_t)c * N];
-      }
+      const int4 q = nl4[(size_t)c * N];
       const int rem = cnt - 4 * c;
-      pair(q.x & kIndexMask, q.x >> kCodeShift);
-      if (rem > 1) pair(q.y & kIndexMask, q.y >> kCodeShift);
-      if (rem > 2) pair(q.z & kIndexMask, q.z >> kCodeShift);
-      if (rem > 3) pair(q.w & kIndexMask, q.w >> kCodeShift);
+      pair(q.x & kIndexMask, entry_code(q.x));
+      if (rem > 1) pair(q.y & kIndexMask, entry_code(q.y));
+      if (rem > 2) pair(q.z & kIndexMask, entry_code(q.z));
+      if (rem > 3) pair(q.w & kIndexMask, entry_code(q.w));
     }
   } else {  // list overflow: scan the cells
     NbrSource<DIM> src;
@@ -556,6 +545,444 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
     if (cand < dtc) dtc = cand;
   }
   block_dt32_and_pairs(v, Ci.inst, active, dtc, (unsigned long long)npair2, cred);
+}
+
+// ---------------------------------------------------------------------------
+// The same for the usual options: Morris viscosity, squared-density gradient, no
+// tensile instability or XSPH, one h, and pair constants (artificial viscosity,
+// masses, flags) the same for every free and every fixed class, taken from the
+// launch (Options::spec32: the dam breaks, the channel). FL 1: without strain
+// rates; 2: with them (LES, Bingham); 3: with the learned closure's sums too.
+//
+// The kernel is bound by instruction issue and the latency of its gathers, so
+//  - a neighbour is three 16-byte records instead of four (PX32: offset and +-1 /
+//    density, negative for a fixed one; V32: velocity and pressure; V32LO: the
+//    velocity's low-order part and the sound speed), what else a pair needs
+//    following from those;
+//  - a lane takes two neighbours at a time: six loads in flight, and every
+//    operation that both need in packed FP32x2 arithmetic (one issue slot for
+//    the two values, each rounded as the scalar operation rounds);
+//  - no branch on the support: outside it kernel and gradient are exact zeros;
+//  - otherwise the general kernel's expressions, rounding by rounding, except
+//    the artificial viscosity (one hardware reciprocal, without the densities);
+//  - the compensated sums are kept apart for the even and the odd neighbours and
+//    joined at the end by an exact two-sum;
+//  - 2^lg lanes share a particle's list.
+// Measured per step (pair kernel alone, before -> now): 6.7M particles with the
+// closure 4330 -> 2740 us, 1.0M without strain rates 485 -> 320 us, 86k in 2D
+// 24.6 -> 20.4 us, the 920-particle channel 34.8 -> 15.4 us. Register caps: 3D
+// 128 (136, 144: 3276; the first form of this kernel at 112: 3173, at 96: 3438).
+// ---------------------------------------------------------------------------
+PSPH_D float2 f2(float a, float b) { return make_float2(a, b); }
+PSPH_D float2 dup(float a) { return make_float2(a, a); }
+PSPH_D float2 operator+(float2 a, float2 b) { return __fadd2_rn(a, b); }
+PSPH_D float2 operator-(float2 a, float2 b) { return __ffma2_rn(b, dup(-1.f), a); }
+PSPH_D float2 operator*(float2 a, float2 b) { return __fmul2_rn(a, b); }
+PSPH_D float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+PSPH_D float rsqrt_ftz(float x) {  // 1/sqrt of a positive normal number, 2 ulp
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+PSPH_D float rcp_ftz(float x) {  // 1/x, 1 ulp
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Two Kahan sums side by side.
+struct Kahan2 {
+  float2 s = make_float2(0.f, 0.f), c = make_float2(0.f, 0.f);
+  PSPH_D void add(float2 x) {
+    const float2 y = x - c;
+    const float2 t = s + y;
+    c = (t - s) - y;
+    s = t;
+  }
+};
+// s - c of two compensated sums joined: the sum of the s with its rounding error
+// (Knuth's two-sum) in c.
+PSPH_D void join(float& s, float& c, float s2, float c2) {
+  const float t = s + s2, b = t - s;
+  const float e = (s - (t - b)) + (s2 - b);
+  c = (c + c2) - e;
+  s = t;
+}
+
+// Kernel and gradient (1/r dW/dr) of two separations in KernF's expressions; exact
+// zeros outside the support.
+template <int DIM, int KT>
+PSPH_D void kern2(float2 q, float2 inv_q, float cwh, float cwg, float2& K, float2& GK) {
+  if (KT == 1) {
+    float2 t = fma2(q, dup(-0.5f), dup(1.f));
+    t.x = fmaxf(t.x, 0.f);
+    t.y = fmaxf(t.y, 0.f);
+    const float2 t2 = t * t;
+    GK = (t2 * t) * dup(cwg * -5.f);
+    K = (dup(cwh) * (t2 * t2)) * fma2(q, dup(2.f), dup(1.f));
+  } else {
+    K = f2(KernF<DIM, KT>::W(q.x, cwh), KernF<DIM, KT>::W(q.y, cwh));
+    GK = f2(KernF<DIM, KT>::GK(q.x, inv_q.x, cwg), KernF<DIM, KT>::GK(q.y, inv_q.y, cwg));
+  }
+}
+
+// On a Shepard step the filter divides SumDen by ZWab: FP32 sums whose rounding
+// goes into the density and, times c^2, into the next step's pressure. They are
+// then taken one neighbour after the other in the order of the cells, a cell's
+// particles by original index, as the general kernel's expressions take them,
+// so that a filtered density depends neither on the pair kernel's lanes nor on
+// the sort's free-first order. (ZWab, SumDen) of particle i, asked for where the
+// filter can apply (ZWab above 0.6); a call, so that one step in 41 takes no
+// registers from the others.
+template <int DIM, int KT>
+__device__ __noinline__ float2 filter_sums(const DevView& v, const int* __restrict__ orig, int i, int cnt, int inst) {
+  const Options& o = v.o;
+  const Spec32& c32 = o.spec32c;
+  const GridDev& g = grid_of(v, inst);
+  const float3 cs = cell_size_f(g);
+  const float4 xi = v.S.PX32[i];
+  const float hi = c32.h, ih = o.inv_h32, ih2 = ih * ih;
+  const float cwh = KernF<DIM, KT>::cw() * (DIM == 2 ? ih2 : ih2 * ih);
+  float zw = 0.f, sd = 0.f;
+  auto one = [&](const int e) {
+    const float4 oj = v.S.PX32[e & kIndexMask];
+    float x0, x1, x2;
+    rel_pos<DIM>(cs, xi, oj, entry_code(e), x0, x1, x2);
+    const float r2 = x0 * x0 + x1 * x1 + x2 * x2;
+    if (r2 > g.cellfac2_32 * hi * hi) return;
+    const float inv_r = (r2 > 0.f) ? rsqrtf(r2) : 0.f;
+    const float q = r2 * inv_r * ih;
+    const float K = KernF<DIM, KT>::W(q, cwh);
+    const float mj = oj.w > 0.f ? c32.m_free : c32.m_wall;
+    const float inv_j = fabsf(oj.w);
+    zw += mj * inv_j * K;
+    sd += mj * K;
+  };
+  auto entry = [&](int k) { return v.S.nl[nl_index(v.nl_stride, i, k)]; };
+  for (int k = 0; k < cnt;) {
+    const int code = entry_code(entry(k));
+    int mid = k, end = k;  // the cell's free particles, then its fixed ones
+    while (end < cnt && entry_code(entry(end)) == code) {
+      if (v.S.PX32[entry(end) & kIndexMask].w > 0.f && mid == end) ++mid;
+      ++end;
+    }
+    int a = k, b = mid;
+    while (a < mid || b < end) {
+      const int ea = a < mid ? entry(a) : 0, eb = b < end ? entry(b) : 0;
+      const bool first = b >= end || (a < mid && orig[ea & kIndexMask] < orig[eb & kIndexMask]);
+      one(first ? ea : eb);
+      if (first) ++a;
+      else ++b;
+    }
+    k = end;
+  }
+  return make_float2(zw, sd);
+}
+
+// ZWab of a particle from its lanes' sums
+PSPH_D float group_zw(float2 zw, int L) {
+  float z = zw.x + zw.y;
+  for (int m = 1; m < L; m <<= 1) z += __shfl_xor_sync(0xffffffffu, z, m);
+  return z;
+}
+
+constexpr int kSumsMax = 20;  // a particle's sums on their way to its thread
+
+template <int DIM, int KT, int FL>
+__global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32_kernel(DevView v, int lg) {
+  // in 3D the partner's mass is folded into the kernel's constants (the closure
+  // flavour does not fit its registers otherwise: 3204 us against 2740)
+  constexpr bool FOLD = DIM == 3;
+  extern __shared__ float staged[];  // kSumsMax rows of (block size >> lg), when lg > 0
+  __shared__ unsigned long long cred[32];
+  const StepScalars* sc = v.sc;
+  if (sc->all_stop) return;
+  const Persist& P = cur_persist(v);
+  const int n = sc->n;
+  const int lane = threadIdx.x & 31, L = 1 << lg, sub = lane & (L - 1);
+  int i = (blockIdx.x * blockDim.x + threadIdx.x) >> lg;
+  const Options& o = v.o;
+  const PClass32* __restrict__ CT = v.cls32;
+  unsigned npair2 = 0;  // 2 per pair with a free partner, 1 per wall partner (the pair is counted once)
+  bool active = false;
+  int cell = -1, ci_cls = 0;
+  if (i < n) {
+    ci_cls = P.cls[i];
+    const bool run = !v.inst[CT[ci_cls].inst].stop;
+    active = run && (CT[ci_cls].flags & CF_FREE);
+    cell = v.S.cellid[i];
+    if (run && !active && sub == 0) {
+      v.S.A4[i] = make_double4_32a(o.gravity[0], o.gravity[1], o.gravity[2], 0.0);
+      v.S.zwab[i] = 1.0;
+    }
+  }
+  const PClass32& Ci = CT[ci_cls];
+  const int inst_i = Ci.inst;
+  const GridDev& g = grid_of(v, inst_i);
+  const InstState& Is = v.inst[inst_i];
+  const int is = active ? i : 0;
+  const float4 xi = v.S.PX32[is];
+  const float4 vi = v.S.V32[is];
+  const float4 vl = v.S.V32LO[is];
+  const float inv_i = xi.w, Pi = vi.w * inv_i * inv_i, snd_i = vl.w;
+  const float mui = o.dyn_mu ? v.S.MU32[is] : o.mu_u32;
+  const bool shep = (Ci.flags & CF_SHEPARD) && (Is.shepard_counter == o.shepard_step);
+  const float3 cs = cell_size_f(g);
+  const Spec32& c32 = o.spec32c;
+  const float reach2 = g.cellfac2_32 * c32.h * c32.h;
+  const float ih2 = o.inv_h32 * o.inv_h32;
+  float cwh = KernF<DIM, KT>::cw() * (DIM == 2 ? ih2 : ih2 * o.inv_h32), cwg = cwh * ih2;
+  if (FOLD) {
+    cwh *= c32.m_free;
+    if (FL == 1) cwg *= c32.m_free;
+  }
+  Kahan2 ax, ay, az, dr;
+  float2 zw = dup(0.f), sd = dup(0.f);
+  // strain-rate sums as sums of products a_r x_c (a = c2 vab); without the
+  // closure (whose vorticity needs the antisymmetric part) the off-diagonal
+  // pairs summed
+  float m00 = 0.f, m11 = 0.f, m22 = 0.f, m01 = 0.f, m02 = 0.f, m12 = 0.f, m10 = 0.f, m20 = 0.f, m21 = 0.f;
+  int nnb = 0;
+  // two neighbours; the second one counts when both is set
+  auto pairs = [&](const int ea, const int eb, const bool both) {
+    const int ja = ea & kIndexMask, jb = eb & kIndexMask;
+    const float4 xa = ld_early(v.S.PX32 + ja), xb = ld_early(v.S.PX32 + jb);
+    const float4 va = ld_early(v.S.V32 + ja), vb = ld_early(v.S.V32 + jb);
+    const float4 la = ld_early(v.S.V32LO + ja), lb = ld_early(v.S.V32LO + jb);
+    const int ca = entry_code(ea), cb = entry_code(eb);
+    float2 x0 = fma2(f2(code_back<0>(ca), code_back<0>(cb)), dup(cs.x), f2(xi.x - xa.x, xi.x - xb.x));
+    float2 x1 = fma2(f2(code_back<1>(ca), code_back<1>(cb)), dup(cs.y), f2(xi.y - xa.y, xi.y - xb.y));
+    float2 x2 = dup(0.f);
+    if (DIM == 3) x2 = fma2(f2(code_back<2>(ca), code_back<2>(cb)), dup(cs.z), f2(xi.z - xa.z, xi.z - xb.z));
+    float2 r2 = fma2(x1, x1, x0 * x0);
+    if (DIM == 3) r2 = fma2(x2, x2, r2);
+    if (!both) r2.y = c32.far2;  // beyond the support: every term of it is zero
+    const bool fa = xa.w > 0.f, fb = xb.w > 0.f;
+    const bool ia = r2.x <= reach2, ib = r2.y <= reach2;
+    npair2 += (ia ? (fa ? 1u : 2u) : 0u) + (ib ? (fb ? 1u : 2u) : 0u);
+    if (FL == 3) nnb += (ia ? 1 : 0) + (ib ? 1 : 0);
+    const float2 inv_r = f2(rsqrt_ftz(fmaxf(r2.x, 1e-30f)), rsqrt_ftz(fmaxf(r2.y, 1e-30f)));
+    const float2 q = r2 * inv_r * dup(o.inv_h32);
+    float2 K, GK;
+    kern2<DIM, KT>(q, inv_r * dup(c32.h), cwh, cwg, K, GK);
+    const float2 inv_j = f2(fabsf(xa.w), fabsf(xb.w));
+    // StrainRate += (m_j / rho_j) S with S = -GK [2 v_a x_a, v_a x_b + v_b x_a, ...]
+    // (Source/Interaction.cpp:114-117, no 1/2): a = c2 vab, S_rc = a_r x_c + a_c x_r;
+    // before the mass is folded in, in the general kernel's roundings: a feature
+    // of the closure near the edge of its range would pick the other model
+    float2 c2 = dup(0.f);
+    if (FL >= 2) {
+      const float ka = fa ? c32.sr_free : c32.sr_wall, kb = fb ? c32.sr_free : c32.sr_wall;  // -1, or 0 where no rate is taken
+      const float2 m = f2(fa ? c32.m_free : c32.m_wall, fb ? c32.m_free : c32.m_wall);
+      c2 = GK * f2(ka, kb) * ((c32.wall_scaled ? m : dup(c32.m_free)) * inv_j);
+      if (FOLD) GK = GK * dup(c32.m_free);
+    }
+    float2 mj = dup(c32.m_free);
+    if (c32.wall_scaled) {
+      if (FOLD) {
+        const float2 w = f2(fa ? 1.f : c32.wall_scale, fb ? 1.f : c32.wall_scale);
+        K = K * w;
+        GK = GK * w;
+      } else {
+        mj = f2(fa ? c32.m_free : c32.m_wall, fb ? c32.m_free : c32.m_wall);
+      }
+    }
+    float2 v0 = f2(vi.x - va.x, vi.x - vb.x) + f2(vl.x - la.x, vl.x - lb.x);
+    float2 v1 = f2(vi.y - va.y, vi.y - vb.y) + f2(vl.y - la.y, vl.y - lb.y);
+    float2 v2 = f2(vi.z - va.z, vi.z - vb.z) + f2(vl.z - la.z, vl.z - lb.z);
+    float2 vx = fma2(v1, x1, v0 * x0);
+    if (DIM == 3) vx = fma2(v2, x2, vx);
+    // pressure and artificial viscosity: (-a c MU + b MU^2) / rho_ij with MU = h v.x / D;
+    // rho_ij = (1/inv_i + 1/inv_j) / 2
+    float2 s = dup(Pi) + f2(va.w, vb.w) * inv_j * inv_j;
+    if (c32.av) {
+      const float2 vm = f2(fminf(vx.x, 0.f), fminf(vx.y, 0.f));
+      const float2 D = r2 + dup(c32.eps2);
+      const float2 ivp = dup(inv_i) * inv_j;
+      const float2 c = (dup(snd_i) + f2(la.w, lb.w)) * ivp;
+      const float2 den = D * (dup(inv_i) + inv_j);
+      float2 num = vm * dup(c32.neg_alpha_h) * c;
+      float2 rc = f2(rcp_ftz(den.x), rcp_ftz(den.y));
+      if (c32.beta_h2 != 0.f) num = fma2(vm * vm * ivp, dup(2.f * c32.beta_h2) * f2(rcp_ftz(D.x), rcp_ftz(D.y)), num);
+      s = fma2(num, rc, s);
+    }
+    s = s * GK * dup(-1.f);
+    float2 c = dup(0.f);
+    float2 w0 = v0, w1 = v1, w2 = v2;
+    {
+      float2 mu2 = dup(2.f * mui);
+      if (o.dyn_mu) {
+        // harmonic mean with a free neighbour, the own viscosity with a wall
+        const float ma = v.S.MU32[ja], mb = v.S.MU32[jb];
+        mu2 = f2(fa ? __fdividef(4.f * mui * ma, mui + ma) : 2.f * mui, fb ? __fdividef(4.f * mui * mb, mui + mb) : 2.f * mui);
+      }
+      c = mu2 * dup(inv_i) * inv_j * GK;
+    }
+    if (!(fa && fb)) {  // walls: their no-slip velocity, or no viscous term where both slip
+      if (!fa) {
+        const float4 ns = v.S.NSV32[ja];
+        w0.x = (vi.x - (2.f * va.x - ns.x)) + (vl.x - 2.f * la.x);
+        w1.x = (vi.y - (2.f * va.y - ns.y)) + (vl.y - 2.f * la.y);
+        w2.x = (vi.z - (2.f * va.z - ns.z)) + (vl.z - 2.f * la.z);
+        if (!c32.wall_visc) c.x = 0.f;
+      }
+      if (!fb) {
+        const float4 ns = v.S.NSV32[jb];
+        w0.y = (vi.x - (2.f * vb.x - ns.x)) + (vl.x - 2.f * lb.x);
+        w1.y = (vi.y - (2.f * vb.y - ns.y)) + (vl.y - 2.f * lb.y);
+        w2.y = (vi.z - (2.f * vb.z - ns.z)) + (vl.z - 2.f * lb.z);
+        if (!c32.wall_visc) c.y = 0.f;
+      }
+    }
+    const float2 md = FOLD ? inv_j : mj * inv_j;
+    if (FL >= 2) {
+      const float2 a0 = c2 * w0, a1 = c2 * w1, a2 = c2 * w2;
+      auto two = [](float& m, float2 a, float2 x) { m = fmaf(a.y, x.y, fmaf(a.x, x.x, m)); };
+      two(m00, a0, x0);
+      two(m11, a1, x1);
+      two(m01, a0, x1);
+      if (DIM == 3) {
+        two(m22, a2, x2);
+        two(m02, a0, x2);
+        two(m12, a1, x2);
+      }
+      two(FL == 3 ? m10 : m01, a1, x0);
+      two(FL == 3 ? m20 : m02, a2, x0);
+      two(FL == 3 ? m21 : m12, a2, x1);
+    }
+    auto times_m = [&](float2 f) { return FOLD ? f : mj * f; };
+    ax.add(times_m(fma2(s, x0, c * w0)));
+    ay.add(times_m(fma2(s, x1, c * w1)));
+    if (DIM == 3) az.add(times_m(fma2(s, x2, c * w2)));
+    dr.add(md * (GK * vx));  // times rho_i at the end
+    zw = fma2(md, K, zw);
+    if (shep) sd = FOLD ? sd + K : fma2(mj, K, sd);
+  };
+  const int cnt = (active && cell >= 0) ? v.S.nl_count[i] : 0;
+  if (cnt >= 0) {
+    // pair p of the list: entries 2p and 2p + 1, half a 16-byte chunk
+    const int2* __restrict__ nl2 = reinterpret_cast<const int2*>(v.S.nl) + 2 * (size_t)nl_slot(i);
+    const size_t N = 2 * (size_t)v.nl_stride;
+    const int np = (cnt + 1) >> 1;
+    int2 next = (sub < np) ? nl2[(sub >> 1) * N + (sub & 1)] : make_int2(0, 0);
+    for (int p = sub; p < np; p += L) {
+      const int2 e = next;
+      const int q = p + L;
+      if (q < np) next = nl2[(size_t)(q >> 1) * N + (q & 1)];
+      const bool both = 2 * p + 1 < cnt;
+      pairs(e.x, both ? e.y : e.x, both);
+    }
+  } else if (sub == 0) {  // list overflow: scan the cells
+    NbrSource<DIM> src;
+    src.init(v, g, i, true, 1.0f);
+    while (true) {
+      int code;
+      const int j = src.next(v, &code);
+      if (j < 0) break;
+      const int e = (int)((unsigned)code << kCodeShift) | j;
+      pairs(e, e, false);
+    }
+  }
+  float2 filtered = dup(0.f);
+  const float zw_all = group_zw(zw, L);
+  const bool filter = shep && active && cell >= 0 && cnt >= 0 && zw_all > 0.599f;
+  if (filter && sub == 0) filtered = filter_sums<DIM, KT>(v, P.orig, i, cnt, inst_i);
+  // even and odd neighbours together, then the lanes of the particle
+  float out[kSumsMax];
+  {
+    Kahan2* const k[4] = {&ax, &ay, &az, &dr};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float ss = k[e]->s.x, cc = k[e]->c.x;
+      join(ss, cc, k[e]->s.y, k[e]->c.y);
+      for (int m = 1; m < L; m <<= 1) {
+        const float s2 = __shfl_xor_sync(0xffffffffu, ss, m), c2 = __shfl_xor_sync(0xffffffffu, cc, m);
+        // the same operands in the same order on both sides
+        const bool up = sub & m;
+        float a = up ? s2 : ss, b = up ? c2 : cc;
+        join(a, b, up ? ss : s2, up ? cc : c2);
+        ss = a;
+        cc = b;
+      }
+      out[2 * e] = ss;
+      out[2 * e + 1] = cc;
+    }
+    out[8] = filter ? filtered.x : zw.x + zw.y;
+    out[9] = filter ? filtered.y : sd.x + sd.y;
+    const float mm[9] = {m00, m11, m22, m01, m02, m12, m10, m20, m21};
+#pragma unroll
+    for (int e = 0; e < 9; ++e) out[10 + e] = mm[e];
+    out[19] = (float)nnb;
+    const int last = FL == 1 ? 10 : (FL == 2 ? 16 : 20);
+#pragma unroll
+    for (int e = 8; e < 20; ++e)
+      if (e < last)
+        for (int m = 1; m < L; m <<= 1) out[e] += __shfl_xor_sync(0xffffffffu, out[e], m);
+    if (lg > 0) {  // one thread per particle from here: full warps for the FP64 conversions
+      const int np = blockDim.x >> lg;
+      if (sub == 0)
+#pragma unroll
+        for (int e = 0; e < 20; ++e)
+          if (e < last) staged[e * np + (threadIdx.x >> lg)] = out[e];
+      __syncthreads();
+      i = blockIdx.x * np + threadIdx.x;
+      active = (int)threadIdx.x < np && i < n;
+      if (active) {
+#pragma unroll
+        for (int e = 0; e < 20; ++e)
+          if (e < last) out[e] = staged[e * np + threadIdx.x];
+        ci_cls = P.cls[i];
+        active = !v.inst[CT[ci_cls].inst].stop && (CT[ci_cls].flags & CF_FREE);
+      }
+    }
+  }
+  const int inst = CT[ci_cls].inst;
+  float dtc = FLT_MAX;
+  if (active) {
+    auto value = [&](int e) { return (double)out[2 * e] - (double)out[2 * e + 1]; };
+    const double axd = o.gb[0] + value(0), ayd = o.gb[1] + value(1), azd = o.gb[2] + value(2);
+    const double drd = value(3) * P.X4[i].w;
+    v.S.A4[i] = make_double4_32a(axd, ayd, azd, drd);
+    v.S.zwab[i] = out[8];
+    if (o.any_shepard) v.S.sumden[i] = out[9];
+    if (FL >= 2) {
+      const float* m = out + 10;
+      // symmetric sums 2 m_rr and m_rc + m_cr; the antisymmetric m_rc - m_cr
+      // (closure) is the vorticity's
+      const float sr0 = 2.f * m[0], sr4 = 2.f * m[1], sr8 = 2.f * m[2];
+      const float sr1 = FL == 3 ? m[3] + m[6] : m[3], sr2 = FL == 3 ? m[4] + m[7] : m[4],
+                  sr5 = FL == 3 ? m[5] + m[8] : m[5];
+      // the 6 distinct sums in FP32 (the FP64 tensor is built on download)
+      float2* q = reinterpret_cast<float2*>(v.S.sr32 + 6 * (size_t)i);
+      q[0] = make_float2(sr0, sr1);
+      q[1] = make_float2(sr2, sr4);
+      q[2] = make_float2(sr5, sr8);
+      // Mat1's ShearRate contraction (Source/Particle.cpp:151-153) of the
+      // symmetric sums, in FP32: the update and the closure take it from here
+      const float temp = sr0 * sr0 + 2.f * sr1 * sr1 + 2.f * sr2 * sr2 + sr4 * sr4 + 2.f * sr5 * sr5 + sr8 * sr8;
+      v.S.cshear[i] = sqrtf(0.5f * temp);
+      if (FL == 3 && (CT[ci_cls].flags & CF_LES)) {
+        const float w01 = m[3] - m[6], w02 = m[4] - m[7], w12 = m[5] - m[8];
+        v.S.cvort[i] = sqrtf(w01 * w01 + w02 * w02 + w12 * w12);
+        v.S.cnnb[i] = out[19];
+        const float det =
+            sr0 * (sr4 * sr8 - sr5 * sr5) - sr1 * (sr1 * sr8 - sr5 * sr2) + sr2 * (sr1 * sr5 - sr4 * sr2);
+        v.S.cr3[i] = temp > 0.f ? det / (temp * sqrtf(temp)) : 0.f;
+      }
+    }
+    // the FP64 sums are finite exactly when their FP32 parts are (checked in FP32)
+    float fin = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) fin += out[e] - out[e];
+    if (!(fin == 0.f)) atomicOr(&v.sc->status, ST_NONFINITE);
+    // this particle's time-step bound sqrt_h_a sqrt(h/|a|) in FP32; the
+    // minimum over particles (FP32 within a warp) and AdaptiveTimeStep stay FP64
+    const float ax32 = d2f_rn(axd), ay32 = d2f_rn(ayd), az32 = d2f_rn(azd);
+    const float an = sqrtf(ax32 * ax32 + ay32 * ay32 + az32 * az32);
+    const float cand = o.sqrt_h_a32 * sqrtf(c32.h / an);
+    if (cand < dtc) dtc = cand;
+  }
+  block_dt32_and_pairs(v, inst, active, dtc, (unsigned long long)npair2, cred);
 }
 
 // ---------------------------------------------------------------------------
@@ -810,6 +1237,22 @@ void prepare32_dispatch(const DevView& v, cudaStream_t st) {
   }
 }
 
+template <int DIM, int KT>
+void spec32_dispatch(const DevView& v, int bt, cudaStream_t st) {
+  // lanes per particle: one, and 4 for the quintic spline, whose lists are more
+  // than twice as long (the 920-particle channel: 24.6 us with one lane, 14.3
+  // with 4; the 1M-particle Wendland dam break: 311 us with one, 365 with two).
+  // As in the FP64 form it depends on nothing that an ensemble changes.
+  constexpr int lg = KT == PSPH_QUINTIC_SPLINE ? 2 : 0;
+  const int per = bt >> lg;
+  const int nb = v.ncap <= 0 ? 1 : (v.ncap + per - 1) / per;
+  const size_t sm = lg > 0 ? sizeof(float) * kSumsMax * per : 0;
+  const Options& o = v.o;
+  if (!o.need_sr) forces_spec32_kernel<DIM, KT, 1><<<nb, bt, sm, st>>>(v, lg);
+  else if (!o.closure) forces_spec32_kernel<DIM, KT, 2><<<nb, bt, sm, st>>>(v, lg);
+  else forces_spec32_kernel<DIM, KT, 3><<<nb, bt, sm, st>>>(v, lg);
+}
+
 template <int DIM>
 void forces32_dispatch(const DevView& v, cudaStream_t st) {
   const int bt = (v.o.pair_block >= 32 && v.o.pair_block <= kMaxPairBlock) ? v.o.pair_block : kFT32;
@@ -822,23 +1265,18 @@ void forces32_dispatch(const DevView& v, cudaStream_t st) {
     }
     return;
   }
-  const Options& o = v.o;
-  const bool spec = o.vis_eq == 0 && o.grad_type == 0 && !o.any_ti && o.xsph == 0.0 && o.uniform_h &&
-                    o.uniform_av && o.uniform_mass && (o.uniform_mu || o.dyn_mu);
-  const int fl = spec ? (o.need_sr ? (o.closure ? 3 : 2) : 1) : 0;
-  switch (o.kt * 4 + fl) {
-    case 0: forces_fluid32_kernel<DIM, 0, 0><<<nb, bt, 0, st>>>(v); break;
-    case 1: forces_fluid32_kernel<DIM, 0, 1><<<nb, bt, 0, st>>>(v); break;
-    case 2: forces_fluid32_kernel<DIM, 0, 2><<<nb, bt, 0, st>>>(v); break;
-    case 3: forces_fluid32_kernel<DIM, 0, 3><<<nb, bt, 0, st>>>(v); break;
-    case 4: forces_fluid32_kernel<DIM, 1, 0><<<nb, bt, 0, st>>>(v); break;
-    case 5: forces_fluid32_kernel<DIM, 1, 1><<<nb, bt, 0, st>>>(v); break;
-    case 6: forces_fluid32_kernel<DIM, 1, 2><<<nb, bt, 0, st>>>(v); break;
-    case 7: forces_fluid32_kernel<DIM, 1, 3><<<nb, bt, 0, st>>>(v); break;
-    case 8: forces_fluid32_kernel<DIM, 2, 0><<<nb, bt, 0, st>>>(v); break;
-    case 9: forces_fluid32_kernel<DIM, 2, 1><<<nb, bt, 0, st>>>(v); break;
-    case 10: forces_fluid32_kernel<DIM, 2, 2><<<nb, bt, 0, st>>>(v); break;
-    default: forces_fluid32_kernel<DIM, 2, 3><<<nb, bt, 0, st>>>(v); break;
+  if (v.o.spec32) {
+    switch (v.o.kt) {
+      case 0: spec32_dispatch<DIM, 0>(v, bt, st); break;
+      case 1: spec32_dispatch<DIM, 1>(v, bt, st); break;
+      default: spec32_dispatch<DIM, 2>(v, bt, st); break;
+    }
+    return;
+  }
+  switch (v.o.kt) {
+    case 0: forces_fluid32_kernel<DIM, 0><<<nb, bt, 0, st>>>(v); break;
+    case 1: forces_fluid32_kernel<DIM, 1><<<nb, bt, 0, st>>>(v); break;
+    default: forces_fluid32_kernel<DIM, 2><<<nb, bt, 0, st>>>(v); break;
   }
 }
 

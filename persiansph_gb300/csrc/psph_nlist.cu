@@ -125,7 +125,7 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
       else if (y < 0 || y >= g.nc[1]) continue;
       const float gy = dy < 0 ? oi.y : (dy > 0 ? cs.y - oi.y : 0.f);
       const int base = g.cell_base + (z * g.nc[1] + y) * g.nc[0];
-      const int cyz = 3 * (dy + 1) + 9 * (dz + 1);
+      const int cyz = (dy + 1) << 2 | (dz + 1) << 4;
       const float cy = -(float)dy * cs.y, cz = -(float)dz * cs.z;  // exact: dy, dz in {-1, 0, 1}
       int slo = -xs, shi = 2 * xs - 1;
       if (cull) {
@@ -144,7 +144,7 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
         const int bin = 2 * ((base + x) * xs + sl);
         int lo = sstart[bin];
         const int hi = sstart[fixed ? bin + 1 : 2 * ((base + x) * xs + s1 + 1)];
-        const int tag = ((dx + 1) + cyz) << kCodeShift;
+        const int tag = (int)((unsigned)((dx + 1) | cyz) << kCodeShift);
         // i's position relative to this cell's origin: x_i - x_j = a - off_j
         // (one rounding away from rel_pos's form, which the pair kernels
         // apply exactly; the list's margin covers the difference)
@@ -298,7 +298,7 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
       const float gya = dy < 0 ? oa.y : (dy > 0 ? cs.y - oa.y : 0.f);
       const float gyb = dy < 0 ? ob.y : (dy > 0 ? cs.y - ob.y : 0.f);
       const int base = g.cell_base + (z * g.nc[1] + y) * g.nc[0];
-      const int cyz = 3 * (dy + 1) + 9 * (dz + 1);
+      const int cyz = (dy + 1) << 2 | (dz + 1) << 4;
       const float cy = -(float)dy * cs.y, cz = -(float)dz * cs.z;
       cand.row(3 * (dz - zlo_) + (dy + 1));
       int slo = -xs, shi = 2 * xs - 1;
@@ -325,7 +325,7 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
         const int hi = sstart[fixed ? bin + 1 : bin + step];
         const bool second = mixed && (bin & 1);
         const float thra = (second && fixed_a) ? -1.f : thr, thrb = (second && fixed_b) ? -1.f : thr;
-        const int tag = ((dx + 1) + cyz) << kCodeShift;
+        const int tag = (int)((unsigned)((dx + 1) | cyz) << kCodeShift);
         const float cx = -(float)dx * cs.x;
         const float axa = oa.x + cx, aya = oa.y + cy, aza = oa.z + cz;
         const float axb = ob.x + cx, ayb = ob.y + cy, azb = ob.z + cz;

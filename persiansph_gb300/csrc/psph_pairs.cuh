@@ -11,8 +11,21 @@
 
 namespace psph {
 
-constexpr int kCodeShift = 26;  // neighbour-list entry: index | code << 26 (index < 2^26)
+// Neighbour-list entry: index | code << 26 (index < 2^26), where code is the cell
+// offset of the neighbour, (dx+1) | (dy+1) << 2 | (dz+1) << 4: two bits an axis,
+// read without divisions; its order is that of the cells' walk.
+constexpr int kCodeShift = 26;
 constexpr int kIndexMask = (1 << kCodeShift) - 1;
+PSPH_HD int entry_code(int e) { return (int)((unsigned)e >> kCodeShift); }
+PSPH_HD int cell_code(int dx, int dy, int dz) { return (dx + 1) | (dy + 1) << 2 | (dz + 1) << 4; }
+constexpr int kCodeMirror = 0x2a;  // the code seen from the neighbour: kCodeMirror - code
+// -dx, -dy, -dz of a code as floats: the upper halves of 1.0f, 0.0f and -1.0f
+// picked by a byte permutation (no conversion, no division)
+template <int AXIS>
+PSPH_D float code_back(int code) {
+  const int sel = (code & (3 << (2 * AXIS))) * (0x2200 >> (2 * AXIS)) + 0x1022;
+  return __uint_as_float(__byte_perm(0x00003f80u, 0x0000bf80u, (unsigned)sel));
+}
 
 // Neighbour-list layout: chunks of 4 consecutive entries of one particle (16
 // bytes), chunk-major across particles: chunk c of particle i is int4 number
@@ -103,12 +116,12 @@ PSPH_D int ref_code(int home, int cand) {
   const int dx = min(max((cand & 1023) - (home & 1023), -1), 1);
   const int dy = min(max(((cand >> 10) & 1023) - ((home >> 10) & 1023), -1), 1);
   const int dz = min(max((cand >> 20) - (home >> 20), -1), 1);
-  return (dx + 1) + 3 * (dy + 1) + 9 * (dz + 1);
+  return cell_code(dx, dy, dz);
 }
 
 // Same rule from a cell-offset code (candidate cell minus home cell, wrapped).
 PSPH_D bool first_of_pair_code(int code, int orig_w, int orig_f) {
-  const int dxc = code % 3 - 1, dyc = (code / 3) % 3 - 1, dzc = code / 9 - 1;
+  const int dxc = (code & 3) - 1, dyc = (code >> 2 & 3) - 1, dzc = (code >> 4) - 1;
   if (dzc != 0) return dzc > 0;
   if (dyc != 0) return dyc > 0;
   if (dxc != 0) return dxc > 0;
@@ -117,7 +130,7 @@ PSPH_D bool first_of_pair_code(int code, int orig_w, int orig_f) {
 
 // Candidate stream over the 3x3(x3) cells around a home cell, one row split
 // into its 3 cells where the periodic x axis wraps; reports each candidate's
-// cell offset code (dx+1) + 3(dy+1) + 9(dz+1) relative to the home cell.
+// cell offset code (cell_code) relative to the home cell.
 template <int DIM>
 struct Cands32 {
   static constexpr int NR = (DIM == 3 ? 9 : 3) * 3;
@@ -150,7 +163,7 @@ struct Cands32 {
     if (g.periodic[1]) y = (y + g.nc[1]) % g.nc[1];
     else if (y < 0 || y >= g.nc[1]) return false;
     base = g.cell_base + (z * g.nc[1] + y) * g.nc[0];
-    code_yz = 3 * (dy + 1) + 9 * (dz + 1);
+    code_yz = (dy + 1) << 2 | (dz + 1) << 4;
     if (!wrapx) {
       if (sub) return false;
       const int x0 = max(cx - 1, 0), x1 = min(cx + 1, g.nc[0] - 1);
@@ -182,10 +195,9 @@ struct Cands32 {
 // x_i - x_j in FP32 from the cell-offset code (cell_j - cell_i) and the offsets.
 template <int DIM>
 PSPH_D void rel_pos(const float3& cs, const float4& oi, const float4& oj, int code, float& x0, float& x1, float& x2) {
-  const int dxc = code % 3 - 1, dyc = (code / 3) % 3 - 1, dzc = code / 9 - 1;
-  x0 = -(float)dxc * cs.x + (oi.x - oj.x);
-  x1 = -(float)dyc * cs.y + (oi.y - oj.y);
-  x2 = (DIM == 3) ? -(float)dzc * cs.z + (oi.z - oj.z) : 0.f;
+  x0 = fmaf(code_back<0>(code), cs.x, oi.x - oj.x);
+  x1 = fmaf(code_back<1>(code), cs.y, oi.y - oj.y);
+  x2 = (DIM == 3) ? fmaf(code_back<2>(code), cs.z, oi.z - oj.z) : 0.f;
 }
 
 PSPH_HD float3 cell_size_f(const GridDev& g) {
@@ -224,7 +236,7 @@ struct NbrSource {
       if (k >= cnt) return -1;
       const int e = v.S.nl[nl_index(v.nl_stride, i, k)];
       ++k;
-      *code = e >> kCodeShift;
+      *code = entry_code(e);
       return e & kIndexMask;
     }
     const float3 csz = cell_size_f(*g);

@@ -1,8 +1,9 @@
-"""FP64 pair kernels at the sizes and options where their lane groups and the
+"""Pair kernels at the sizes and options where their lane groups and the
 constant-parameter form can go wrong, one step against the oracle: particle
 counts that leave groups, warps and blocks partly filled, lists longer than
 their capacity (the cell scan), every kernel, beta and wall masses, free-slip
-walls, and tensile stresses (the tolerance is the FP64 form's parity bound)."""
+walls, and tensile stresses. The tolerances are the forms' parity bounds: 1e-12
+(FP64) and 1e-5 (FP32C) of each particle's sum of term magnitudes."""
 import numpy as np
 import pytest
 
@@ -72,3 +73,44 @@ def test_soil_2d(gpu, hfac, ti, alpha):
     s[free, 1, 1] += rng.uniform(-400.0, 400.0, len(free))
     p.set("sigma", s)
     one_step(dom, dt, f"soil hfac {hfac} ti {ti}")
+
+
+@pytest.mark.parametrize("les", [False, True])
+@pytest.mark.parametrize("dim,kernel,hfac,beta,fpmassc,slip", [
+    (2, 0, 1.2, 0.0, 1.0, False), (2, 0, 3.2, 0.2, 1.0, False), (2, 2, 1.1, 0.0, 0.8, False),
+    (2, 1, 1.3, 0.1, 1.0, True), (3, 1, 1.3, 0.0, 1.0, False), (3, 1, 1.9, 0.2, 0.7, False),
+    (3, 0, 1.3, 0.0, 1.0, True), (3, 2, 1.0, 0.0, 1.0, False)])
+def test_fluid_fp32c(gpu, dim, kernel, hfac, beta, fpmassc, slip, les):
+    if dim == 2:
+        dx = 0.031
+        dom, dt, _ = scenarios.dam_break_2d(dx=dx, L=0.4, H=0.7, TL=1.1, TH=0.9, kernel=kernel, hfac=hfac)
+    else:
+        dx = 0.05
+        dom, dt, _ = scenarios.dam_break_3d(dx=dx, L=0.3, H=0.35, W=0.25, TL=0.6, TH=0.4, TW=0.25, kernel=kernel,
+                                            hfac=hfac)
+    p = dom.particles
+    p.set("beta", beta)
+    p.set("fpmassc", fpmassc)
+    if slip:
+        p.set("no_slip", 0)
+    if les:
+        p.set("les", 1)
+        p.set("csmag", 0.17)
+    stir(p, dx, 7, dim, 0.5)
+    o = OracleDomain(dom.config(dt), p, initial=True)
+    o.step(1)
+    a_scale, dr_scale = o.scales()
+    ref = o.download()
+    cfg = dom.config(dt)
+    cfg.precision = 1
+    gd = GpuDomain(cfg)
+    gd.upload(p)
+    gd.step(1)
+    got = gd.download_fields()
+    free = ref["is_free"] == 1
+    assert np.max(np.linalg.norm(got["a"] - ref["a"], axis=1)[free] / a_scale[free]) <= 1e-5
+    assert np.max(np.abs(got["ddensity"] - ref["ddensity"])[free] / (dr_scale[free] + 1e-300)) <= 1e-5
+    if les:
+        s = np.abs(ref["strain_rate"][free]).max()
+        assert np.max(np.abs(got["strain_rate"] - ref["strain_rate"])[free]) <= 1e-5 * s
+    gd.close()
