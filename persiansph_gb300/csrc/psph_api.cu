@@ -559,6 +559,26 @@ void derive_class_options(const std::vector<PClass>& classes, bool mixed, bool d
     o.spec32 = o.fp32 && o.vis_eq == PSPH_MORRIS && o.grad_type == PSPH_SQUARED_DENSITY && o.uniform_h &&
                o.uniform_av && o.uniform_mass && (o.uniform_mu || dyn_mu) && !o.any_ti && o.xsph == 0.0 &&
                !o.has_solid && one;
+    // the FP32C 2D soil kernel's: also one sound speed and tensile instability, and
+    // one free mass per instance
+    bool soil = o.fp32 && o.dim == 2 && o.grad_type == PSPH_SQUARED_DENSITY && o.xsph == 0.0 && o.uniform_h &&
+                o.uniform_av && one && !o.ti_always && !mixed;
+    std::vector<double> m_inst;
+    double fpm = -1.0;
+    for (const PClass& C : classes) {
+      soil = soil && C.material == 3 && C.cs == C0.cs && C.ti == C0.ti && C.tin == C0.tin && C.tid == C0.tid;
+      if (!C.is_free) {
+        soil = soil && (fpm < 0.0 || C.fpmassc == fpm);
+        fpm = C.fpmassc;
+        continue;
+      }
+      if ((size_t)C.inst >= m_inst.size()) m_inst.resize(C.inst + 1, -1.0);
+      soil = soil && (m_inst[C.inst] < 0.0 || m_inst[C.inst] == C.mass);
+      m_inst[C.inst] = C.mass;
+    }
+    o.soil32 = soil;
+    o.soil_noslip = ((ff | fw) & CF_NOSLIP) != 0;
+    if (soil) o.fpm_wall32 = fpm < 0.0 ? 1.f : (float)fpm;
     Spec32& f = o.spec32c;
     f.h = (float)C0.h;
     f.m_free = o.m_free32;
@@ -963,12 +983,12 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
     if (lf && (st = dalloc(c, &P->H4b, N))) return st;
     if (dyn_mu && (st = dalloc(c, &P->mu, N))) return st;
     if (inout && (st = dalloc(c, &P->io, N))) return st;
-    if (o.has_solid) {
-      if ((st = dalloc(c, &P->sigma, 9 * N)) || (st = dalloc(c, &P->sigma_h, 9 * N)) ||
-          (st = dalloc(c, &P->strain, 9 * N)) || (st = dalloc(c, &P->strain_h, 9 * N)) ||
-          (st = dalloc(c, &P->shear, 9 * N)) || (st = dalloc(c, &P->shear_h, 9 * N)) ||
-          (st = dalloc(c, &P->tir, 9 * N)))
-        return st;
+  }
+  if (o.has_solid) {  // one array each for both buffers
+    for (double* Persist::*t : {&Persist::sigma, &Persist::sigma_h, &Persist::strain, &Persist::strain_h,
+                                &Persist::shear, &Persist::shear_h, &Persist::tir}) {
+      if ((st = dalloc(c, &(c->PA.*t), 9 * N))) return st;
+      c->PB.*t = c->PA.*t;
     }
   }
   Scratch& S = c->S;
@@ -976,7 +996,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
   const size_t NB = 2 * NC * kMaxXsub;  // sort bins at the finest x-slab split, free and fixed apart
   if ((st = dalloc(c, &S.key, N)) || (st = dalloc(c, &S.count, NB + 2)) || (st = dalloc(c, &S.start, NC + 3)) ||
       (st = dalloc(c, &S.sstart, NB + 3)) ||
-      (st = dalloc(c, &S.tmp_perm, N)) || (st = dalloc(c, &S.perm, N)) || (st = dalloc(c, &S.cellid, N)) ||
+      (st = dalloc(c, &S.tmp_perm, N)) || (st = dalloc(c, &S.slot, N)) || (st = dalloc(c, &S.cellid, N)) ||
       (st = dalloc(c, &S.block_sums, (NB + 2 + 1023) / 1024 + 1)) ||
       (st = dalloc(c, &S.OFF32, N)) || (st = dalloc(c, &S.D4, N)) || (st = dalloc(c, &S.nl_count, N)) ||
       (st = dalloc(c, &S.A4, N)) || (st = dalloc(c, &S.zwab, N)) || (st = dalloc(c, &S.sumden, N)) ||
@@ -1011,6 +1031,8 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
       return st;
   }
   if (o.fp32 && o.has_solid) {
+    if (o.soil32 && (st = dalloc(c, &S.PX32, N))) return st;
+    if ((st = dalloc(c, &S.rates32, 3 * N))) return st;
     if ((st = dalloc(c, &S.SIG32, 2 * N)) || (st = dalloc(c, &S.VB32, N))) return st;
     if (o.any_ti && (st = dalloc(c, &S.TIR32, 2 * N))) return st;
   }
@@ -1086,21 +1108,6 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
       CUDA_TRY(c, cudaMemcpyAsync(c->PA.io, parts[0].in_out, NP * sizeof(int), cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (o.has_solid) {
-      // Mat3 neither reads nor writes the ShearStress history: a soil domain
-      // whose uploaded history is zero does not carry it through the sort
-      o.carry_shear_h = 1;
-      if (o.soil_pairs) {
-        o.carry_shear_h = 0;
-        for (int q = 0; q < ninst && !o.carry_shear_h; ++q) {
-          const double* hs = lf ? parts[q].shear_stressa : parts[q].shear_stressb;
-          if (hs)
-            for (size_t e = 0; e < 9 * (size_t)parts[q].n; ++e)
-              if (hs[e] != 0.0) {
-                o.carry_shear_h = 1;
-                break;
-              }
-        }
-      }
       for (int q = 0; q < ninst; ++q) {
         const psph_particles* p = &parts[q];
         const double* srcs[7] = {p->sigma, lf ? p->sigmaa : p->sigmab, p->strain, lf ? p->straina : p->strainb,
@@ -1710,6 +1717,12 @@ psph_status alive_of(psph_ctx* c, int q, std::vector<std::pair<int, int>>& order
 // original index among the instance's alive particles, Array::DelItems'
 // order), then per requested field one gather into a staging buffer laid out
 // as the caller's array and one copy into that array.
+// Whether an array is one of the tensors that keep their place in the sort.
+bool keeps_place(const Persist& P, const double* a) {
+  return a && (a == P.sigma || a == P.sigma_h || a == P.strain || a == P.strain_h || a == P.shear || a == P.shear_h ||
+               a == P.tir);
+}
+
 __global__ void dl_flag_kernel(const uint8_t* __restrict__ alive, const int* __restrict__ orig, int n, int lo,
                                int hi, int* __restrict__ flag) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1720,23 +1733,28 @@ __global__ void dl_row_kernel(const uint8_t* __restrict__ alive, const int* __re
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < n) row[s] = (alive[s] && orig[s] >= lo && orig[s] < hi) ? rank[orig[s] - lo] : -1;
 }
-// dst[row * width + e] = src[s * stride + off + e]
+// dst[row * width + e] = src[s * stride + off + e], or of place[s] (tensors keep
+// their place: the original index)
 __global__ void dl_gather_kernel(const double* __restrict__ src, int stride, int off, int width,
-                                 double* __restrict__ dst, const int* __restrict__ row, int n) {
+                                 double* __restrict__ dst, const int* __restrict__ row, int n,
+                                 const int* __restrict__ place) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const int r = row[s];
   if (r < 0) return;
-  for (int e = 0; e < width; ++e) dst[(size_t)r * width + e] = src[(size_t)s * stride + off + e];
+  const size_t at = (size_t)(place ? place[s] : s) * stride + off;
+  for (int e = 0; e < width; ++e) dst[(size_t)r * width + e] = src[at + e];
 }
 // psph_patch: the caller's row r = row[s] back into slot s (dl_gather_kernel's reverse)
 __global__ void patch_scatter_kernel(double* __restrict__ dst, int stride, int off, int width,
-                                     const double* __restrict__ src, const int* __restrict__ row, int n) {
+                                     const double* __restrict__ src, const int* __restrict__ row, int n,
+                                     const int* __restrict__ place) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const int r = row[s];
   if (r < 0) return;
-  for (int e = 0; e < width; ++e) dst[(size_t)s * stride + off + e] = src[(size_t)r * width + e];
+  const size_t at = (size_t)(place ? place[s] : s) * stride + off;
+  for (int e = 0; e < width; ++e) dst[at + e] = src[(size_t)r * width + e];
 }
 __global__ void patch_scatter_int_kernel(int* __restrict__ dst, const int* __restrict__ src,
                                          const int* __restrict__ row, int n) {
@@ -1877,9 +1895,10 @@ psph_status download_impl(psph_ctx* c, int q, psph_particles* out) {
       if (batch_of[a] != b) continue;
       const F& f = *act[a];
       // the FP32C fluid kernel keeps its strain-rate sums in FP32: expand them first
-      if (f.dev == c->S.strain_rate && c->S.sr32) launch_expand_sr32(view(c), n, s);
+      if ((f.dev == c->S.strain_rate && (c->S.sr32 || c->S.rates32)) || (f.dev == c->S.rotation_rate && c->S.rates32))
+        launch_expand_sr32(view(c), n, s);
       dl_gather_kernel<<<nb, 256, 0, s>>>(f.dev, f.stride, f.off, f.width, c->dl_buf + (size_t)seg[a] * m,
-                                          c->dl_row, n);
+                                          c->dl_row, n, keeps_place(P, f.dev) ? P.orig : nullptr);
     }
   };
   if (nbatch > 0) gather_batch(0);
@@ -2064,7 +2083,8 @@ psph_status patch_impl(psph_ctx* c, const psph_particles* p) {
   for (const F& f : fields) {
     if (!f.in || !f.dev) continue;
     CUDA_TRY(c, cudaMemcpyAsync(c->dl_buf, f.in, (size_t)m * f.width * sizeof(double), cudaMemcpyHostToDevice, s));
-    patch_scatter_kernel<<<nb, 256, 0, s>>>(f.dev, f.stride, f.off, f.width, c->dl_buf, c->dl_row, n);
+    patch_scatter_kernel<<<nb, 256, 0, s>>>(f.dev, f.stride, f.off, f.width, c->dl_buf, c->dl_row, n,
+                                            keeps_place(P, f.dev) ? P.orig : nullptr);
   }
   CUDA_TRY(c, cudaGetLastError());
 

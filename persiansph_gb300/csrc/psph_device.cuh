@@ -15,7 +15,10 @@ struct Persist {
   int* orig;     // original particle index
   int* io;       // in/out-flow state (Particle::InOut: 0, 1 in-flow, 2 out-flow); null without the boundary
   double* mu;    // dynamic viscosity (LES / Bingham); null when constant per class
-  // soil / solid tensors (9 doubles per particle, row-major); null without solids
+  // soil / solid tensors (9 doubles per particle, row-major); null without solids.
+  // They keep one place each, at the particle's original index (tensor_row), in
+  // both buffers: moving them every step cost more than the indirection does
+  // (1.0M soil particles: sort 332 us a step with, 110 without).
   double* sigma;
   double* sigma_h;   // leapfrog Sigmaa | MVerlet Sigmab
   double* strain;
@@ -32,7 +35,7 @@ struct Scratch {
   int* start;      // ncells + 3 exclusive prefix: cell c's particles are [start[c], start[c+1])
   int* sstart;     // 2 ncells * xsub + 3 exclusive prefix over the x-slabs of the cells, free and fixed apart
   int* tmp_perm;
-  int* perm;
+  int* slot;       // a particle's place in its segment before the ranking
   int* cellid;     // cell of each sorted particle (orphan/dead: -1)
   int* block_sums;
   // per-step derived / outputs
@@ -84,6 +87,7 @@ struct Scratch {
   float* cnnb;           // neighbours inside the support
   float* cshear;         // FP32C: ShearRate of the strain-rate sums
   float* sr32;           // FP32C fluid: the strain-rate sums xx, xy, xz, yy, yz, zz (6 per particle)
+  float4* rates32;       // FP32C soil / solids: strain- and rotation-rate sums, 3 float4 per particle
   float* cr3;            // FP32C: det(StrainRate) / (StrainRate:StrainRate)^(3/2)
   float* cfeat;          // raw network features, 6 per particle
   double* nut;           // eddy viscosity from the network; -1 = use Smagorinsky
@@ -131,7 +135,6 @@ struct Options {
   int couple_solid;   // fluid + solid: CalcForce12
   int fsi;            // Domain::FSI: the solid's interpolated pressure and velocity
   int swi;            // Domain::SWIType
-  int carry_shear_h;  // the sort moves the ShearStress history (Mat2, or a non-zero upload)
   int uniform_h;      // every particle has the same h
   int any_periodic;   // some instance has a periodic axis
   int any_periodic_x; // some instance has a periodic x axis (no staged neighbour scan)
@@ -143,6 +146,8 @@ struct Options {
   int spec64;         // the FP64 fluid pair kernel's SPEC form applies, with these constants
   Spec64 spec;
   int spec32;         // the FP32C fluid pair kernel's
+  int soil32;         // the FP32C 2D soil pair kernel's constant-parameter form applies
+  int soil_noslip;    // (with it) a wall or its partner is no-slip
   Spec32 spec32c;
   double mu_u;        // that viscosity
   double inv_h;       // 1/h when uniform
@@ -194,7 +199,20 @@ struct DevView {
 PSPH_D const GridDev& grid_of(const DevView& v, int inst) { return v.grids[inst]; }
 
 PSPH_D const Persist& cur_persist(const DevView& v) { return v.sc->buf ? v.PB : v.PA; }
+// A particle's row in the tensor arrays.
+PSPH_D size_t tensor_row(const Persist& P, int s) { return 9 * (size_t)P.orig[s]; }
 PSPH_D const Persist& next_persist(const DevView& v) { return v.sc->buf ? v.PA : v.PB; }
+
+// A soil or solid particle's FP32 rate sums (rates32) as the FP64 tensors.
+PSPH_D void widen_rates(const float4* __restrict__ q, double* __restrict__ sr, double* __restrict__ rr) {
+  const float4 a = q[0], b = q[1], c = q[2];
+  sr[0] = a.x; sr[1] = a.y; sr[2] = a.z;
+  sr[3] = a.y; sr[4] = a.w; sr[5] = b.x;
+  sr[6] = a.z; sr[7] = b.x; sr[8] = b.y;
+  rr[0] = 0.0; rr[1] = b.z; rr[2] = b.w;
+  rr[3] = -(double)b.z; rr[4] = 0.0; rr[5] = c.x;
+  rr[6] = -(double)b.w; rr[7] = -(double)c.x; rr[8] = 0.0;
+}
 
 // Launch wrappers (defined in the .cu files).
 void launch_sort(const DevView& v, cudaStream_t st);      // bin + scan + scatter + rank + reorder + flip
@@ -206,7 +224,7 @@ void nlist_configure();                                   // once, outside strea
 void launch_prepare(const DevView& v, cudaStream_t st);   // per-particle derived quantities, TIR
 void launch_prepare32(const DevView& v, cudaStream_t st); // FP32C form: copies + wall interpolation
 void launch_forces32(const DevView& v, cudaStream_t st);  // FP32C form: fluid pair forces
-void launch_expand_sr32(const DevView& v, int n, cudaStream_t st);  // sr32 -> the FP64 strain_rate tensors
+void launch_expand_sr32(const DevView& v, int n, cudaStream_t st);  // sr32 / rates32 -> the FP64 rate tensors
 void launch_wall(const DevView& v, cudaStream_t st);      // wall interpolation
 void launch_forces(const DevView& v, cudaStream_t st);    // pair forces + per-block dt minimum
 void launch_saturation(const DevView& v, cudaStream_t st); // fluid-soil: saturation check and weight switch

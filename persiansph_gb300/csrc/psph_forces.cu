@@ -160,7 +160,7 @@ constexpr int kInfoCls = 0xffff, kInfoFree = 1 << 16, kInfoList = 1 << 17, kInfo
 // kInfoTir of particle w, from its tensile-instability stress
 PSPH_D int tir_bit(const DevView& v, const Persist& P, int w) {
   if (!v.o.any_ti || !P.tir) return 0;
-  const double* T = P.tir + 9 * (size_t)w;
+  const double* T = P.tir + tensor_row(P, w);
   long long b = 0;
 #pragma unroll
   for (int e = 0; e < 9; ++e) b |= __double_as_longlong(T[e]);
@@ -235,7 +235,7 @@ PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int f
     sk += K;
     if (mat < 3) p += vf.w * K + (gx * x0 + gy * x1 + gz * x2) * xf.w * K;
     if (mat > 1) {
-      const double* sf = P.sigma + 9 * (size_t)f;
+      const double* sf = P.sigma + tensor_row(P, f);
 #pragma unroll
       for (int e = 0; e < 9; ++e) sig[e] += sf[e] * K;
     }
@@ -302,16 +302,16 @@ PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int f
     const double is = (sk != 0.0 && mat > 1) ? 1.0 / sk : 1.0;
 #pragma unroll
     for (int e = 0; e < 9; ++e) sig[e] = f[5 + e] * is;
-    double* sw = P.sigma + 9 * (size_t)w;
+    double* sw = P.sigma + tensor_row(P, w);
 #pragma unroll
     for (int e = 0; e < 9; ++e) sw[e] = sig[e];
     if (P.shear) {
-      double* tw = P.shear + 9 * (size_t)w;
+      double* tw = P.shear + tensor_row(P, w);
 #pragma unroll
       for (int e = 0; e < 9; ++e) tw[e] = 0.0;
     }
     if (sk != 0.0 && mat > 1 && Cw.ti > 0.0) {
-      tensile_tir<DIM>(sig, Cw.ti, xw.w, P.tir + 9 * (size_t)w);
+      tensile_tir<DIM>(sig, Cw.ti, xw.w, P.tir + tensor_row(P, w));
       if (v.S.pair_info) v.S.pair_info[w] = (v.S.pair_info[w] & ~kInfoTir) | tir_bit(v, P, w);
     }
   }
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v, int lg, in
       const double pr = P.V4[q].w;
       v.S.D4[q] = make_double4_32a(inv, pr * inv * inv, sound_speed(C.pres_eq, C.cs, rho, C.rho0), rho);
       if (o.has_solid && C.material > 1 && C.ti > 0.0)
-        tensile_tir<DIM>(P.sigma + 9 * (size_t)q, C.ti, rho, P.tir + 9 * (size_t)q);
+        tensile_tir<DIM>(P.sigma + tensor_row(P, q), C.ti, rho, P.tir + tensor_row(P, q));
     }
     // (the FP32C pair kernels have copies of their own)
     if (v.S.pair_info)
@@ -961,10 +961,10 @@ __global__ void __launch_bounds__(kFT) forces_solid_kernel(DevView v, int lg) {
   const double4_32a di4 = v.S.D4[is];
   const double di = xi.w, inv_i = di4.x, mi = Ci.mass, hi = Ci.h;
   const bool shep = Ci.shepard && (Is.shepard_counter == o.shepard_step);
-  const double* __restrict__ Ti = P.tir + 9 * (size_t)is;
+  const double* __restrict__ Ti = P.tir + tensor_row(P, is);
   double Si[9];  // the own stress, over density squared for the squared-density gradient
   {
-    const double* __restrict__ S = P.sigma + 9 * (size_t)is;
+    const double* __restrict__ S = P.sigma + tensor_row(P, is);
     const double c = (o.grad_type == 0) ? inv_i * inv_i : 1.0;
 #pragma unroll
     for (int e = 0; e < 9; ++e) Si[e] = S[e] * c;
@@ -1056,7 +1056,7 @@ __global__ void __launch_bounds__(kFT) forces_solid_kernel(DevView v, int lg) {
       const double4_32a vbj = (o.scheme == PSPH_MVERLET) ? P.H4[j] : P.H4b[j];
       vab0 = vi.x - vbj.x; vab1 = vi.y - vbj.y; vab2 = vi.z - vbj.z;
     }
-    const double* __restrict__ Sj = P.sigma + 9 * (size_t)j;
+    const double* __restrict__ Sj = P.sigma + tensor_row(P, j);
     double M[9];
     if (o.grad_type == 0) {
       const double cj2 = inv_j * inv_j;
@@ -1071,7 +1071,7 @@ __global__ void __launch_bounds__(kFT) forces_solid_kernel(DevView v, int lg) {
     if (o.any_ti && (Ci.ti > 0.0 || Cj.ti > 0.0) && (o.ti_always || ((tir_i | v.S.pair_info[j]) & kInfoTir))) {
       const double Wd = Kern<DIM, KT>::W((Ci.tid + Cj.tid) / (2.0 * hb), cwh);
       const double TIs = pow(K / Wd, (Ci.tin + Cj.tin) / 2.0);
-      const double* __restrict__ Tj = P.tir + 9 * (size_t)j;
+      const double* __restrict__ Tj = P.tir + tensor_row(P, j);
 #pragma unroll
       for (int e = 0; e < 9; ++e) M[e] += (Ti[e] + Tj[e]) * TIs;
     }
@@ -1374,7 +1374,7 @@ PSPH_D void seepage_pair(const DevView& v, const Persist& P, const InstState& Is
     double kp = Cs.kp, kp2 = Cs.kp2;
     if (Cs.var_por && Cs.is_free && !Is.k_initial) {
       // VarPorosity: the permeabilities of the strain the last update left
-      const double* E = P.strain + 9 * (size_t)s;
+      const double* E = P.strain + tensor_row(P, s);
       const double ev = (E[0] + E[4] + E[8]);
       permeability(Cs.seep_type, (Cs.n0 + ev) / (1.0 + ev), Cs.dgrain, &kp, &kp2);
     }

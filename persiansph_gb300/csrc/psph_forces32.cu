@@ -1013,21 +1013,45 @@ __global__ void __launch_bounds__(kFT32) solid_copies32_kernel(DevView v) {
   const double4_32a vv = P.V4[w];
   float lx, ly, lz;
   const float vx = d2f_split(vv.x, &lx), vy = d2f_split(vv.y, &ly), vz = d2f_split(vv.z, &lz);
-  v.S.V32[w] = make_float4(vx, vy, vz, d2f_rn(vv.w));
   // the velocity's low-order part: near-rigid motion (a column settling as one
   // body) makes v_i - v_j far smaller than v, and the pair differences take
   // (hi_i - hi_j) + (lo_i - lo_j), exact to ~2^-48 of |v|
-  v.S.V32LO[w] = make_float4(lx, ly, lz, 0.f);
   const double4_32a d = v.S.D4[w];
-  v.S.D32[w] = make_float4(d2f_rn(d.x), d2f_rn(d.y), d2f_rn(d.z), d2f_rn(d.w));
-  sym_store(v.S.SIG32, (size_t)w, P.sigma + 9 * (size_t)w);
-  if (v.o.any_ti) sym_store(v.S.TIR32, (size_t)w, P.tir + 9 * (size_t)w);
+  const double* sg = P.sigma + tensor_row(P, w);
+  if (v.o.soil32) {  // the three records of forces_soil32_kernel
+    const double* t = P.tir + tensor_row(P, w);
+    const bool tens = v.o.any_ti && (t[0] != 0.0 || t[1] != 0.0 || t[4] != 0.0);
+    const float4 x = v.S.OFF32[w];
+    const bool fr = C.flags & CF_FREE;
+    const float inv = d2f_rn(d.x);
+    v.S.PX32[w] = make_float4(x.x, x.y, d2f_rn(sg[0]), d2f_rn(sg[1]));
+    v.S.V32[w] = make_float4(vx, vy, d2f_rn(sg[4]), fr ? inv : -inv);
+    v.S.V32LO[w] = make_float4(lx, ly, vz, tens ? 1.f : 0.f);
+    if (tens) v.S.TIR32[2 * (size_t)w] = make_float4(d2f_rn(t[0]), d2f_rn(t[1]), 0.f, d2f_rn(t[4]));
+  } else {
+    v.S.V32[w] = make_float4(vx, vy, vz, d2f_rn(vv.w));
+    v.S.V32LO[w] = make_float4(lx, ly, lz, 0.f);
+    v.S.D32[w] = make_float4(d2f_rn(d.x), d2f_rn(d.y), d2f_rn(d.z), d2f_rn(d.w));
+    sym_store(v.S.SIG32, (size_t)w, sg);
+    if (v.o.any_ti) sym_store(v.S.TIR32, (size_t)w, P.tir + tensor_row(P, w));
+  }
   if (!(C.flags & CF_FREE)) {
     const double4_32a vb = (v.o.scheme == PSPH_MVERLET) ? P.H4[w] : P.H4b[w];
     v.S.VB32[w] = make_float4(d2f_rn(vb.x), d2f_rn(vb.y), d2f_rn(vb.z), 0.f);
     const double4_32a ns = v.S.nsv4[w];
     v.S.NSV32[w] = make_float4(d2f_rn(ns.x), d2f_rn(ns.y), d2f_rn(ns.z), 0.f);
   }
+}
+
+// The strain-rate (00 01 02 11 12 22) and rotation-rate (01 02 12) sums of a
+// soil or solid particle, in FP32 as they are summed: the update widens them
+// (36 bytes instead of two FP64 tensors), a download expands them.
+PSPH_D void store_rates32(const DevView& v, int i, float s0, float s1, float s2, float s3, float s4, float s5,
+                          float r0, float r1, float r2) {
+  float4* q = v.S.rates32 + 3 * (size_t)i;
+  q[0] = make_float4(s0, s1, s2, s3);
+  q[1] = make_float4(s4, s5, r0, r1);
+  q[2] = make_float4(r2, 0.f, 0.f, 0.f);
 }
 
 template <int DIM, int KT>
@@ -1205,14 +1229,7 @@ __global__ void __maxnreg__(128) forces_solid32_kernel(DevView v) {
     v.S.zwab[i] = zw;
     if (o.any_shepard) v.S.sumden[i] = sd;
     if (xsph_on) v.S.vxsph4[i] = make_double4_32a(xs0, xs1, xs2, 0.0);
-    double* out = v.S.strain_rate + 9 * (size_t)i;
-    out[0] = sr0; out[1] = sr1; out[2] = sr2;
-    out[3] = sr1; out[4] = sr3; out[5] = sr4;
-    out[6] = sr2; out[7] = sr4; out[8] = sr5;
-    double* ro = v.S.rotation_rate + 9 * (size_t)i;
-    ro[0] = 0.0; ro[1] = rr0; ro[2] = rr1;
-    ro[3] = -(double)rr0; ro[4] = 0.0; ro[5] = rr2;
-    ro[6] = -(double)rr1; ro[7] = -(double)rr2; ro[8] = 0.0;
+    store_rates32(v, i, sr0, sr1, sr2, sr3, sr4, sr5, rr0, rr1, rr2);
     if (!(isfinite(axd) && isfinite(ayd) && isfinite(azd) && isfinite(drd))) atomicOr(&v.sc->status, ST_NONFINITE);
     // this particle's time-step bound sqrt_h_a sqrt(h/|a|) in FP32; the
     // minimum over particles and AdaptiveTimeStep stay FP64
@@ -1222,6 +1239,199 @@ __global__ void __maxnreg__(128) forces_solid32_kernel(DevView v) {
     if (cand < dtc) dtc = cand;
   }
   block_dt_and_pairs<0>(v, Ci.inst, active, dtc, npair2, red, cred);
+}
+
+// The same for soil domains in 2D whose classes share their pair constants
+// (Options::soil32: one h, artificial viscosity, sound speed, tensile-instability
+// constants and flags; one free mass per instance): the granular columns. As in
+// forces_spec32_kernel a lane takes two neighbours at a time in packed FP32x2
+// arithmetic, and a neighbour is three 16-byte records (solid_copies32_kernel):
+//   PX32  x, y, Sigma00, Sigma01      V32  vx, vy, Sigma11, +-1/density (- fixed)
+//   V32LO the low-order parts of vx and vy, vz, whether its TIR is non-zero
+// In 2D the entries with a z index meet a zero separation in the acceleration.
+// The tensile-instability power is evaluated only where one of the two carries a
+// tensile stress (elsewhere it multiplies a zero).
+// 1.0M particles in ten columns: 513 us before (nine loads a neighbour and the
+// power for every pair), 197 us now.
+template <int KT>
+__global__ void __maxnreg__(112) forces_soil32_kernel(DevView v) {
+  __shared__ unsigned long long cred[32];
+  const StepScalars* sc = v.sc;
+  if (sc->all_stop) return;
+  const Persist& P = cur_persist(v);
+  const int n = sc->n;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const Options& o = v.o;
+  const PClass32* __restrict__ CT = v.cls32;
+  float dtc = FLT_MAX;
+  unsigned npair2 = 0;  // 2 per pair with a free partner, 1 per wall partner (the pair is counted once)
+  bool active = false;
+  int cell = -1, ci_cls = 0;
+  if (i < n) {
+    ci_cls = P.cls[i];
+    const bool run = !v.inst[CT[ci_cls].inst].stop;
+    active = run && (CT[ci_cls].flags & CF_FREE);
+    cell = v.S.cellid[i];
+    if (run && !active) {
+      v.S.A4[i] = make_double4_32a(o.gravity[0], o.gravity[1], o.gravity[2], 0.0);
+      v.S.zwab[i] = 1.0;
+    }
+  }
+  const PClass32& Ci = CT[ci_cls];
+  const GridDev& g = grid_of(v, Ci.inst);
+  const InstState& Is = v.inst[Ci.inst];
+  const int is = active ? i : 0;
+  const float4 xi = v.S.PX32[is], vi = v.S.V32[is], vl = v.S.V32LO[is];
+  const float inv_i = fabsf(vi.w), mi = Ci.mass, h = Ci.h, ih = 1.f / h, ih2 = ih * ih;
+  const float cwh = KernF<2, KT>::cw() * ih2, cwg = cwh * ih2;
+  const float ci2 = inv_i * inv_i;
+  const float P00 = xi.z * ci2, P01 = xi.w * ci2, P11 = vi.z * ci2;  // the own stress over density squared
+  const bool shep = (Ci.flags & CF_SHEPARD) && (Is.shepard_counter == o.shepard_step);
+  const float fpm = o.fpm_wall32;
+  const bool wall_scaled = fpm != 1.f, av = Ci.alpha != 0.f || Ci.beta != 0.f;
+  const float ac = Ci.alpha * Ci.cs;
+  const float3 cs = cell_size_f(g);
+  const float reach2 = g.cellfac2_32 * h * h, far2 = 100.f * h * h, eps2 = 0.01f * h * h;
+  const bool noslip = o.soil_noslip;
+  Kahan2 ax, ay, dr;
+  float2 zw = dup(0.f), sd = dup(0.f);
+  float2 s00 = dup(0.f), s01 = dup(0.f), s11 = dup(0.f), r01 = dup(0.f), s02 = dup(0.f), s12 = dup(0.f);
+  auto pairs = [&](const int ea, const int eb, const bool both) {
+    const int ja = ea & kIndexMask, jb = eb & kIndexMask;
+    const float4 xa = ld_early(v.S.PX32 + ja), xb = ld_early(v.S.PX32 + jb);
+    const float4 va = ld_early(v.S.V32 + ja), vb = ld_early(v.S.V32 + jb);
+    const float4 la = ld_early(v.S.V32LO + ja), lb = ld_early(v.S.V32LO + jb);
+    const int ca = entry_code(ea), cb = entry_code(eb);
+    const float2 x0 = fma2(f2(code_back<0>(ca), code_back<0>(cb)), dup(cs.x), f2(xi.x - xa.x, xi.x - xb.x));
+    const float2 x1 = fma2(f2(code_back<1>(ca), code_back<1>(cb)), dup(cs.y), f2(xi.y - xa.y, xi.y - xb.y));
+    float2 r2 = fma2(x1, x1, x0 * x0);
+    if (!both) r2.y = far2;  // beyond the support: every term of it is zero
+    const bool fa = va.w > 0.f, fb = vb.w > 0.f;
+    const bool ia = r2.x <= reach2, ib = r2.y <= reach2;
+    npair2 += (ia ? (fa ? 1u : 2u) : 0u) + (ib ? (fb ? 1u : 2u) : 0u);
+    const float2 inv_r = f2(rsqrt_ftz(fmaxf(r2.x, 1e-30f)), rsqrt_ftz(fmaxf(r2.y, 1e-30f)));
+    float2 K, GK;
+    kern2<2, KT>(r2 * inv_r * dup(ih), inv_r * dup(h), cwh, cwg, K, GK);
+    // soil walls take the partner's density (Source/Interaction.cpp:201-205)
+    const float2 inv_j = f2(fa ? va.w : inv_i, fb ? vb.w : inv_i);
+    float2 mj = dup(mi);
+    if (wall_scaled) mj = f2(fa ? mi : fpm * mi, fb ? mi : fpm * mi);
+    const float2 v0 = f2(vi.x - va.x, vi.x - vb.x) + f2(vl.x - la.x, vl.x - lb.x);
+    const float2 v1 = f2(vi.y - va.y, vi.y - vb.y) + f2(vl.y - la.y, vl.y - lb.y);
+    const float2 vx = fma2(v1, x1, v0 * x0);
+    const float2 cj2 = inv_j * inv_j;
+    float2 M00 = fma2(f2(xa.z, xb.z), cj2, dup(P00));
+    const float2 M01_ = fma2(f2(xa.w, xb.w), cj2, dup(P01));
+    float2 M11 = fma2(f2(va.z, vb.z), cj2, dup(P11));
+    float2 M01 = M01_;
+    if (av) {  // PIij = PI I, PI = (a c MU + b MU^2) / rho_ij with MU = h v.x / D
+      const float2 t = f2(fminf(vx.x, 0.f), fminf(vx.y, 0.f)) * dup(h);
+      const float2 D = r2 + dup(eps2);
+      const float2 ivp = dup(2.f * inv_i) * inv_j;  // rho_ij = (1/inv_i + 1/inv_j) / 2
+      const float2 den = D * D * (dup(inv_i) + inv_j);
+      const float2 PI = t * fma2(dup(Ci.beta), t, dup(ac) * D) * ivp * f2(rcp_ftz(den.x), rcp_ftz(den.y));
+      M00 = M00 + PI;
+      M11 = M11 + PI;
+    }
+    if (vl.w + la.w + lb.w > 0.f) {  // a tensile stress on either side of one of the pairs
+      const float Wd = KernF<2, KT>::W(Ci.tid * ih, cwh);
+      auto add = [&](float k, int j, float tj, float& m00, float& m01, float& m11) {
+        if (!(vl.w + tj > 0.f)) return;
+        const float f = powf(k / Wd, Ci.tin);
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (vl.w > 0.f) t = v.S.TIR32[2 * (size_t)is];
+        if (tj > 0.f) {
+          const float4 u = v.S.TIR32[2 * (size_t)j];
+          t.x += u.x; t.y += u.y; t.w += u.w;
+        }
+        m00 += t.x * f;
+        m01 += t.y * f;
+        m11 += t.w * f;
+      };
+      add(K.x, ja, la.w, M00.x, M01.x, M11.x);
+      add(K.y, jb, lb.w, M00.y, M01.y, M11.y);
+    }
+    const float2 g0 = GK * x0, g1 = GK * x1;
+    // row vector (GK x_ij) times M (Mult, External/matvec.h:806)
+    ax.add(mj * fma2(g1, M01, g0 * M00));
+    ay.add(mj * fma2(g1, M11, g0 * M01));
+    const float2 md = mj * inv_j;
+    dr.add(md * fma2(v1, g1, v0 * g0));  // times rho_i at the end
+    zw = fma2(md, K, zw);
+    if (shep) sd = fma2(mj, K, sd);
+    float2 w0 = v0, w1 = v1, w2 = f2(vl.z - la.z, vl.z - lb.z);
+    if (!(fa && fb)) {
+      auto wall = [&](int j, float4 vj, float4 lj, float& a0, float& a1, float& a2) {
+        if (noslip) {
+          const float4 ns = v.S.NSV32[j];
+          a0 = vi.x - (2.f * vj.x - ns.x);
+          a1 = vi.y - (2.f * vj.y - ns.y);
+          a2 = vl.z - (2.f * lj.z - ns.z);
+        } else {
+          const float4 q = v.S.VB32[j];
+          a0 = vi.x - q.x; a1 = vi.y - q.y; a2 = vl.z - q.z;
+        }
+      };
+      if (!fa) wall(ja, va, la, w0.x, w1.x, w2.x);
+      if (!fb) wall(jb, vb, lb, w0.y, w1.y, w2.y);
+    }
+    const float2 c2 = dup(-0.5f) * GK * md;
+    const float2 p01 = w0 * x1, p10 = w1 * x0;
+    s00 = fma2(c2, w0 * x0, s00);
+    s11 = fma2(c2, w1 * x1, s11);
+    s01 = fma2(c2, p01 + p10, s01);
+    r01 = fma2(c2, p01 - p10, r01);
+    s02 = fma2(c2, w2 * x0, s02);
+    s12 = fma2(c2, w2 * x1, s12);
+  };
+  const int cnt = (active && cell >= 0) ? v.S.nl_count[i] : 0;
+  if (cnt >= 0) {
+    // pair p of the list: entries 2p and 2p + 1, half a 16-byte chunk
+    const int2* __restrict__ nl2 = reinterpret_cast<const int2*>(v.S.nl) + 2 * (size_t)nl_slot(i);
+    const size_t N = 2 * (size_t)v.nl_stride;
+    const int np = (cnt + 1) >> 1;
+    int2 next = np > 0 ? nl2[0] : make_int2(0, 0);
+    for (int p = 0; p < np; ++p) {
+      const int2 e = next;
+      if (p + 1 < np) next = nl2[(size_t)((p + 1) >> 1) * N + ((p + 1) & 1)];
+      const bool both = 2 * p + 1 < cnt;
+      pairs(e.x, both ? e.y : e.x, both);
+    }
+  } else {  // list overflow: scan the cells
+    NbrSource<2> src;
+    src.init(v, g, i, true, 1.0f);
+    while (true) {
+      int code;
+      const int j = src.next(v, &code);
+      if (j < 0) break;
+      const int e = (int)((unsigned)code << kCodeShift) | j;
+      pairs(e, e, false);
+    }
+  }
+  if (active) {
+    auto value = [](Kahan2& k) {
+      join(k.s.x, k.c.x, k.s.y, k.c.y);
+      return (double)k.s.x - (double)k.c.x;
+    };
+    const double axd = o.gb[0] + value(ax), ayd = o.gb[1] + value(ay), azd = o.gb[2];
+    const double drd = value(dr) * P.X4[i].w;
+    v.S.A4[i] = make_double4_32a(axd, ayd, azd, drd);
+    v.S.zwab[i] = zw.x + zw.y;
+    if (o.any_shepard) v.S.sumden[i] = sd.x + sd.y;
+    const float t02 = s02.x + s02.y, t12 = s12.x + s12.y;
+    store_rates32(v, i, 2.f * (s00.x + s00.y), s01.x + s01.y, t02, 2.f * (s11.x + s11.y), t12, 0.f, r01.x + r01.y,
+                  -t02, -t12);
+    const float fin = (ax.s.x - ax.s.x) + (ax.c.x - ax.c.x) + (ay.s.x - ay.s.x) + (ay.c.x - ay.c.x) +
+                      (dr.s.x - dr.s.x) + (dr.c.x - dr.c.x);
+    if (!(fin == 0.f)) atomicOr(&v.sc->status, ST_NONFINITE);
+    // this particle's time-step bound sqrt_h_a sqrt(h/|a|) in FP32; the
+    // minimum over particles and AdaptiveTimeStep stay FP64
+    const float ax32 = d2f_rn(axd), ay32 = d2f_rn(ayd), az32 = d2f_rn(azd);
+    const float an = sqrtf(ax32 * ax32 + ay32 * ay32 + az32 * az32);
+    const float cand = (float)o.sqrt_h_a * sqrtf(h / an);
+    if (cand < dtc) dtc = cand;
+  }
+  block_dt32_and_pairs(v, Ci.inst, active, dtc, (unsigned long long)npair2, cred);
 }
 
 inline int nblk32(int n) { return n <= 0 ? 1 : (n + kFT32 - 1) / kFT32; }
@@ -1257,6 +1467,14 @@ template <int DIM>
 void forces32_dispatch(const DevView& v, cudaStream_t st) {
   const int bt = (v.o.pair_block >= 32 && v.o.pair_block <= kMaxPairBlock) ? v.o.pair_block : kFT32;
   const int nb = v.ncap <= 0 ? 1 : (v.ncap + bt - 1) / bt;
+  if (DIM == 2 && v.o.soil32) {
+    switch (v.o.kt) {
+      case 0: forces_soil32_kernel<0><<<nb, bt, 0, st>>>(v); break;
+      case 1: forces_soil32_kernel<1><<<nb, bt, 0, st>>>(v); break;
+      default: forces_soil32_kernel<2><<<nb, bt, 0, st>>>(v); break;
+    }
+    return;
+  }
   if (v.o.has_solid) {
     switch (v.o.kt) {
       case 0: forces_solid32_kernel<DIM, 0><<<nb, bt, 0, st>>>(v); break;
@@ -1306,7 +1524,17 @@ __global__ void expand_sr32_kernel(const float* __restrict__ sr32, double* __res
 }
 }  // namespace
 
+namespace {
+__global__ void expand_rates32_kernel(const float4* __restrict__ r, double* __restrict__ sr, double* __restrict__ rr,
+                                      int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) widen_rates(r + 3 * (size_t)i, sr + 9 * (size_t)i, rr + 9 * (size_t)i);
+}
+}  // namespace
+
 void launch_expand_sr32(const DevView& v, int n, cudaStream_t st) {
+  if (n > 0 && v.S.rates32)
+    expand_rates32_kernel<<<(n + 255) / 256, 256, 0, st>>>(v.S.rates32, v.S.strain_rate, v.S.rotation_rate, n);
   if (n > 0 && v.S.sr32 && v.S.strain_rate)
     expand_sr32_kernel<<<(n + 255) / 256, 256, 0, st>>>(v.S.sr32, v.S.strain_rate, n);
 }

@@ -103,9 +103,9 @@ __global__ void out_gather_kernel(DevView v, int lo, int hi, const int* __restri
   f[unit(10) * N + r] = (float)C.h;
   float* sg = f + unit(11) * N + 6 * r;
   float* sn = f + unit(12) * N + 6 * r;
-  if (P.sigma) sym6(sg, P.sigma + 9 * (size_t)s);
+  if (P.sigma) sym6(sg, P.sigma + tensor_row(P, s));
   else for (int k = 0; k < 6; ++k) sg[k] = 0.f;
-  if (P.strain) sym6(sn, P.strain + 9 * (size_t)s);
+  if (P.strain) sym6(sn, P.strain + tensor_row(P, s));
   else for (int k = 0; k < 6; ++k) sn[k] = 0.f;
 }
 

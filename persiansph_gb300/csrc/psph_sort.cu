@@ -23,6 +23,7 @@
 //            scan handles one per lane, and the new counts and buffer.
 // Six launches (eleven with separate clearing, scan of totals, ranking and
 // finish kernels): 57 -> 44 us for 86k particles, where launches are what counts.
+#include <algorithm>
 #include <cstdio>
 
 #include "psph_device.cuh"
@@ -181,9 +182,8 @@ __global__ void scatter_kernel(const int* __restrict__ key, const int* __restric
 
 // One thread per scattered particle i: its place s is its segment's start plus
 // the number of the segment's particles with a smaller original index; then its
-// fields move there. perm[s] = i serves the solids' tensors.
-__global__ void reorder_kernel(DevView v, const int* __restrict__ tmp_perm, int* __restrict__ perm,
-                               const int* __restrict__ key, const int* __restrict__ start, int* __restrict__ cellid,
+// fields move there (a solid's 3x3 tensors stay where they are: tensor_row).
+__global__ void reorder_kernel(DevView v, const int* __restrict__ tmp_perm, const int* __restrict__ key, const int* __restrict__ start, int* __restrict__ cellid,
                                uint8_t* __restrict__ alive, const StepScalars* sc, int nbins, int xsub, int dyn_mu) {
   if (sc->all_stop || !sc->rebuild) return;
   const Persist& src = cur_persist(v);
@@ -196,7 +196,6 @@ __global__ void reorder_kernel(DevView v, const int* __restrict__ tmp_perm, int*
     const int mine = src.orig[i];
     int s = lo;
     for (int t = lo; t < hi; ++t) s += src.orig[tmp_perm[t]] < mine;
-    perm[s] = i;
     dst.X4[s] = src.X4[i];
     dst.V4[s] = src.V4[i];
     dst.H4[s] = src.H4[i];
@@ -225,40 +224,6 @@ __global__ void reorder_kernel(DevView v, const int* __restrict__ tmp_perm, int*
     cellid[s] = (k < nbins) ? k / (2 * xsub) : -1;
     alive[s] = 1;
     if (dyn_mu) dst.mu[s] = src.mu[i];
-  }
-}
-
-// The 3x3 tensors of solids (9 doubles a row) in the new order, a warp per 32
-// rows: lane l moves words l, l+32, ... of the warp's 288, so the stores are
-// contiguous and the loads too wherever the permutation keeps neighbours
-// together (it mostly does: particles move little between steps).
-__global__ void reorder_tensors_kernel(DevView v, const int* __restrict__ perm, const int* __restrict__ start,
-                                       const StepScalars* sc, int nbins) {
-  if (sc->all_stop || !sc->rebuild) return;
-  const Persist& src = cur_persist(v);
-  const Persist& dst = next_persist(v);
-  const int n_new = start[nbins + 1];
-  const int lane = threadIdx.x & 31;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const double* srcs[7] = {src.sigma, src.sigma_h, src.strain, src.strain_h, src.shear, src.tir, src.shear_h};
-  double* dsts[7] = {dst.sigma, dst.sigma_h, dst.strain, dst.strain_h, dst.shear, dst.tir, dst.shear_h};
-  // the ShearStress history serves Mat2 only (a zero history of a soil domain stays behind)
-  const int nt = v.o.carry_shear_h ? 7 : 6;
-  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; 32 * w < n_new; w += nwarps) {
-    const int base = 32 * w;
-    const int rows = min(32, n_new - base);
-    const int mine = lane < rows ? perm[base + lane] : 0;  // the source row of this lane's destination row
-    for (int a = 0; a < nt; ++a) {
-      const double* __restrict__ sa = srcs[a];
-      double* __restrict__ da = dsts[a] + 9 * (size_t)base;
-#pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        const int word = lane + 32 * k;       // of the warp's 288
-        const int r = word / 9, e = word - 9 * r;
-        const int from = __shfl_sync(0xffffffffu, mine, r & 31);
-        if (r < rows) da[word] = sa[9 * (size_t)from + e];
-      }
-    }
   }
 }
 
@@ -367,17 +332,17 @@ void launch_sort(const DevView& v, cudaStream_t st) {
   const int xsub = v.o.xsub;
   const int nbins = 2 * ncells * xsub;
   const int len = nbins + 2;
-  const int gp = grid_for(v.ncap);
-  // S.count is zero here (allocated so, and cleared behind every scan); S.perm
-  // holds the slots until the reorder writes the permutation
-  bin_kernel<<<gp, kBT, 0, st>>>(v, v.alive, S.key, S.count, S.perm, v.sc, v.o.dim, xsub);
+  // with a skin most steps skip the sort: few enough blocks that skipping is cheap
+  // (6.7M particles: 67 us a step for the skipped launches, 25 so)
+  const int gp = v.o.skin > 0.f ? std::min(grid_for(v.ncap), 4096) : grid_for(v.ncap);
+  // S.count is zero here (allocated so, and cleared behind every scan)
+  bin_kernel<<<gp, kBT, 0, st>>>(v, v.alive, S.key, S.count, S.slot, v.sc, v.o.dim, xsub);
   const int nb = scan_blocks_for(len);
   scan_blocks<<<nb, 1024, 0, st>>>(S.count, S.sstart, S.block_sums, len, v.sc);
   scan_add<<<nb, 1024, 0, st>>>(S.sstart, S.block_sums, len, S.count, v.sc);
-  scatter_kernel<<<gp, kBT, 0, st>>>(S.key, S.sstart, S.perm, S.tmp_perm, v.sc);
-  reorder_kernel<<<gp, kBT, 0, st>>>(v, S.tmp_perm, S.perm, S.key, S.sstart, S.cellid, v.alive, v.sc, nbins, xsub,
+  scatter_kernel<<<gp, kBT, 0, st>>>(S.key, S.sstart, S.slot, S.tmp_perm, v.sc);
+  reorder_kernel<<<gp, kBT, 0, st>>>(v, S.tmp_perm, S.key, S.sstart, S.cellid, v.alive, v.sc, nbins, xsub,
                                      v.o.dyn_mu);
-  if (v.o.has_solid) reorder_tensors_kernel<<<gp, kBT, 0, st>>>(v, S.perm, S.sstart, v.sc, nbins);
   cell_starts_kernel<<<grid_for(ncells + 3), kBT, 0, st>>>(S.sstart, S.start, ncells, xsub, v.sc, S.tmp_perm, v.ncap);
 }
 

@@ -393,13 +393,22 @@ __global__ void __launch_bounds__(kUT) update_kernel(DevView v) {
       }
     }
   } else {
-    const double* SR = v.S.strain_rate + 9 * (size_t)s;
-    const double* RR = v.S.rotation_rate + 9 * (size_t)s;
-    double* Sig = P.sigma + 9 * (size_t)s;
-    double* Sh = P.sigma_h + 9 * (size_t)s;
+    const size_t home = tensor_row(P, s);
+    double SR[9], RR[9];
+    if (v.S.rates32) {  // FP32C: the pair kernel's FP32 sums
+      widen_rates(v.S.rates32 + 3 * (size_t)s, SR, RR);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 9; ++e) {
+        SR[e] = v.S.strain_rate[9 * (size_t)s + e];
+        RR[e] = v.S.rotation_rate[9 * (size_t)s + e];
+      }
+    }
+    double* Sig = P.sigma + home;
+    double* Sh = P.sigma_h + home;
     double* So = v.S.sigma_o + 9 * (size_t)s;
-    double* E = P.strain + 9 * (size_t)s;
-    double* Eh = P.strain_h + 9 * (size_t)s;
+    double* E = P.strain + home;
+    double* Eh = P.strain_h + home;
     double* Eo = v.S.strain_o + 9 * (size_t)s;
     const double I22 = (DIM == 2) ? 0.0 : 1.0;
     const bool lf = (o.scheme != PSPH_MVERLET);
@@ -407,8 +416,8 @@ __global__ void __launch_bounds__(kUT) update_kernel(DevView v) {
     if (mat == 2) {
       // Mat2Leapfrog / Mat2MVerlet (Source/Particle.cpp:598-639 / :276-318)
       p = eos(C.pres_eq, C.cs, C.p0, rho, C.rho0);
-      double* SS = P.shear + 9 * (size_t)s;
-      double* SSh = P.shear_h + 9 * (size_t)s;
+      double* SS = P.shear + home;
+      double* SSh = P.shear_h + home;
       double* SSo = v.S.shear_o + 9 * (size_t)s;
       double X9[9];
       mat2_rate(SR, RR, SS, C.g_mod, X9);
@@ -438,7 +447,7 @@ __global__ void __launch_bounds__(kUT) update_kernel(DevView v) {
         for (int e = 0; e < 9; ++e) SS[e] = (SSh[e] + SSo[e]) * (1.0 / 2.0);
       for (int e = 0; e < 9; ++e) Sig[e] = OIe(e) * -p + SS[e];
     } else {
-      double* SS = P.shear ? P.shear + 9 * (size_t)s : nullptr;
+      double* SS = P.shear ? P.shear + home : nullptr;
       plane = (DIM == 2) && plane_zeros(SR, RR, Sig, Sh, E, Eh);
       if (plane) mat3_update<true>(C, I22, lf, first, ct, dt, SR, RR, Sig, Sh, So, SS);
       else mat3_update<false>(C, I22, lf, first, ct, dt, SR, RR, Sig, Sh, So, SS);
@@ -488,7 +497,7 @@ void launch_update(const DevView& v, cudaStream_t st) {
   else update_kernel<3><<<nb > 0 ? nb : 1, kUT, 0, st>>>(v);
 }
 
-// begin, bin, 2 scan, scatter, reorder (+ the solids' tensors), cell starts, neighbour lists, prepare (2 in the FP32C form: copies + walls),
+// begin, bin, 2 scan, scatter, reorder, cell starts, neighbour lists, prepare (2 in the FP32C form: copies + walls),
 // forces, closure, dt, update, end
 namespace {
 __global__ void class_constants_kernel(PClass* cls, int n, int dim) {
@@ -536,7 +545,7 @@ void launch_upload_pack(const double* sx, const double* sd, const double* sp, co
 }
 
 int launches_per_step(const DevView& v) {
-  return (v.o.fp32 ? 14 : 13) + (v.o.closure ? 1 : 0) + (v.o.has_solid ? 1 : 0) + (v.o.fp64_half ? 1 : 0) +
+  return (v.o.fp32 ? 14 : 13) + (v.o.closure ? 1 : 0) + (v.o.fp64_half ? 1 : 0) +
          (v.o.mixed ? 2 : 0) + (v.o.couple_soil && v.o.swi != 2 ? 2 : 0) + (v.o.fsi ? 1 : 0) +
          (v.o.skin > 0.f ? 1 : 0);
 }

@@ -114,3 +114,39 @@ def test_fluid_fp32c(gpu, dim, kernel, hfac, beta, fpmassc, slip, les):
         s = np.abs(ref["strain_rate"][free]).max()
         assert np.max(np.abs(got["strain_rate"] - ref["strain_rate"])[free]) <= 1e-5 * s
     gd.close()
+
+
+@pytest.mark.parametrize("kernel", [0, 1, 2])
+@pytest.mark.parametrize("hfac,ti,alpha,fpmassc,slip", [
+    (1.2, 0.5, 0.1, 1.0, False), (3.2, 0.5, 0.1, 0.9, False), (1.2, 0.0, 0.0, 1.0, True)])
+def test_soil_fp32c(gpu, kernel, hfac, ti, alpha, fpmassc, slip):
+    dx = 0.013
+    dom, dt, info = scenarios.granular_column(dx=dx, aspect=0.8, cohesion=1.0e3, hfac=hfac, ti=ti, alpha=alpha)
+    dom.Kernel_Set(kernel)
+    p = dom.particles
+    p.set("fpmassc", fpmassc)
+    if slip:
+        p.set("no_slip", 0)
+    stir(p, dx, 8, 2, 0.5)
+    rng = np.random.default_rng(9)
+    free = np.flatnonzero(p.get("is_free") != 0)
+    s = p.get("sigma")
+    for r, c in ((0, 0), (1, 1)):
+        s[free, r, c] += rng.uniform(-400.0, 400.0, len(free))
+    p.set("sigma", s)
+    o = OracleDomain(dom.config(dt), p, initial=True)
+    o.step(1)
+    a_scale, dr_scale = o.scales()
+    ref = o.download()
+    cfg = dom.config(dt)
+    cfg.precision = 1
+    gd = GpuDomain(cfg)
+    gd.upload(p)
+    gd.step(1)
+    got = gd.download_fields()
+    f = ref["is_free"] == 1
+    assert np.max(np.linalg.norm(got["a"] - ref["a"], axis=1)[f] / a_scale[f]) <= 1e-5
+    assert np.max(np.abs(got["ddensity"] - ref["ddensity"])[f] / (dr_scale[f] + 1e-300)) <= 1e-5
+    for k in ("strain_rate", "rotation_rate", "sigma", "strain"):
+        assert np.max(np.abs(got[k] - ref[k])[f]) <= 1e-5 * np.abs(ref[k][f]).max(), k
+    gd.close()
