@@ -897,7 +897,14 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
         return set_err(c, PSPH_ERR_UNSUPPORTED, "periodic axis %d spans fewer than 3 cells", d);
     }
     gd.hmax = g.hmax;
-    for (int d = 0; d < 3; ++d) gd.inv_cell_size32[d] = (float)(1.0 / g.cell_size[d]);
+    for (int d = 0; d < 3; ++d) {
+      gd.inv_cell_size32[d] = (float)(1.0 / g.cell_size[d]);
+      gd.blpf32[d] = (float)g.blpf[d];
+      // a coordinate truncated to FP32 moves by less than 2^-22 of its magnitude
+      const double m = 1e-6 * std::max(std::fabs(g.blpf[d]), std::fabs(g.trpr[d])) + 1e-37;
+      gd.in_lo32[d] = (float)(g.blpf[d] + m);
+      gd.in_hi32[d] = (float)(g.trpr[d] - m);
+    }
     for (int d = 0; d < 3; ++d) gd.cell_size32[d] = (float)g.cell_size[d];
     gd.cellfac = (cf.kernel_type == PSPH_QUINTIC_SPLINE) ? 3.0 : 2.0;
     gd.cellfac2_32 = (float)(gd.cellfac * gd.cellfac);
@@ -1498,7 +1505,7 @@ __global__ void offsets32_kernel(DevView v) {
   const Persist& P = cur_persist(v);
   const double4_32a xs = P.X4[s];
   const PClass& C = v.cls[P.cls[s]];
-  const float h = (float)C.h;
+  const float h = C.is_free ? (float)C.h : -(float)C.h;
   const int cell = v.S.cellid[s];
   if (cell >= 0) {
     const GridDev& g = grid_of(v, C.inst);

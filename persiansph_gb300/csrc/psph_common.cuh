@@ -87,6 +87,7 @@ PSPH_HD void permeability(int type, double n, double d, double* k, double* k2) {
 // instance for a single Domain, or many independent instances for an ensemble.
 struct InstState {
   double time, deltat, deltatint, deltatmin, t_stop;
+  double dt2, half_dt2;  // 2 dt and dt^2 / 2 of the step (set with deltat)
   long long steps;
   unsigned long long dtmin_bits;  // running minimum of the acceleration time-step bound (ordered bits)
   int first_step, ct, shepard_counter, stop;
@@ -161,13 +162,28 @@ __host__ __device__ inline float psph_fbits(unsigned u) {
 #endif
 }
 
+// The conversion instructions, out of line: inlined they are predicated, and a
+// predicated-off instruction takes its FP64 issue slot all the same.
+__host__ __device__
+#ifdef __CUDACC__
+__noinline__
+#endif
+inline float2 d2f_split_slow(double x) {
+  const float h = (float)x;
+  return make_float2(h, (float)(x - (double)h));
+}
+
 __host__ __device__ inline float d2f_split(double x, float* lo) {
   const unsigned long long b = psph_dbits(x);
   const unsigned E = (unsigned)(b >> 52) & 0x7ffu;
+  if ((b << 1) == 0ull) {  // zero, either sign (walls at rest): no conversion instruction
+    if (lo) *lo = 0.f;
+    return psph_fbits((unsigned)(b >> 32));
+  }
   if (E < 949u || E > 1149u) {
-    const float h = (float)x;
-    if (lo) *lo = (float)(x - (double)h);
-    return h;
+    const float2 r = d2f_split_slow(x);
+    if (lo) *lo = r.y;
+    return r.x;
   }
   const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
   const unsigned long long m = b & 0xfffffffffffffull;
@@ -178,7 +194,10 @@ __host__ __device__ inline float d2f_split(double x, float* lo) {
     const float scale = psph_fbits((E - 948u) << 23);  // 2^(E-1075)
     int q = (int)(up ? rem - 0x20000000u : rem);
     if (sign) q = -q;
-    *lo = (float)q * scale;  // +0 when exact, as x - (double)hi gives
+    // q (30 bits) as 2^15 qh + ql, each exactly a float by its bits: one rounding
+    const float qh = psph_fbits(0x4b400000u + (unsigned)(q >> 15)) - 12582912.f;
+    const float ql = psph_fbits(0x4b000000u | ((unsigned)q & 0x7fffu)) - 8388608.f;
+    *lo = fmaf(qh, 32768.f, ql) * scale;  // +0 when exact, as x - (double)hi gives
   }
   return psph_fbits(hb);
 }
@@ -189,19 +208,25 @@ __host__ __device__ inline float d2f_rn(double x) { return d2f_split(x, nullptr)
 // estimate: with the estimate's relative residual e, the series of 1/(1-e) and
 // 1/sqrt(1-e) to e^2 leave |e|^3 < 2^-57. Within 1 ulp; 3 to 5 FP64 instructions
 // on a part with 2 FP64 lanes per SM. sqrt(0) = 0, and 1/sqrt(0) is returned as
-// 0 (a pair of coincident particles); NaN stays NaN.
+// 0 (a pair of coincident particles).
 PSPH_D double rcp_newton(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-x, y, 1.0);
   return fma(y, fma(e, e, e), y);
 }
+// rcp_newton with one Newton step more: correctly rounded but for a few in 2^50
+PSPH_D double rcp_refined(double x) {
+  const double y = rcp_newton(x);
+  return fma(fma(-x, y, 1.0), y, y);
+}
+// (below 2^-1006, where the estimate flushes to zero, a separation is none: 0)
 PSPH_D double rsqrt_newton(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-x * y, y, 1.0);
   const double r = fma(y * e, fma(e, 0.375, 0.5), y);
-  return __double_as_longlong(x) == 0ll ? 0.0 : r;
+  return __double2hiint(x) < 0x01100000 ? 0.0 : r;
 }
 PSPH_D double sqrt_newton(double x) {
   double y;
@@ -209,14 +234,32 @@ PSPH_D double sqrt_newton(double x) {
   const double t = x * y;
   const double e = fma(-t, y, 1.0);
   const double r = fma(t * e, fma(e, 0.375, 0.5), t);
-  return __double_as_longlong(x) == 0ll ? 0.0 : r;
+  return __double2hiint(x) < 0x01100000 ? 0.0 : r;
 }
+// sqrt_newton for any argument (tiny, negative): the library's function there
+__device__ __noinline__ inline double sqrt_small(double x) { return sqrt(x); }
+PSPH_D double sqrt_any(double x) { return __double2hiint(x) < 0x01100000 ? sqrt_small(x) : sqrt_newton(x); }
 
 // Signs and comparisons of doubles on the integer pipe (an FP64 comparison
 // takes an FP64 issue slot): x < 0 (true for -0.0 too), and a > b for
 // non-negative a and b (true for NaN a).
 PSPH_D bool negative(double x) { return __double2hiint(x) < 0; }
 PSPH_D bool above(double a, double b) { return __double_as_longlong(a) > __double_as_longlong(b); }
+
+// A non-negative integer and a float as doubles, exactly, on the integer pipe (the conversion instructions run on the FP64 pipe).
+PSPH_D double i2d_small(int c) {
+  const int e = 31 - __clz(c | 1);
+  const unsigned long long m = ((unsigned long long)(unsigned)c << (52 - e)) & 0xfffffffffffffull;
+  const double r = __longlong_as_double((long long)(((unsigned long long)(1023 + e) << 52) | m));
+  return c == 0 ? 0.0 : r;
+}
+__device__ __noinline__ inline double f2d_slow(float f) { return (double)f; }
+PSPH_D double f2d_bits(float f) {
+  const unsigned u = __float_as_uint(f), e = (u >> 23) & 0xffu, s = u & 0x80000000u;
+  if ((u << 1) == 0u) return __hiloint2double((int)s, 0);
+  if (e == 0u || e == 255u) return f2d_slow(f);  // denormals, infinities, NaN
+  return __hiloint2double((int)(s | ((e + 896u) << 20) | ((u >> 3) & 0xfffffu)), (int)(u << 29));
+}
 
 struct GridDev {
   double blpf[3], trpr[3], cell_size[3], dom_size[3];
@@ -229,6 +272,8 @@ struct GridDev {
   float inv_cell_size32[3];  // 1 / cell_size in FP32 (cell-index estimate of the sort)
   float cell_size32[3];      // cell_size rounded to FP32 (on the host)
   float cellfac2_32;         // Cellfac^2 in FP32
+  float blpf32[3];           // blpf rounded to FP32
+  float in_lo32[3], in_hi32[3];  // strictly inside (blpf, trpr) whatever FP32 truncation does to a coordinate
   float skin_disp2;          // with a skin: (half the skin)^2, the displacement that forces a rebuild
 };
 
@@ -362,6 +407,22 @@ PSPH_HD double density_solid(int eq, double cs, double p0, double p, double rho0
 // ---------------------------------------------------------------------------
 // Cell indexing
 // ---------------------------------------------------------------------------
+// ListGenerate's floor((x - BLPF) / CellSize) (Source/Domain.cpp:669-691) along
+// axis d. An FP32 estimate (the coordinate truncated on the integer pipe) decides
+// it unless the quotient lies within the estimate's error of an integer; only
+// then the FP64 subtraction and division run (a division costs tens of
+// operations on the FP64 pipe).
+__device__ __noinline__ inline int cell_floor_exact(double x, double blpf, double size) {
+  return (int)floor((x - blpf) / size);
+}
+PSPH_D int cell_floor(const GridDev& g, int d, double x) {
+  const float xf = d2f_bits(x), inv = g.inv_cell_size32[d], b = g.blpf32[d];
+  const float t = (xf - b) * inv;
+  const float ft = floorf(t), fr = t - ft;
+  const float tol = 1e-6f + 4e-7f * (fabsf(t) + (fabsf(xf) + fabsf(b)) * inv);
+  if (fr >= tol && fr <= 1.f - tol) return (int)ft;
+  return cell_floor_exact(x, g.blpf[d], g.cell_size[d]);
+}
 PSPH_HD int cell_linear(const GridDev& g, int cx, int cy, int cz) { return (cz * g.nc[1] + cy) * g.nc[0] + cx; }
 
 }  // namespace psph

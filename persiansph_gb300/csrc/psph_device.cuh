@@ -39,7 +39,7 @@ struct Scratch {
   int* cellid;     // cell of each sorted particle (orphan/dead: -1)
   int* block_sums;
   // per-step derived / outputs
-  float4* OFF32;     // (position - cell origin, h) in FP32, written by the reorder
+  float4* OFF32;     // (position - cell origin, +-h) in FP32, negative for a fixed particle, written by the reorder
   float4* OFFREF;    // with a skin: the position at the last rebuild in FP32 (displacements are measured from it)
   int* refcell;      // with a skin: each particle's cell in the reference's grid (x | y << 10 | z << 20),
                      // for the wall pressure's pair orientation

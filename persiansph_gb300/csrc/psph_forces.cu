@@ -167,6 +167,25 @@ PSPH_D int tir_bit(const DevView& v, const Persist& P, int w) {
   return (b << 1) ? kInfoTir : 0;
 }
 
+// The FP32C 2D soil pair kernel's three records of particle w (forces_soil32_kernel),
+// and a wall's no-slip or history velocity.
+PSPH_D void soil_records(const DevView& v, const Persist& P, int w, bool fixed, const double4_32a& vel, double inv,
+                         const double* sg) {
+  const double* t = P.tir + tensor_row(P, w);
+  const bool tens = v.o.any_ti && ((__double_as_longlong(t[0]) | __double_as_longlong(t[1]) |
+                                    __double_as_longlong(t[4])) << 1) != 0ll;
+  const float4 x = v.S.OFF32[w];
+  const float i32 = d2f_rn(inv);
+  float lx, ly;
+  // the velocity's low-order part: near-rigid motion (a column settling as one
+  // body) makes v_i - v_j far smaller than v
+  const float vx = d2f_split(vel.x, &lx), vy = d2f_split(vel.y, &ly);
+  v.S.PX32[w] = make_float4(x.x, x.y, d2f_rn(sg[0]), d2f_rn(sg[1]));
+  v.S.V32[w] = make_float4(vx, vy, d2f_rn(sg[4]), fixed ? -i32 : i32);
+  v.S.V32LO[w] = make_float4(lx, ly, d2f_rn(vel.z), tens ? 1.f : 0.f);
+  if (tens) v.S.TIR32[2 * (size_t)w] = make_float4(d2f_rn(t[0]), d2f_rn(t[1]), 0.f, d2f_rn(t[4]));
+}
+
 // ---------------------------------------------------------------------------
 // Per-particle preparation and wall interpolation
 // ---------------------------------------------------------------------------
@@ -321,8 +340,15 @@ PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int f
     rw = density_solid(Ce.pres_eq, Ce.cs, Ce.p0, p, Ce.rho0);
     cwv = sound_speed(Ce.pres_eq, Ce.cs, rw, Ce.rho0);
   }
-  const double inv = 1.0 / rw;
-  v.S.D4[w] = make_double4_32a(inv, p * inv * inv, cwv, rw);
+  const double inv = rcp_refined(rw);
+  if (DIM == 2 && o.soil32) {
+    soil_records(v, P, w, true, vw, inv, sig);
+    const double4_32a vb = (o.scheme == PSPH_MVERLET) ? P.H4[w] : P.H4b[w];
+    v.S.VB32[w] = make_float4(d2f_rn(vb.x), d2f_rn(vb.y), d2f_rn(vb.z), 0.f);
+    v.S.NSV32[w] = make_float4(d2f_rn(n0), d2f_rn(n1), d2f_rn(n2), 0.f);
+  } else {
+    v.S.D4[w] = make_double4_32a(inv, p * inv * inv, cwv, rw);
+  }
 }
 
 template <int DIM, int KT>
@@ -345,11 +371,12 @@ __global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v, int lg, in
     wall_q = !C.is_free;
     if (C.is_free) {
       const double rho = P.X4[q].w;
-      const double inv = 1.0 / rho;
-      const double pr = P.V4[q].w;
-      v.S.D4[q] = make_double4_32a(inv, pr * inv * inv, sound_speed(C.pres_eq, C.cs, rho, C.rho0), rho);
+      const double inv = rcp_refined(rho);
+      const double4_32a vel = P.V4[q];
       if (o.has_solid && C.material > 1 && C.ti > 0.0)
         tensile_tir<DIM>(P.sigma + tensor_row(P, q), C.ti, rho, P.tir + tensor_row(P, q));
+      if (DIM == 2 && o.soil32) soil_records(v, P, q, false, vel, inv, P.sigma + tensor_row(P, q));
+      else v.S.D4[q] = make_double4_32a(inv, vel.w * inv * inv, sound_speed(C.pres_eq, C.cs, rho, C.rho0), rho);
     }
     // (the FP32C pair kernels have copies of their own)
     if (v.S.pair_info)
@@ -1166,6 +1193,8 @@ __global__ void dt_finalize_kernel(DevView v) {
     if (dti > dtmin) dt = (dt < dtmin) ? 2.0 * dt * dtmin / (dt + dtmin) : dtmin;
     else dt = (dti != dt) ? 2.0 * dt * dti / (dt + dti) : dti;
     I.deltat = dt;
+    I.dt2 = 2.0 * dt;
+    I.half_dt2 = 0.5 * dt * dt;
     if (dt < (dti / 1.0e5)) {
       atomicOr(&sc->status, ST_DT_COLLAPSE);
       I.stop = 1;  // the reference throws here (Source/Domain.cpp:150-151)

@@ -57,6 +57,12 @@ PSPH_D float4 ld_early_coherent(const float4* p) {
   return r;
 }
 
+PSPH_D float ld_early_coherent(const float* p) {
+  float r;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(p));
+  return r;
+}
+
 template <int DIM, int KT>
 struct KernF {
   static constexpr float cw() { return (float)Kern<DIM, KT>::cw(); }
@@ -187,14 +193,13 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
   const int winst = (w < n) ? CT[P.cls[w]].inst : 0;
   const GridDev& g = grid_of(v, winst);
   bool wall = false, noslip = false;
-  int cell = -1, ow = 0, mat = 0;
+  int cell = -1, ow = 0;
   float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
   if (w < n && !v.inst[winst].stop) {
     const PClass32& C = CT[P.cls[w]];
     if (!(C.flags & CF_FREE)) {
       wall = true;
       noslip = C.flags & CF_NOSLIP;
-      mat = C.material;
       ow = P.orig[w];
       cell = v.S.cellid[w];
       oi = v.S.OFF32[w];
@@ -206,17 +211,10 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
   const bool skin = o.skin > 0.f;
   const int rc_w = (skin && need_orient && wall) ? v.S.refcell[w] : 0;
   float sk = 0.f, p = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
-  const float hw = oi.w;
-  // one fluid neighbour of the same material: its position, velocity and
-  // density loads go out together (this kernel writes the walls' own V32 /
-  // D32, which the class test then rejects, so those two take the coherent path)
-  auto visit = [&](const int f, const int code) {
-    const int clsf = ld_early(P.cls + f);
-    const float4 of = v.S.OFF32[f];
-    const float4 vf = ld_early_coherent(v.S.V32 + f);
-    const float4 df = ld_early_coherent(v.S.D32 + f);
-    const PClass32& Cf = CT[clsf];
-    if (!(Cf.flags & CF_FREE) || Cf.material != mat) return;
+  const float hw = fabsf(oi.w);
+  // One neighbour, loaded: free particles contribute (OFF32.w is negative for a
+  // fixed one; an FP32C domain has one material).
+  auto visit = [&](const int f, const int code, const float4 of, const float4 vf, const float rho) {
     float x0, x1, x2;
     rel_pos<DIM>(cs, oi, of, code, x0, x1, x2);  // x_wall - x_fluid
     if (need_orient) {
@@ -233,21 +231,33 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
     const float K = KernF<DIM, KT>::W(q, KernF<DIM, KT>::cw() * (DIM == 2 ? ih * ih : ih * ih * ih));
     if (K == 0.f) return;
     sk += K;
-    p += vf.w * K + (gx * x0 + gy * x1 + gz * x2) * df.w * K;
+    p += vf.w * K + (gx * x0 + gy * x1 + gz * x2) * rho * K;
     if (noslip) { n0 += vf.x * K; n1 += vf.y * K; n2 += vf.z * K; }
   };
   const int cnt = (wall && cell >= 0) ? v.S.nl_count[w] : 0;
-  if (cnt >= 0) {  // the neighbour list, 4 entries per 16-byte load
+  if (cnt >= 0) {
+    // the neighbour list, 4 entries per 16-byte load, whose 12 loads go out
+    // together (this kernel writes the walls' own V32 / D32, which the test then
+    // rejects, so those two take the coherent path)
     const int4* __restrict__ nl4 = reinterpret_cast<const int4*>(v.S.nl) + nl_slot(w);
     const size_t N = (size_t)v.nl_stride;
     const int nch = (cnt + 3) >> 2;
     for (int c = 0; c < nch; ++c) {
       const int4 q = nl4[(size_t)c * N];
       const int rem = cnt - 4 * c;
-      visit(q.x & kIndexMask, entry_code(q.x));
-      if (rem > 1) visit(q.y & kIndexMask, entry_code(q.y));
-      if (rem > 2) visit(q.z & kIndexMask, entry_code(q.z));
-      if (rem > 3) visit(q.w & kIndexMask, entry_code(q.w));
+      const int e[4] = {q.x, rem > 1 ? q.y : q.x, rem > 2 ? q.z : q.x, rem > 3 ? q.w : q.x};
+      float4 of[4], vf[4];
+      float rho[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const int f = e[t] & kIndexMask;
+        of[t] = ld_early(v.S.OFF32 + f);
+        vf[t] = ld_early_coherent(v.S.V32 + f);
+        rho[t] = ld_early_coherent(&v.S.D32[f].w);
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        if (t < rem && of[t].w > 0.f) visit(e[t] & kIndexMask, entry_code(e[t]), of[t], vf[t], rho[t]);
     }
   } else {  // list overflow: scan the cells
     NbrSource<DIM> src;
@@ -256,7 +266,8 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
       int code;
       const int f = src.next(v, &code);
       if (f < 0) break;
-      visit(f, code);
+      const float4 of = v.S.OFF32[f];
+      if (of.w > 0.f) visit(f, code, of, ld_early_coherent(v.S.V32 + f), ld_early_coherent(&v.S.D32[f].w));
     }
   }
   if (!wall) return;
@@ -272,9 +283,9 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
   v.S.sumkernel[w] = sk;
   v.S.nsv4[w] = make_double4_32a(n0, n1, n2, 0.0);
   v.S.NSV32[w] = make_float4(n0, n1, n2, 0.f);
-  v.S.V32[w] = make_float4((float)vw.x, (float)vw.y, (float)vw.z, p);
+  v.S.V32[w] = make_float4(d2f_rn(vw.x), d2f_rn(vw.y), d2f_rn(vw.z), p);
   const PClass32& Ce = CT[o.eos_cls];
-  float rw = (float)P.X4[w].w, cwv = 0.f;
+  float rw = d2f_rn(P.X4[w].w), cwv = 0.f;
   if (o.uniform_eos) {
     // DensitySolid / SoundSpeed of the fluid's EOS (Source/Functions.cpp:214-264), FP32
     const float cs2 = Ce.cs * Ce.cs, r0 = Ce.rho0, p0 = Ce.p0;
@@ -286,7 +297,10 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
   }
   const float inv = 1.f / rw;
   if (o.spec32) {
-    v.S.PX32[w] = make_float4(oi.x, oi.y, oi.z, -inv);
+    // a wall without a free particle in its support has none to meet, but may
+    // stand in a list (their margin): its terms are zeros times finite numbers
+    const bool odd = sk == 0.f && !(fabsf(inv) <= FLT_MAX);
+    v.S.PX32[w] = make_float4(oi.x, oi.y, oi.z, odd ? -1.f : -inv);
     v.S.V32LO[w].w = cwv;
   } else {
     v.S.D32[w] = make_float4(inv, p * inv * inv, cwv, rw);
@@ -333,7 +347,7 @@ __global__ void __maxnreg__(128) forces_fluid32_kernel(DevView v) {
   const float4 vil = v.S.V32LO[is];
   const float4 di4 = v.S.D32[is];
   const float di = di4.w, inv_i = di4.x, Pi = di4.y, ci_snd = di4.z, pi = vi.w;
-  const float mi = Ci.mass, hi = oi.w;
+  const float mi = Ci.mass, hi = fabsf(oi.w);
   const float mui = o.dyn_mu ? v.S.MU32[is] : Ci.mu0;
   const int fi = Ci.flags;
   const bool shep = (fi & CF_SHEPARD) && (Is.shepard_counter == o.shepard_step);
@@ -367,7 +381,7 @@ __global__ void __maxnreg__(128) forces_fluid32_kernel(DevView v) {
     const int clsj = wj & 0xffff;
     float x0, x1, x2;
     rel_pos<DIM>(cs, oi, oj, code, x0, x1, x2);
-    const float hb = 0.5f * (hi + oj.w);
+    const float hb = 0.5f * (hi + fabsf(oj.w));
     const float r2 = x0 * x0 + x1 * x1 + x2 * x2;
     // the list's own support test (exact in FP32; lists with a skin hold more)
     if (r2 > cf2 * hb * hb) return;
@@ -1018,23 +1032,11 @@ __global__ void __launch_bounds__(kFT32) solid_copies32_kernel(DevView v) {
   // (hi_i - hi_j) + (lo_i - lo_j), exact to ~2^-48 of |v|
   const double4_32a d = v.S.D4[w];
   const double* sg = P.sigma + tensor_row(P, w);
-  if (v.o.soil32) {  // the three records of forces_soil32_kernel
-    const double* t = P.tir + tensor_row(P, w);
-    const bool tens = v.o.any_ti && (t[0] != 0.0 || t[1] != 0.0 || t[4] != 0.0);
-    const float4 x = v.S.OFF32[w];
-    const bool fr = C.flags & CF_FREE;
-    const float inv = d2f_rn(d.x);
-    v.S.PX32[w] = make_float4(x.x, x.y, d2f_rn(sg[0]), d2f_rn(sg[1]));
-    v.S.V32[w] = make_float4(vx, vy, d2f_rn(sg[4]), fr ? inv : -inv);
-    v.S.V32LO[w] = make_float4(lx, ly, vz, tens ? 1.f : 0.f);
-    if (tens) v.S.TIR32[2 * (size_t)w] = make_float4(d2f_rn(t[0]), d2f_rn(t[1]), 0.f, d2f_rn(t[4]));
-  } else {
-    v.S.V32[w] = make_float4(vx, vy, vz, d2f_rn(vv.w));
-    v.S.V32LO[w] = make_float4(lx, ly, lz, 0.f);
-    v.S.D32[w] = make_float4(d2f_rn(d.x), d2f_rn(d.y), d2f_rn(d.z), d2f_rn(d.w));
-    sym_store(v.S.SIG32, (size_t)w, sg);
-    if (v.o.any_ti) sym_store(v.S.TIR32, (size_t)w, P.tir + tensor_row(P, w));
-  }
+  v.S.V32[w] = make_float4(vx, vy, vz, d2f_rn(vv.w));
+  v.S.V32LO[w] = make_float4(lx, ly, lz, 0.f);
+  v.S.D32[w] = make_float4(d2f_rn(d.x), d2f_rn(d.y), d2f_rn(d.z), d2f_rn(d.w));
+  sym_store(v.S.SIG32, (size_t)w, sg);
+  if (v.o.any_ti) sym_store(v.S.TIR32, (size_t)w, P.tir + tensor_row(P, w));
   if (!(C.flags & CF_FREE)) {
     const double4_32a vb = (v.o.scheme == PSPH_MVERLET) ? P.H4[w] : P.H4b[w];
     v.S.VB32[w] = make_float4(d2f_rn(vb.x), d2f_rn(vb.y), d2f_rn(vb.z), 0.f);
@@ -1088,7 +1090,7 @@ __global__ void __maxnreg__(128) forces_solid32_kernel(DevView v) {
   const float4 vil = v.S.V32LO[is];
   const float4 di4 = v.S.D32[is];
   const float di = di4.w, inv_i = di4.x, ci_snd = di4.z;
-  const float mi = Ci.mass, hi = oi.w;
+  const float mi = Ci.mass, hi = fabsf(oi.w);
   const bool shep = (Ci.flags & CF_SHEPARD) && (Is.shepard_counter == o.shepard_step);
   const float4 sa = v.S.SIG32[2 * (size_t)is], sb = v.S.SIG32[2 * (size_t)is + 1];
   const float Si[6] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y};
@@ -1116,7 +1118,7 @@ __global__ void __maxnreg__(128) forces_solid32_kernel(DevView v) {
     const float4 oj = v.S.OFF32[j];
     float x0, x1, x2;
     rel_pos<DIM>(cs, oi, oj, code, x0, x1, x2);
-    const float hb = 0.5f * (hi + oj.w);
+    const float hb = 0.5f * (hi + fabsf(oj.w));
     const float r2 = x0 * x0 + x1 * x1 + x2 * x2;
     if (r2 > cf2 * hb * hb) continue;  // the support test (the list holds a margin)
     const PClass32& Cj = CT[P.cls[j]];
@@ -1245,7 +1247,8 @@ __global__ void __maxnreg__(128) forces_solid32_kernel(DevView v) {
 // (Options::soil32: one h, artificial viscosity, sound speed, tensile-instability
 // constants and flags; one free mass per instance): the granular columns. As in
 // forces_spec32_kernel a lane takes two neighbours at a time in packed FP32x2
-// arithmetic, and a neighbour is three 16-byte records (solid_copies32_kernel):
+// arithmetic, and a neighbour is three 16-byte records
+// (written by prepare_wall_kernel)
 //   PX32  x, y, Sigma00, Sigma01      V32  vx, vy, Sigma11, +-1/density (- fixed)
 //   V32LO the low-order parts of vx and vy, vz, whether its TIR is non-zero
 // In 2D the entries with a z index meet a zero separation in the acceleration.
@@ -1503,6 +1506,7 @@ void forces32_dispatch(const DevView& v, cudaStream_t st) {
 void launch_prepare32(const DevView& v, cudaStream_t st) {
   if (v.o.has_solid) {  // FP64 wall stress interpolation and TIR, then the FP32 copies
     launch_prepare(v, st);
+    if (v.o.soil32) return;  // which wrote the pair kernel's records too
     const int nb = nblk32(v.ncap);
     if (v.o.dim == 2) solid_copies32_kernel<2><<<nb, kFT32, 0, st>>>(v);
     else solid_copies32_kernel<3><<<nb, kFT32, 0, st>>>(v);

@@ -98,7 +98,8 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
   const GridDev& g = grid_of(v, C.inst);
   const bool fixed = !C.is_free && !v.o.list_all;  // its list holds free particles only (it has no other pairs)
   const float3 cs = cell_size_f(g);
-  const float4 oi = v.S.OFF32[i];
+  float4 oi = v.S.OFF32[i];
+  oi.w = fabsf(oi.w);  // (its sign says whether the particle is fixed)
   const float cf = (float)g.cellfac;
   // support test r^2 <= (Cellfac hb)^2 margin; with one h everywhere it is a constant
   const float thr_u = cf * cf * oi.w * oi.w * margin;
@@ -154,7 +155,7 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
           const float x0 = ax - oj.x, x1 = ay - oj.y, x2 = (DIM == 3) ? az - oj.z : 0.f;
           float thr = thr_u;
           if (!UNIFORM_H) {
-            const float hb = 0.5f * (oi.w + oj.w);
+            const float hb = 0.5f * (oi.w + fabsf(oj.w));
             thr = cf * cf * hb * hb * margin;
           }
           return x0 * x0 + x1 * x1 + x2 * x2 <= thr;

@@ -227,6 +227,7 @@ struct NbrSource {
     if (on && cnt < 0) {
       cs.init(grid, v.S.cellid[i]);
       oi = v.S.OFF32[i];
+      oi.w = fabsf(oi.w);  // (its sign says whether the particle is fixed)
     } else {
       cs.init(grid, -1);
     }
@@ -248,7 +249,7 @@ struct NbrSource {
       const float4 oj = v.S.OFF32[j];
       float x0, x1, x2;
       rel_pos<DIM>(csz, oi, oj, *code, x0, x1, x2);
-      const float hb = 0.5f * (oi.w + oj.w);
+      const float hb = 0.5f * (oi.w + fabsf(oj.w));
       if (x0 * x0 + x1 * x1 + x2 * x2 <= cf * cf * hb * hb * margin) return j;
     }
   }

@@ -52,20 +52,9 @@ __global__ void bin_kernel(DevView v, const uint8_t* __restrict__ alive, int* __
       const double4_32a x = P.X4[i];
       const double xs[3] = {x.x, x.y, x.z};
       int c[3] = {0, 0, 0};
-      double a0 = 0.0;  // x - BLPF_x
       bool orphan = false, out = false;
       for (int d = 0; d < dim; ++d) {
-        // ListGenerate's floor((x - BLPF) / CellSize) (Source/Domain.cpp:669-691).
-        // An FP32 estimate (the difference converted on the integer pipe)
-        // decides it unless the quotient lies within the estimate's error of
-        // an integer; only then the FP64 division runs (a division costs tens
-        // of operations on the FP64 pipe).
-        const double a = xs[d] - g.blpf[d];
-        if (d == 0) a0 = a;
-        const float t = d2f_bits(a) * g.inv_cell_size32[d];
-        const float ft = floorf(t), fr = t - ft, tol = 1e-3f + 4e-7f * fabsf(t);
-        int cd = (int)ft;
-        if (!(fr >= tol && fr <= 1.f - tol)) cd = (int)floor(a / g.cell_size[d]);
+        int cd = cell_floor(g, d, xs[d]);  // ListGenerate's rule
         if (cd < 0) {
           if ((g.blpf[d] - xs[d]) <= g.hmax) cd = 0;
           else out = true;
@@ -85,7 +74,7 @@ __global__ void bin_kernel(DevView v, const uint8_t* __restrict__ alive, int* __
       } else {
         int slab = 0;
         if (xsub > 1) {  // x-slab inside the cell (clamped for particles outside it), in FP32
-          const float ox = d2f_bits(a0) - (float)c[0] * g.cell_size32[0];
+          const float ox = d2f_bits(x.x - g.blpf[0]) - (float)c[0] * g.cell_size32[0];
           slab = min(max((int)floorf(ox * (float)xsub * g.inv_cell_size32[0]), 0), xsub - 1);
         }
         k = 2 * ((g.cell_base + (c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0]) * xsub + slab) + (C.is_free ? 0 : 1);
@@ -205,14 +194,14 @@ __global__ void reorder_kernel(DevView v, const int* __restrict__ tmp_perm, cons
     {
       // FP32 offset from the cell origin (absolute position outside any cell)
       const double4_32a xs = src.X4[i];
-      const float h = d2f_rn(v.cls[cls].h);
+      const float h = v.cls[cls].is_free ? d2f_rn(v.cls[cls].h) : -d2f_rn(v.cls[cls].h);
       if (k < nbins) {
         const GridDev& g = grid_of(v, v.cls[cls].inst);
         const int lk = k / (2 * xsub) - g.cell_base;
         const int cx = lk % g.nc[0], t = lk / g.nc[0], cy = t % g.nc[1], cz = t / g.nc[1];
-        v.S.OFF32[s] = make_float4(d2f_rn(xs.x - (g.blpf[0] + cx * g.cell_size[0])),
-                                   d2f_rn(xs.y - (g.blpf[1] + cy * g.cell_size[1])),
-                                   v.o.dim == 3 ? d2f_rn(xs.z - (g.blpf[2] + cz * g.cell_size[2])) : 0.f, h);
+        v.S.OFF32[s] = make_float4(d2f_rn(xs.x - (g.blpf[0] + i2d_small(cx) * g.cell_size[0])),
+                                   d2f_rn(xs.y - (g.blpf[1] + i2d_small(cy) * g.cell_size[1])),
+                                   v.o.dim == 3 ? d2f_rn(xs.z - (g.blpf[2] + i2d_small(cz) * g.cell_size[2])) : 0.f, h);
       } else {
         v.S.OFF32[s] = make_float4(d2f_rn(xs.x), d2f_rn(xs.y), d2f_rn(xs.z), h);
       }
@@ -275,29 +264,23 @@ __global__ void skin_offsets_kernel(DevView v) {
   const Persist& P = cur_persist(v);
   const PClass& C = v.cls[P.cls[s]];
   const double4_32a xs = P.X4[s];
-  const float h = (float)C.h;
+  const float h = C.is_free ? d2f_rn(C.h) : -d2f_rn(C.h);
   const int cell = v.S.cellid[s];
   if (cell >= 0) {
     const GridDev& g = grid_of(v, C.inst);
     const int lk = cell - g.cell_base;
     const int cx = lk % g.nc[0], t = lk / g.nc[0], cy = t % g.nc[1], cz = t / g.nc[1];
-    v.S.OFF32[s] = make_float4((float)(xs.x - (g.blpf[0] + cx * g.cell_size[0])),
-                               (float)(xs.y - (g.blpf[1] + cy * g.cell_size[1])),
-                               (float)(v.o.dim == 3 ? xs.z - (g.blpf[2] + cz * g.cell_size[2]) : 0.0), h);
+    v.S.OFF32[s] = make_float4(d2f_rn(xs.x - (g.blpf[0] + i2d_small(cx) * g.cell_size[0])),
+                               d2f_rn(xs.y - (g.blpf[1] + i2d_small(cy) * g.cell_size[1])),
+                               v.o.dim == 3 ? d2f_rn(xs.z - (g.blpf[2] + i2d_small(cz) * g.cell_size[2])) : 0.f, h);
   } else {
-    v.S.OFF32[s] = make_float4((float)xs.x, (float)xs.y, (float)xs.z, h);
+    v.S.OFF32[s] = make_float4(d2f_rn(xs.x), d2f_rn(xs.y), d2f_rn(xs.z), h);
   }
   const GridDev& r = v.grids_ref[C.inst];
   const double xd[3] = {xs.x, xs.y, xs.z};
   int q[3] = {0, 0, 0};
   for (int d = 0; d < v.o.dim; ++d) {
-    // floor((x - BLPF) / CellSize) from an FP32 estimate, with the FP64
-    // division only near a cell face (as the sort's bin_kernel)
-    const double a = xd[d] - r.blpf[d];
-    const float t = d2f_bits(a) * r.inv_cell_size32[d];
-    const float ft = floorf(t), fr = t - ft, tol = 1e-3f + 4e-7f * fabsf(t);
-    int k = (int)ft;
-    if (!(fr >= tol && fr <= 1.f - tol)) k = (int)floor(a / r.cell_size[d]);
+    const int k = cell_floor(r, d, xd[d]);
     q[d] = min(max(k, 0), r.cn_ref[d] - 1);  // clamped as ListGenerate clamps the particles just outside
   }
   v.S.refcell[s] = q[0] | (q[1] << 10) | (q[2] << 20);

@@ -102,7 +102,7 @@ PSPH_D void mat3_rate(const double* SR, const double* RR, const double* Sg, doub
 
 PSPH_D double dp_apex(double* S, double alpha, double kf) {
   double I1 = S[0] + S[4] + S[8];
-  if ((kf - alpha * I1) < 0.0) {
+  if (negative(kf - alpha * I1)) {
     const double Ratio = (alpha == 0.0) ? 0.0 : kf / alpha;
     S[0] -= 1.0 / 3.0 * (I1 - Ratio);
     S[4] -= 1.0 / 3.0 * (I1 - Ratio);
@@ -142,21 +142,22 @@ PSPH_D void dp_return(const PClass& C, double I22, double* Sig, const double* Sn
   double I1 = dp_apex(Sig, alpha, kf);
   deviator<PL>(Sig, I1, SS);
   double J2 = J2of_t<PL>(SS);
-  if ((sqrt(J2) + alpha * I1 - kf) > 0.0) {
+  if ((sqrt_any(J2) + alpha * I1 - kf) > 0.0) {
     deviator<PL>(Sn, Sn[0] + Sn[4] + Sn[8], SS);
     J2 = J2of_t<PL>(SS);
-    if (sqrt(J2) > 0.0) {
+    const double root = sqrt_any(J2);
+    if (root > 0.0) {
       double sum = SS[0] * SR[0];
 #pragma unroll
       for (int e = 1; e < 9; ++e)
         if (live<PL>(e)) sum = sum + SS[e] * SR[e];
-      const double gj = G / sqrt(J2);
+      const double gj = G * rcp_refined(root);
       double dL, s;
       if (C.fail == 2) {
-        dL = 1.0 / (9.0 * alpha * alpha * K + G) * ((3.0 * alpha * K * I1strain) + (G / sqrt(J2)) * sum);
+        dL = rcp_refined(9.0 * alpha * alpha * K + G) * ((3.0 * alpha * K * I1strain) + gj * sum);
         s = 3.0 * alpha * K;
       } else {
-        dL = 1.0 / (9.0 * alpha * K * 3.0 * C.dp_sin_psi + G) * ((3.0 * alpha * K * I1strain) + (G / sqrt(J2)) * sum);
+        dL = rcp_refined(9.0 * alpha * K * 3.0 * C.dp_sin_psi + G) * ((3.0 * alpha * K * I1strain) + gj * sum);
         s = 3.0 * 3.0 * C.dp_sin_psi * K;
       }
 #pragma unroll
@@ -169,8 +170,9 @@ PSPH_D void dp_return(const PClass& C, double I22, double* Sig, const double* Sn
     I1 = dp_apex(Sig, alpha, kf);
     deviator<PL>(Sig, I1, SS);
     J2 = J2of_t<PL>(SS);
-    if ((sqrt(J2) + alpha * I1 - kf) > 0.0 && sqrt(J2) > 0.0) {
-      const double s1 = I1 / 3.0, s2 = (kf - alpha * I1) / sqrt(J2);
+    const double root2 = sqrt_any(J2);
+    if ((root2 + alpha * I1 - kf) > 0.0 && root2 > 0.0) {
+      const double s1 = I1 / 3.0, s2 = (kf - alpha * I1) * rcp_refined(root2);
 #pragma unroll
       for (int e = 0; e < 9; ++e)
         if (live<PL>(e)) Sig[e] = OIe(e) * s1 + SS[e] * s2;
@@ -242,8 +244,11 @@ PSPH_D void strain_update(bool lf, int first, int ct, double dt, const double* S
   }
 }
 
-template <int DIM>
-__global__ void __launch_bounds__(kUT) update_kernel(DevView v) {
+// SOLID: the domain holds soil or solid particles. Without it the kernel is
+// compiled without their stress update, whose registers would leave it a sixth
+// of its warps (1.0M fluid particles: 75 us with, FLUIDNOW us without).
+template <int DIM, bool SOLID>
+__global__ void __launch_bounds__(kUT, SOLID ? 4 : 8) update_kernel(DevView v) {
   const StepScalars* sc = v.sc;
   if (sc->all_stop) return;
   const Persist& P = cur_persist(v);
@@ -278,12 +283,14 @@ __global__ void __launch_bounds__(kUT) update_kernel(DevView v) {
   double rho = X.w;
   if (o.scheme == PSPH_MVERLET) {
     // Move_MVerlet (Source/Particle.cpp:189-274)
-    double vx[3] = {0.0, 0.0, 0.0};
+    const double hdt2 = Is.half_dt2;
     if (o.xsph != 0.0) {
       const double4_32a w = v.S.vxsph4[s];
-      vx[0] = w.x; vx[1] = w.y; vx[2] = w.z;
+      const double vx[3] = {w.x, w.y, w.z};
+      for (int d = 0; d < 3; ++d) x[d] += dt * (vel[d] + vx[d]) + hdt2 * a[d];
+    } else {
+      for (int d = 0; d < 3; ++d) x[d] += dt * vel[d] + hdt2 * a[d];
     }
-    for (int d = 0; d < 3; ++d) x[d] += dt * (vel[d] + vx[d]) + 0.5 * dt * dt * a[d];
     const bool shep = C.shepard && (Is.shepard_counter == o.shepard_step);
     const double zw = v.S.zwab[s];
     double rhob = H.w;
@@ -308,12 +315,12 @@ __global__ void __launch_bounds__(kUT) update_kernel(DevView v) {
         rho = sd / zw;
       } else {
         const double dens = rho;
-        rho = rhob + 2.0 * dt * drho;
+        rho = rhob + Is.dt2 * drho;
         rhob = dens;
       }
       for (int d = 0; d < 3; ++d) {
         const double t = vel[d];
-        vel[d] = vb[d] + 2 * dt * a[d];
+        vel[d] = vb[d] + Is.dt2 * a[d];
         vb[d] = t;
       }
     }
@@ -340,16 +347,16 @@ __global__ void __launch_bounds__(kUT) update_kernel(DevView v) {
     P.H4b[s] = make_double4_32a(vb[0], vb[1], vb[2], rhob);
   }
   double p = V.w;
-  const int mat = C.material;
-  if (mat == 1) {
+  const int mat = SOLID ? C.material : 1;
+  if (!SOLID || mat == 1) {
     // Mat1 (Source/Particle.cpp:146-186)
     if (o.fp32 && C.pres_eq == 1) {
       // FP32C: the Tait pressure from d = rho/rho0 - 1 (FP64) as p0 + B ((1+d)^7 - 1)
       // with the power expanded, 7d + 21d^2 + ... + d^7, in FP32: no cancellation
       // near rho0, ~1e-7 relative, 5 FP64 operations instead of two divisions
-      const float e = (float)((rho - C.rho0) * C.eos_inv_rho0);
+      const float e = d2f_rn((rho - C.rho0) * C.eos_inv_rho0);
       const float poly = e * (7.f + e * (21.f + e * (35.f + e * (35.f + e * (21.f + e * (7.f + e))))));
-      p = C.p0 + (double)(C.eos_b32 * poly);
+      p = C.p0 + f2d_bits(C.eos_b32 * poly);
     } else {
       p = eos(C.pres_eq, C.cs, C.p0, rho, C.rho0);
     }
@@ -358,7 +365,7 @@ __global__ void __launch_bounds__(kUT) update_kernel(DevView v) {
       if (o.need_sr && o.fp32 && !o.has_solid) {
         // FP32C fluid pair kernel: its FP32 contraction of its FP32 sums (two
         // FP64 square roots per particle less); Sbar = sqrt(2 temp) = 2 ShearRate
-        shear_rate = (double)v.S.cshear[s];
+        shear_rate = f2d_bits(v.S.cshear[s]);
         sbar = 2.0 * shear_rate;
       } else if (o.need_sr) {
         const double* S = v.S.strain_rate + 9 * (size_t)s;
@@ -459,6 +466,10 @@ __global__ void __launch_bounds__(kUT) update_kernel(DevView v) {
   // periodic wrap (Source/Particle.cpp:128-142) and CheckParticleLeave's test
   bool out = false;
   for (int d = 0; d < 3; ++d) {
+    // well inside by its FP32 value: neither applies (a comparison of doubles
+    // takes the FP64 pipe as long as an addition)
+    const float xf = d2f_bits(x[d]);
+    if (xf > g.in_lo32[d] && xf < g.in_hi32[d]) continue;
     if (g.dom_size[d] > 0.0) {
       if (x[d] > g.trpr[d]) x[d] -= g.dom_size[d];
       if (x[d] < g.blpf[d]) x[d] += g.dom_size[d];
@@ -493,8 +504,14 @@ __global__ void __launch_bounds__(kUT) update_kernel(DevView v) {
 
 void launch_update(const DevView& v, cudaStream_t st) {
   const int nb = (v.ncap + kUT - 1) / kUT;
-  if (v.o.dim == 2) update_kernel<2><<<nb > 0 ? nb : 1, kUT, 0, st>>>(v);
-  else update_kernel<3><<<nb > 0 ? nb : 1, kUT, 0, st>>>(v);
+  const int grid = nb > 0 ? nb : 1;
+  if (v.o.has_solid) {
+    if (v.o.dim == 2) update_kernel<2, true><<<grid, kUT, 0, st>>>(v);
+    else update_kernel<3, true><<<grid, kUT, 0, st>>>(v);
+  } else {
+    if (v.o.dim == 2) update_kernel<2, false><<<grid, kUT, 0, st>>>(v);
+    else update_kernel<3, false><<<grid, kUT, 0, st>>>(v);
+  }
 }
 
 // begin, bin, 2 scan, scatter, reorder, cell starts, neighbour lists, prepare (2 in the FP32C form: copies + walls),
