@@ -1005,7 +1005,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
       (st = dalloc(c, &S.sstart, NB + 3)) ||
       (st = dalloc(c, &S.tmp_perm, N)) || (st = dalloc(c, &S.slot, N)) || (st = dalloc(c, &S.cellid, N)) ||
       (st = dalloc(c, &S.block_sums, (NB + 2 + 1023) / 1024 + 1)) ||
-      (st = dalloc(c, &S.OFF32, N)) || (st = dalloc(c, &S.D4, N)) || (st = dalloc(c, &S.nl_count, N)) ||
+      (st = dalloc(c, &S.OFF32, N + 4)) || (st = dalloc(c, &S.D4, N)) || (st = dalloc(c, &S.nl_count, N)) ||
       (st = dalloc(c, &S.A4, N)) || (st = dalloc(c, &S.zwab, N)) || (st = dalloc(c, &S.sumden, N)) ||
       (st = dalloc(c, &S.sumkernel, N)) || (st = dalloc(c, &S.nsv4, N)) || (st = dalloc(c, &S.vxsph4, N)) ||
       (st = dalloc(c, &S.shear_rate, N)) || (st = dalloc(c, &S.sbar, N)))

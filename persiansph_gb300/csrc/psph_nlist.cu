@@ -34,6 +34,7 @@ namespace psph {
 namespace {
 
 constexpr int kNT = 128;
+constexpr int kOver = 4;  // a masked group reads up to 3 candidates past its cell's end: room behind the offsets
 
 // Shared pieces of both scans. The 8-slot entry ring of a lane is
 // lane-interleaved (slot s of lane l at ring[s][l], so the per-candidate
@@ -260,11 +261,10 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
   const PClass& C = v.cls[P.cls[ia]];
   const GridDev& g = grid_of(v, C.inst);
   // a fixed particle lists free candidates only: two fixed ones scan the free
-  // half of each slab, a free and a fixed one scan both, the fixed one with a
-  // threshold nothing meets in the fixed half
+  // half of each cell (one slab per cell), otherwise the candidates' signs tell
   const bool fixed_a = !C.is_free && !v.o.list_all;
   const bool fixed_b = pair ? !v.cls[P.cls[ib]].is_free && !v.o.list_all : fixed_a;
-  const bool fixed = fixed_a && fixed_b, mixed = fixed_a != fixed_b;
+  const bool free_half = fixed_a && fixed_b && v.o.xsub == 1, by_sign = (fixed_a || fixed_b) && !free_half;
   const float3 cs = cell_size_f(g);
   // particle b far away when it is not paired: its tests always fail
   constexpr float kFar = 1e18f;
@@ -285,6 +285,8 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
   const int xs = v.o.xsub;
   const int* __restrict__ sstart = v.S.sstart;  // two bins per slab: its free, then its fixed particles
   const float inv_sw = (float)xs / cs.x;
+  const float2 AXm = make_float2(oa.x + cs.x, ob.x + cs.x), AX0 = make_float2(oa.x, ob.x),
+               AXp = make_float2(oa.x - cs.x, ob.x - cs.x);
   const int zlo = (DIM == 3) ? -1 : 0, zhi = (DIM == 3) ? 1 : 0;
   for (int dz = zlo; dz <= zhi; ++dz) {
     int z = c.z + dz;
@@ -313,30 +315,53 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
         slo = max(slo, la);
         shi = min(shi, ha);
       }
-      for (int dx = -1; dx <= 1; ++dx) {
+      // The row's three cells as candidate ranges, walked in one loop: the lanes
+      // of a warp lie in neighbouring cells of one row, whose sums over three cells
+      // are nearly equal where the single cells' counts are not (a lattice puts two
+      // or three planes into a cell's width). A group of 4 candidates never spans
+      // two cells; the last one of a cell is partly masked. Bound by issue slots:
+      // with a loop per cell 21 of 32 lanes were active (1.0M particles in 3D: 420 us,
+      // this walk 360; 86k: 143, now 110).
+      int lo0, hi0, lo1, hi1, lo2, hi2;
+      auto range = [&](int dx, int& lo, int& hi) {
+        lo = hi = 0;
         int x = c.x + dx;
         if (g.periodic[0]) x = (x + g.nc[0]) % g.nc[0];
-        else if (x < 0 || x >= g.nc[0]) continue;
+        else if (x < 0 || x >= g.nc[0]) return;
         const int s0 = max(slo - dx * xs, 0), s1 = min(shi - dx * xs, xs - 1);
-        if (s0 > s1) continue;
-        const int bin0 = 2 * ((base + x) * xs + s0), bin1 = 2 * ((base + x) * xs + s1 + 1);
-        const int step = fixed ? 2 : (mixed ? 1 : bin1 - bin0);  // two free ones: the slabs in one range
-        for (int bin = bin0; bin < bin1; bin += step) {
-        int lo = sstart[bin];
-        const int hi = sstart[fixed ? bin + 1 : bin + step];
-        const bool second = mixed && (bin & 1);
-        const float thra = (second && fixed_a) ? -1.f : thr, thrb = (second && fixed_b) ? -1.f : thr;
-        const int tag = (int)((unsigned)((dx + 1) | cyz) << kCodeShift);
-        const float cx = -(float)dx * cs.x;
-        const float axa = oa.x + cx, aya = oa.y + cy, aza = oa.z + cz;
-        const float axb = ob.x + cx, ayb = ob.y + cy, azb = ob.z + cz;
-        // both particles' separations in packed FP32x2 arithmetic: a - off_j
-        // as fma(off_j, -1, a) (one rounding, the subtraction's), then the
-        // squared distances, one instruction for both particles' values
-        const float2 AX = make_float2(axa, axb), AY = make_float2(aya, ayb), AZ = make_float2(aza, azb);
-        const float2 M1 = make_float2(-1.f, -1.f);
-        auto test = [&](int j, bool& ina, bool& inb) {
-          const float4 oj = cand.at(j);
+        if (s0 > s1) return;
+        const int bin = 2 * ((base + x) * xs + s0);
+        lo = sstart[bin];
+        hi = sstart[free_half ? bin + 1 : 2 * ((base + x) * xs + s1 + 1)];
+      };
+      range(-1, lo0, hi0);
+      range(0, lo1, hi1);
+      range(1, lo2, hi2);
+      const bool home = dy == 0 && dz == 0;  // neither particle lists itself
+      const float2 AY = make_float2(oa.y + cy, ob.y + cy), AZ = make_float2(oa.z + cz, ob.z + cz);
+      const float2 M1 = make_float2(-1.f, -1.f);
+      float2 AX = AXm;
+      int tag = (int)((unsigned)cyz << kCodeShift), cell_k = 0, j = lo0, end = hi0;
+      auto next_cell = [&]() {
+        while (j >= end && cell_k < 2) {
+          ++cell_k;
+          j = cell_k == 1 ? lo1 : lo2;
+          end = cell_k == 1 ? hi1 : hi2;
+          AX = cell_k == 1 ? AX0 : AXp;
+          tag += 1 << kCodeShift;
+        }
+      };
+      next_cell();
+      while (j < end) {
+        const int m = end - j;  // candidates left in the cell
+        bool ia_[4], ib_[4];
+        float w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          // both particles' separations in packed FP32x2 arithmetic: a - off_j
+          // as fma(off_j, -1, a) (one rounding, the subtraction's), then the
+          // squared distances, one instruction for both particles' values
+          const float4 oj = cand.at(j + e);  // (past the cell's end: another particle's, masked)
           const float2 ex = __ffma2_rn(make_float2(oj.x, oj.x), M1, AX);
           const float2 ey = __ffma2_rn(make_float2(oj.y, oj.y), M1, AY);
           float2 d2 = __fmul2_rn(ex, ex);
@@ -345,49 +370,35 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
             const float2 ez = __ffma2_rn(make_float2(oj.z, oj.z), M1, AZ);
             d2 = __ffma2_rn(ez, ez, d2);
           }
-          ina = d2.x <= thra;
-          inb = d2.y <= thrb;
-        };
-        auto one = [&](int j, bool ena, bool enb) {
-          bool ina, inb;
-          test(j, ina, inb);
-          const int ka = wa.k, kb = wb.k;
-          wa.put(j | tag, ina && ena);
-          wb.put(j | tag, inb && enb);
-          wa.flush(ka, cap, N);
-          wb.flush(kb, cap, N);
-        };
-        if (dx == 0 && dy == 0 && dz == 0) {  // the home cell: neither particle lists itself
-          const int e0 = min(ia, hi);
-          for (int j = lo; j < e0; ++j) one(j, true, true);
-          if (lo <= ia && ia < hi) one(ia, false, true);
-          int nx = ia + 1;
-          if (pair) {
-            if (lo <= ib && ib < hi) one(ib, true, false);
-            nx = ib + 1;
+          ia_[e] = d2.x <= thr && m > e;
+          ib_[e] = d2.y <= thr && m > e;
+          w[e] = oj.w;
+        }
+        if (home) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            ia_[e] = ia_[e] && j + e != ia;
+            ib_[e] = ib_[e] && j + e != ib;
           }
-          lo = max(lo, nx);
         }
-        int j = lo;
-        for (; j + 4 <= hi; j += 4) {
-          bool a0, a1, a2, a3, b0, b1, b2, b3;
-          test(j, a0, b0);
-          test(j + 1, a1, b1);
-          test(j + 2, a2, b2);
-          test(j + 3, a3, b3);
-          const int ka = wa.k, kb = wb.k;
-          wa.put(j | tag, a0);
-          wa.put((j + 1) | tag, a1);
-          wa.put((j + 2) | tag, a2);
-          wa.put((j + 3) | tag, a3);
-          wb.put(j | tag, b0);
-          wb.put((j + 1) | tag, b1);
-          wb.put((j + 2) | tag, b2);
-          wb.put((j + 3) | tag, b3);
-          wa.flush(ka, cap, N);
-          wb.flush(kb, cap, N);
+        if (by_sign) {  // fixed particles among the candidates of a fixed one (their h is negative)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            ia_[e] = ia_[e] && !(fixed_a && w[e] < 0.f);
+            ib_[e] = ib_[e] && !(fixed_b && w[e] < 0.f);
+          }
         }
-        for (; j < hi; ++j) one(j, true, true);
+        const int ka = wa.k, kb = wb.k;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) wa.put((j + e) | tag, ia_[e]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) wb.put((j + e) | tag, ib_[e]);
+        wa.flush(ka, cap, N);
+        wb.flush(kb, cap, N);
+        j += 4;
+        if (j >= end) {
+          j = end;
+          next_cell();
         }
       }
     }
@@ -519,7 +530,7 @@ int sm_count() {
 }  // namespace
 
 void nlist_configure() {
-  const int bytes = kStageCapMax * (int)sizeof(float4);
+  const int bytes = (kStageCapMax + kOver) * (int)sizeof(float4);
   cudaFuncSetAttribute(nlist_staged_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   cudaFuncSetAttribute(nlist_staged_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
@@ -535,7 +546,7 @@ void launch_nlist(const DevView& v, cudaStream_t st) {
     const int nb = nr + (half > 0 ? (half + kNT - 1) / kNT : 1);
     const int cap = min(v.o.nlist_stage, kStageCapMax);
     if (cap > 0 && !v.o.any_periodic_x) {
-      const size_t smem = (size_t)cap * sizeof(float4);
+      const size_t smem = (size_t)(cap + kOver) * sizeof(float4);
       if (v.o.dim == 2) nlist_staged_kernel<2><<<nb, kNT, smem, st>>>(v, margin, nr, cap);
       else nlist_staged_kernel<3><<<nb, kNT, smem, st>>>(v, margin, nr, cap);
       return;
