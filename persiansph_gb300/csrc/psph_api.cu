@@ -1003,13 +1003,14 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
   const size_t NB = 2 * NC * kMaxXsub;  // sort bins at the finest x-slab split, free and fixed apart
   if ((st = dalloc(c, &S.key, N)) || (st = dalloc(c, &S.count, NB + 2)) || (st = dalloc(c, &S.start, NC + 3)) ||
       (st = dalloc(c, &S.sstart, NB + 3)) ||
-      (st = dalloc(c, &S.tmp_perm, N)) || (st = dalloc(c, &S.slot, N)) || (st = dalloc(c, &S.cellid, N)) ||
+      (st = dalloc(c, &S.tmp_perm, N)) || (st = dalloc(c, &S.slot, N)) || (st = dalloc(c, &S.rest, N)) || (st = dalloc(c, &S.cellid, N)) ||
       (st = dalloc(c, &S.block_sums, (NB + 2 + 1023) / 1024 + 1)) ||
       (st = dalloc(c, &S.OFF32, N + 4)) || (st = dalloc(c, &S.D4, N)) || (st = dalloc(c, &S.nl_count, N)) ||
       (st = dalloc(c, &S.A4, N)) || (st = dalloc(c, &S.zwab, N)) || (st = dalloc(c, &S.sumden, N)) ||
       (st = dalloc(c, &S.sumkernel, N)) || (st = dalloc(c, &S.nsv4, N)) || (st = dalloc(c, &S.vxsph4, N)) ||
       (st = dalloc(c, &S.shear_rate, N)) || (st = dalloc(c, &S.sbar, N)))
     return st;
+  S.walls = S.slot;
   if (o.couple_soil && o.swi == 1 && (st = dalloc(c, &S.s_acc, N))) return st;
   if (o.couple_soil && o.swi != 2 && (st = dalloc(c, &S.satcheck, N))) return st;
   if (o.couple_solid && ((st = dalloc(c, &S.fsi_p, N)) || (st = dalloc(c, &S.fsi_nsv, N)))) return st;
@@ -1032,6 +1033,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
         (st = dalloc(c, &S.V32LO, N)))
       return st;
     if (o.spec32 && (st = dalloc(c, &S.PX32, N))) return st;
+    if (o.spec32) S.RC32 = reinterpret_cast<float2*>(S.D32);
     if (dyn_mu && (st = dalloc(c, &S.MU32, N))) return st;
     if (o.need_sr && !o.has_solid &&  // FP32 ShearRate and strain-rate sums of the fluid kernel
         ((st = dalloc(c, &S.cshear, N)) || (st = dalloc(c, &S.sr32, 6 * N))))
@@ -1567,6 +1569,7 @@ psph_status split_steps(psph_ctx* c, int64_t nsteps, long long* launched, bool o
     }
     {
       const DevView v = view(c);
+      launch_copies32(v, s);  // the in-flow and the hook may have changed what the sort copied
       if (v.o.fp32) launch_prepare32(v, s);
       else launch_prepare(v, s);
       if (v.o.couple_soil && v.o.swi != 2) launch_saturation(v, s);

@@ -108,6 +108,8 @@ struct StepScalars {
   int launches;
   unsigned long long closure_eval, closure_fallback;  // closure evaluations / Smagorinsky fallbacks
   int nl_rest;    // particles the neighbour-list scan handles one per lane (set by the sort)
+  int n_walls;    // fixed particles (Scratch::walls, set by the sort)
+  int n_old;      // n before the sort removed particles (its scatter's range)
   // neighbour lists with a skin (FP32C form, Options::skin > 0): the cell sort
   // and the lists are rebuilt only when a particle has moved half the skin
   int rebuild;             // this step sorts and lists (always, without a skin)

@@ -36,6 +36,8 @@ struct Scratch {
   int* sstart;     // 2 ncells * xsub + 3 exclusive prefix over the x-slabs of the cells, free and fixed apart
   int* tmp_perm;
   int* slot;       // a particle's place in its segment before the ranking
+  int* walls;      // the fixed particles, in nearly sorted order (the same memory as slot, whose use is over)
+  int* rest;       // the particles the neighbour-list scan handles one per lane
   int* cellid;     // cell of each sorted particle (orphan/dead: -1)
   int* block_sums;
   // per-step derived / outputs
@@ -49,6 +51,7 @@ struct Scratch {
   float4* PX32;      // FP32C form, Options::spec32: (position - cell origin, +-1/density), negative for a fixed one
   float4* V32;       // FP32C form: (v, pressure)
   float4* D32;       // FP32C form: (1/density, pressure/density^2, sound speed, density)
+  float2* RC32;      // FP32C form, Options::spec32, in D32's place: (density, refcell with a skin) of the free ones
   float4* SIG32;     // FP32C solids: symmetric Sigma, 2 per particle (00 01 02 11 | 12 22 - -)
   float4* TIR32;     // FP32C solids with TI: symmetric TIR, same layout
   float4* VB32;      // FP32C solids: wall history velocity (MVerlet vb / leapfrog vb)
@@ -199,6 +202,8 @@ struct DevView {
 PSPH_D const GridDev& grid_of(const DevView& v, int inst) { return v.grids[inst]; }
 
 PSPH_D const Persist& cur_persist(const DevView& v) { return v.sc->buf ? v.PB : v.PA; }
+// A free particle's FP32 density (FP32C form).
+PSPH_D float rho32(const DevView& v, int s) { return v.o.spec32 ? v.S.RC32[s].x : v.S.D32[s].w; }
 // A particle's row in the tensor arrays.
 PSPH_D size_t tensor_row(const Persist& P, int s) { return 9 * (size_t)P.orig[s]; }
 PSPH_D const Persist& next_persist(const DevView& v) { return v.sc->buf ? v.PA : v.PB; }
@@ -215,14 +220,17 @@ PSPH_D void widen_rates(const float4* __restrict__ q, double* __restrict__ sr, d
 }
 
 // Launch wrappers (defined in the .cu files).
-void launch_sort(const DevView& v, cudaStream_t st);      // bin + scan + scatter + rank + reorder + flip
+void launch_sort(const DevView& v, cudaStream_t st);      // bin + scan + scatter + reorder
+int sort_launches(const DevView& v);
 void launch_nlist(const DevView& v, cudaStream_t st);     // per-step neighbour lists
 void launch_skin_offsets(const DevView& v, cudaStream_t st);  // lists with a skin: FP32 offsets, reference cells
 // the next cell sort runs (now, a sort outside a step) / the next step rebuilds its lists
 void launch_mark_rebuild(const DevView& v, bool now, bool next_step, cudaStream_t st);
 void nlist_configure();                                   // once, outside stream capture: shared-memory limits
 void launch_prepare(const DevView& v, cudaStream_t st);   // per-particle derived quantities, TIR
-void launch_prepare32(const DevView& v, cudaStream_t st); // FP32C form: copies + wall interpolation
+void launch_prepare32(const DevView& v, cudaStream_t st); // FP32C form: wall interpolation (solids: and copies)
+// FP32C fluids: the copies again, where the state changed after the sort (hooks, in/out-flow)
+void launch_copies32(const DevView& v, cudaStream_t st);
 void launch_forces32(const DevView& v, cudaStream_t st);  // FP32C form: fluid pair forces
 void launch_expand_sr32(const DevView& v, int n, cudaStream_t st);  // sr32 / rates32 -> the FP64 rate tensors
 void launch_wall(const DevView& v, cudaStream_t st);      // wall interpolation

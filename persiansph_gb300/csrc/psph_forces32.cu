@@ -12,9 +12,10 @@
 //  - the acceleration and density-rate sums are Kahan-compensated in FP32;
 //  - integration, material update and the dt reduction stay in FP64
 //    (psph_update.cu, dt_finalize_kernel).
+#include <algorithm>
 #include <cfloat>
 
-#include "psph_pairs.cuh"
+#include "psph_copies.cuh"
 
 namespace psph {
 
@@ -57,6 +58,11 @@ PSPH_D float4 ld_early_coherent(const float4* p) {
   return r;
 }
 
+PSPH_D float2 ld_early_coherent(const float2* p) {
+  float2 r;
+  asm volatile("ld.global.v2.f32 {%0,%1}, [%2];" : "=f"(r.x), "=f"(r.y) : "l"(p));
+  return r;
+}
 PSPH_D float ld_early_coherent(const float* p) {
   float r;
   asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(p));
@@ -141,92 +147,61 @@ struct KernF {
 // ---------------------------------------------------------------------------
 // Preparation (FP32 copies, partner-visible wall state) and wall interpolation
 // ---------------------------------------------------------------------------
-template <int DIM>
 __global__ void __launch_bounds__(kFT32) copies32_kernel(DevView v) {
   const StepScalars* sc = v.sc;
   if (sc->all_stop) return;
   const Persist& P = cur_persist(v);
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= sc->n) return;
-  const PClass32& C = v.cls32[P.cls[w]];
-  if (v.inst[C.inst].stop) return;
-  const double4_32a vv = P.V4[w];
-  // every conversion on the integer pipe (d2f_rn / d2f_split: the values of
-  // the conversion instruction, which runs on the FP64 pipe)
-  const float p = d2f_rn(vv.w);
-  float lx, ly, lz;
-  const float vx = d2f_split(vv.x, &lx), vy = d2f_split(vv.y, &ly), vz = d2f_split(vv.z, &lz);
-  v.S.V32[w] = make_float4(vx, vy, vz, p);
-  // the velocity's low-order part: in a smooth flow v_i - v_j is far smaller
-  // than v, and the pair differences take (hi_i - hi_j) + (lo_i - lo_j), exact
-  // to ~2^-48 of |v|; the class index and its flags ride along in .w (class |
-  // flags << 16: one load per pair, and no class-table load when the pair
-  // constants are uniform)
-  float lw = __int_as_float(P.cls[w] | (C.flags << 16));
-  if (C.flags & CF_FREE) {
-    const float rho = d2f_rn(P.X4[w].w);
-    const float inv = 1.f / rho;
-    const float ratio = rho / C.rho0;
-    const float c = (C.pres_eq == 1) ? C.cs * ratio * ratio * ratio : C.cs;
-    v.S.D32[w] = make_float4(inv, p * inv * inv, c, rho);
-    if (v.o.spec32) {  // the constant-parameter pair kernel's record (the walls' comes with their pressure)
-      const float4 x = v.S.OFF32[w];
-      v.S.PX32[w] = make_float4(x.x, x.y, x.z, inv);
-      lw = c;
-    }
-  }
-  v.S.V32LO[w] = make_float4(lx, ly, lz, lw);
-  // FP32 copy of a per-particle viscosity: the pair loop then converts nothing
-  // (a double-to-float conversion runs on the FP64 pipe, 1/64 of the FP32 rate)
-  if (v.o.dyn_mu) v.S.MU32[w] = d2f_rn(P.mu[w]);
+  if (w < sc->n) fluid_copies32(v, P, w, P.cls[w], P.X4[w].w, P.V4[w], v.S.OFF32[w], v.o.skin > 0.f ? v.S.refcell[w] : 0);
 }
 
+// Wall interpolation, bound by the neighbours' gathers. 2D: 4 lanes to a wall,
+// each a 16-byte chunk of its list at a time, over the sort's list of the fixed
+// particles (920 particles 10 us where one lane takes 14, 86k 11 and 14). 3D: a lane to a particle, the free ones' idle: a warp's
+// walls then gather the same neighbours at the same time (1.0M particles 82 us;
+// over the list of the fixed ones, whose warps lie less close, 93, with 2 and 4
+// lanes to a wall 129 and 177).
+template <int DIM>
+constexpr int kWallLanesLog2 = DIM == 2 ? 2 : 0;
+
 template <int DIM, int KT>
-__global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
-  const StepScalars* sc = v.sc;
-  if (sc->all_stop) return;
-  const Persist& P = cur_persist(v);
-  const int n = sc->n;
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+PSPH_D void interpolate_wall32(const DevView& v, const Persist& P, int w, int sub) {
   const Options& o = v.o;
   const PClass32* __restrict__ CT = v.cls32;
-  const int winst = (w < n) ? CT[P.cls[w]].inst : 0;
-  const GridDev& g = grid_of(v, winst);
-  bool wall = false, noslip = false;
-  int cell = -1, ow = 0;
-  float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (w < n && !v.inst[winst].stop) {
-    const PClass32& C = CT[P.cls[w]];
-    if (!(C.flags & CF_FREE)) {
-      wall = true;
-      noslip = C.flags & CF_NOSLIP;
-      ow = P.orig[w];
-      cell = v.S.cellid[w];
-      oi = v.S.OFF32[w];
-    }
-  }
+  const bool wall = w >= 0;
+  const PClass32& C = CT[wall ? P.cls[w] : 0];
+  const GridDev& g = grid_of(v, C.inst);
+  const bool noslip = wall && (C.flags & CF_NOSLIP);
+  const int ow = wall ? P.orig[w] : 0, cell = wall ? v.S.cellid[w] : -1;
+  const float4 oi = wall ? v.S.OFF32[w] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float3 cs = cell_size_f(g);
   const float gx = o.gravity32[0], gy = o.gravity32[1], gz = o.gravity32[2];
   const bool need_orient = !o.wallp_physical && (gx != 0.f || gy != 0.f || gz != 0.f);
   const bool skin = o.skin > 0.f;
   const int rc_w = (skin && need_orient && wall) ? v.S.refcell[w] : 0;
   float sk = 0.f, p = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
-  const float hw = fabsf(oi.w);
+  const float hw = fabsf(oi.w), ihw = 1.f / hw;
+  // a free neighbour's density and, with a skin, its cell in the reference's grid
+  auto density_and_cell = [&](int f) {
+    return o.spec32 ? ld_early_coherent(v.S.RC32 + f)
+                    : make_float2(ld_early_coherent(&v.S.D32[f].w),
+                                  skin && need_orient ? __int_as_float(v.S.refcell[f]) : 0.f);
+  };
   // One neighbour, loaded: free particles contribute (OFF32.w is negative for a
   // fixed one; an FP32C domain has one material).
-  auto visit = [&](const int f, const int code, const float4 of, const float4 vf, const float rho) {
+  auto visit = [&](const int f, const int code, const float4 of, const float4 vf, const float2 rr) {
+    const float rho = rr.x;
     float x0, x1, x2;
     rel_pos<DIM>(cs, oi, of, code, x0, x1, x2);  // x_wall - x_fluid
     if (need_orient) {
       // the pair's cell offset in the reference's grid (with a skin the lists'
       // cells are coarser): it decides which particle the reference lists first
-      const int cd = skin ? ref_code(rc_w, v.S.refcell[f]) : code;
+      const int cd = skin ? ref_code(rc_w, __float_as_int(rr.y)) : code;
       if (!first_of_pair_code(cd, ow, P.orig[f])) {
         x0 = -x0; x1 = -x1; x2 = -x2;
       }
     }
-    const float hb = 0.5f * (hw + of.w);
-    const float ih = 1.f / hb;
+    const float ih = o.uniform_h ? ihw : 1.f / (0.5f * (hw + of.w));
     const float q = sqrtf(x0 * x0 + x1 * x1 + x2 * x2) * ih;
     const float K = KernF<DIM, KT>::W(q, KernF<DIM, KT>::cw() * (DIM == 2 ? ih * ih : ih * ih * ih));
     if (K == 0.f) return;
@@ -242,24 +217,24 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
     const int4* __restrict__ nl4 = reinterpret_cast<const int4*>(v.S.nl) + nl_slot(w);
     const size_t N = (size_t)v.nl_stride;
     const int nch = (cnt + 3) >> 2;
-    for (int c = 0; c < nch; ++c) {
+    for (int c = sub; c < nch; c += 1 << kWallLanesLog2<DIM>) {
       const int4 q = nl4[(size_t)c * N];
       const int rem = cnt - 4 * c;
       const int e[4] = {q.x, rem > 1 ? q.y : q.x, rem > 2 ? q.z : q.x, rem > 3 ? q.w : q.x};
       float4 of[4], vf[4];
-      float rho[4];
+      float2 rr[4];
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
         const int f = e[t] & kIndexMask;
         of[t] = ld_early(v.S.OFF32 + f);
         vf[t] = ld_early_coherent(v.S.V32 + f);
-        rho[t] = ld_early_coherent(&v.S.D32[f].w);
+        rr[t] = density_and_cell(f);
       }
 #pragma unroll
       for (int t = 0; t < 4; ++t)
-        if (t < rem && of[t].w > 0.f) visit(e[t] & kIndexMask, entry_code(e[t]), of[t], vf[t], rho[t]);
+        if (t < rem && of[t].w > 0.f) visit(e[t] & kIndexMask, entry_code(e[t]), of[t], vf[t], rr[t]);
     }
-  } else {  // list overflow: scan the cells
+  } else if (sub == 0) {  // list overflow: scan the cells
     NbrSource<DIM> src;
     src.init(v, g, w, true, 1.0f);
     while (true) {
@@ -267,10 +242,18 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
       const int f = src.next(v, &code);
       if (f < 0) break;
       const float4 of = v.S.OFF32[f];
-      if (of.w > 0.f) visit(f, code, of, ld_early_coherent(v.S.V32 + f), ld_early_coherent(&v.S.D32[f].w));
+      if (of.w > 0.f) visit(f, code, of, ld_early_coherent(v.S.V32 + f), density_and_cell(f));
     }
   }
-  if (!wall) return;
+#pragma unroll
+  for (int d = 1; d < 1 << kWallLanesLog2<DIM>; d <<= 1) {  // the lanes' sums together
+    sk += __shfl_xor_sync(0xffffffffu, sk, d);
+    p += __shfl_xor_sync(0xffffffffu, p, d);
+    n0 += __shfl_xor_sync(0xffffffffu, n0, d);
+    n1 += __shfl_xor_sync(0xffffffffu, n1, d);
+    n2 += __shfl_xor_sync(0xffffffffu, n2, d);
+  }
+  if (!wall || sub != 0) return;
   if (sk != 0.f) {
     p = p / sk;
     if (noslip) { n0 /= sk; n1 /= sk; n2 /= sk; }
@@ -305,6 +288,19 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
   } else {
     v.S.D32[w] = make_float4(inv, p * inv * inv, cwv, rw);
   }
+}
+
+template <int DIM, int KT>
+__global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
+  const StepScalars* sc = v.sc;
+  if (sc->all_stop) return;
+  const Persist& P = cur_persist(v);
+  const int t = blockIdx.x * kFT32 + threadIdx.x, sub = t & ((1 << kWallLanesLog2<DIM>) - 1);
+  int w = t >> kWallLanesLog2<DIM>;
+  if (DIM == 2) w = w < sc->n_walls ? v.S.walls[w] : -1;
+  else if (w >= sc->n || (v.cls32[P.cls[w]].flags & CF_FREE)) w = -1;
+  if (w >= 0 && v.inst[v.cls32[P.cls[w]].inst].stop) w = -1;
+  if (__any_sync(0xffffffffu, w >= 0)) interpolate_wall32<DIM, KT>(v, P, w, sub);  // (a wall's lanes sum together)
 }
 
 // ---------------------------------------------------------------------------
@@ -1441,8 +1437,7 @@ inline int nblk32(int n) { return n <= 0 ? 1 : (n + kFT32 - 1) / kFT32; }
 
 template <int DIM>
 void prepare32_dispatch(const DevView& v, cudaStream_t st) {
-  const int nb = nblk32(v.ncap);
-  copies32_kernel<DIM><<<nb, kFT32, 0, st>>>(v);
+  const int nb = nblk32(v.ncap << kWallLanesLog2<DIM>);  // (how many walls there are is known on the device only)
   switch (v.o.kt) {
     case 0: prepare32_kernel<DIM, 0><<<nb, kFT32, 0, st>>>(v); break;
     case 1: prepare32_kernel<DIM, 1><<<nb, kFT32, 0, st>>>(v); break;
@@ -1502,6 +1497,10 @@ void forces32_dispatch(const DevView& v, cudaStream_t st) {
 }
 
 }  // namespace
+
+void launch_copies32(const DevView& v, cudaStream_t st) {
+  if (v.o.fp32 && !v.o.has_solid) copies32_kernel<<<nblk32(v.ncap), kFT32, 0, st>>>(v);
+}
 
 void launch_prepare32(const DevView& v, cudaStream_t st) {
   if (v.o.has_solid) {  // FP64 wall stress interpolation and TIR, then the FP32 copies

@@ -224,7 +224,7 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
 // when they share a cell. Both scan the same cell block, so each candidate is
 // loaded once and tested against both, and the rows and slabs walked are the
 // union of the two particles' reach. The odd particles whose cell starts at
-// them (listed by the sort, nl_rest of them in S.tmp_perm) get a lane of their
+// them (listed by the sort, nl_rest of them in S.rest) get a lane of their
 // own in the first nr blocks of the grid, which the hardware starts first, so
 // their scans run beside the pairs instead of after them.
 template <int DIM>
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kNT, 8) nlist_pair_kernel(DevView v, float mar
   if ((int)blockIdx.x < nr) {
     const int m = min(sc->nl_rest, v.ncap);
     for (int q = blockIdx.x * kNT + threadIdx.x; q < m; q += nr * kNT)
-      list_one<DIM, true>(v, v.S.tmp_perm[q], margin, &ring[0][0][threadIdx.x]);
+      list_one<DIM, true>(v, v.S.rest[q], margin, &ring[0][0][threadIdx.x]);
     return;
   }
   const int n = sc->n;
@@ -321,7 +321,7 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
       // or three planes into a cell's width). A group of 4 candidates never spans
       // two cells; the last one of a cell is partly masked. Bound by issue slots:
       // with a loop per cell 21 of 32 lanes were active (1.0M particles in 3D: 420 us,
-      // this walk 360; 86k: 143, now 110).
+      // this walk 360; 177k: 143, now 110).
       int lo0, hi0, lo1, hi1, lo2, hi2;
       auto range = [&](int dx, int& lo, int& hi) {
         lo = hi = 0;
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kNT, 4) nlist_staged_kernel(DevView v, float m
   if ((int)blockIdx.x < nr) {
     const int m = min(sc->nl_rest, v.ncap);
     for (int q = blockIdx.x * kNT + threadIdx.x; q < m; q += nr * kNT)
-      list_one<DIM, true>(v, v.S.tmp_perm[q], margin, &ring[0][0][threadIdx.x]);
+      list_one<DIM, true>(v, v.S.rest[q], margin, &ring[0][0][threadIdx.x]);
     return;
   }
   const int n = sc->n;

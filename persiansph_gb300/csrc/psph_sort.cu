@@ -12,21 +12,21 @@
 //            would drop into a periodic ghost column (it then sits in no list),
 //            nbins+1 for one that CheckParticleLeave removed. The counting
 //            atomic's old value is the particle's slot inside its segment.
-//   scan     exclusive prefix of the counts (block scans, then each block adds
-//            the totals before it and clears the counts for the next sort).
-//   scatter  into the slots.
+//   scan     exclusive prefix of the counts; the sorted state's particle counts.
+//   scatter  into the slots; per-cell segment starts (start[c] = start of c's
+//            first slab) for everything that walks whole cells, the particles
+//            the neighbour-list scan handles one per lane, the counts cleared.
 //   reorder  deterministic order inside each segment: by original index, so the
 //            sorted state depends only on positions, never on atomic timing;
-//            each particle's fields move to that place (HBM-bound).
-//   starts   per-cell segment starts (start[c] = start of c's first slab) for
-//            everything that walks whole cells, the particles the neighbour-list
-//            scan handles one per lane, and the new counts and buffer.
-// Six launches (eleven with separate clearing, scan of totals, ranking and
-// finish kernels): 57 -> 44 us for 86k particles, where launches are what counts.
+//            each particle's fields move to that place (HBM-bound), with its
+//            FP32 copies and the list of the fixed particles.
+// Four launches (five with more than 131,072 bins): launches are what counts up
+// to 100k particles. With six 5k particles took 40 us, so 31; 920 in the FP32C
+// form, their copies included, 37 and 25.
 #include <algorithm>
 #include <cstdio>
 
-#include "psph_device.cuh"
+#include "psph_copies.cuh"
 
 namespace psph {
 
@@ -40,7 +40,7 @@ __global__ void bin_kernel(DevView v, const uint8_t* __restrict__ alive, int* __
   const Persist& P = cur_persist(v);
   const int n = sc->n;
   const int nbins = 2 * v.total_cells * xsub;
-  if (blockIdx.x == 0 && threadIdx.x == 0) sc->nl_rest = 0;  // cell_starts_kernel counts them
+  if (blockIdx.x == 0 && threadIdx.x == 0) sc->nl_rest = sc->n_walls = 0;  // counted by the scatter and the reorder
   const int orphan_key = nbins, dead_key = nbins + 1;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     int k;
@@ -92,19 +92,16 @@ __global__ void bin_kernel(DevView v, const uint8_t* __restrict__ alive, int* __
   }
 }
 
-// Phase 1: in-block exclusive scan of `in` (len entries), block totals to sums.
-// A thread takes kScanPer consecutive entries, a block kScanBlock: few enough
-// totals that phase 2 needs no scan of them in between.
+// Exclusive scan of `in` (len entries): a thread takes kScanPer consecutive
+// entries, a block kScanBlock.
 constexpr int kScanPer = 8, kScanBlock = 1024 * kScanPer;
-__global__ void __launch_bounds__(1024) scan_blocks(const int* __restrict__ in, int* __restrict__ out,
-                                                    int* __restrict__ sums, int len, const StepScalars* sc) {
-  if (sc && (sc->all_stop || !sc->rebuild)) return;  // the cell sort's scan, on a step without a rebuild
-  __shared__ int warp_tot[32];
+
+// A block's scan: v[] the thread's entries; returns the exclusive prefix of the
+// thread's first one in the block, *total the block's sum (in every thread).
+__device__ __forceinline__ int block_scan(const int (&v)[kScanPer], int* total) {
+  __shared__ int warp_tot[33];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  const int first = blockIdx.x * kScanBlock + t * kScanPer;
-  int v[kScanPer], own = 0;
-#pragma unroll
-  for (int e = 0; e < kScanPer; ++e) v[e] = (first + e < len) ? in[first + e] : 0;
+  int own = 0;
 #pragma unroll
   for (int e = 0; e < kScanPer; ++e) own += v[e];
   int incl = own;
@@ -124,10 +121,75 @@ __global__ void __launch_bounds__(1024) scan_blocks(const int* __restrict__ in, 
       if (lane >= o) si += y;
     }
     warp_tot[lane] = si - s;  // exclusive warp offsets
-    if (lane == 31) sums[blockIdx.x] = si;
+    if (lane == 31) warp_tot[32] = si;
   }
   __syncthreads();
-  int at = incl - own + warp_tot[w];
+  *total = warp_tot[32];
+  return incl - own + warp_tot[w];
+}
+
+// The sum of `part` over the block, in every thread.
+__device__ __forceinline__ int block_sum(int part) {
+  __shared__ int warp_sum[32];
+  const int lane = threadIdx.x & 31;
+  part = __reduce_add_sync(0xffffffffu, part);
+  if (lane == 0) warp_sum[threadIdx.x >> 5] = part;
+  __syncthreads();
+  return __reduce_add_sync(0xffffffffu, warp_sum[lane]);
+}
+
+// The cell sort's scan knows the sorted state's counts, and makes its buffer the
+// current one: nothing but the reorder, which knows, reads it in between.
+__device__ __forceinline__ void sorted_counts(StepScalars* sc, int i, int len, int at) {
+  if (i == len - 2) sc->n_cells = at;  // len = bins + 2: the orphans' and the removed particles' segments come last
+  if (i == len - 1) {
+    sc->n_old = sc->n;
+    sc->n = at;
+    sc->buf ^= 1;
+  }
+}
+
+// Few blocks: each sums the entries before its own itself, so that one launch
+// does it (up to 16 blocks, 131,072 bins: the last one reads 480 KB, 3 us, where
+// a second launch costs as much).
+constexpr int kScanWhole = 16;
+__global__ void __launch_bounds__(1024) scan_whole(const int* __restrict__ in, int* __restrict__ out, int len,
+                                                   StepScalars* sc) {
+  if (sc && (sc->all_stop || !sc->rebuild)) return;  // the cell sort's scan, on a step without a rebuild
+  const int t = threadIdx.x, first = blockIdx.x * kScanBlock + t * kScanPer;
+  int before = 0;
+#pragma unroll 4
+  for (int i = t; i < (int)blockIdx.x * (kScanBlock / 4); i += 1024) {
+    const int4 q = reinterpret_cast<const int4*>(in)[i];
+    before += q.x + q.y + q.z + q.w;
+  }
+  int v[kScanPer], total;
+#pragma unroll
+  for (int e = 0; e < kScanPer; ++e) v[e] = (first + e < len) ? in[first + e] : 0;
+  before = block_sum(before);
+  int at = before + block_scan(v, &total);
+#pragma unroll
+  for (int e = 0; e < kScanPer; ++e) {
+    const int i = first + e;
+    if (i < len) {
+      out[i] = at;
+      if (sc) sorted_counts(sc, i, len, at);
+    }
+    at += v[e];
+  }
+  if (blockIdx.x == gridDim.x - 1 && t == 0) out[len] = before + total;
+}
+
+// Many blocks, phase 1: each block's own scan, its total to sums.
+__global__ void __launch_bounds__(1024) scan_blocks(const int* __restrict__ in, int* __restrict__ out,
+                                                    int* __restrict__ sums, int len, const StepScalars* sc) {
+  if (sc && (sc->all_stop || !sc->rebuild)) return;
+  const int first = blockIdx.x * kScanBlock + threadIdx.x * kScanPer;
+  int v[kScanPer], total;
+#pragma unroll
+  for (int e = 0; e < kScanPer; ++e) v[e] = (first + e < len) ? in[first + e] : 0;
+  int at = block_scan(v, &total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
 #pragma unroll
   for (int e = 0; e < kScanPer; ++e) {
     if (first + e < len) out[first + e] = at;
@@ -136,24 +198,20 @@ __global__ void __launch_bounds__(1024) scan_blocks(const int* __restrict__ in, 
 }
 
 // Phase 2: every block adds the totals of the blocks before it; the last one
-// writes the grand total. clear (if given): entries set to zero behind the scan.
+// writes the grand total.
 __global__ void __launch_bounds__(1024) scan_add(int* __restrict__ out, const int* __restrict__ sums, int len,
-                                                 int* __restrict__ clear, const StepScalars* sc) {
+                                                 StepScalars* sc) {
   if (sc && (sc->all_stop || !sc->rebuild)) return;
-  __shared__ int part[32];
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int t = threadIdx.x;
   int before = 0;
   for (int b = t; b < (int)blockIdx.x; b += 1024) before += sums[b];
-  before = __reduce_add_sync(0xffffffffu, before);
-  if (lane == 0) part[w] = before;
-  __syncthreads();
-  before = __reduce_add_sync(0xffffffffu, part[lane]);
-#pragma unroll
+  before = block_sum(before);
   for (int e = 0; e < kScanPer; ++e) {
     const int i = blockIdx.x * kScanBlock + e * 1024 + t;
     if (i < len) {
-      out[i] += before;
-      if (clear) clear[i] = 0;
+      const int at = out[i] + before;
+      out[i] = at;
+      if (sc) sorted_counts(sc, i, len, at);
     }
   }
   if (blockIdx.x == gridDim.x - 1 && t == 0) out[len] = before + sums[blockIdx.x];
@@ -161,98 +219,138 @@ __global__ void __launch_bounds__(1024) scan_add(int* __restrict__ out, const in
 
 inline int scan_blocks_for(int len) { return len > kScanBlock ? (len - 1) / kScanBlock + 1 : 1; }
 
-__global__ void scatter_kernel(const int* __restrict__ key, const int* __restrict__ start,
-                               const int* __restrict__ slot_of, int* __restrict__ tmp_perm, const StepScalars* sc) {
+void scan_launch(const int* in, int* out, int len, int* sums, StepScalars* sc, cudaStream_t st) {
+  const int nb = scan_blocks_for(len);
+  if (nb <= kScanWhole) {
+    scan_whole<<<nb, 1024, 0, st>>>(in, out, len, sc);
+  } else {
+    scan_blocks<<<nb, 1024, 0, st>>>(in, out, sums, len, sc);
+    scan_add<<<nb, 1024, 0, st>>>(out, sums, len, sc);
+  }
+}
+
+// Particles into their slots; and what the scan makes known: per-cell segment
+// starts from the bin starts (start[c] = sstart[c * 2 xsub] for c <= ncells, and
+// the orphan / dead / total boundaries after them), and the particles the
+// two-per-lane neighbour-list scan leaves to a lane of their own: lanes take
+// sorted particles 2t and 2t+1 together when they share a cell, so the odd
+// particles left are exactly the cells' first particles at odd indices (into
+// rest, at most cap). The counts are cleared for the next sort.
+__global__ void scatter_kernel(const int* __restrict__ key, const int* __restrict__ sstart,
+                               const int* __restrict__ slot_of, int* __restrict__ tmp_perm, int* __restrict__ count,
+                               int* __restrict__ start, int ncells, int xsub, StepScalars* sc,
+                               int* __restrict__ rest, int cap) {
   if (sc->all_stop || !sc->rebuild) return;
-  const int n = sc->n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    tmp_perm[start[key[i]] + slot_of[i]] = i;
+  const int n = sc->n_old;  // (the scan has counted the sorted state's n)
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31;
+  for (int i = tid; i < n; i += stride) tmp_perm[sstart[key[i]] + slot_of[i]] = i;
+  const size_t per = 2 * (size_t)xsub, nbins = per * ncells;
+  for (size_t i = tid; i < nbins + 2; i += stride) count[i] = 0;
+  for (int c0 = tid - lane; c0 < ncells + 3; c0 += stride) {
+    const int c = c0 + lane;
+    if (c <= ncells) start[c] = sstart[c * per];
+    else if (c <= ncells + 2) start[c] = sstart[nbins + (c - ncells)];
+    bool odd_first = false;
+    int s0 = 0;
+    if (c < ncells) {
+      s0 = sstart[c * per];
+      odd_first = (s0 & 1) && sstart[(c + 1) * per] > s0;
+    }
+    const unsigned want = __ballot_sync(0xffffffffu, odd_first);  // (c0 is the warp's)
+    if (odd_first) {  // one atomic per warp
+      const int leader = __ffs(want) - 1;
+      int base = 0;
+      if (lane == leader) base = atomicAdd(&sc->nl_rest, __popc(want));
+      base = __shfl_sync(want, base, leader);
+      const int slot = base + __popc(want & ((1u << lane) - 1u));
+      if (slot < cap) rest[slot] = s0;
+    }
+  }
 }
 
 // One thread per scattered particle i: its place s is its segment's start plus
 // the number of the segment's particles with a smaller original index; then its
 // fields move there (a solid's 3x3 tensors stay where they are: tensor_row).
-__global__ void reorder_kernel(DevView v, const int* __restrict__ tmp_perm, const int* __restrict__ key, const int* __restrict__ start, int* __restrict__ cellid,
-                               uint8_t* __restrict__ alive, const StepScalars* sc, int nbins, int xsub, int dyn_mu) {
+// With it go the FP32 offset from the cell's origin, an FP32C fluid's copies, and
+// the list of the fixed particles (written by warps of places that ascend, so
+// that a warp of the list lies close together).
+__global__ void __launch_bounds__(kBT) reorder_kernel(DevView v, const int* __restrict__ tmp_perm, const int* __restrict__ key, const int* __restrict__ start, int* __restrict__ cellid,
+                               uint8_t* __restrict__ alive, StepScalars* sc, int nbins, int xsub, int dyn_mu) {
   if (sc->all_stop || !sc->rebuild) return;
-  const Persist& src = cur_persist(v);
-  const Persist& dst = next_persist(v);
-  const int n_new = start[nbins + 1];  // the removed particles' segment comes last
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n_new; q += gridDim.x * blockDim.x) {
-    const int i = tmp_perm[q];
-    const int k = key[i];
-    const int lo = start[k], hi = start[k + 1];
-    const int mine = src.orig[i];
-    int s = lo;
-    for (int t = lo; t < hi; ++t) s += src.orig[tmp_perm[t]] < mine;
-    dst.X4[s] = src.X4[i];
-    dst.V4[s] = src.V4[i];
-    dst.H4[s] = src.H4[i];
-    if (src.H4b) dst.H4b[s] = src.H4b[i];
-    const int cls = src.cls[i];
-    dst.cls[s] = cls;
-    {
+  const Persist& src = next_persist(v);  // (the scan has made the sorted state's buffer the current one)
+  const Persist& dst = cur_persist(v);
+  const int n_new = sc->n;  // the removed particles' segment comes last
+  const bool fluid32 = v.o.fp32 && !v.o.has_solid;
+  const bool copies = fluid32 && v.o.skin == 0.f;  // (with a skin: skin_offsets_kernel)
+  const bool list_walls = fluid32 && v.o.dim == 2;
+  __shared__ int before[kBT / 32];  // walls of the block's warps before each
+  __shared__ int list_at;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int q0 = blockIdx.x * kBT; q0 < n_new; q0 += gridDim.x * kBT) {
+    const int q = q0 + threadIdx.x;
+    int wall = -1;  // this thread's particle, if fixed
+    if (q < n_new) {
+      const int i = tmp_perm[q];
+      const int k = key[i];
+      const int lo = start[k], hi = start[k + 1];
+      const int mine = src.orig[i];
+      int s = lo;
+      for (int t = lo; t < hi; ++t) s += src.orig[tmp_perm[t]] < mine;
+      const double4_32a xs = src.X4[i], vs = src.V4[i];
+      dst.X4[s] = xs;
+      dst.V4[s] = vs;
+      dst.H4[s] = src.H4[i];
+      if (src.H4b) dst.H4b[s] = src.H4b[i];
+      const int cls = src.cls[i];
+      dst.cls[s] = cls;
+      if (dyn_mu) dst.mu[s] = src.mu[i];
+      const bool is_free = v.cls[cls].is_free;
       // FP32 offset from the cell origin (absolute position outside any cell)
-      const double4_32a xs = src.X4[i];
-      const float h = v.cls[cls].is_free ? d2f_rn(v.cls[cls].h) : -d2f_rn(v.cls[cls].h);
+      const float h = is_free ? d2f_rn(v.cls[cls].h) : -d2f_rn(v.cls[cls].h);
+      float4 off;
       if (k < nbins) {
         const GridDev& g = grid_of(v, v.cls[cls].inst);
         const int lk = k / (2 * xsub) - g.cell_base;
         const int cx = lk % g.nc[0], t = lk / g.nc[0], cy = t % g.nc[1], cz = t / g.nc[1];
-        v.S.OFF32[s] = make_float4(d2f_rn(xs.x - (g.blpf[0] + i2d_small(cx) * g.cell_size[0])),
-                                   d2f_rn(xs.y - (g.blpf[1] + i2d_small(cy) * g.cell_size[1])),
-                                   v.o.dim == 3 ? d2f_rn(xs.z - (g.blpf[2] + i2d_small(cz) * g.cell_size[2])) : 0.f, h);
+        off = make_float4(d2f_rn(xs.x - (g.blpf[0] + i2d_small(cx) * g.cell_size[0])),
+                          d2f_rn(xs.y - (g.blpf[1] + i2d_small(cy) * g.cell_size[1])),
+                          v.o.dim == 3 ? d2f_rn(xs.z - (g.blpf[2] + i2d_small(cz) * g.cell_size[2])) : 0.f, h);
       } else {
-        v.S.OFF32[s] = make_float4(d2f_rn(xs.x), d2f_rn(xs.y), d2f_rn(xs.z), h);
+        off = make_float4(d2f_rn(xs.x), d2f_rn(xs.y), d2f_rn(xs.z), h);
       }
+      v.S.OFF32[s] = off;
       if (v.o.skin > 0.f)  // displacements are measured from here (FP32, truncated)
         v.S.OFFREF[s] = make_float4(d2f_bits(xs.x), d2f_bits(xs.y), d2f_bits(xs.z), 0.f);
+      if (copies) fluid_copies32(v, dst, s, cls, xs.w, vs, off, 0);
+      dst.orig[s] = mine;
+      if (src.io) dst.io[s] = src.io[i];
+      cellid[s] = (k < nbins) ? k / (2 * xsub) : -1;
+      alive[s] = 1;
+      if (!is_free) wall = s;
     }
-    dst.orig[s] = mine;
-    if (src.io) dst.io[s] = src.io[i];
-    cellid[s] = (k < nbins) ? k / (2 * xsub) : -1;
-    alive[s] = 1;
-    if (dyn_mu) dst.mu[s] = src.mu[i];
+    if (!list_walls) continue;
+    // the block's walls, by one atomic: parts of some hundred in sorted order
+    const unsigned m = __ballot_sync(0xffffffffu, wall >= 0);
+    if (lane == 0) before[warp] = __popc(m);
+    if (__syncthreads_or(m != 0) == 0) continue;
+    if (threadIdx.x == 0) {
+      int sum = 0;
+      for (int w = 0; w < kBT / 32; ++w) {
+        const int c = before[w];
+        before[w] = sum;
+        sum += c;
+      }
+      list_at = atomicAdd(&sc->n_walls, sum);
+    }
+    __syncthreads();
+    if (wall >= 0) v.S.walls[list_at + before[warp] + __popc(m & ((1u << lane) - 1u))] = wall;
+    __syncthreads();
   }
 }
 
-// Per-cell segment starts from the bin starts: start[c] = sstart[c * 2 xsub] for
-// c <= ncells, and the orphan / dead / total boundaries after them; the sorted
-// state's counts and buffer. Also lists the particles the two-per-lane
-// neighbour-list scan leaves to a lane of their own: lanes take sorted particles
-// 2t and 2t+1 together when they share a cell, so the odd particles left are
-// exactly the cells' first particles at odd indices (into rest, at most cap).
-__global__ void cell_starts_kernel(const int* __restrict__ sstart, int* __restrict__ start, int ncells, int xsub,
-                                   StepScalars* sc, int* __restrict__ rest, int cap) {
-  if (sc->all_stop || !sc->rebuild) return;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t per = 2 * (size_t)xsub, nbins = per * ncells;
-  if (c <= ncells) start[c] = sstart[c * per];
-  else if (c <= ncells + 2) start[c] = sstart[nbins + (c - ncells)];
-  if (c == 0) {
-    sc->n_cells = sstart[nbins];
-    sc->n = sstart[nbins + 1];
-    sc->buf ^= 1;
-  }
-  bool odd_first = false;
-  int s0 = 0;
-  if (c < ncells) {
-    s0 = sstart[c * per];
-    odd_first = (s0 & 1) && sstart[(c + 1) * per] > s0;
-  }
-  const unsigned want = __ballot_sync(0xffffffffu, odd_first);  // every lane of the grid gets here
-  if (odd_first) {  // one atomic per warp
-    const int lane = threadIdx.x & 31, leader = __ffs(want) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(&sc->nl_rest, __popc(want));
-    base = __shfl_sync(want, base, leader);
-    const int slot = base + __popc(want & ((1u << lane) - 1u));
-    if (slot < cap) rest[slot] = s0;
-  }
-}
-
-// Neighbour lists with a skin: on every step the FP32 offsets of the
-// particles from their cells' origins (the cells of the last rebuild), and
+// Neighbour lists with a skin: on every step an FP32C fluid's copies, the FP32
+// offsets of the particles from their cells' origins (the cells of the last rebuild), and
 // each particle's cell in the reference's grid (ListGenerate's floor and
 // clamp on the FP64 position, Source/Domain.cpp:669-691), which orients the
 // wall pressure's pairs as the reference's neighbour search does.
@@ -266,16 +364,18 @@ __global__ void skin_offsets_kernel(DevView v) {
   const double4_32a xs = P.X4[s];
   const float h = C.is_free ? d2f_rn(C.h) : -d2f_rn(C.h);
   const int cell = v.S.cellid[s];
+  float4 off;
   if (cell >= 0) {
     const GridDev& g = grid_of(v, C.inst);
     const int lk = cell - g.cell_base;
     const int cx = lk % g.nc[0], t = lk / g.nc[0], cy = t % g.nc[1], cz = t / g.nc[1];
-    v.S.OFF32[s] = make_float4(d2f_rn(xs.x - (g.blpf[0] + i2d_small(cx) * g.cell_size[0])),
-                               d2f_rn(xs.y - (g.blpf[1] + i2d_small(cy) * g.cell_size[1])),
-                               v.o.dim == 3 ? d2f_rn(xs.z - (g.blpf[2] + i2d_small(cz) * g.cell_size[2])) : 0.f, h);
+    off = make_float4(d2f_rn(xs.x - (g.blpf[0] + i2d_small(cx) * g.cell_size[0])),
+                      d2f_rn(xs.y - (g.blpf[1] + i2d_small(cy) * g.cell_size[1])),
+                      v.o.dim == 3 ? d2f_rn(xs.z - (g.blpf[2] + i2d_small(cz) * g.cell_size[2])) : 0.f, h);
   } else {
-    v.S.OFF32[s] = make_float4(d2f_rn(xs.x), d2f_rn(xs.y), d2f_rn(xs.z), h);
+    off = make_float4(d2f_rn(xs.x), d2f_rn(xs.y), d2f_rn(xs.z), h);
   }
+  v.S.OFF32[s] = off;
   const GridDev& r = v.grids_ref[C.inst];
   const double xd[3] = {xs.x, xs.y, xs.z};
   int q[3] = {0, 0, 0};
@@ -283,7 +383,9 @@ __global__ void skin_offsets_kernel(DevView v) {
     const int k = cell_floor(r, d, xd[d]);
     q[d] = min(max(k, 0), r.cn_ref[d] - 1);  // clamped as ListGenerate clamps the particles just outside
   }
-  v.S.refcell[s] = q[0] | (q[1] << 10) | (q[2] << 20);
+  const int rc = q[0] | (q[1] << 10) | (q[2] << 20);
+  v.S.refcell[s] = rc;
+  if (v.o.fp32 && !v.o.has_solid) fluid_copies32(v, P, s, P.cls[s], xs.w, P.V4[s], off, rc);
 }
 
 // now: the next cell sort runs (a sort outside the step loop); next_step:
@@ -320,14 +422,14 @@ void launch_sort(const DevView& v, cudaStream_t st) {
   const int gp = v.o.skin > 0.f ? std::min(grid_for(v.ncap), 4096) : grid_for(v.ncap);
   // S.count is zero here (allocated so, and cleared behind every scan)
   bin_kernel<<<gp, kBT, 0, st>>>(v, v.alive, S.key, S.count, S.slot, v.sc, v.o.dim, xsub);
-  const int nb = scan_blocks_for(len);
-  scan_blocks<<<nb, 1024, 0, st>>>(S.count, S.sstart, S.block_sums, len, v.sc);
-  scan_add<<<nb, 1024, 0, st>>>(S.sstart, S.block_sums, len, S.count, v.sc);
-  scatter_kernel<<<gp, kBT, 0, st>>>(S.key, S.sstart, S.slot, S.tmp_perm, v.sc);
+  scan_launch(S.count, S.sstart, len, S.block_sums, v.sc, st);
+  scatter_kernel<<<gp, kBT, 0, st>>>(S.key, S.sstart, S.slot, S.tmp_perm, S.count, S.start, ncells, xsub, v.sc, S.rest,
+                                     v.ncap);
   reorder_kernel<<<gp, kBT, 0, st>>>(v, S.tmp_perm, S.key, S.sstart, S.cellid, v.alive, v.sc, nbins, xsub,
                                      v.o.dyn_mu);
-  cell_starts_kernel<<<grid_for(ncells + 3), kBT, 0, st>>>(S.sstart, S.start, ncells, xsub, v.sc, S.tmp_perm, v.ncap);
 }
+
+int sort_launches(const DevView& v) { return scan_blocks_for(2 * v.total_cells * v.o.xsub + 2) <= kScanWhole ? 4 : 5; }
 
 }  // namespace psph
 
@@ -337,9 +439,7 @@ namespace psph {
 // block_sums (>= ceil(len/1024) entries) as scratch. Used by the pair export
 // that takes its scratch from caller-owned or static device memory.
 void launch_exclusive_scan(const int* in, int* out, int len, int* block_sums, cudaStream_t st) {
-  const int nb = scan_blocks_for(len);
-  scan_blocks<<<nb, 1024, 0, st>>>(in, out, block_sums, len, nullptr);
-  scan_add<<<nb, 1024, 0, st>>>(out, block_sums, len, nullptr, nullptr);
+  scan_launch(in, out, len, block_sums, nullptr, st);
 }
 
 }  // namespace psph

@@ -514,8 +514,6 @@ void launch_update(const DevView& v, cudaStream_t st) {
   }
 }
 
-// begin, bin, 2 scan, scatter, reorder, cell starts, neighbour lists, prepare (2 in the FP32C form: copies + walls),
-// forces, closure, dt, update, end
 namespace {
 __global__ void class_constants_kernel(PClass* cls, int n, int dim) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -562,9 +560,10 @@ void launch_upload_pack(const double* sx, const double* sd, const double* sp, co
 }
 
 int launches_per_step(const DevView& v) {
-  return (v.o.fp32 ? 14 : 13) + (v.o.closure ? 1 : 0) + (v.o.fp64_half ? 1 : 0) +
-         (v.o.mixed ? 2 : 0) + (v.o.couple_soil && v.o.swi != 2 ? 2 : 0) + (v.o.fsi ? 1 : 0) +
-         (v.o.skin > 0.f ? 1 : 0);
+  // begin, sort, neighbour lists, prepare, forces, dt, update, end
+  return 7 + sort_launches(v) + (v.o.fp32 && v.o.has_solid && !v.o.soil32 ? 1 : 0) + (v.o.closure ? 1 : 0) +
+         (v.o.fp64_half ? 1 : 0) + (v.o.mixed ? 2 : 0) + (v.o.couple_soil && v.o.swi != 2 ? 2 : 0) +
+         (v.o.fsi ? 1 : 0) + (v.o.skin > 0.f ? 1 : 0);
 }
 
 }  // namespace psph
