@@ -34,7 +34,7 @@ struct Scratch {
   int* count;      // ncells + 2 counters
   int* start;      // ncells + 3 exclusive prefix: cell c's particles are [start[c], start[c+1])
   int* sstart;     // 2 ncells * xsub + 3 exclusive prefix over the x-slabs of the cells, free and fixed apart
-  int* tmp_perm;
+  int2* tmp_perm;  // scattered particles: (place before the sort, original index)
   int* slot;       // a particle's place in its segment before the ranking
   int* walls;      // the fixed particles, in nearly sorted order (the same memory as slot, whose use is over)
   int* rest;       // the particles the neighbour-list scan handles one per lane
@@ -155,6 +155,7 @@ struct Options {
   double mu_u;        // that viscosity
   double inv_h;       // 1/h when uniform
   int nl_cap;         // neighbour-list capacity per particle
+  int fused_tail;     // the update takes the time step from the dt minimum and ends the step itself
   int list_all;       // fixed particles' lists hold fixed candidates too (a hook may have freed some of them)
   int pair_block;     // threads per block of the FP32C pair kernels (psph_autotune)
   int xsub;           // x-slabs per cell in the sort (1, 2 or 4; psph_autotune)
@@ -217,6 +218,45 @@ PSPH_D void widen_rates(const float4* __restrict__ q, double* __restrict__ sr, d
   rr[0] = 0.0; rr[1] = b.z; rr[2] = b.w;
   rr[3] = -(double)b.z; rr[4] = 0.0; rr[5] = c.x;
   rr[6] = -(double)b.w; rr[7] = -(double)c.x; rr[8] = 0.0;
+}
+
+// LastComputeAcceleration's minimum (Source/Domain.cpp:1280-1296) and
+// AdaptiveTimeStep (Source/Domain.cpp:133-152) of an instance.
+struct StepDt {
+  double deltat, deltatmin;
+  bool collapse;  // the reference throws here (Source/Domain.cpp:150-151)
+};
+PSPH_D StepDt adaptive_dt(const InstState& I) {
+  const double m = __longlong_as_double((long long)I.dtmin_bits);
+  double dtmin = I.deltatint;
+  if (dtmin > m) dtmin = m;
+  double dt = I.deltat;
+  const double dti = I.deltatint;
+  if (dti > dtmin) dt = (dt < dtmin) ? 2.0 * dt * dtmin / (dt + dtmin) : dtmin;
+  else dt = (dti != dt) ? 2.0 * dt * dti / (dt + dti) : dti;
+  return {dt, dtmin, dt < (dti / 1.0e5)};
+}
+PSPH_D void store_dt(InstState& I, const StepDt& d, StepScalars* sc) {
+  I.deltatmin = d.deltatmin;
+  I.deltat = d.deltat;
+  I.dt2 = 2.0 * d.deltat;
+  I.half_dt2 = 0.5 * d.deltat * d.deltat;
+  if (d.collapse) {
+    atomicOr(&sc->status, ST_DT_COLLAPSE);
+    I.stop = 1;
+  }
+}
+// End of step: Time += deltat and the per-particle counters, once per instance.
+PSPH_D void end_step(InstState& I, const Options& o) {
+  if (I.stop) return;
+  I.time += I.deltat;
+  I.steps += 1;
+  if (o.scheme == PSPH_MVERLET) {
+    I.ct = (I.ct == 30) ? 0 : I.ct + 1;
+    I.shepard_counter = (I.shepard_counter == o.shepard_step) ? 0 : I.shepard_counter + 1;
+  }
+  I.first_step = 0;
+  I.k_initial = 0;
 }
 
 // Launch wrappers (defined in the .cu files).

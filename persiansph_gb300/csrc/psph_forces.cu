@@ -1176,30 +1176,11 @@ __global__ void __launch_bounds__(kFT) forces_solid_kernel(DevView v, int lg) {
 }
 
 // Per-instance step control, one block looping over the instances.
-// dt: LastComputeAcceleration's minimum (Source/Domain.cpp:1280-1296) and
-// AdaptiveTimeStep (Source/Domain.cpp:133-152).
 __global__ void dt_finalize_kernel(DevView v) {
   StepScalars* sc = v.sc;
   if (sc->all_stop) return;
-  for (int k = threadIdx.x; k < v.ninst; k += blockDim.x) {
-    InstState& I = v.inst[k];
-    if (I.stop) continue;
-    const double m = __longlong_as_double((long long)I.dtmin_bits);
-    double dtmin = I.deltatint;
-    if (dtmin > m) dtmin = m;
-    I.deltatmin = dtmin;
-    double dt = I.deltat;
-    const double dti = I.deltatint;
-    if (dti > dtmin) dt = (dt < dtmin) ? 2.0 * dt * dtmin / (dt + dtmin) : dtmin;
-    else dt = (dti != dt) ? 2.0 * dt * dti / (dt + dti) : dti;
-    I.deltat = dt;
-    I.dt2 = 2.0 * dt;
-    I.half_dt2 = 0.5 * dt * dt;
-    if (dt < (dti / 1.0e5)) {
-      atomicOr(&sc->status, ST_DT_COLLAPSE);
-      I.stop = 1;  // the reference throws here (Source/Domain.cpp:150-151)
-    }
-  }
+  for (int k = threadIdx.x; k < v.ninst; k += blockDim.x)
+    if (!v.inst[k].stop) store_dt(v.inst[k], adaptive_dt(v.inst[k]), sc);
 }
 
 // Begin of step: Solve's `Time < tf` test per instance, Move_MVerlet's
@@ -1231,21 +1212,9 @@ __global__ void begin_kernel(DevView v) {
   }
 }
 
-// End of step: Time += deltat and the per-particle counters, once per instance.
 __global__ void end_kernel(DevView v) {
   if (v.sc->all_stop) return;
-  for (int k = threadIdx.x; k < v.ninst; k += blockDim.x) {
-    InstState& I = v.inst[k];
-    if (I.stop) continue;
-    I.time += I.deltat;
-    I.steps += 1;
-    if (v.o.scheme == PSPH_MVERLET) {
-      I.ct = (I.ct == 30) ? 0 : I.ct + 1;
-      I.shepard_counter = (I.shepard_counter == v.o.shepard_step) ? 0 : I.shepard_counter + 1;
-    }
-    I.first_step = 0;
-    I.k_initial = 0;
-  }
+  for (int k = threadIdx.x; k < v.ninst; k += blockDim.x) end_step(v.inst[k], v.o);
 }
 
 // Pair export: candidate (which=0) or in-support (which=1) pairs in reference
@@ -1762,11 +1731,15 @@ void launch_coupling(const DevView& v, cudaStream_t st) { by_dim_kernel<Coupling
 
 void launch_fsi(const DevView& v, cudaStream_t st) { by_dim_kernel<FsiLaunch>(v, st); }
 
-void launch_dt(const DevView& v, cudaStream_t st) { dt_finalize_kernel<<<1, 256, 0, st>>>(v); }
+void launch_dt(const DevView& v, cudaStream_t st) {
+  if (!v.o.fused_tail) dt_finalize_kernel<<<1, 256, 0, st>>>(v);
+}
 
 void launch_begin(const DevView& v, cudaStream_t st) { begin_kernel<<<1, 256, 0, st>>>(v); }
 
-void launch_end(const DevView& v, cudaStream_t st) { end_kernel<<<1, 256, 0, st>>>(v); }
+void launch_end(const DevView& v, cudaStream_t st) {
+  if (!v.o.fused_tail) end_kernel<<<1, 256, 0, st>>>(v);
+}
 
 void launch_pairs_export(const DevView& v, int which, long long* out, long long cap, unsigned long long* counter,
                          cudaStream_t st) {

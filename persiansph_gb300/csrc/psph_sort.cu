@@ -229,22 +229,24 @@ void scan_launch(const int* in, int* out, int len, int* sums, StepScalars* sc, c
   }
 }
 
-// Particles into their slots; and what the scan makes known: per-cell segment
+// Particles into their slots, each with its original index (which the reorder ranks
+// by: a read of it through the slot was a second wait per member); and what the scan makes known: per-cell segment
 // starts from the bin starts (start[c] = sstart[c * 2 xsub] for c <= ncells, and
 // the orphan / dead / total boundaries after them), and the particles the
 // two-per-lane neighbour-list scan leaves to a lane of their own: lanes take
 // sorted particles 2t and 2t+1 together when they share a cell, so the odd
 // particles left are exactly the cells' first particles at odd indices (into
 // rest, at most cap). The counts are cleared for the next sort.
-__global__ void scatter_kernel(const int* __restrict__ key, const int* __restrict__ sstart,
-                               const int* __restrict__ slot_of, int* __restrict__ tmp_perm, int* __restrict__ count,
+__global__ void scatter_kernel(DevView v, const int* __restrict__ key, const int* __restrict__ sstart,
+                               const int* __restrict__ slot_of, int2* __restrict__ tmp_perm, int* __restrict__ count,
                                int* __restrict__ start, int ncells, int xsub, StepScalars* sc,
                                int* __restrict__ rest, int cap) {
   if (sc->all_stop || !sc->rebuild) return;
   const int n = sc->n_old;  // (the scan has counted the sorted state's n)
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
-  for (int i = tid; i < n; i += stride) tmp_perm[sstart[key[i]] + slot_of[i]] = i;
+  const int* __restrict__ orig = next_persist(v).orig;  // (the scan has made the sorted state's buffer the current one)
+  for (int i = tid; i < n; i += stride) tmp_perm[sstart[key[i]] + slot_of[i]] = make_int2(i, orig[i]);
   const size_t per = 2 * (size_t)xsub, nbins = per * ncells;
   for (size_t i = tid; i < nbins + 2; i += stride) count[i] = 0;
   for (int c0 = tid - lane; c0 < ncells + 3; c0 += stride) {
@@ -275,7 +277,7 @@ __global__ void scatter_kernel(const int* __restrict__ key, const int* __restric
 // With it go the FP32 offset from the cell's origin, an FP32C fluid's copies, and
 // the list of the fixed particles (written by warps of places that ascend, so
 // that a warp of the list lies close together).
-__global__ void __launch_bounds__(kBT) reorder_kernel(DevView v, const int* __restrict__ tmp_perm, const int* __restrict__ key, const int* __restrict__ start, int* __restrict__ cellid,
+__global__ void __launch_bounds__(kBT) reorder_kernel(DevView v, const int2* __restrict__ tmp_perm, const int* __restrict__ key, const int* __restrict__ start, int* __restrict__ cellid,
                                uint8_t* __restrict__ alive, StepScalars* sc, int nbins, int xsub, int dyn_mu) {
   if (sc->all_stop || !sc->rebuild) return;
   const Persist& src = next_persist(v);  // (the scan has made the sorted state's buffer the current one)
@@ -291,12 +293,12 @@ __global__ void __launch_bounds__(kBT) reorder_kernel(DevView v, const int* __re
     const int q = q0 + threadIdx.x;
     int wall = -1;  // this thread's particle, if fixed
     if (q < n_new) {
-      const int i = tmp_perm[q];
+      const int2 own = tmp_perm[q];
+      const int i = own.x, mine = own.y;
       const int k = key[i];
       const int lo = start[k], hi = start[k + 1];
-      const int mine = src.orig[i];
       int s = lo;
-      for (int t = lo; t < hi; ++t) s += src.orig[tmp_perm[t]] < mine;
+      for (int t = lo; t < hi; ++t) s += tmp_perm[t].y < mine;
       const double4_32a xs = src.X4[i], vs = src.V4[i];
       dst.X4[s] = xs;
       dst.V4[s] = vs;
@@ -423,7 +425,7 @@ void launch_sort(const DevView& v, cudaStream_t st) {
   // S.count is zero here (allocated so, and cleared behind every scan)
   bin_kernel<<<gp, kBT, 0, st>>>(v, v.alive, S.key, S.count, S.slot, v.sc, v.o.dim, xsub);
   scan_launch(S.count, S.sstart, len, S.block_sums, v.sc, st);
-  scatter_kernel<<<gp, kBT, 0, st>>>(S.key, S.sstart, S.slot, S.tmp_perm, S.count, S.start, ncells, xsub, v.sc, S.rest,
+  scatter_kernel<<<gp, kBT, 0, st>>>(v, S.key, S.sstart, S.slot, S.tmp_perm, S.count, S.start, ncells, xsub, v.sc, S.rest,
                                      v.ncap);
   reorder_kernel<<<gp, kBT, 0, st>>>(v, S.tmp_perm, S.key, S.sstart, S.cellid, v.alive, v.sc, nbins, xsub,
                                      v.o.dyn_mu);

@@ -1,7 +1,9 @@
-"""The two-particle list scan walks a row's three cells in groups of four
-candidates, the last group of a cell partly masked: cells of every fill from
-empty upwards (a shaken lattice), cell splits, the staged copy, and a tall
-support, one step against the oracle at the FP64 form's parity bound."""
+"""The neighbour-list scans on cells of every fill from empty upwards (a shaken
+lattice), one step against the oracle at the FP64 form's parity bound: a lane to
+a cell (few particles), the walk of a row's three cells in groups of four with
+the last of a cell partly masked (many, or the staged copy), cell splits, a tall
+support, cells fuller than a lane's bits, and a grid whose bins take more than
+one launch to scan."""
 import numpy as np
 import pytest
 
@@ -13,6 +15,29 @@ from tests.gpu_helpers import assert_step_parity
 pytestmark = pytest.mark.gpu
 
 
+def shaken(p, dx, dim, by=0.6, seed=7):
+    rng = np.random.default_rng(seed)
+    free = p.get("is_free") != 0
+    x = p.get("x")
+    x[free, :dim] += by * dx * (rng.random((int(free.sum()), dim)) - 0.5)
+    p.set("x", x)
+
+
+def one_step(dom, dt, label, tuning=None):
+    cfg = dom.config(dt)
+    o = OracleDomain(cfg, dom.particles, initial=True)
+    gd = GpuDomain(cfg)
+    gd.upload(dom.particles)
+    if tuning:
+        gd.set_tuning(128, *tuning)
+    assert set(map(tuple, gd.pairs(1).tolist())) == set(map(tuple, o.pairs(3).tolist()))
+    o.step(1)
+    gd.step(1)
+    a_scale, dr_scale = o.scales()
+    assert_step_parity(gd.download_fields(), o.download(), a_scale, dr_scale, dt, label=label)
+    gd.close()
+
+
 @pytest.mark.parametrize("split,stage", [(1, 0), (2, 0), (4, 0), (1, 3072), (4, 4096)])
 @pytest.mark.parametrize("dim,hfac", [(2, 1.2), (2, 2.2), (3, 1.3)])
 def test_shaken_lattice(gpu, dim, hfac, split, stage):
@@ -21,20 +46,33 @@ def test_shaken_lattice(gpu, dim, hfac, split, stage):
         dom, dt, _ = scenarios.dam_break_2d(dx=dx, L=0.5, H=0.65, TL=1.0, TH=0.8, hfac=hfac)
     else:
         dom, dt, _ = scenarios.dam_break_3d(dx=dx, L=0.3, H=0.35, W=0.25, TL=0.5, TH=0.4, TW=0.25, hfac=hfac)
-    p = dom.particles
-    rng = np.random.default_rng(7)
-    free = p.get("is_free") != 0
-    x = p.get("x")
-    x[free, :dim] += 0.6 * dx * (rng.random((int(free.sum()), dim)) - 0.5)
-    p.set("x", x)
-    cfg = dom.config(dt)
-    o = OracleDomain(cfg, p, initial=True)
-    gd = GpuDomain(cfg)
-    gd.upload(p)
-    gd.set_tuning(128, split, stage)
-    assert set(map(tuple, gd.pairs(1).tolist())) == set(map(tuple, o.pairs(3).tolist()))
-    o.step(1)
-    gd.step(1)
-    a_scale, dr_scale = o.scales()
-    assert_step_parity(gd.download_fields(), o.download(), a_scale, dr_scale, dt, label=f"{dim}D {hfac} {split} {stage}")
-    gd.close()
+    shaken(dom.particles, dx, dim)
+    one_step(dom, dt, f"{dim}D {hfac} {split} {stage}", (split, stage))
+
+
+@pytest.mark.parametrize("dim,split", [(2, 1), (2, 4), (3, 1), (3, 4)])
+def test_more_than_the_lanes_to_a_cell(gpu, dim, split):
+    if dim == 2:
+        dx = 0.01
+        dom, dt, _ = scenarios.dam_break_2d(dx=dx, L=1.2, H=1.6, TL=2.0, TH=2.0)
+    else:
+        dx = 0.03
+        dom, dt, _ = scenarios.dam_break_3d(dx=dx, L=0.7, H=0.5, W=0.6, TL=1.0, TH=0.6, TW=0.6)
+    assert dom.particles.n > 152 * 2048 >> (4 if dim == 2 else 5)
+    shaken(dom.particles, dx, dim)
+    one_step(dom, dt, f"{dim}D split {split}", (split, 0))
+
+
+def test_cells_fuller_than_a_lanes_bits(gpu):
+    dx = 0.05
+    dom, dt, _ = scenarios.dam_break_2d(dx=dx, L=1.0, H=1.0, TL=1.4, TH=1.2, hfac=4.5)  # 9 x 9 particles to a cell
+    shaken(dom.particles, dx, 2, 0.2)
+    one_step(dom, dt, "full cells")
+
+
+@pytest.mark.parametrize("split", [1, 4])
+def test_sparse_grid(gpu, split):
+    dx = 0.05
+    dom, dt, _ = scenarios.dam_break_2d(dx=dx, L=0.5, H=0.65, TL=16.5, TH=16.5)
+    shaken(dom.particles, dx, 2)
+    one_step(dom, dt, f"sparse {split}", (split, 0))
