@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -44,10 +45,18 @@ namespace {
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float sigm(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float silu(float z) { return z * sigm(z); }
-__device__ __forceinline__ float dsilu(float z) {
-  const float s = sigm(z);
-  return s * (1.f + z * (1.f - s));
+// The same sigmoid for the training epilogues, which evaluate 64 a thread in a
+// row: the division's special cases are a branch that keeps them one after the
+// other. The reciprocal here is the hardware's estimate and one Newton step
+// (within 1e-6 ulp of half an ulp); past 8e37 (z < -87) it is zero.
+__device__ __forceinline__ float sigm_row(float z) {
+  const float x = 1.f + expf(-z);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fminf(x, 8e37f)));
+  r = fmaf(fmaf(-x, r, 1.f), r, r);
+  return x < 8e37f ? r : (x == x ? 0.f : x);
 }
+__device__ __forceinline__ float dsilu_of(float z, float s) { return s * (1.f + z * (1.f - s)); }
 // SiLU of the tensor-core inference epilogues: hardware exp2 and reciprocal
 // approximations (relative error ~1e-6, far below the BF16 rounding of the
 // activations that follows). z is clamped at -80 so 1 + exp(-z) stays a
@@ -500,59 +509,60 @@ constexpr int kTrainThreads = 128;
 // samples: part[chunk][param] (W2 and W3 come from the tensor cores). Threads
 // of a warp take consecutive parameters, so the activation reads of a weight
 // row are contiguous.
-__global__ void train_wgrad_kernel(const float* __restrict__ U, const float* __restrict__ Z1,
-                                   const float* __restrict__ Z2, const float* __restrict__ Z3,
-                                   const float* __restrict__ G4, const float* __restrict__ D1,
-                                   const float* __restrict__ D2, const float* __restrict__ D3, int B, int chunk,
-                                   float* part) {
-  const int pidx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pidx >= kNParams) return;
-  const int b0 = blockIdx.y * chunk, b1 = min(B, b0 + chunk);
+// Bound by the wait for the loads: 16 samples' go out together, the sums keep the
+// samples' order (a load at a time, and silu's division between them, took 66 us for 4,096
+// samples, this 14).
+constexpr int kWgParams = kMlpH * kMlpIn + 4 * kMlpH + 1;  // W1, B1, B2, B3, W4, B4
+
+// acc += f(0) + f(1) + ... in order, the loads of 16 ahead of their sums
+template <class F>
+__device__ __forceinline__ float sum_in_order(int n, F&& f) {
   float acc = 0.f;
-  if (pidx < kOB1) {
-    const int nn = pidx / kMlpIn, k = pidx % kMlpIn;
-    for (int b = b0; b < b1; ++b) acc += D1[(size_t)kMlpH * b + nn] * U[(size_t)8 * b + k];
-  } else if (pidx < kOW2) {
-    const int nn = pidx - kOB1;
-    for (int b = b0; b < b1; ++b) acc += D1[(size_t)kMlpH * b + nn];
-  } else if (pidx < kOB2) {  // W2: the tensor-core partials
-  } else if (pidx < kOW3) {
-    const int nn = pidx - kOB2;
-    for (int b = b0; b < b1; ++b) acc += D2[(size_t)kMlpH * b + nn];
-  } else if (pidx < kOB3) {  // W3: the tensor-core partials
-  } else if (pidx < kOW4) {
-    const int nn = pidx - kOB3;
-    for (int b = b0; b < b1; ++b) acc += D3[(size_t)kMlpH * b + nn];
-  } else if (pidx < kOB4) {
-    const int k = pidx - kOW4;
-    for (int b = b0; b < b1; ++b) acc += G4[b] * silu(Z3[(size_t)kMlpH * b + k]);
-  } else {
-    for (int b = b0; b < b1; ++b) acc += G4[b];
+  int i = 0;
+  for (; i + 16 <= n; i += 16) {
+    float2 q[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) q[e] = f(i + e);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) acc = fmaf(q[e].x, q[e].y, acc);
   }
-  part[(size_t)blockIdx.y * kNParams + pidx] = acc;
+  for (; i < n; ++i) {
+    const float2 q = f(i);
+    acc = fmaf(q.x, q.y, acc);
+  }
+  return acc;
 }
 
-// Sums the per-chunk partials of the CUDA-core parameters and, for W2 and W3,
-// the per-CTA tensor-core partials (mma[cta][0] = dW3, mma[cta][1] = dW2, row =
-// output unit, column = input unit), each in a fixed order.
-__global__ void train_reduce_kernel(const float* __restrict__ part, int nchunks, const float* __restrict__ mma,
-                                    int nctas, float* grad) {
-  const int pidx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pidx >= kNParams) return;
-  float s = 0.f;
-  const bool w2 = pidx >= kOW2 && pidx < kOB2, w3 = pidx >= kOW3 && pidx < kOB3;
-  if (w2 || w3) {
-    const int q = w2 ? pidx - kOW2 : pidx - kOW3;
-    for (int c = 0; c < nctas; ++c) s += mma[((size_t)c * 2 + (w2 ? 1 : 0)) * kMlpH * kMlpH + q];
-  } else {
-    for (int c = 0; c < nchunks; ++c) s += part[(size_t)c * kNParams + pidx];
+__global__ void __launch_bounds__(128) train_wgrad_kernel(
+    const float* __restrict__ U, const float* __restrict__ A3, const float* __restrict__ G4,
+    const float* __restrict__ D1, const float* __restrict__ D2, const float* __restrict__ D3, int B, int chunk,
+    float* __restrict__ part) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= kWgParams) return;
+  const size_t b0 = (size_t)blockIdx.y * chunk;
+  const int n = min(B - (int)b0, chunk);
+  float* out = part + (size_t)blockIdx.y * kNParams;
+  if (t < kMlpH * kMlpIn) {
+    const float* d = D1 + kMlpH * b0 + t / kMlpIn;
+    const float* u = U + 8 * b0 + t % kMlpIn;
+    out[kOW1 + t] = sum_in_order(n, [&](int i) { return make_float2(d[kMlpH * i], u[8 * i]); });
+    return;
   }
-  grad[pidx] = s;
+  const int q = t - kMlpH * kMlpIn, k = q % kMlpH;
+  if (q < 3 * kMlpH) {  // the biases of the three layers
+    const int layer = q / kMlpH;
+    const float* d = (layer == 0 ? D1 : layer == 1 ? D2 : D3) + kMlpH * b0 + k;
+    const float s = sum_in_order(n, [&](int i) { return make_float2(d[kMlpH * i], 1.f); });
+    out[(layer == 0 ? kOB1 : layer == 1 ? kOB2 : kOB3) + k] = s;
+  } else if (q < 4 * kMlpH) {
+    const float *g = G4 + b0, *z = A3 + kMlpH * b0 + k;
+    out[kOW4 + k] = sum_in_order(n, [&](int i) { return make_float2(g[i], z[kMlpH * i]); });
+  } else {
+    const float* g = G4 + b0;
+    out[kOB4] = sum_in_order(n, [&](int i) { return make_float2(g[i], 1.f); });
+  }
 }
 
-// ---------------------------------------------------------------------------
-// training on the tensor cores
-// ---------------------------------------------------------------------------
 // The operand images of one optimizer step, built on the device from the FP32
 // master parameters: W1 (K padded to 16), W2 and W3 (row = output unit, K =
 // input unit) for the forward pass; W2^T and W3^T (row = input unit, K =
@@ -576,6 +586,131 @@ __global__ void train_images_kernel(const float* __restrict__ p, TrainImages* im
   *reinterpret_cast<__nv_bfloat16*>(img->w[im] + sw128_offset(r, k)) = __float2bfloat16_rn(w);
 }
 
+// An optimizer step's update, done by the thread that has a parameter's gradient.
+struct AdamStep {
+  float *params, *m, *v;  // (params null: the gradient alone)
+  TrainImages* img;       // the next step's operand images
+  float lr, b1, b2, c1, c2, eps;
+  int* status;            // [0] a tensor-core wait gave up: no update; [1] the updates done
+  float* loss;            // the minibatch's mean loss (null: not wanted)
+};
+
+__device__ __forceinline__ void put_bf16(uint8_t* img, int r, int k, float w) {
+  *reinterpret_cast<__nv_bfloat16*>(img + sw128_offset(r, k)) = __float2bfloat16_rn(w);
+}
+
+// Sums the per-chunk partials of the CUDA-core parameters and, for W2 and W3,
+// the per-CTA tensor-core partials (mma[cta][0] = dW3, mma[cta][1] = dW2, row =
+// output unit, column = input unit), each in a fixed order; then Adam and the
+// parameter's entries of the operand images (two launches more before). The last block sums the loss.
+__global__ void __launch_bounds__(128) train_reduce_kernel(const float* __restrict__ part, int nchunks,
+                                                           const float* __restrict__ mma, int nctas, float* grad,
+                                                           const double* __restrict__ loss_part, int B, AdamStep a) {
+  if (blockIdx.x == gridDim.x - 1) {
+    if (threadIdx.x >= 32) return;
+    if (a.loss) {
+      double s = 0.0;
+      for (int t = threadIdx.x; t < nchunks; t += 32) s += loss_part[t];
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (threadIdx.x == 0) *a.loss = (float)(s / B);
+    }
+    if (threadIdx.x == 0 && a.params && !a.status[0]) a.status[1] += 1;
+    return;
+  }
+  const int pidx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pidx >= kNParams) return;
+  float s = 0.f;
+  const bool w2 = pidx >= kOW2 && pidx < kOB2, w3 = pidx >= kOW3 && pidx < kOB3;
+  const int q = w2 ? pidx - kOW2 : pidx - kOW3;
+  if (w2 || w3) {
+    for (int c = 0; c < nctas; ++c) s += mma[((size_t)c * 2 + (w2 ? 1 : 0)) * kMlpH * kMlpH + q];
+  } else {
+    for (int c = 0; c < nchunks; ++c) s += part[(size_t)c * kNParams + pidx];
+  }
+  grad[pidx] = s;
+  if (!a.params || a.status[0]) return;
+  const float mk = a.b1 * a.m[pidx] + (1.f - a.b1) * s;
+  const float vk = a.b2 * a.v[pidx] + (1.f - a.b2) * s * s;
+  a.m[pidx] = mk;
+  a.v[pidx] = vk;
+  const float w = a.params[pidx] - a.lr * (mk / a.c1) / (sqrtf(vk / a.c2) + a.eps);
+  a.params[pidx] = w;
+  if (pidx < kOB1) {
+    put_bf16(a.img->w[0], pidx / kMlpIn, pidx % kMlpIn, w);
+  } else if (w2 || w3) {
+    put_bf16(a.img->w[w2 ? 1 : 2], q / kMlpH, q % kMlpH, w);
+    put_bf16(a.img->w[w2 ? 3 : 4], q % kMlpH, q / kMlpH, w);
+  }
+}
+
+// The inference image of the current parameters.
+__global__ void infer_image_kernel(const float* __restrict__ p, const float* __restrict__ norm, MlpImage* img) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < 3 * kMlpH * kMlpH) {
+    const int im = t / (kMlpH * kMlpH), r = (t / kMlpH) % kMlpH, k = t % kMlpH;
+    if (im == 0) put_bf16(img->w1, r, k, k < kMlpIn ? p[kOW1 + r * kMlpIn + k] : 0.f);  // K padded
+    else if (im == 1) put_bf16(img->w2, r, k, p[kOW2 + r * kMlpH + k]);
+    else put_bf16(img->w3, r, k, p[kOW3 + r * kMlpH + k]);
+  }
+  if (t < kMlpH) {
+    img->b1[t] = p[kOB1 + t];
+    img->b2[t] = p[kOB2 + t];
+    img->b3[t] = p[kOB3 + t];
+    img->w4[t] = p[kOW4 + t];
+  }
+  if (t == 0) {
+    img->b4 = p[kOB4];
+    img->pad0 = img->pad1 = img->pad2 = 0.f;
+  }
+  if (t < PSPH_MLP_NNORM) img->mean[t] = norm[t];  // mean, 1/std, lo, hi follow one another
+}
+
+// ---------------------------------------------------------------------------
+// The samples' order of a training pass: a Fisher-Yates shuffle with the seeded
+// generator, step i = n - 1 .. 1 swapping entries i and j_i = draw % (i + 1). The
+// generator counts, so every j_i is known at once; and an entry's value can be
+// traced back without making the swaps. Entry p is final after step p, which
+// took what stood at x = j_p; that came there by the last step before with
+// j = x, the smallest i > p of them, which put there what stood at i before
+// step i; and so on with the smallest i' > i with j_i' = i, until none. The steps
+// are linked by their j (a list has ln n of them at most on average), and every
+// entry traces its value by itself. The same order as the loop's, 200,000 samples
+// 1.2 ms on the host, 36 us here.
+// ---------------------------------------------------------------------------
+constexpr uint64_t kSplitmixStep = 0x9e3779b97f4a7c15ull;
+__host__ __device__ inline uint64_t splitmix_at(uint64_t z) {
+  z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+  z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+  return z ^ (z >> 31);
+}
+__device__ __forceinline__ int shuffle_draw(uint64_t state, int n, int i) {
+  return (int)(splitmix_at(state + (uint64_t)(n - i) * kSplitmixStep) % (uint64_t)(i + 1));
+}
+__global__ void shuffle_link_kernel(uint64_t state, int n, int* __restrict__ head, int* __restrict__ next) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 1 || i >= n) return;
+  next[i] = atomicExch(&head[shuffle_draw(state, n, i)], i);
+}
+// the first step after `after` (the smallest larger i) that swaps with entry x, or INT_MAX
+__device__ __forceinline__ int first_swap(const int* __restrict__ head, const int* __restrict__ next, int x,
+                                          int after) {
+  int k = INT_MAX;
+  for (int i = head[x]; i >= 0; i = next[i])
+    if (i > after && i < k) k = i;
+  return k;
+}
+__global__ void shuffle_trace_kernel(uint64_t state, int n, const int* __restrict__ head, const int* __restrict__ next,
+                                     const int* __restrict__ prior, int* __restrict__ out) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  int x = p > 0 ? shuffle_draw(state, n, p) : 0;
+  for (int k = first_swap(head, next, x, p); k != INT_MAX; k = first_swap(head, next, x, x)) x = k;
+  out[p] = prior ? prior[x] : x;  // (no order before the first pass: the samples' own)
+}
+
+// ---------------------------------------------------------------------------
+// training on the tensor cores
+// ---------------------------------------------------------------------------
 // shared memory of train_tc_kernel (offsets from a 1024-byte aligned base)
 constexpr int kTrA = 0;                            // A tile: 128 rows x 64 BF16 (16 KB)
 constexpr int kTrW = kTrA + kMlpTile * 128;        // the five operand images (40 KB)
@@ -623,6 +758,16 @@ __device__ __forceinline__ void tmem_row64(uint32_t taddr, int col, float* z) {
   tmem_wait_ld();
 }
 
+// a sample's row of 64 values in global memory (16-byte accesses: a row is 256 bytes)
+__device__ __forceinline__ void row64_store(float* base, int b, const float* x) {
+  float4* p = reinterpret_cast<float4*>(base + (size_t)kMlpH * b);
+#pragma unroll
+  for (int k = 0; k < kMlpH / 4; ++k) p[k] = make_float4(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
+}
+__device__ __forceinline__ float4 row64_load4(const float* base, int b, int k) {
+  return reinterpret_cast<const float4*>(base + (size_t)kMlpH * b)[k];
+}
+
 // column c of a transposed operand ([rows] x 128 samples, two 64-wide
 // sub-tiles of sub_bytes): 64 values of this thread's sample
 __device__ __forceinline__ void store_col64(uint8_t* t, int sub_bytes, int c, const float* x) {
@@ -635,12 +780,14 @@ __device__ __forceinline__ void store_col64(uint8_t* t, int sub_bytes, int c, co
 
 // One CTA of 128 threads per tile of 128 samples (thread t = sample t of the
 // tile), looping over tiles; writes the activations and deltas the CUDA-core
-// gradients need (U, Z1..Z4, G4, D1..D3), the loss partial of each tile, and
-// its tensor-core partials of dW3 and dW2 (mma[cta][2][64][64]).
+// gradients need (U, Z1, Z2, layer 3's activations A3, Z4, G4, D1..D3), the loss partial of each tile, and
+// its tensor-core partials of dW3 and dW2 (mma[cta][2][64][64]). A chain of six
+// products and the epilogues between them: 4,096 samples 92 us with scalar row
+// accesses and the division's branches in the sigmoids, 50 without.
 __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
     const TrainImages* __restrict__ img, const float* __restrict__ params, const float* __restrict__ norm,
     const float* __restrict__ X, const float* __restrict__ Y, const float* __restrict__ W, const int* __restrict__ idx,
-    int B, float* U, float* Z1, float* Z2, float* Z3, float* Z4, float* G4, float* D1, float* D2, float* D3,
+    int B, float* U, float* Z1, float* Z2, float* A3, float* Z4, float* G4, float* D1, float* D2, float* D3,
     double* loss_part, float* mma, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bars[2];
@@ -661,7 +808,7 @@ __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
   uint8_t* at2 = AT;
   uint8_t* at1 = AT + 2 * kAsub;
   if (tid == 0) {
-    err = 0;
+    err = *status;  // (a step before gave up: the ones after it do nothing)
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
     mbar_init_fence();
@@ -716,11 +863,14 @@ __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
 #pragma unroll
     for (int k = 0; k < kMlpH; ++k) z[k] += b1[k];
     if (valid) {
-      for (int k = 0; k < kMlpH; ++k) Z1[(size_t)kMlpH * b + k] = z[k];
-      for (int k = 0; k < 8; ++k) U[(size_t)8 * b + k] = k < kMlpIn ? u[k] : 0.f;
+      row64_store(Z1, b, z);
+      static_assert(kMlpIn == 6, "u[6], u[7] are zero");
+      float4* pu = reinterpret_cast<float4*>(U + (size_t)8 * b);
+      pu[0] = make_float4(u[0], u[1], u[2], u[3]);
+      pu[1] = make_float4(u[4], u[5], 0.f, 0.f);
     }
 #pragma unroll
-    for (int k = 0; k < kMlpH; ++k) z[k] = bf16r(silu(z[k]));
+    for (int k = 0; k < kMlpH; ++k) z[k] = bf16r(z[k] * sigm_row(z[k]));
     store_row64(A, tid, z);
     store_col64(at1, kAsub, tid, z);
     // layer 2
@@ -729,10 +879,9 @@ __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
     tmem_row64(taddr, 0, z);
 #pragma unroll
     for (int k = 0; k < kMlpH; ++k) z[k] += b2[k];
-    if (valid)
-      for (int k = 0; k < kMlpH; ++k) Z2[(size_t)kMlpH * b + k] = z[k];
+    if (valid) row64_store(Z2, b, z);
 #pragma unroll
-    for (int k = 0; k < kMlpH; ++k) z[k] = bf16r(silu(z[k]));
+    for (int k = 0; k < kMlpH; ++k) z[k] = bf16r(z[k] * sigm_row(z[k]));
     store_row64(A, tid, z);
     store_col64(at2, kAsub, tid, z);
     // layer 3 and the output
@@ -741,9 +890,16 @@ __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
     tmem_row64(taddr, 0, z);
     float o = f[4 * kMlpH];
 #pragma unroll
-    for (int k = 0; k < kMlpH; ++k) {
-      z[k] += b3[k];
-      o += w4[k] * silu(z[k]);
+    for (int k = 0; k < kMlpH; ++k) z[k] += b3[k];
+#pragma unroll
+    for (int k = 0; k < kMlpH; ++k) d[k] = sigm_row(z[k]);
+    {
+      float a3[kMlpH];
+#pragma unroll
+      for (int k = 0; k < kMlpH; ++k) a3[k] = z[k] * d[k];
+#pragma unroll
+      for (int k = 0; k < kMlpH; ++k) o += w4[k] * a3[k];
+      if (valid) row64_store(A3, b, a3);
     }
     // loss and its gradient (mean over the minibatch)
     double lp = 0.0;
@@ -755,15 +911,13 @@ __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
       lp = (double)w * (double)e * (double)e;
       Z4[b] = o;
       G4[b] = g;
-      for (int k = 0; k < kMlpH; ++k) Z3[(size_t)kMlpH * b + k] = z[k];
     }
     for (int off = 16; off > 0; off >>= 1) lp += __shfl_down_sync(0xffffffffu, lp, off);
     if ((tid & 31) == 0) lred[tid >> 5] = lp;
     // delta of layer 3
 #pragma unroll
-    for (int k = 0; k < kMlpH; ++k) d[k] = g * w4[k] * dsilu(z[k]);
-    if (valid)
-      for (int k = 0; k < kMlpH; ++k) D3[(size_t)kMlpH * b + k] = d[k];
+    for (int k = 0; k < kMlpH; ++k) d[k] = g * w4[k] * dsilu_of(z[k], d[k]);
+    if (valid) row64_store(D3, b, d);
     store_row64(A, tid, d);
     store_col64(dt3, kDsub, tid, d);
     // delta of layer 2: (d3 W3) o silu'(z2)
@@ -776,17 +930,31 @@ __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
     }
     tmem_row64(taddr, 0, d);
 #pragma unroll
-    for (int k = 0; k < kMlpH; ++k) d[k] *= dsilu(valid ? Z2[(size_t)kMlpH * b + k] : 0.f);
-    if (valid)
-      for (int k = 0; k < kMlpH; ++k) D2[(size_t)kMlpH * b + k] = d[k];
+    for (int k = 0; k < kMlpH / 4; ++k) {
+      const float4 q = valid ? row64_load4(Z2, b, k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      d[4 * k] *= dsilu_of(q.x, sigm_row(q.x));
+      d[4 * k + 1] *= dsilu_of(q.y, sigm_row(q.y));
+      d[4 * k + 2] *= dsilu_of(q.z, sigm_row(q.z));
+      d[4 * k + 3] *= dsilu_of(q.w, sigm_row(q.w));
+    }
+    if (valid) row64_store(D2, b, d);
     store_row64(A, tid, d);
     store_col64(dt2, kDsub, tid, d);
     // delta of layer 1: (d2 W2) o silu'(z1)
     if (!tc_sync_mma(&bars[1], phase, &err, [&] { tc_mma_chain(taddr, A, 0, Wi + 3 * kImgBytes, 0, 4, false); }))
       break;
     tmem_row64(taddr, 0, d);
-    if (valid)
-      for (int k = 0; k < kMlpH; ++k) D1[(size_t)kMlpH * b + k] = d[k] * dsilu(Z1[(size_t)kMlpH * b + k]);
+    if (valid) {
+#pragma unroll
+      for (int k = 0; k < kMlpH / 4; ++k) {
+        const float4 q = row64_load4(Z1, b, k);
+        d[4 * k] *= dsilu_of(q.x, sigm_row(q.x));
+        d[4 * k + 1] *= dsilu_of(q.y, sigm_row(q.y));
+        d[4 * k + 2] *= dsilu_of(q.z, sigm_row(q.z));
+        d[4 * k + 3] *= dsilu_of(q.w, sigm_row(q.w));
+      }
+      row64_store(D1, b, d);
+    }
     // dW3 += d3^T a2 and dW2 += d2^T a1 over this tile's samples (K = 128)
     const bool acc = !first;
     if (!tc_sync_mma(&bars[1], phase, &err, [&] {
@@ -800,9 +968,9 @@ __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
   if (!err && !first && tid < kMlpH) {
     float* out = mma + (size_t)blockIdx.x * 2 * kMlpH * kMlpH;
     tmem_row64(taddr, 64, z);
-    for (int k = 0; k < kMlpH; ++k) out[(size_t)tid * kMlpH + k] = z[k];
+    row64_store(out, tid, z);
     tmem_row64(taddr, 128, z);
-    for (int k = 0; k < kMlpH; ++k) out[(size_t)(kMlpH + tid) * kMlpH + k] = z[k];
+    row64_store(out, kMlpH + tid, z);
   } else if (!err && first && tid < kMlpH) {  // no tile: zero partials
     float* out = mma + (size_t)blockIdx.x * 2 * kMlpH * kMlpH;
     for (int k = 0; k < 2 * kMlpH; ++k) out[(size_t)(k / kMlpH * kMlpH + tid) * kMlpH + k % kMlpH] = 0.f;
@@ -814,44 +982,10 @@ __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
   if (tid < 32) tmem_dealloc(taddr, kTrCols);
 }
 
-__global__ void adam_kernel(float* params, const float* grad, float* m, float* v, float lr, float b1, float b2,
-                            float c1, float c2, float eps) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= kNParams) return;
-  const float g = grad[k];
-  const float mk = b1 * m[k] + (1.f - b1) * g;
-  const float vk = b2 * v[k] + (1.f - b2) * g * g;
-  m[k] = mk;
-  v[k] = vk;
-  params[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
-}
-
 // ---------------------------------------------------------------------------
 // host helpers
 // ---------------------------------------------------------------------------
-uint16_t bf16_bits(float f) {  // round to nearest even
-  uint32_t u;
-  std::memcpy(&u, &f, 4);
-  if ((u & 0x7f800000u) == 0x7f800000u) return (uint16_t)((u >> 16) | ((u & 0xffffu) ? 0x40u : 0u));
-  u += 0x7fffu + ((u >> 16) & 1u);
-  return (uint16_t)(u >> 16);
-}
-
-void put_operand(uint8_t* img, const float* W, int rows, int cols) {  // W[rows][cols] -> swizzled K-major
-  std::memset(img, 0, kImgBytes);
-  for (int r = 0; r < rows; ++r)
-    for (int k = 0; k < cols; ++k) {
-      const uint16_t b = bf16_bits(W[r * cols + k]);
-      std::memcpy(img + sw128_offset(r, k), &b, 2);
-    }
-}
-
-uint64_t splitmix(uint64_t& s) {
-  uint64_t z = (s += 0x9e3779b97f4a7c15ull);
-  z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
-  z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
-  return z ^ (z >> 31);
-}
+uint64_t splitmix(uint64_t& s) { return splitmix_at(s += kSplitmixStep); }
 double uniform01(uint64_t& s) { return (double)(splitmix(s) >> 11) * (1.0 / 9007199254740992.0); }
 
 int num_sms() {
@@ -930,8 +1064,11 @@ struct psph_mlp {
   int64_t n_data = 0;
   // minibatch scratch
   int cap = 0, nchunk_cap = 0;
-  int* d_idx = nullptr;
-  float *d_U = nullptr, *d_Z1 = nullptr, *d_Z2 = nullptr, *d_Z3 = nullptr, *d_Z4 = nullptr, *d_G4 = nullptr;
+  // training passes: the samples' order (two, the last pass's and the next), the shuffle's lists
+  int *d_order[2] = {nullptr, nullptr}, *d_head = nullptr, *d_next = nullptr;
+  int64_t order_cap = 0;
+  float* d_losses = nullptr;  // kLossRun of them
+  float *d_U = nullptr, *d_Z1 = nullptr, *d_Z2 = nullptr, *d_A3 = nullptr, *d_Z4 = nullptr, *d_G4 = nullptr;
   float *d_D1 = nullptr, *d_D2 = nullptr, *d_D3 = nullptr, *d_part = nullptr;
   float* d_mma = nullptr;            // per-CTA tensor-core partials of dW3, dW2
   TrainImages* d_timg = nullptr;     // operand images of the current parameters
@@ -979,16 +1116,14 @@ psph_status ensure_batch(psph_mlp* m, int B) {
     m->mma_cap = nctas;
   }
   if (B <= m->cap && nchunk <= m->nchunk_cap) return PSPH_OK;
-  for (float** p : {&m->d_U, &m->d_Z1, &m->d_Z2, &m->d_Z3, &m->d_Z4, &m->d_G4, &m->d_D1, &m->d_D2, &m->d_D3,
+  for (float** p : {&m->d_U, &m->d_Z1, &m->d_Z2, &m->d_A3, &m->d_Z4, &m->d_G4, &m->d_D1, &m->d_D2, &m->d_D3,
                     &m->d_part})
     dfree(*p);
-  dfree(m->d_idx);
   dfree(m->d_loss);
   const size_t b = (size_t)B;
-  MLP_TRY(m, cudaMalloc(&m->d_idx, b * sizeof(int)));
   MLP_TRY(m, cudaMalloc(&m->d_U, 8 * b * sizeof(float)));
   MLP_TRY(m, cudaMemset(m->d_U, 0, 8 * b * sizeof(float)));
-  for (float** p : {&m->d_Z1, &m->d_Z2, &m->d_Z3, &m->d_D1, &m->d_D2, &m->d_D3})
+  for (float** p : {&m->d_Z1, &m->d_Z2, &m->d_A3, &m->d_D1, &m->d_D2, &m->d_D3})
     MLP_TRY(m, cudaMalloc(p, (size_t)kMlpH * b * sizeof(float)));
   MLP_TRY(m, cudaMalloc(&m->d_Z4, b * sizeof(float)));
   MLP_TRY(m, cudaMalloc(&m->d_G4, b * sizeof(float)));
@@ -999,59 +1134,52 @@ psph_status ensure_batch(psph_mlp* m, int B) {
   return PSPH_OK;
 }
 
-// Loss and gradient of one minibatch (rows idx of X/Y, or the first B rows).
-psph_status batch_grad(psph_mlp* m, const float* dX, const float* dY, const float* dW, const int* d_idx, int B,
-                       double* loss) {
+// Most losses kept on the device before they are fetched.
+constexpr int64_t kLossRun = 1 << 16;
+
+// The status of the training kernels since it was cleared.
+psph_status training_status(psph_mlp* m, int* steps_done) {
+  int status[2];
+  MLP_TRY(m, cudaMemcpy(status, m->d_status, sizeof status, cudaMemcpyDeviceToHost));
+  if (steps_done) *steps_done = status[1];
+  if (status[0]) return mlp_err(m, PSPH_ERR_CUDA, "training: a tensor-core completion wait gave up");
+  return PSPH_OK;
+}
+
+// Before a run of minibatches of at most B samples.
+psph_status begin_batches(psph_mlp* m, int B) {
   psph_status st = ensure_batch(m, B);
   if (st) return st;
-  const int nb = (B + kTrainThreads - 1) / kTrainThreads;
   MLP_TRY(m, ensure_train_attrs());
-  // tensor cores: forward, loss gradient, deltas, dW2 / dW3
   train_images_kernel<<<(5 * kMlpH * kMlpH + 255) / 256, 256>>>(m->d_params, m->d_timg);
-  MLP_TRY(m, cudaMemset(m->d_status, 0, sizeof(int)));
+  MLP_TRY(m, cudaMemsetAsync(m->d_status, 0, 2 * sizeof(int)));
+  return PSPH_OK;
+}
+
+// Loss and gradient of one minibatch (rows idx of X/Y, or the first B rows), and
+// the update (if any), as launches.
+psph_status batch_grad(psph_mlp* m, const float* dX, const float* dY, const float* dW, const int* d_idx, int B,
+                       const AdamStep& step) {
+  // tensor cores: forward, loss gradient, deltas, dW2 / dW3
   const int nctas = train_ctas(B);
   train_tc_kernel<<<nctas, kTcThreads, kTrSmemBytes>>>(m->d_timg, m->d_params, m->d_norm, dX, dY, dW, d_idx, B,
-                                                       m->d_U, m->d_Z1, m->d_Z2, m->d_Z3, m->d_Z4, m->d_G4, m->d_D1,
+                                                       m->d_U, m->d_Z1, m->d_Z2, m->d_A3, m->d_Z4, m->d_G4, m->d_D1,
                                                        m->d_D2, m->d_D3, m->d_loss, m->d_mma, m->d_status);
   // CUDA cores: W1, the biases and the output layer, per chunk of samples
   const int chunk = 128, nchunk = (B + chunk - 1) / chunk;
-  dim3 grid((kNParams + 127) / 128, nchunk);
-  train_wgrad_kernel<<<grid, 128>>>(m->d_U, m->d_Z1, m->d_Z2, m->d_Z3, m->d_G4, m->d_D1, m->d_D2, m->d_D3, B, chunk,
-                                    m->d_part);
-  train_reduce_kernel<<<(kNParams + 127) / 128, 128>>>(m->d_part, nchunk, m->d_mma, nctas, m->d_grad);
+  static_assert(kMlpTile == 128 && kTrainThreads == 128, "a loss partial per chunk");
+  train_wgrad_kernel<<<dim3((kWgParams + 127) / 128, nchunk), 128>>>(m->d_U, m->d_A3, m->d_G4, m->d_D1, m->d_D2,
+                                                                     m->d_D3, B, chunk, m->d_part);
+  train_reduce_kernel<<<(kNParams + 127) / 128 + 1, 128>>>(m->d_part, nchunk, m->d_mma, nctas, m->d_grad, m->d_loss,
+                                                           B, step);
   MLP_TRY(m, cudaGetLastError());
-  int tstatus = 0;
-  MLP_TRY(m, cudaMemcpy(&tstatus, m->d_status, sizeof(int), cudaMemcpyDeviceToHost));
-  if (tstatus) return mlp_err(m, PSPH_ERR_CUDA, "training: a tensor-core completion wait gave up");
-  if (loss) {
-    std::vector<double> parts(nb);
-    MLP_TRY(m, cudaMemcpy(parts.data(), m->d_loss, nb * sizeof(double), cudaMemcpyDeviceToHost));
-    double s = 0.0;
-    for (double x : parts) s += x;
-    *loss = s / B;
-  }
   return PSPH_OK;
 }
 
 psph_status build_image(psph_mlp* m) {
   if (!m->img_dirty) return PSPH_OK;
-  std::vector<float> p(kNParams);
-  MLP_TRY(m, cudaMemcpy(p.data(), m->d_params, kNParams * sizeof(float), cudaMemcpyDeviceToHost));
-  std::vector<uint8_t> buf(sizeof(MlpImage), 0);
-  MlpImage* img = reinterpret_cast<MlpImage*>(buf.data());
-  std::vector<float> w1(kMlpH * 16, 0.f);  // K padded to one 16-wide MMA step
-  for (int r = 0; r < kMlpH; ++r)
-    for (int k = 0; k < kMlpIn; ++k) w1[r * 16 + k] = p[kOW1 + r * kMlpIn + k];
-  put_operand(img->w1, w1.data(), kMlpH, 16);
-  put_operand(img->w2, &p[kOW2], kMlpH, kMlpH);
-  put_operand(img->w3, &p[kOW3], kMlpH, kMlpH);
-  std::memcpy(img->b1, &p[kOB1], kMlpH * 4);
-  std::memcpy(img->b2, &p[kOB2], kMlpH * 4);
-  std::memcpy(img->b3, &p[kOB3], kMlpH * 4);
-  std::memcpy(img->w4, &p[kOW4], kMlpH * 4);
-  img->b4 = p[kOB4];
-  std::memcpy(img->mean, m->norm.data(), PSPH_MLP_NNORM * 4);
-  MLP_TRY(m, cudaMemcpy(m->d_img, buf.data(), sizeof(MlpImage), cudaMemcpyHostToDevice));
+  infer_image_kernel<<<(3 * kMlpH * kMlpH + 255) / 256, 256>>>(m->d_params, m->d_norm, m->d_img);
+  MLP_TRY(m, cudaGetLastError());
   m->img_dirty = false;
   return PSPH_OK;
 }
@@ -1063,6 +1191,7 @@ psph_status psph_mlp_image(const psph_mlp* mlp, const MlpImage** dev_image) {
   if (!m || !dev_image) return PSPH_ERR_INVALID_ARGUMENT;
   psph_status st = build_image(m);
   if (st) return st;
+  MLP_TRY(m, cudaStreamSynchronize(0));  // the caller's stream is another one
   *dev_image = m->d_img;
   return PSPH_OK;
 }
@@ -1081,7 +1210,7 @@ psph_status psph_mlp_create(uint64_t seed, psph_mlp** out) {
   MLP_TRY(m, cudaMalloc(&m->d_grad, kNParams * sizeof(float)));
   MLP_TRY(m, cudaMalloc(&m->d_norm, PSPH_MLP_NNORM * sizeof(float)));
   MLP_TRY(m, cudaMalloc(&m->d_img, sizeof(MlpImage)));
-  MLP_TRY(m, cudaMalloc(&m->d_status, sizeof(int)));
+  MLP_TRY(m, cudaMalloc(&m->d_status, 2 * sizeof(int)));
   MLP_TRY(m, cudaMemset(m->d_m, 0, kNParams * sizeof(float)));
   MLP_TRY(m, cudaMemset(m->d_v, 0, kNParams * sizeof(float)));
   // uniform(-1/sqrt(fan_in), 1/sqrt(fan_in)) weights and biases; the output
@@ -1115,12 +1244,16 @@ void psph_mlp_destroy(psph_mlp* m) {
   if (!m) return;
   cudaDeviceSynchronize();
   for (float** p : {&m->d_params, &m->d_m, &m->d_v, &m->d_grad, &m->d_norm, &m->d_X, &m->d_Y, &m->d_W, &m->d_U, &m->d_Z1,
-                    &m->d_Z2, &m->d_Z3, &m->d_Z4, &m->d_G4, &m->d_D1, &m->d_D2, &m->d_D3, &m->d_part})
+                    &m->d_Z2, &m->d_A3, &m->d_Z4, &m->d_G4, &m->d_D1, &m->d_D2, &m->d_D3, &m->d_part})
     dfree(*p);
   dfree(m->d_img);
   dfree(m->d_timg);
   dfree(m->d_mma);
-  dfree(m->d_idx);
+  dfree(m->d_order[0]);
+  dfree(m->d_order[1]);
+  dfree(m->d_head);
+  dfree(m->d_next);
+  dfree(m->d_losses);
   dfree(m->d_loss);
   dfree(m->d_status);
   delete m;
@@ -1205,54 +1338,85 @@ psph_status psph_mlp_set_weights(psph_mlp* m, const float* w) {
 psph_status psph_mlp_train(psph_mlp* m, int64_t steps, int batch, float lr, uint64_t seed, float* losses) {
   if (!m || steps < 0 || batch < 1 || !(lr > 0.f)) return PSPH_ERR_INVALID_ARGUMENT;
   if (!m->n_data) return mlp_err(m, PSPH_ERR_STATE, "psph_mlp_train before psph_mlp_set_data");
-  const int B = (int)std::min<int64_t>(batch, m->n_data);
-  std::vector<int> perm(m->n_data);
-  for (int64_t i = 0; i < m->n_data; ++i) perm[i] = (int)i;
-  uint64_t rs = seed;
-  int64_t pos = m->n_data;  // forces a shuffle on the first step
-  psph_status st = ensure_batch(m, B);
+  const int n = (int)m->n_data, B = (int)std::min<int64_t>(batch, n);
+  psph_status st = begin_batches(m, B);
   if (st) return st;
+  if (n > m->order_cap) {
+    for (int** p : {&m->d_order[0], &m->d_order[1], &m->d_head, &m->d_next}) dfree(*p);
+    m->order_cap = 0;
+    for (int** p : {&m->d_order[0], &m->d_order[1], &m->d_head, &m->d_next})
+      MLP_TRY(m, cudaMalloc(p, (size_t)n * sizeof(int)));
+    m->order_cap = n;
+  }
+  if (losses && !m->d_losses) MLP_TRY(m, cudaMalloc(&m->d_losses, kLossRun * sizeof(float)));
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  const int* order = nullptr;  // (the first pass shuffles the samples as they are)
+  uint64_t rs = seed;
+  int pos = n;  // forces a shuffle on the first step
+  const long long t0 = m->adam_t;
+  m->img_dirty = true;
+  int64_t fetched = 0;
+  // every step is launches alone; what they left is read back at the end, or when the losses' room is full
+  auto settle = [&](int64_t upto) {
+    int done = 0;
+    psph_status q = training_status(m, &done);
+    m->adam_t = t0 + fetched + done;
+    if (q) return q;
+    if (losses) {
+      const cudaError_t e = cudaMemcpy(losses + fetched, m->d_losses, (size_t)(upto - fetched) * sizeof(float),
+                                       cudaMemcpyDeviceToHost);
+      if (e != cudaSuccess) return mlp_err(m, PSPH_ERR_CUDA, "losses: %s", cudaGetErrorString(e));
+    }
+    fetched = upto;
+    const cudaError_t e = cudaMemsetAsync(m->d_status, 0, 2 * sizeof(int));
+    return e == cudaSuccess ? PSPH_OK : mlp_err(m, PSPH_ERR_CUDA, "status: %s", cudaGetErrorString(e));
+  };
   for (int64_t step = 0; step < steps; ++step) {
-    if (pos + B > m->n_data) {  // new pass: Fisher-Yates with the seeded generator
-      for (int64_t i = m->n_data - 1; i > 0; --i) {
-        const int64_t j = (int64_t)(splitmix(rs) % (uint64_t)(i + 1));
-        std::swap(perm[i], perm[j]);
-      }
+    if (pos > n - B) {  // new pass
+      int* to = m->d_order[order == m->d_order[0] ? 1 : 0];
+      MLP_TRY(m, cudaMemsetAsync(m->d_head, 0xff, (size_t)n * sizeof(int)));
+      const int nb = (int)(((int64_t)n + 255) / 256);
+      shuffle_link_kernel<<<nb, 256>>>(rs, n, m->d_head, m->d_next);
+      shuffle_trace_kernel<<<nb, 256>>>(rs, n, m->d_head, m->d_next, order, to);
+      rs += (uint64_t)(n - 1) * kSplitmixStep;
+      order = to;
       pos = 0;
     }
-    MLP_TRY(m, cudaMemcpy(m->d_idx, perm.data() + pos, B * sizeof(int), cudaMemcpyHostToDevice));
+    const double t = (double)(t0 + step + 1);
+    AdamStep a{m->d_params, m->d_m, m->d_v, m->d_timg, lr, b1, b2, (float)(1.0 - std::pow((double)b1, t)),
+               (float)(1.0 - std::pow((double)b2, t)), eps, m->d_status,
+               losses ? m->d_losses + (step - fetched) : nullptr};
+    if ((st = batch_grad(m, m->d_X, m->d_Y, m->d_W, order + pos, B, a))) return st;
     pos += B;
-    double loss = 0.0;
-    if ((st = batch_grad(m, m->d_X, m->d_Y, m->d_W, m->d_idx, B, losses ? &loss : nullptr))) return st;
-    m->adam_t += 1;
-    const float c1 = (float)(1.0 - std::pow((double)b1, (double)m->adam_t));
-    const float c2 = (float)(1.0 - std::pow((double)b2, (double)m->adam_t));
-    adam_kernel<<<(kNParams + 255) / 256, 256>>>(m->d_params, m->d_grad, m->d_m, m->d_v, lr, b1, b2, c1, c2, eps);
-    MLP_TRY(m, cudaGetLastError());
-    if (losses) losses[step] = (float)loss;
+    if (step + 1 - fetched == kLossRun && (st = settle(step + 1))) return st;
   }
+  if (fetched < steps && (st = settle(steps))) return st;
   MLP_TRY(m, cudaDeviceSynchronize());
-  m->img_dirty = true;
   return PSPH_OK;
 }
 
 psph_status psph_mlp_loss_grad(psph_mlp* m, const float* x, const float* y, int64_t n, double* loss, float* grad) {
   if (!m || !x || !y || n < 1 || n > (1 << 24)) return PSPH_ERR_INVALID_ARGUMENT;
+  if (loss) *loss = 0.0;
   float *dX = nullptr, *dY = nullptr;
   MLP_TRY(m, cudaMalloc(&dX, (size_t)n * kMlpIn * sizeof(float)));
   MLP_TRY(m, cudaMalloc(&dY, (size_t)n * sizeof(float)));
   MLP_TRY(m, cudaMemcpy(dX, x, (size_t)n * kMlpIn * sizeof(float), cudaMemcpyHostToDevice));
   MLP_TRY(m, cudaMemcpy(dY, y, (size_t)n * sizeof(float), cudaMemcpyHostToDevice));
-  double l = 0.0;
-  psph_status st = batch_grad(m, dX, dY, nullptr, nullptr, (int)n, &l);
-  if (!st && grad) {
-    cudaError_t e = cudaMemcpy(grad, m->d_grad, kNParams * sizeof(float), cudaMemcpyDeviceToHost);
+  psph_status st = begin_batches(m, (int)n);
+  if (!st) st = batch_grad(m, dX, dY, nullptr, nullptr, (int)n, AdamStep{});
+  if (!st) st = training_status(m, nullptr);
+  if (!st) {
+    std::vector<double> parts((n + kTrainThreads - 1) / kTrainThreads);
+    cudaError_t e = cudaMemcpy(parts.data(), m->d_loss, parts.size() * sizeof(double), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && grad) e = cudaMemcpy(grad, m->d_grad, kNParams * sizeof(float), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) st = mlp_err(m, PSPH_ERR_CUDA, "gradient copy: %s", cudaGetErrorString(e));
+    double l = 0.0;
+    for (double q : parts) l += q;
+    if (!st && loss) *loss = l / (double)n;
   }
   cudaFree(dX);
   cudaFree(dY);
-  if (loss) *loss = l;
   return st;
 }
 
