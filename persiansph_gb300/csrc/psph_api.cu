@@ -70,7 +70,8 @@ struct psph_ctx {
   GridDev* d_grids_ref = nullptr;       // the reference's grids (CellInitiate)
   int total_cells_ref = 0;
   InstState* d_inst = nullptr;
-  InstState* h_inst = nullptr;  // pinned mirror
+  InstState* h_inst = nullptr;  // pinned mirror (behind h_sc, as d_inst behind d_sc: one copy fetches both)
+  char* h_stage = nullptr;      // pinned, kStageBytes: small downloads land here
   StepScalars* d_sc = nullptr;
   StepScalars* h_sc = nullptr;  // pinned mirror
   uint8_t* d_alive = nullptr;
@@ -145,6 +146,12 @@ psph_status dalloc(psph_ctx* c, T** p, size_t count) {
   return PSPH_OK;
 }
 
+// The instances' states behind the scalars, on the device and in the mirror.
+constexpr size_t kInstAt = (sizeof(StepScalars) + 255) / 256 * 256;
+// A download of at most this much goes through pinned memory: a copy into pageable
+// memory is a wait of its own, some 10 us, per field.
+constexpr size_t kStageBytes = 1 << 20;
+
 void free_all(psph_ctx* c) {
   if (c->graph) cudaGraphExecDestroy(c->graph);
   c->graph = nullptr;
@@ -152,8 +159,9 @@ void free_all(psph_ctx* c) {
   c->allocs.clear();
   if (c->h_sc) cudaFreeHost(c->h_sc);
   c->h_sc = nullptr;
-  if (c->h_inst) cudaFreeHost(c->h_inst);
   c->h_inst = nullptr;
+  if (c->h_stage) cudaFreeHost(c->h_stage);
+  c->h_stage = nullptr;
 }
 
 // Particle constructor defaults (Source/Particle.cpp:25-117) for NULL arrays.
@@ -361,26 +369,39 @@ __global__ void rearm_kernel(InstState* inst, int ninst, StepScalars* sc) {
 }
 
 psph_status sync_scalars(psph_ctx* c) {
-  CUDA_TRY(c, cudaMemcpyAsync(c->h_sc, c->d_sc, sizeof(StepScalars), cudaMemcpyDeviceToHost, c->stream));
-  CUDA_TRY(c, cudaMemcpyAsync(c->h_inst, c->d_inst, sizeof(InstState) * c->ninst, cudaMemcpyDeviceToHost, c->stream));
+  CUDA_TRY(c, cudaMemcpyAsync(c->h_sc, c->d_sc, kInstAt + sizeof(InstState) * c->ninst, cudaMemcpyDeviceToHost,
+                              c->stream));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   return PSPH_OK;
 }
 
 // Sets each instance's stop time (t_stop[q], or t_all when t_stop is NULL)
-// and clears the stop flags and the status word before a run of steps.
-psph_status arm(psph_ctx* c, const double* t_stop, double t_all) {
-  psph_status st = sync_scalars(c);
-  if (st) return st;
-  for (int q = 0; q < c->ninst; ++q) {
-    c->h_inst[q].t_stop = t_stop ? t_stop[q] : t_all;
-    c->h_inst[q].stop = 0;
+// and clears the stop flags and the status word before a run of steps: on the
+// device, in stream order, with nothing to wait for.
+__global__ void arm_kernel(InstState* inst, int ninst, StepScalars* sc, double t_all, int keep_t) {
+  for (int k = threadIdx.x; k < ninst; k += blockDim.x) {
+    if (!keep_t) inst[k].t_stop = t_all;
+    inst[k].stop = 0;
+    inst[k].steps0 = inst[k].steps;
   }
-  c->h_sc->status = 0;
-  c->h_sc->all_stop = 0;
-  CUDA_TRY(c, cudaMemcpyAsync(c->d_inst, c->h_inst, sizeof(InstState) * c->ninst, cudaMemcpyHostToDevice, c->stream));
-  CUDA_TRY(c, cudaMemcpyAsync(c->d_sc, c->h_sc, sizeof(StepScalars), cudaMemcpyHostToDevice, c->stream));
-  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  if (threadIdx.x == 0) {
+    sc->status = 0;
+    sc->all_stop = 0;
+  }
+}
+
+psph_status arm(psph_ctx* c, const double* t_stop, double t_all) {
+  if (t_stop && c->ninst == 1) {
+    t_all = t_stop[0];
+  } else if (t_stop) {
+    psph_status st = sync_scalars(c);
+    if (st) return st;
+    for (int q = 0; q < c->ninst; ++q) c->h_inst[q].t_stop = t_stop[q];
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_inst, c->h_inst, sizeof(InstState) * c->ninst, cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  }
+  arm_kernel<<<1, 256, 0, c->stream>>>(c->d_inst, c->ninst, c->d_sc, t_all, t_stop && c->ninst > 1);
+  CUDA_TRY(c, cudaGetLastError());
   return PSPH_OK;
 }
 
@@ -1058,14 +1079,16 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
         (st = dalloc(c, &S.strain_o, 9 * N)) || (st = dalloc(c, &S.shear_o, 9 * N)))
       return st;
   }
+  char* state = nullptr;
   c->cls_cap = (int)c->classes.size() + (inout ? 256 : 0);  // recycled in-flow particles may need new classes
-  if ((st = dalloc(c, &c->d_cls, (size_t)c->cls_cap)) || (st = dalloc(c, &c->d_sc, 1)) ||
+  if ((st = dalloc(c, &c->d_cls, (size_t)c->cls_cap)) || (st = dalloc(c, &state, kInstAt + sizeof(InstState) * ninst)) ||
       (st = dalloc(c, &c->d_alive, N)) || (st = dalloc(c, &c->d_grids, (size_t)ninst)) ||
-      (st = dalloc(c, &c->d_grids_ref, (size_t)ninst)) ||
-      (st = dalloc(c, &c->d_inst, (size_t)ninst)))
+      (st = dalloc(c, &c->d_grids_ref, (size_t)ninst)))
     return st;
-  CUDA_TRY(c, cudaMallocHost(&c->h_sc, sizeof(StepScalars)));
-  CUDA_TRY(c, cudaMallocHost(&c->h_inst, sizeof(InstState) * ninst));
+  c->d_sc = reinterpret_cast<StepScalars*>(state);
+  c->d_inst = reinterpret_cast<InstState*>(state + kInstAt);
+  CUDA_TRY(c, cudaMallocHost(&c->h_sc, kInstAt + sizeof(InstState) * ninst));
+  c->h_inst = reinterpret_cast<InstState*>(reinterpret_cast<char*>(c->h_sc) + kInstAt);
   {
     std::vector<PClass32> c32(c->classes.size());
     for (size_t q = 0; q < c->classes.size(); ++q) {
@@ -1629,10 +1652,9 @@ psph_status step_impl(psph_ctx* c, int64_t nsteps, const double* t_stop, double 
   psph_status st;
   if (nsteps <= 0) return c->timing ? PSPH_OK : build_graph(c);
   if ((st = arm(c, t_stop, t_all))) return st;
-  std::vector<long long> steps0(c->ninst);
-  for (int q = 0; q < c->ninst; ++q) steps0[q] = c->h_inst[q].steps;
   for (int e = 0; e < kNumPhases; ++e) c->phase_ms[e] = 0.0;
   long long launched = 0;
+  bool fetched = false;  // the scalars as the steps left them
   if (c->out_requested && (c->inout || c->hook_fn)) {
     c->out_requested = false;
     if ((st = split_steps(c, nsteps, &launched, true))) return st;
@@ -1681,12 +1703,13 @@ psph_status step_impl(psph_ctx* c, int64_t nsteps, const double* t_stop, double 
       left -= chunk;
       launched += chunk * launches_per_step(view(c));
       if ((st = sync_scalars(c))) return st;
+      fetched = true;
       if (c->h_sc->all_stop || c->h_sc->status) break;
     }
   }
-  if ((st = sync_scalars(c))) return st;
+  if (!fetched && (st = sync_scalars(c))) return st;
   if (steps_done)
-    for (int q = 0; q < c->ninst; ++q) steps_done[q] = c->h_inst[q].steps - steps0[q];
+    for (int q = 0; q < c->ninst; ++q) steps_done[q] = c->h_inst[q].steps - c->h_inst[q].steps0;
   c->last_launches = launched;
   const uint32_t status = c->h_sc->status;
   // the root cause first: a non-finite state also throws particles off the grid
@@ -1746,27 +1769,42 @@ bool keeps_place(const Persist& P, const double* a) {
                a == P.tir);
 }
 
-__global__ void dl_flag_kernel(const uint8_t* __restrict__ alive, const int* __restrict__ orig, int n, int lo,
-                               int hi, int* __restrict__ flag) {
+__global__ void dl_flag_kernel(DevView v, int lo, int hi, int* __restrict__ flag) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < n && alive[s] && orig[s] >= lo && orig[s] < hi) flag[orig[s] - lo] = 1;
+  if (s >= v.sc->n) return;
+  const int o = cur_persist(v).orig[s];
+  if (v.alive[s] && o >= lo && o < hi) flag[o - lo] = 1;
 }
-__global__ void dl_row_kernel(const uint8_t* __restrict__ alive, const int* __restrict__ orig, int n, int lo, int hi,
-                              const int* __restrict__ rank, int* __restrict__ row) {
+__global__ void dl_row_kernel(DevView v, int lo, int hi, const int* __restrict__ rank, int* __restrict__ row) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < n) row[s] = (alive[s] && orig[s] >= lo && orig[s] < hi) ? rank[orig[s] - lo] : -1;
+  if (s == 0) v.sc->rows = rank[hi - lo];
+  if (s >= v.sc->n) return;
+  const int o = cur_persist(v).orig[s];
+  row[s] = (v.alive[s] && o >= lo && o < hi) ? rank[o - lo] : -1;
 }
-// dst[row * width + e] = src[s * stride + off + e], or of place[s] (tensors keep
-// their place: the original index)
-__global__ void dl_gather_kernel(const double* __restrict__ src, int stride, int off, int width,
-                                 double* __restrict__ dst, const int* __restrict__ row, int n,
-                                 const int* __restrict__ place) {
+// The fields of one batch of a download: dst[row * width + e] = src[s * stride +
+// off + e], or of place[s] (tensors keep their place: the original index).
+struct DlField {
+  const double* src;
+  const int* place;
+  double* dst;
+  int stride, off, width;
+};
+constexpr int kDlFields = 16;
+struct DlBatch {
+  DlField f[kDlFields];
+  int count;
+};
+__global__ void dl_gather_kernel(DlBatch b, const int* __restrict__ row, int n) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const int r = row[s];
   if (r < 0) return;
-  const size_t at = (size_t)(place ? place[s] : s) * stride + off;
-  for (int e = 0; e < width; ++e) dst[(size_t)r * width + e] = src[at + e];
+  for (int k = 0; k < b.count; ++k) {
+    const DlField& f = b.f[k];
+    const size_t at = (size_t)(f.place ? f.place[s] : s) * f.stride + f.off;
+    for (int e = 0; e < f.width; ++e) f.dst[(size_t)r * f.width + e] = f.src[at + e];
+  }
 }
 // psph_patch: the caller's row r = row[s] back into slot s (dl_gather_kernel's reverse)
 __global__ void patch_scatter_kernel(double* __restrict__ dst, int stride, int off, int width,
@@ -1818,9 +1856,6 @@ __global__ void dl_class_kernel(const PClass* __restrict__ tab, const int* __res
 // original order (leavers and other instances: -1); *m receives the row count.
 psph_status download_rows(psph_ctx* c, int q, int64_t* m) {
   psph_status st;
-  if ((st = sync_scalars(c))) return st;
-  const int n = c->h_sc->n;
-  const Persist& P = c->h_sc->buf ? c->PB : c->PA;
   cudaStream_t s = c->stream;
   const size_t N = (size_t)c->ncap;
   // (an in/out-flow domain's appended particles take original indices past the upload's)
@@ -1833,15 +1868,15 @@ psph_status download_rows(psph_ctx* c, int q, int64_t* m) {
       return st;
     c->dl_cap = cap;
   }
-  const int nb = n > 0 ? (n + 255) / 256 : 1;
+  const int nb = c->ncap > 0 ? (c->ncap + 255) / 256 : 1;
+  const DevView v = view(c);
   CUDA_TRY(c, cudaMemsetAsync(c->dl_flag, 0, sizeof(int) * (size_t)(len + 1), s));
-  if (n > 0) dl_flag_kernel<<<nb, 256, 0, s>>>(c->d_alive, P.orig, n, lo, hi, c->dl_flag);
+  dl_flag_kernel<<<nb, 256, 0, s>>>(v, lo, hi, c->dl_flag);
   launch_exclusive_scan(c->dl_flag, c->dl_rank, len, c->dl_bs, s);
-  if (n > 0) dl_row_kernel<<<nb, 256, 0, s>>>(c->d_alive, P.orig, n, lo, hi, c->dl_rank, c->dl_row);
-  int m32 = 0;
-  CUDA_TRY(c, cudaMemcpyAsync(&m32, c->dl_rank + len, sizeof(int), cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(c, cudaStreamSynchronize(s));
-  *m = m32;
+  dl_row_kernel<<<nb, 256, 0, s>>>(v, lo, hi, c->dl_rank, c->dl_row);
+  CUDA_TRY(c, cudaGetLastError());
+  if ((st = sync_scalars(c))) return st;  // (the count, and what the caller needs to know of the state)
+  *m = c->h_sc->rows;
   return PSPH_OK;
 }
 
@@ -1914,18 +1949,27 @@ psph_status download_impl(psph_ctx* c, int q, psph_particles* out) {
     c->dl_width = stage;
   }
   auto gather_batch = [&](int b) {
+    DlBatch g;
+    g.count = 0;
     for (size_t a = 0; a < act.size(); ++a) {
       if (batch_of[a] != b) continue;
       const F& f = *act[a];
       // the FP32C fluid kernel keeps its strain-rate sums in FP32: expand them first
       if ((f.dev == c->S.strain_rate && (c->S.sr32 || c->S.rates32)) || (f.dev == c->S.rotation_rate && c->S.rates32))
         launch_expand_sr32(view(c), n, s);
-      dl_gather_kernel<<<nb, 256, 0, s>>>(f.dev, f.stride, f.off, f.width, c->dl_buf + (size_t)seg[a] * m,
-                                          c->dl_row, n, keeps_place(P, f.dev) ? P.orig : nullptr);
+      // (a batch is at most kStageWidth values wide: no more fields than that)
+      g.f[g.count++] = {f.dev, keeps_place(P, f.dev) ? P.orig : nullptr, c->dl_buf + (size_t)seg[a] * m,
+                        f.stride, f.off, f.width};
     }
+    if (g.count) dl_gather_kernel<<<nb, 256, 0, s>>>(g, c->dl_row, n);
   };
+  static_assert(kStageWidth <= kDlFields, "a batch's fields");
+  size_t values = 0;
+  for (const F* f : act) values += f->width;
+  const bool staged = values * (size_t)m * sizeof(double) <= kStageBytes;
+  if (staged && !c->h_stage) CUDA_TRY(c, cudaMallocHost(&c->h_stage, kStageBytes));
   if (nbatch > 0) gather_batch(0);
-  {
+  if (!staged) {
     // Fresh output pages are populated here by host threads in parallel (one
     // write per page; the copies overwrite them): a device copy into
     // untouched pageable memory would take each page fault in turn.
@@ -1943,12 +1987,21 @@ psph_status download_impl(psph_ctx* c, int q, psph_particles* out) {
         }
       });
   }
+  char* to = c->h_stage;  // staged: batch after batch
   for (int b = 0; b < nbatch; ++b) {
     if (b > 0) gather_batch(b);  // after the previous batch's copies (same stream)
+    size_t width_b = 0;
     for (size_t a = 0; a < act.size(); ++a) {
       if (batch_of[a] != b) continue;
-      CUDA_TRY(c, cudaMemcpyAsync(act[a]->out, c->dl_buf + (size_t)seg[a] * m,
-                                  (size_t)m * act[a]->width * sizeof(double), cudaMemcpyDeviceToHost, s));
+      width_b += act[a]->width;
+      if (!staged)
+        CUDA_TRY(c, cudaMemcpyAsync(act[a]->out, c->dl_buf + (size_t)seg[a] * m,
+                                    (size_t)m * act[a]->width * sizeof(double), cudaMemcpyDeviceToHost, s));
+    }
+    if (staged) {
+      const size_t bytes = width_b * (size_t)m * sizeof(double);
+      CUDA_TRY(c, cudaMemcpyAsync(to, c->dl_buf, bytes, cudaMemcpyDeviceToHost, s));
+      to += bytes;
     }
   }
   if (out->in_out && P.io) {  // Particle::InOut (in/out-flow domains)
@@ -1988,6 +2041,14 @@ psph_status download_impl(psph_ctx* c, int q, psph_particles* out) {
   }
   CUDA_TRY(c, cudaStreamSynchronize(s));
   CUDA_TRY(c, cudaGetLastError());
+  if (staged) {  // (the batches hold the fields in their order)
+    const char* from = c->h_stage;
+    for (const F* f : act) {
+      const size_t bytes = (size_t)m * f->width * sizeof(double);
+      std::memcpy(f->out, from, bytes);
+      from += bytes;
+    }
+  }
   return PSPH_OK;
 }
 

@@ -89,6 +89,7 @@ struct InstState {
   double time, deltat, deltatint, deltatmin, t_stop;
   double dt2, half_dt2;  // 2 dt and dt^2 / 2 of the step (set with deltat)
   long long steps;
+  long long steps0;  // steps when the run of steps began
   unsigned long long dtmin_bits;  // running minimum of the acceleration time-step bound (ordered bits)
   int first_step, ct, shepard_counter, stop;
   int k_initial;  // the first step after an initial upload: permeabilities are InitialChecks' values
@@ -109,6 +110,7 @@ struct StepScalars {
   unsigned long long closure_eval, closure_fallback;  // closure evaluations / Smagorinsky fallbacks
   int nl_rest;    // particles the neighbour-list scan handles one per lane (set by the sort)
   int n_walls;    // fixed particles (Scratch::walls, set by the sort)
+  int rows;       // particles the last count of an instance's rows found
   int n_old;      // n before the sort removed particles (its scatter's range)
   // neighbour lists with a skin (FP32C form, Options::skin > 0): the cell sort
   // and the lists are rebuilt only when a particle has moved half the skin
