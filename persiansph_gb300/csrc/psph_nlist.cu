@@ -12,8 +12,9 @@
 // work; the pair kernels then walk lists of nearly equal length instead of
 // branching per candidate.
 //
-// With one h everywhere (nlist_pair_kernel) a lane scans for two particles of
-// one cell at once; otherwise (nlist_kernel) a lane scans for one particle.
+// With one h everywhere and many particles (nlist_pair_kernel) a lane scans for two
+// particles of one cell at once; otherwise (nlist_kernel) for one particle, and
+// with few particles (nlist_cells_kernel) a lane takes one cell of one particle.
 //
 // Staged form (nlist_staged_kernel, one h everywhere, x not periodic): a block
 // first copies the candidate positions of its particles' neighbour cells into
@@ -97,7 +98,8 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
   const Persist& P = cur_persist(v);
   const PClass& C = v.cls[P.cls[i]];
   const GridDev& g = grid_of(v, C.inst);
-  const bool fixed = !C.is_free && !v.o.list_all;  // its list holds free particles only (it has no other pairs)
+  // a fixed particle's list holds free particles only (it has no other pairs)
+  const bool fixed = !C.is_free && !v.o.list_all, free_half = fixed && v.o.xsub == 1, by_sign = fixed && !free_half;
   const float3 cs = cell_size_f(g);
   float4 oi = v.S.OFF32[i];
   oi.w = fabsf(oi.w);  // (its sign says whether the particle is fixed)
@@ -136,51 +138,65 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
         slo = max(slo, lo_);
         shi = min(shi, hi_);
       }
-      for (int dx = -1; dx <= 1; ++dx) {
+      // the row's three cells in one walk, as in scan_two
+      int lo0, hi0, lo1, hi1, lo2, hi2;
+      auto range = [&](int dx, int& lo, int& hi) {
+        lo = hi = 0;
         int x = c.x + dx;
         if (g.periodic[0]) x = (x + g.nc[0]) % g.nc[0];
-        else if (x < 0 || x >= g.nc[0]) continue;
+        else if (x < 0 || x >= g.nc[0]) return;
         const int s0 = max(slo - dx * xs, 0), s1 = min(shi - dx * xs, xs - 1);
-        if (s0 > s1) continue;
-        for (int sl = s0; sl <= s1; sl += fixed ? 1 : xs) {  // a free particle's slabs in one range
-        const int bin = 2 * ((base + x) * xs + sl);
-        int lo = sstart[bin];
-        const int hi = sstart[fixed ? bin + 1 : 2 * ((base + x) * xs + s1 + 1)];
-        const int tag = (int)((unsigned)((dx + 1) | cyz) << kCodeShift);
-        // i's position relative to this cell's origin: x_i - x_j = a - off_j
-        // (one rounding away from rel_pos's form, which the pair kernels
-        // apply exactly; the list's margin covers the difference)
-        const float ax = oi.x - (float)dx * cs.x, ay = oi.y + cy, az = oi.z + cz;
-        auto inside = [&](int j) {
-          const float4 oj = off[j];
-          const float x0 = ax - oj.x, x1 = ay - oj.y, x2 = (DIM == 3) ? az - oj.z : 0.f;
+        if (s0 > s1) return;
+        const int bin = 2 * ((base + x) * xs + s0);
+        lo = sstart[bin];
+        hi = sstart[free_half ? bin + 1 : 2 * ((base + x) * xs + s1 + 1)];
+      };
+      range(-1, lo0, hi0);
+      range(0, lo1, hi1);
+      range(1, lo2, hi2);
+      const bool home = dy == 0 && dz == 0;
+      // i's position relative to a cell's origin: x_i - x_j = a - off_j (one
+      // rounding away from rel_pos's form, which the pair kernels apply exactly;
+      // the list's margin covers the difference)
+      const float ay = oi.y + cy, az = oi.z + cz;
+      float ax = oi.x + cs.x;
+      int tag = (int)((unsigned)cyz << kCodeShift), cell_k = 0, j = lo0, end = hi0;
+      auto next_cell = [&]() {
+        while (j >= end && cell_k < 2) {
+          ++cell_k;
+          j = cell_k == 1 ? lo1 : lo2;
+          end = cell_k == 1 ? hi1 : hi2;
+          ax = cell_k == 1 ? oi.x : oi.x - cs.x;
+          tag += 1 << kCodeShift;
+        }
+      };
+      next_cell();
+      while (j < end) {
+        const int m = end - j;
+        bool in[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float4 oj = off[j + e];  // (past the cell's end: another particle's, masked)
+          const float x0 = ax - oj.x, x1 = ay - oj.y, x2 = az - oj.z;
+          float d2 = __fmaf_rn(x1, x1, x0 * x0);
+          if (DIM == 3) d2 = __fmaf_rn(x2, x2, d2);
           float thr = thr_u;
           if (!UNIFORM_H) {
             const float hb = 0.5f * (oi.w + fabsf(oj.w));
             thr = cf * cf * hb * hb * margin;
           }
-          return x0 * x0 + x1 * x1 + x2 * x2 <= thr;
-        };
-        auto one = [&](int j) {
-          const int k0 = w.k;
-          w.put(j | tag, inside(j));
-          w.flush(k0, cap, N);
-        };
-        if (dx == 0 && dy == 0 && dz == 0 && lo <= i && i < hi) {  // the home cell: skip i itself
-          for (int j = lo; j < i; ++j) one(j);
-          lo = i + 1;
+          in[e] = d2 <= thr && m > e;
+          if (home) in[e] = in[e] && j + e != i;
+          if (by_sign) in[e] = in[e] && !(oj.w < 0.f);
         }
-        int j = lo;
-        for (; j + 4 <= hi; j += 4) {  // groups of 4: one chunk check per group
-          const bool in0 = inside(j), in1 = inside(j + 1), in2 = inside(j + 2), in3 = inside(j + 3);
-          const int k0 = w.k;
-          w.put(j | tag, in0);
-          w.put((j + 1) | tag, in1);
-          w.put((j + 2) | tag, in2);
-          w.put((j + 3) | tag, in3);
-          w.flush(k0, cap, N);
-        }
-        for (; j < hi; ++j) one(j);
+        const int k0 = w.k;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w.put((j + e) | tag, in[e]);
+        w.flush(k0, cap, N);
+        j += 4;
+        if (j >= end) {
+          j = end;
+          next_cell();
         }
       }
     }
@@ -639,6 +655,16 @@ void launch_nlist(const DevView& v, cudaStream_t st) {
     else if (v.o.dim == 2) nlist_cells_kernel<2, false><<<nb, kNT, 0, st>>>(v, margin);
     else if (v.o.uniform_h) nlist_cells_kernel<3, true><<<nb, kNT, 0, st>>>(v, margin);
     else nlist_cells_kernel<3, false><<<nb, kNT, 0, st>>>(v, margin);
+    return;
+  }
+  // A lane to a particle while the lanes of two particles would fit the SMs at once
+  // (1,024 an SM): then there are too few of them to cover each other's waits
+  // (86k particles in 2D 18 us against 23, 177k in 3D 87 against 107), where more
+  // take the shared loads and tests of two (1.0M in 3D 390 and 355).
+  if (v.o.uniform_h && v.o.nlist_stage == 0 && v.ncap <= 2048ll * sm_count()) {
+    const int nb = (v.ncap + kNT - 1) / kNT;
+    if (v.o.dim == 2) nlist_kernel<2, true><<<nb, kNT, 0, st>>>(v, margin);
+    else nlist_kernel<3, true><<<nb, kNT, 0, st>>>(v, margin);
     return;
   }
   if (v.o.uniform_h) {  // two particles per lane; the leftovers' blocks first

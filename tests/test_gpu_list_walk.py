@@ -9,7 +9,7 @@ import pytest
 
 from oracle.oracle import OracleDomain
 from persiansph_gb300 import scenarios
-from persiansph_gb300.solver import GpuDomain
+from persiansph_gb300.solver import GpuEnsemble, GpuDomain
 from tests.gpu_helpers import assert_step_parity
 
 pytestmark = pytest.mark.gpu
@@ -51,7 +51,7 @@ def test_shaken_lattice(gpu, dim, hfac, split, stage):
 
 
 @pytest.mark.parametrize("dim,split", [(2, 1), (2, 4), (3, 1), (3, 4)])
-def test_more_than_the_lanes_to_a_cell(gpu, dim, split):
+def test_more_than_the_lanes_to_a_cell(gpu, dim, split):  # a lane to a particle
     if dim == 2:
         dx = 0.01
         dom, dt, _ = scenarios.dam_break_2d(dx=dx, L=1.2, H=1.6, TL=2.0, TH=2.0)
@@ -76,3 +76,34 @@ def test_sparse_grid(gpu, split):
     dom, dt, _ = scenarios.dam_break_2d(dx=dx, L=0.5, H=0.65, TL=16.5, TH=16.5)
     shaken(dom.particles, dx, 2)
     one_step(dom, dt, f"sparse {split}", (split, 0))
+
+
+@pytest.mark.parametrize("dim,split", [(2, 1), (2, 4), (3, 1)])
+def test_two_particles_to_a_lane(gpu, dim, split):
+    """Many instances (two particles to a lane) give each the bits it has alone
+    (a lane to a cell, or to a particle): the same lists in the same order."""
+    dx = 0.02 if dim == 2 else 0.04
+    doms = []
+    for seed in range(3):
+        if dim == 2:
+            dom, dt, _ = scenarios.dam_break_2d(dx=dx, L=1.2, H=1.6, TL=2.0, TH=2.0)
+        else:
+            dom, dt, _ = scenarios.dam_break_3d(dx=dx, L=0.7, H=0.5, W=0.6, TL=1.0, TH=0.6, TW=0.6)
+        shaken(dom.particles, dx, dim, seed=seed)
+        doms.append(dom)
+    copies = 152 * 2048 // (3 * doms[0].particles.n) + 2
+    assert 3 * copies * doms[0].particles.n > 152 * 2048
+    b = GpuEnsemble([doms[q % 3].config(dt) for q in range(3 * copies)])
+    b.upload([doms[q % 3].particles for q in range(3 * copies)])
+    b.set_tuning(128, split)
+    b.step(2)
+    for seed, q in ((0, 0), (1, 3 * copies - 2), (2, 3 * copies // 2 // 3 * 3 + 2)):
+        g = GpuDomain(doms[seed].config(dt))
+        g.upload(doms[seed].particles)
+        g.set_tuning(128, split)
+        g.step(2)
+        one, many = g.download_fields(("x", "v", "density", "a")), b.download_fields(q, ("x", "v", "density", "a"))
+        for f in one:
+            assert np.array_equal(one[f], many[f]), f
+        g.close()
+    b.close()
