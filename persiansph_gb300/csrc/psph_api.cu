@@ -1604,7 +1604,8 @@ psph_status split_steps(psph_ctx* c, int64_t nsteps, long long* launched, bool o
       if (c->hook_set_x) offsets32_kernel<<<n > 0 ? (n + 255) / 256 : 1, 256, 0, s>>>(view(c));
     }
     {
-      const DevView v = view(c);
+      DevView v = view(c);
+      v.o.list_all = before && c->hook_freed;  // the sort's list of the fixed particles is not theirs any more
       launch_copies32(v, s);  // the in-flow and the hook may have changed what the sort copied
       if (v.o.fp32) launch_prepare32(v, s);
       else launch_prepare(v, s);

@@ -16,6 +16,7 @@
 //   forces_solid  CalcForce2233 (Source/Interaction.cpp:186-377)
 //   dt_finalize   LastComputeAcceleration's minimum (Source/Domain.cpp:1280-1296)
 //                 and AdaptiveTimeStep (Source/Domain.cpp:133-152)
+#include <algorithm>
 #include <cfloat>
 
 #include "psph_pairs.cuh"
@@ -189,15 +190,17 @@ PSPH_D void soil_records(const DevView& v, const Persist& P, int w, bool fixed, 
 // ---------------------------------------------------------------------------
 // Per-particle preparation and wall interpolation
 // ---------------------------------------------------------------------------
-// The wall interpolation of particles first .. first + (kFT >> lg) - 1 (those
-// that are fixed), 2^lg lanes each; every thread of the block calls it.
+// The wall interpolation of the fixed particles first .. first + (kFT >> lg) - 1 of
+// the sort's list of them (Options::list_all: of all particles, those that are
+// fixed), 2^lg lanes each; every thread of the block calls it.
 template <int DIM, int KT>
 PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int first, int n, double (*sums)[14]) {
   const LaneGroup G(lg);
   const Options& o = v.o;
   const PClass* __restrict__ CT = v.cls;
-  int w = first + (threadIdx.x >> lg);
-  const int winst = (w < n) ? CT[P.cls[w]].inst : 0;
+  auto particle = [&](int k) { return k >= n ? -1 : (o.list_all ? k : v.S.walls[k]); };
+  int w = particle(first + (threadIdx.x >> lg));
+  const int winst = (w >= 0) ? CT[P.cls[w]].inst : 0;
   const GridDev& g = grid_of(v, winst);
   bool wall = false;
   int mat = 0;
@@ -209,7 +212,7 @@ PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int f
   int ow = 0, cell = -1;
   double hw = 0.0;
   bool noslip = false;
-  if (w < n && !v.inst[winst].stop && !CT[P.cls[w]].is_free) {
+  if (w >= 0 && !v.inst[winst].stop && !CT[P.cls[w]].is_free) {
     const PClass& Cw = CT[P.cls[w]];
     wall = true;
     mat = Cw.material;
@@ -296,9 +299,10 @@ PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int f
     }
   }
   __syncthreads();  // (the next batch's barrier at its start keeps its sums off these)
-  w = first + threadIdx.x;
-  if ((int)threadIdx.x >= (kFT >> lg) || w >= n) return;
-  const PClass& Cw = CT[P.cls[w]];
+  w = (int)threadIdx.x < (kFT >> lg) ? particle(first + threadIdx.x) : -1;
+  if (w < 0) return;
+  const int cls_w = P.cls[w];
+  const PClass& Cw = CT[cls_w];
   if (Cw.is_free || v.inst[Cw.inst].stop) return;
   mat = Cw.material;
   noslip = Cw.no_slip;
@@ -329,11 +333,10 @@ PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int f
 #pragma unroll
       for (int e = 0; e < 9; ++e) tw[e] = 0.0;
     }
-    if (sk != 0.0 && mat > 1 && Cw.ti > 0.0) {
-      tensile_tir<DIM>(sig, Cw.ti, xw.w, P.tir + tensor_row(P, w));
-      if (v.S.pair_info) v.S.pair_info[w] = (v.S.pair_info[w] & ~kInfoTir) | tir_bit(v, P, w);
-    }
+    if (sk != 0.0 && mat > 1 && Cw.ti > 0.0) tensile_tir<DIM>(sig, Cw.ti, xw.w, P.tir + tensor_row(P, w));
   }
+  if (v.S.pair_info)  // (the FP32C pair kernels have copies of their own)
+    v.S.pair_info[w] = cls_w | (v.S.cellid[w] >= 0 && v.S.nl_count[w] >= 0 ? kInfoList : 0) | tir_bit(v, P, w);
   // density, 1/density, p/density^2 and sound speed the partners see (Source/Interaction.cpp:41-61)
   double rw = xw.w, cwv = 0.0;
   if (o.uniform_eos && mat != 3) {
@@ -351,41 +354,40 @@ PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int f
   }
 }
 
+// What partners see of every particle. The first wall_blocks blocks interpolate the
+// walls, the others take the free particles, a thread each: neither reads what the
+// other writes, and neither waits for the other. (With both in every block, its
+// walls' lanes after its free particles, blocks waited at their barriers: ten
+// soil columns of 1.0M particles 201 us, so 133; 86k particles in 2D 33 and 24, 177k
+// in 3D, half of them walls, 121 and 112.)
 template <int DIM, int KT>
-__global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v, int lg, int per_block) {
+__global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v, int lg, int wall_blocks) {
   __shared__ double sums[kFT >> kMinLanesLog2][14];  // per wall: kernel, pressure, velocity (3), stress (9) sums
   const StepScalars* sc = v.sc;
   if (sc->all_stop) return;
   const Persist& P = cur_persist(v);
-  const int n = sc->n;
   const Options& o = v.o;
-  const PClass* __restrict__ CT = v.cls;
-  // every particle of the block's range, one thread each: what partners see of
-  // the free ones
-  const int first = blockIdx.x * per_block;
-  const int q = first + threadIdx.x;
-  bool wall_q = false;
-  if ((int)threadIdx.x < per_block && q < n && !v.inst[CT[P.cls[q]].inst].stop) {
-    const int cls = P.cls[q];
-    const PClass& C = CT[cls];
-    wall_q = !C.is_free;
-    if (C.is_free) {
-      const double rho = P.X4[q].w;
-      const double inv = rcp_refined(rho);
-      const double4_32a vel = P.V4[q];
-      if (o.has_solid && C.material > 1 && C.ti > 0.0)
-        tensile_tir<DIM>(P.sigma + tensor_row(P, q), C.ti, rho, P.tir + tensor_row(P, q));
-      if (DIM == 2 && o.soil32) soil_records(v, P, q, false, vel, inv, P.sigma + tensor_row(P, q));
-      else v.S.D4[q] = make_double4_32a(inv, vel.w * inv * inv, sound_speed(C.pres_eq, C.cs, rho, C.rho0), rho);
-    }
-    // (the FP32C pair kernels have copies of their own)
-    if (v.S.pair_info)
-      v.S.pair_info[q] = cls | (C.is_free ? kInfoFree : 0) |
-                         (v.S.cellid[q] >= 0 && v.S.nl_count[q] >= 0 ? kInfoList : 0) | tir_bit(v, P, q);
+  if ((int)blockIdx.x < wall_blocks) {
+    const int n = o.list_all ? sc->n : sc->n_walls, per = kFT >> lg;
+    for (int at = blockIdx.x * per; at < n; at += wall_blocks * per)
+      wall_interpolation<DIM, KT>(v, P, lg, at, n, sums);
+    return;
   }
-  if (__syncthreads_or(wall_q) == 0) return;
-  // the fixed ones, 2^lg lanes each, as many at a time as the block's threads serve
-  for (int at = 0; at < per_block; at += kFT >> lg) wall_interpolation<DIM, KT>(v, P, lg, first + at, n, sums);
+  const int q = (blockIdx.x - wall_blocks) * kFT + threadIdx.x;
+  if (q >= sc->n) return;
+  const int cls = P.cls[q];
+  const PClass& C = v.cls[cls];
+  if (!C.is_free || v.inst[C.inst].stop) return;
+  const double rho = P.X4[q].w;
+  const double inv = rcp_refined(rho);
+  const double4_32a vel = P.V4[q];
+  if (o.has_solid && C.material > 1 && C.ti > 0.0)
+    tensile_tir<DIM>(P.sigma + tensor_row(P, q), C.ti, rho, P.tir + tensor_row(P, q));
+  if (DIM == 2 && o.soil32) soil_records(v, P, q, false, vel, inv, P.sigma + tensor_row(P, q));
+  else v.S.D4[q] = make_double4_32a(inv, vel.w * inv * inv, sound_speed(C.pres_eq, C.cs, rho, C.rho0), rho);
+  if (v.S.pair_info)
+    v.S.pair_info[q] =
+        cls | kInfoFree | (v.S.cellid[q] >= 0 && v.S.nl_count[q] >= 0 ? kInfoList : 0) | tir_bit(v, P, q);
 }
 
 // ---------------------------------------------------------------------------
@@ -1637,17 +1639,12 @@ int lanes_log2(int kt) { return kt == PSPH_QUINTIC_SPLINE ? 3 : 2; }
 template <int DIM>
 void prepare_dispatch(const DevView& v, cudaStream_t st) {
   const int lg = lanes_log2(v.o.kt);
-  // particles per block: as many as its lanes serve at once, so that the walls
-  // spread over the chip; large soil domains, mostly free particles with a
-  // tensile-instability test each, one per thread (ten columns, 1.0M particles:
-  // 371 us against 268; the 177k-particle dam break, half of it walls: 187
-  // against 273)
-  const int per = (v.o.has_solid && v.ncap >= kFT * 1024) ? kFT : kFT >> lg;
-  const int nb = nblk(v.ncap, per);
+  const int walls = std::min(nblk(v.ncap, kFT >> lg), 32 * 152);  // (how many there are is known on the device)
+  const int nb = walls + nblk(v.ncap, kFT);
   switch (v.o.kt) {
-    case 0: prepare_wall_kernel<DIM, 0><<<nb, kFT, 0, st>>>(v, lg, per); break;
-    case 1: prepare_wall_kernel<DIM, 1><<<nb, kFT, 0, st>>>(v, lg, per); break;
-    default: prepare_wall_kernel<DIM, 2><<<nb, kFT, 0, st>>>(v, lg, per); break;
+    case 0: prepare_wall_kernel<DIM, 0><<<nb, kFT, 0, st>>>(v, lg, walls); break;
+    case 1: prepare_wall_kernel<DIM, 1><<<nb, kFT, 0, st>>>(v, lg, walls); break;
+    default: prepare_wall_kernel<DIM, 2><<<nb, kFT, 0, st>>>(v, lg, walls); break;
   }
 }
 

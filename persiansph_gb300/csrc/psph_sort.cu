@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kBT) reorder_kernel(DevView v, const int2* __r
   const int n_new = sc->n;  // the removed particles' segment comes last
   const bool fluid32 = v.o.fp32 && !v.o.has_solid;
   const bool copies = fluid32 && v.o.skin == 0.f;  // (with a skin: skin_offsets_kernel)
-  const bool list_walls = fluid32 && v.o.dim == 2;
+  const bool list_walls = !fluid32 || v.o.dim == 2;  // (the 3D FP32C walls are interpolated where they lie)
   __shared__ int before[kBT / 32];  // walls of the block's warps before each
   __shared__ int list_at;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
