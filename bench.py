@@ -66,25 +66,23 @@ REF_BUDGET_S = 90.0
 # CalcForce11 does once per unordered pair (Source/Interaction.cpp:139-145).
 FLOPS_PER_PAIR = 106
 # Algorithmic HBM bytes per particle of one FP32C fluid pair-kernel launch:
-# read each particle's inputs once (offset+h 16, v+p 16, 1/rho, p/rho^2, c, rho
-# 16, class 4, cell 4) and write its outputs once (a + drho 32, zwab 8, sumden
+# read each particle's inputs once (offset and 1/rho 16, v+p 16, v's low-order
+# part and c 16, class 4, cell 4) and write its outputs once (a + drho 32, zwab 8, sumden
 # 8) = 104 B; with LES and the closure also the viscosity (4), the strain-rate
 # sums (6 x 4) and the closure's four features (16) = 148 B.
 FORCE32_BYTES_PER_PARTICLE = {False: 104, True: 148}
 # DRAM bytes per particle one launch actually moved: ncu captures of the same
 # kernels on the same tank at dx = 10 mm (1,021,104 particles),
-# dram__bytes_read.sum + dram__bytes_write.sum per particle (LES + closure
-# flavour with the 5 % list skin the autotuner picks: 276.56 + 54.12 MB; without
-# LES: an earlier capture of that flavour, lists every step); the traffic grows
+# dram__bytes per particle (LES + closure flavour with the 5 % list skin the
+# autotuner picks: 340.8 MB; without LES, lists every step: 324.6 MB); the traffic grows
 # with the particle count, so a full-size launch moves this x n. Most of the
 # excess over the algorithmic bytes is the neighbour list (~80 entries x 4 B a
 # particle).
-FORCE32_TRAFFIC_BYTES_PER_PARTICLE = {False: 304.6, True: 323.9}
+FORCE32_TRAFFIC_BYTES_PER_PARTICLE = {False: 317.9, True: 333.8}
 # Pipe activity of that launch (LES + closure flavour, list skin) and of the FP64
-# pair kernel (pass A) in the same capture series (sm__pipe_*_cycles_active, % of
-# peak).
-FORCE32_NCU = {"issue_active": 0.573, "fma_pipe": 0.297, "fp64_pipe": 0.040, "warps_active": 0.298}
-FORCE64_NCU_FP64_PIPE = 0.834
+# pair kernel (pass A, 177,156 particles; sm__pipe_fp64_cycles_active, % of peak).
+FORCE32_NCU = {"issue_active": 0.609, "l1_wavefronts": 0.557, "fp64_pipe": 0.066, "warps_active": 0.239}
+FORCE64_NCU_FP64_PIPE = 0.785
 
 
 def peaks():
@@ -527,11 +525,11 @@ def main():
         "fp32c_closure_over_fp64_steps_per_s": m32["steps_per_s"] / m64["steps_per_s"],
         "roofline": {"bound": "hbm", "achieved": achieved_gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved_gbs / pk["hbm_gbs"], "traffic": traffic,
-                     "kernel": "forces_fluid32_kernel", "peak_source": pk["src"],
+                     "kernel": "forces_spec32_kernel", "peak_source": pk["src"],
                      "bytes_per_particle": FORCE32_BYTES_PER_PARTICLE[cl],
-                     "note": "latency-bound gather kernel (neither HBM nor tensor bound); ncu pipe activity of "
+                     "note": "bound by issue slots and L1 gathers (neither HBM nor tensor bound); ncu activity of "
                              "the same kernel at dx=10 mm in ncu_small_case "
-                             "(profiles/pair_kernel_skin_dam3d_10mm.md)",
+                             "(profiles/step_kernels_small_cases.md)",
                      "ncu_small_case": FORCE32_NCU},
         "roofline_fp64": {"bound": "fp64", "kernel": "forces_fluid_kernel", "achieved": fp64_tflops,
                           "peak": fp64.value, "unit": "TFLOP/s",
@@ -540,7 +538,7 @@ def main():
                           "fp64_pipe_active_ncu_small_case": FORCE64_NCU_FP64_PIPE,
                           "note": "frac counts 106 algorithmic FP64 flops per pair-interaction (one evaluation "
                                   "and the partner's terms, each pair once) against the DFMA rate; the FP64 pipe "
-                                  "itself is ~83 % busy (square roots, divisions, conversions, idle lanes)"},
+                                  "itself is ~78 % busy (square roots, divisions, conversions, idle lanes)"},
         "clocks": m32["clocks"],
         "e2e": {"value": e2e_v, "unit": UNIT, "h2d_bytes_per_step": h2d / max(done_e, 1),
                 "d2h_bytes_per_step": d2h / max(done_e, 1), "steps": done_e,

@@ -105,7 +105,7 @@ struct StepScalars {
   int all_stop;   // every instance has reached its stop time
   int buf;        // which persistent buffer (A=0 / B=1) holds the current sorted state
   unsigned long long pairs_x2;  // 2 x pair-interactions evaluated since upload
-  unsigned int work;            // tile counter of the persistent pair kernels
+  unsigned int work;            // blocks of the update that have finished (Options::fused_tail; zero between steps)
   int launches;
   unsigned long long closure_eval, closure_fallback;  // closure evaluations / Smagorinsky fallbacks
   int nl_rest;    // particles the neighbour-list scan handles one per lane (set by the sort)

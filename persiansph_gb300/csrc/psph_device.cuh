@@ -45,7 +45,7 @@ struct Scratch {
   float4* OFFREF;    // with a skin: the position at the last rebuild in FP32 (displacements are measured from it)
   int* refcell;      // with a skin: each particle's cell in the reference's grid (x | y << 10 | z << 20),
                      // for the wall pressure's pair orientation
-  int* nl;           // per-step neighbour lists, entry k of particle i at nl[k*ncap + i]:
+  int* nl;           // per-step neighbour lists, entry k of particle i at nl[nl_index(stride, i, k)]:
                      // index | cell-offset code << 26
   int* nl_count;     // list length, or -1 when it exceeded the capacity (scan instead)
   float4* PX32;      // FP32C form, Options::spec32: (position - cell origin, +-1/density), negative for a fixed one
