@@ -107,3 +107,14 @@ def test_two_particles_to_a_lane(gpu, dim, split):
             assert np.array_equal(one[f], many[f]), f
         g.close()
     b.close()
+
+
+@pytest.mark.parametrize("dx,split", [(0.05, 1), (0.05, 4), (0.01, 2)])
+def test_unlike_smoothing_lengths(gpu, dx, split):  # a lane to a cell, and to a particle
+    dom, dt, _ = scenarios.dam_break_2d(dx=dx, L=0.5 if dx > 0.02 else 1.2, H=0.65 if dx > 0.02 else 1.6, TL=2.0, TH=2.0)
+    p = dom.particles
+    shaken(p, dx, 2)
+    h = p.get("h")
+    h *= 1.0 + 0.15 * np.random.default_rng(9).random(len(h))
+    p.set("h", h)
+    one_step(dom, dt, f"h, dx {dx}", (split, 0))
