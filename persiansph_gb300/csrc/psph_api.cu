@@ -2256,10 +2256,9 @@ psph_status patch_impl(psph_ctx* c, const psph_particles* p) {
     CUDA_TRY(c, cudaMemcpyAsync(c->d_cls, c->classes.data(), c->classes.size() * sizeof(PClass),
                                 cudaMemcpyHostToDevice, s));
     launch_class_constants(c->d_cls, (int)c->classes.size(), o.dim, s);
-    // constants the pair kernel takes from the launch may no longer be shared
-    c->opt.spec64 = o1.spec64;
-    c->opt.ti_always = o1.ti_always;
-    c->opt.spec = o1.spec;
+    // every option that follows from the parameter sets, not some of them: constants
+    // that a kernel takes from one particle or from the launch may no longer be shared
+    c->opt = o1;
     c->opt.nclasses = (int)c->classes.size();
     int* dnext = reinterpret_cast<int*>(c->dl_buf);
     CUDA_TRY(c, cudaMemcpyAsync(dnext, next.data(), (size_t)m * sizeof(int), cudaMemcpyHostToDevice, s));
