@@ -24,6 +24,7 @@
 #include <mutex>
 #include <vector>
 
+#include "psph_bins.cuh"
 #include "psph_device.cuh"
 #include "psph_inout.cuh"
 #include "psph_mlp.cuh"
@@ -34,8 +35,6 @@ using namespace psph;
 // Phases timed by psph_phase_times: sort, neighbour lists, prepare, pair
 // forces, closure, dt, update.
 constexpr int kNumPhases = 7;
-// Finest split of the cells into x-slabs in the sort (Options::xsub).
-constexpr int kMaxXsub = 4;
 // Deepest staging of the neighbour search (Options::nlist_stage, candidates per block).
 constexpr int kMaxStage = 4096;
 constexpr int kMaxSkinPermille = 150;  // list skins up to 15 % of the support (the lists' capacity)
@@ -939,11 +938,11 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
     gd.cellfac2_32 = (float)(gd.cellfac * gd.cellfac);
     g.cellfac = gd.cellfac;
     const long long nci = (long long)gd.nc[0] * gd.nc[1] * gd.nc[2];
-    if (nci > (1LL << 28)) return set_err(c, PSPH_ERR_UNSUPPORTED, "grid has more than 2^28 cells");
+    if (nci > kMaxCells) return set_err(c, PSPH_ERR_UNSUPPORTED, "grid has more than 2^28 cells");
     gd.ncells = (int)nci;
     gd.cell_base = (int)cell_base;
     cell_base += nci;
-    if (cell_base > (1LL << 28))
+    if (cell_base > kMaxCells)
       return set_err(c, PSPH_ERR_UNSUPPORTED, "the instances' grids hold more than 2^28 cells");
   }
   c->total_cells = (int)cell_base;

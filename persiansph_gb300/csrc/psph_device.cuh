@@ -30,7 +30,7 @@ struct Persist {
 
 // Per-step arrays (sorted order of the current step; not reordered).
 struct Scratch {
-  int* key;        // cell key per particle (pre-sort order)
+  unsigned* key;   // sort bin per particle (pre-sort order)
   int* count;      // ncells + 2 counters
   int* start;      // ncells + 3 exclusive prefix: cell c's particles are [start[c], start[c+1])
   int* sstart;     // 2 ncells * xsub + 3 exclusive prefix over the x-slabs of the cells, free and fixed apart

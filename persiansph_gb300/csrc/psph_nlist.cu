@@ -147,9 +147,9 @@ __device__ __forceinline__ void list_one(const DevView& v, int i, float margin, 
         else if (x < 0 || x >= g.nc[0]) return;
         const int s0 = max(slo - dx * xs, 0), s1 = min(shi - dx * xs, xs - 1);
         if (s0 > s1) return;
-        const int bin = 2 * ((base + x) * xs + s0);
+        const unsigned bin = sort_bin(base + x, xs, s0);
         lo = sstart[bin];
-        hi = sstart[free_half ? bin + 1 : 2 * ((base + x) * xs + s1 + 1)];
+        hi = sstart[free_half ? bin + 1 : sort_bin(base + x, xs, s1 + 1)];
       };
       range(-1, lo0, hi0);
       range(0, lo1, hi1);
@@ -434,9 +434,9 @@ __device__ __forceinline__ void scan_two(const DevView& v, int ia, int n, float 
         else if (x < 0 || x >= g.nc[0]) return;
         const int s0 = max(slo - dx * xs, 0), s1 = min(shi - dx * xs, xs - 1);
         if (s0 > s1) return;
-        const int bin = 2 * ((base + x) * xs + s0);
+        const unsigned bin = sort_bin(base + x, xs, s0);
         lo = sstart[bin];
-        hi = sstart[free_half ? bin + 1 : 2 * ((base + x) * xs + s1 + 1)];
+        hi = sstart[free_half ? bin + 1 : sort_bin(base + x, xs, s1 + 1)];
       };
       range(-1, lo0, hi0);
       range(0, lo1, hi1);

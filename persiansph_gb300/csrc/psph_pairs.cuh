@@ -7,6 +7,7 @@
 #include <cfloat>
 #include <climits>
 
+#include "psph_bins.cuh"
 #include "psph_device.cuh"
 
 namespace psph {

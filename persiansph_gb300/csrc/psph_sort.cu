@@ -20,6 +20,8 @@
 //            sorted state depends only on positions, never on atomic timing;
 //            each particle's fields move to that place (HBM-bound), with its
 //            FP32 copies and the list of the fixed particles.
+// A cell takes 64 bytes: 8 bins (4 slabs, free and fixed) in the counts and in their
+// scan, 17 GB at the limit of 2^28 cells (half of it with one bin for both kinds).
 // Four launches (five with more than 131,072 bins): launches are what counts up
 // to 100k particles. With six 5k particles took 40 us, so 31; 920 in the FP32C
 // form, their copies included, 37 and 25.
@@ -34,16 +36,16 @@ namespace {
 
 constexpr int kBT = 256;
 
-__global__ void bin_kernel(DevView v, const uint8_t* __restrict__ alive, int* __restrict__ key,
+__global__ void bin_kernel(DevView v, const uint8_t* __restrict__ alive, unsigned* __restrict__ key,
                            int* __restrict__ count, int* __restrict__ slot_of, StepScalars* sc, int dim, int xsub) {
   if (sc->all_stop || !sc->rebuild) return;
   const Persist& P = cur_persist(v);
   const int n = sc->n;
-  const int nbins = 2 * v.total_cells * xsub;
+  const unsigned nbins = sort_bin(v.total_cells, xsub, 0);
   if (blockIdx.x == 0 && threadIdx.x == 0) sc->nl_rest = sc->n_walls = 0;  // counted by the scatter and the reorder
-  const int orphan_key = nbins, dead_key = nbins + 1;
+  const unsigned orphan_key = nbins, dead_key = nbins + 1;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    int k;
+    unsigned k;
     if (!alive[i]) {
       k = dead_key;
     } else {
@@ -77,7 +79,7 @@ __global__ void bin_kernel(DevView v, const uint8_t* __restrict__ alive, int* __
           const float ox = d2f_bits(x.x - g.blpf[0]) - (float)c[0] * g.cell_size32[0];
           slab = min(max((int)floorf(ox * (float)xsub * g.inv_cell_size32[0]), 0), xsub - 1);
         }
-        k = 2 * ((g.cell_base + (c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0]) * xsub + slab) + (C.is_free ? 0 : 1);
+        k = sort_bin(g.cell_base + (c[2] * g.nc[1] + c[1]) * g.nc[0] + c[0], xsub, slab) + (C.is_free ? 0 : 1);
       }
     }
     key[i] = k;
@@ -92,39 +94,37 @@ __global__ void bin_kernel(DevView v, const uint8_t* __restrict__ alive, int* __
   }
 }
 
-// Exclusive scan of `in` (len entries): a thread takes kScanPer consecutive
-// entries, a block kScanBlock.
-constexpr int kScanPer = 8, kScanBlock = 1024 * kScanPer;
+// Exclusive scan of `in` (len entries; psph_bins.cuh has its shape).
 
 // A thread's entries, from `first` (a multiple of 8), as 16-byte accesses: entry by
 // entry a warp's accesses are 32 bytes apart (the sort of 86k particles into 167k bins
 // 41 us, so 37; of 957k into 2.4M 117 and 109).
-__device__ __forceinline__ void load_entries(const int* __restrict__ in, int first, int len, int (&v)[kScanPer]) {
+__device__ __forceinline__ void load_entries(const int* __restrict__ in, unsigned first, unsigned len, int (&v)[kScanPer]) {
   static_assert(kScanPer == 8, "two int4");
-  if (first + kScanPer <= len) {
+  if (scan_full(first, kScanPer, len)) {
     const int4 a = *reinterpret_cast<const int4*>(in + first), b = *reinterpret_cast<const int4*>(in + first + 4);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
   } else {
 #pragma unroll
-    for (int e = 0; e < kScanPer; ++e) v[e] = (first + e < len) ? in[first + e] : 0;
+    for (unsigned e = 0; e < kScanPer; ++e) v[e] = (first + e < len) ? in[first + e] : 0;
   }
 }
 // their exclusive prefixes from `at`
-__device__ __forceinline__ void store_prefixes(int* __restrict__ out, int first, int len, int at,
+__device__ __forceinline__ void store_prefixes(int* __restrict__ out, unsigned first, unsigned len, int at,
                                                const int (&v)[kScanPer]) {
   int p[kScanPer];
 #pragma unroll
-  for (int e = 0; e < kScanPer; ++e) {
+  for (unsigned e = 0; e < kScanPer; ++e) {
     p[e] = at;
     at += v[e];
   }
-  if (first + kScanPer <= len) {
+  if (scan_full(first, kScanPer, len)) {
     *reinterpret_cast<int4*>(out + first) = make_int4(p[0], p[1], p[2], p[3]);
     *reinterpret_cast<int4*>(out + first + 4) = make_int4(p[4], p[5], p[6], p[7]);
   } else {
 #pragma unroll
-    for (int e = 0; e < kScanPer; ++e)
+    for (unsigned e = 0; e < kScanPer; ++e)
       if (first + e < len) out[first + e] = p[e];
   }
 }
@@ -136,7 +136,7 @@ __device__ __forceinline__ int block_scan(const int (&v)[kScanPer], int* total) 
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   int own = 0;
 #pragma unroll
-  for (int e = 0; e < kScanPer; ++e) own += v[e];
+  for (unsigned e = 0; e < kScanPer; ++e) own += v[e];
   int incl = own;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -175,7 +175,7 @@ __device__ __forceinline__ int block_sum(int part) {
 // current one: nothing but the reorder, which knows, reads it in between. at is
 // the prefix of entry i (len = bins + 2: the orphans' and the removed particles'
 // segments come last).
-__device__ __forceinline__ void sorted_counts(StepScalars* sc, int i, int len, int at) {
+__device__ __forceinline__ void sorted_counts(StepScalars* sc, unsigned i, unsigned len, int at) {
   if (i == len - 2) sc->n_cells = at;
   if (i == len - 1) {
     sc->n_old = sc->n;
@@ -183,7 +183,7 @@ __device__ __forceinline__ void sorted_counts(StepScalars* sc, int i, int len, i
     sc->buf ^= 1;
   }
 }
-__device__ __forceinline__ void sorted_counts4(StepScalars* sc, int i, int len, int4 at) {
+__device__ __forceinline__ void sorted_counts4(StepScalars* sc, unsigned i, unsigned len, int4 at) {
   if (i + 4 < len - 1 || i >= len) return;
   sorted_counts(sc, i, len, at.x);
   sorted_counts(sc, i + 1, len, at.y);
@@ -194,14 +194,14 @@ __device__ __forceinline__ void sorted_counts4(StepScalars* sc, int i, int len, 
 // Few blocks: each sums the entries before its own itself, so that one launch
 // does it (up to 16 blocks, 131,072 bins: the last one reads 480 KB, 3 us, where
 // a second launch costs as much).
-constexpr int kScanWhole = 16;
-__global__ void __launch_bounds__(1024) scan_whole(const int* __restrict__ in, int* __restrict__ out, int len,
+constexpr unsigned kScanWhole = 16;
+__global__ void __launch_bounds__(1024) scan_whole(const int* __restrict__ in, int* __restrict__ out, unsigned len,
                                                    StepScalars* sc) {
   if (sc && (sc->all_stop || !sc->rebuild)) return;  // the cell sort's scan, on a step without a rebuild
-  const int t = threadIdx.x, first = blockIdx.x * kScanBlock + t * kScanPer;
+  const unsigned t = threadIdx.x, first = scan_first(blockIdx.x, t);
   int before = 0;
 #pragma unroll 4
-  for (int i = t; i < (int)blockIdx.x * (kScanBlock / 4); i += 1024) {
+  for (unsigned i = t; i < blockIdx.x * (kScanBlock / 4); i += 1024) {
     const int4 q = reinterpret_cast<const int4*>(in)[i];
     before += q.x + q.y + q.z + q.w;
   }
@@ -220,9 +220,9 @@ __global__ void __launch_bounds__(1024) scan_whole(const int* __restrict__ in, i
 
 // Many blocks, phase 1: each block's own scan, its total to sums.
 __global__ void __launch_bounds__(1024) scan_blocks(const int* __restrict__ in, int* __restrict__ out,
-                                                    int* __restrict__ sums, int len, const StepScalars* sc) {
+                                                    int* __restrict__ sums, unsigned len, const StepScalars* sc) {
   if (sc && (sc->all_stop || !sc->rebuild)) return;
-  const int first = blockIdx.x * kScanBlock + threadIdx.x * kScanPer;
+  const unsigned first = scan_first(blockIdx.x, threadIdx.x);
   int v[kScanPer], total;
   load_entries(in, first, len, v);
   const int at = block_scan(v, &total);
@@ -232,18 +232,18 @@ __global__ void __launch_bounds__(1024) scan_blocks(const int* __restrict__ in, 
 
 // Phase 2: every block adds the totals of the blocks before it; the last one
 // writes the grand total.
-__global__ void __launch_bounds__(1024) scan_add(int* __restrict__ out, const int* __restrict__ sums, int len,
+__global__ void __launch_bounds__(1024) scan_add(int* __restrict__ out, const int* __restrict__ sums, unsigned len,
                                                  StepScalars* sc) {
   if (sc && (sc->all_stop || !sc->rebuild)) return;
-  const int t = threadIdx.x;
+  const unsigned t = threadIdx.x;
   int before = 0;
-  for (int b = t; b < (int)blockIdx.x; b += 1024) before += sums[b];
+  for (unsigned b = t; b < blockIdx.x; b += 1024) before += sums[b];
   before = block_sum(before);
   // four consecutive entries, twice: 16-byte accesses that follow one another
 #pragma unroll
-  for (int h = 0; h < kScanPer / 4; ++h) {
-    const int i = blockIdx.x * kScanBlock + h * 4096 + 4 * t;
-    if (i + 4 <= len) {
+  for (unsigned h = 0; h < kScanPer / 4; ++h) {
+    const unsigned i = blockIdx.x * kScanBlock + h * 4096 + 4 * t;
+    if (scan_full(i, 4, len)) {
       int4 q = *reinterpret_cast<int4*>(out + i);
       q.x += before; q.y += before; q.z += before; q.w += before;
       *reinterpret_cast<int4*>(out + i) = q;
@@ -251,17 +251,15 @@ __global__ void __launch_bounds__(1024) scan_add(int* __restrict__ out, const in
     } else {
       int4 q = make_int4(0, 0, 0, 0);
       int* const e = &q.x;
-      for (int k = 0; k < 4 && i + k < len; ++k) out[i + k] = e[k] = out[i + k] + before;
+      for (unsigned k = 0; k < 4 && i + k < len; ++k) out[i + k] = e[k] = out[i + k] + before;
       if (sc) sorted_counts4(sc, i, len, q);
     }
   }
   if (blockIdx.x == gridDim.x - 1 && t == 0) out[len] = before + sums[blockIdx.x];
 }
 
-inline int scan_blocks_for(int len) { return len > kScanBlock ? (len - 1) / kScanBlock + 1 : 1; }
-
-void scan_launch(const int* in, int* out, int len, int* sums, StepScalars* sc, cudaStream_t st) {
-  const int nb = scan_blocks_for(len);
+void scan_launch(const int* in, int* out, unsigned len, int* sums, StepScalars* sc, cudaStream_t st) {
+  const unsigned nb = scan_blocks_for(len);
   if (nb <= kScanWhole) {
     scan_whole<<<nb, 1024, 0, st>>>(in, out, len, sc);
   } else {
@@ -278,7 +276,7 @@ void scan_launch(const int* in, int* out, int len, int* sums, StepScalars* sc, c
 // sorted particles 2t and 2t+1 together when they share a cell, so the odd
 // particles left are exactly the cells' first particles at odd indices (into
 // rest, at most cap). The counts are cleared for the next sort.
-__global__ void scatter_kernel(DevView v, const int* __restrict__ key, const int* __restrict__ sstart,
+__global__ void scatter_kernel(DevView v, const unsigned* __restrict__ key, const int* __restrict__ sstart,
                                const int* __restrict__ slot_of, int2* __restrict__ tmp_perm, int* __restrict__ count,
                                int* __restrict__ start, int ncells, int xsub, StepScalars* sc,
                                int* __restrict__ rest, int cap) {
@@ -318,8 +316,8 @@ __global__ void scatter_kernel(DevView v, const int* __restrict__ key, const int
 // With it go the FP32 offset from the cell's origin, an FP32C fluid's copies, and
 // the list of the fixed particles (written by warps of places that ascend, so
 // that a warp of the list lies close together).
-__global__ void __launch_bounds__(kBT) reorder_kernel(DevView v, const int2* __restrict__ tmp_perm, const int* __restrict__ key, const int* __restrict__ start, int* __restrict__ cellid,
-                               uint8_t* __restrict__ alive, StepScalars* sc, int nbins, int xsub, int dyn_mu) {
+__global__ void __launch_bounds__(kBT) reorder_kernel(DevView v, const int2* __restrict__ tmp_perm, const unsigned* __restrict__ key, const int* __restrict__ start, int* __restrict__ cellid,
+                               uint8_t* __restrict__ alive, StepScalars* sc, unsigned nbins, int xsub, int dyn_mu) {
   if (sc->all_stop || !sc->rebuild) return;
   const Persist& src = next_persist(v);  // (the scan has made the sorted state's buffer the current one)
   const Persist& dst = cur_persist(v);
@@ -336,7 +334,7 @@ __global__ void __launch_bounds__(kBT) reorder_kernel(DevView v, const int2* __r
     if (q < n_new) {
       const int2 own = tmp_perm[q];
       const int i = own.x, mine = own.y;
-      const int k = key[i];
+      const unsigned k = key[i];
       const int lo = start[k], hi = start[k + 1];
       int s = lo;
       for (int t = lo; t < hi; ++t) s += tmp_perm[t].y < mine;
@@ -354,7 +352,7 @@ __global__ void __launch_bounds__(kBT) reorder_kernel(DevView v, const int2* __r
       float4 off;
       if (k < nbins) {
         const GridDev& g = grid_of(v, v.cls[cls].inst);
-        const int lk = k / (2 * xsub) - g.cell_base;
+        const int lk = (int)(k / sort_bin(1, xsub, 0)) - g.cell_base;
         const int cx = lk % g.nc[0], t = lk / g.nc[0], cy = t % g.nc[1], cz = t / g.nc[1];
         off = make_float4(d2f_rn(xs.x - (g.blpf[0] + i2d_small(cx) * g.cell_size[0])),
                           d2f_rn(xs.y - (g.blpf[1] + i2d_small(cy) * g.cell_size[1])),
@@ -368,7 +366,7 @@ __global__ void __launch_bounds__(kBT) reorder_kernel(DevView v, const int2* __r
       if (copies) fluid_copies32(v, dst, s, cls, xs.w, vs, off, 0);
       dst.orig[s] = mine;
       if (src.io) dst.io[s] = src.io[i];
-      cellid[s] = (k < nbins) ? k / (2 * xsub) : -1;
+      cellid[s] = (k < nbins) ? (int)(k / sort_bin(1, xsub, 0)) : -1;
       alive[s] = 1;
       if (!is_free) wall = s;
     }
@@ -458,8 +456,7 @@ void launch_sort(const DevView& v, cudaStream_t st) {
   const Scratch& S = v.S;
   const int ncells = v.total_cells;
   const int xsub = v.o.xsub;
-  const int nbins = 2 * ncells * xsub;
-  const int len = nbins + 2;
+  const unsigned nbins = sort_bin(ncells, xsub, 0), len = nbins + 2;
   // with a skin most steps skip the sort: few enough blocks that skipping is cheap
   // (6.7M particles: 67 us a step for the skipped launches, 25 so)
   const int gp = v.o.skin > 0.f ? std::min(grid_for(v.ncap), 4096) : grid_for(v.ncap);
@@ -472,7 +469,7 @@ void launch_sort(const DevView& v, cudaStream_t st) {
                                      v.o.dyn_mu);
 }
 
-int sort_launches(const DevView& v) { return scan_blocks_for(2 * v.total_cells * v.o.xsub + 2) <= kScanWhole ? 4 : 5; }
+int sort_launches(const DevView& v) { return scan_blocks_for(sort_bin(v.total_cells, v.o.xsub, 0) + 2) <= kScanWhole ? 4 : 5; }
 
 }  // namespace psph
 
