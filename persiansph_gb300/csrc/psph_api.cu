@@ -584,9 +584,10 @@ void derive_class_options(const std::vector<PClass>& classes, bool mixed, bool d
     }
     if (ff < 0) ff = 0;
     if (fw < 0) fw = 0;
-    o.spec32 = o.fp32 && o.vis_eq == PSPH_MORRIS && o.grad_type == PSPH_SQUARED_DENSITY && o.uniform_h &&
-               o.uniform_av && o.uniform_mass && (o.uniform_mu || dyn_mu) && !o.any_ti && o.xsph == 0.0 &&
-               !o.has_solid && one;
+    o.flavours32 = o.fp32 && o.vis_eq == PSPH_MORRIS && o.grad_type == PSPH_SQUARED_DENSITY && o.uniform_h &&
+                   o.uniform_av && o.uniform_mass && (o.uniform_mu || dyn_mu) && !o.any_ti && o.xsph == 0.0 &&
+                   !o.has_solid;
+    o.spec32 = o.flavours32 && one;
     // the FP32C 2D soil kernel's: also one sound speed and tensile instability, and
     // one free mass per instance
     bool soil = o.fp32 && o.dim == 2 && o.grad_type == PSPH_SQUARED_DENSITY && o.xsph == 0.0 && o.uniform_h &&

@@ -148,7 +148,8 @@ struct Options {
   float alpha32, beta32, m_free32, fpm_wall32;
   int spec64;         // the FP64 fluid pair kernel's SPEC form applies, with these constants
   Spec64 spec;
-  int spec32;         // the FP32C fluid pair kernel's
+  int flavours32;     // the FP32C fluid pair kernel's compiled flavours apply
+  int spec32;         // its constant-parameter form too: every free and every fixed class has the same flags
   int soil32;         // the FP32C 2D soil pair kernel's constant-parameter form applies
   int soil_noslip;    // (with it) a wall or its partner is no-slip
   Spec32 spec32c;

@@ -306,12 +306,25 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
 // ---------------------------------------------------------------------------
 // Fluid pair force, FP32 with compensated sums, over the neighbour lists
 // ---------------------------------------------------------------------------
-// Every option read at run time (forces_spec32_kernel serves the usual ones).
+// FL 0: every option read at run time. FL 1, 2 and 3: Morris viscosity,
+// squared-density gradient, no tensile instability or XSPH, one h, and pair
+// constants (artificial viscosity, masses) the same for every class, taken from
+// the launch (Options::flavours32), without (1) or with (2) the strain-rate sums
+// of LES and Bingham, or with the learned closure's vorticity too (3); the
+// classes' flags may differ (a slip lid over no-slip walls, LES on part of the
+// fluid), where forces_spec32_kernel wants them alike and is faster.
 // The list walk is a counted loop so that the next neighbour's loads can be
 // issued before this one's arithmetic; each pair issues all of its neighbour
 // loads before the support test (ld_early).
-template <int DIM, int KT>
-__global__ void __maxnreg__(128) forces_fluid32_kernel(DevView v) {
+// Register caps measured on the 6.7M-particle dam break (64 to 112 swept): the
+// strain-rate flavours run best at 96 (20 warps/SM), the plain one at 80, the
+// general one at 128. A tank with a slip lid, 1.0M particles, through FL 0 and its
+// flavour: 916 and 495 us without rates, 1049 and 606 with LES, 1012 and 606 with
+// the closure; 86k in 2D 44 and 25.
+template <int DIM, int KT, int FL>
+__global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_kernel(DevView v) {
+  constexpr bool SPEC = FL != 0;
+  constexpr bool CLOSURE = FL == 3;
   __shared__ unsigned long long cred[32];
   const StepScalars* sc = v.sc;
   if (sc->all_stop) return;
@@ -348,13 +361,13 @@ __global__ void __maxnreg__(128) forces_fluid32_kernel(DevView v) {
   const int fi = Ci.flags;
   const bool shep = (fi & CF_SHEPARD) && (Is.shepard_counter == o.shepard_step);
   const bool sr_self = fi & (CF_T0 | CF_LES);
-  const bool use_sr = o.need_sr;
-  const bool xsph_on = o.xsph != 0.0;
+  const bool use_sr = SPEC ? (FL >= 2) : (bool)o.need_sr;
+  const bool xsph_on = SPEC ? false : o.xsph != 0.0;
   const float xsph = o.xsph32;
   const float3 cs = cell_size_f(g);
   const float mu_u = o.mu_u32;
   const bool uniform_mu = o.uniform_mu, dyn_mu = o.dyn_mu;
-  const int vis_eq = o.vis_eq, grad_type = o.grad_type;
+  const int vis_eq = SPEC ? 0 : o.vis_eq, grad_type = SPEC ? 0 : o.grad_type;
   Kahan ax, ay, az, dr;
   float zw = 0.f, sd = 0.f, xs0 = 0.f, xs1 = 0.f, xs2 = 0.f;
   // strain-rate sums as sums of products a_r x_c (a = c2 vab): diagonal
@@ -363,8 +376,9 @@ __global__ void __maxnreg__(128) forces_fluid32_kernel(DevView v) {
   // apart (m01, m10, ...)
   float m00 = 0.f, m11 = 0.f, m22 = 0.f, m01 = 0.f, m02 = 0.f, m12 = 0.f, m10 = 0.f, m20 = 0.f, m21 = 0.f;
   int nnb = 0;
-  const bool closure = o.closure && (fi & CF_LES);
-  const bool split_sr = closure;
+  const bool closure = SPEC ? (CLOSURE && (fi & CF_LES)) : (o.closure && (fi & CF_LES));
+  // the closure flavour always keeps the antisymmetric sums apart
+  const bool split_sr = SPEC ? CLOSURE : closure;
   const float cf2 = g.cellfac2_32;
   const bool uniform_h = o.uniform_h;
   const float ih_u = o.inv_h32;
@@ -377,11 +391,11 @@ __global__ void __maxnreg__(128) forces_fluid32_kernel(DevView v) {
     const int clsj = wj & 0xffff;
     float x0, x1, x2;
     rel_pos<DIM>(cs, oi, oj, code, x0, x1, x2);
-    const float hb = 0.5f * (hi + fabsf(oj.w));
+    const float hb = SPEC ? hi : 0.5f * (hi + fabsf(oj.w));  // one h: (h + h) / 2 = h exactly
     const float r2 = x0 * x0 + x1 * x1 + x2 * x2;
     // the list's own support test (exact in FP32; lists with a skin hold more)
     if (r2 > cf2 * hb * hb) return;
-    const PClass32& Cj = CT[clsj];
+    const PClass32& Cj = CT[SPEC ? 0 : clsj];
     const int fjf = wj >> 16;
     const bool fj = fjf & CF_FREE;
     npair2 += fj ? 1u : 2u;
@@ -397,20 +411,20 @@ __global__ void __maxnreg__(128) forces_fluid32_kernel(DevView v) {
     const float GK = KernF<DIM, KT>::GK(q, inv_q, cwg);
     const float K = KernF<DIM, KT>::W(q, cwh);
     const float dj = dj4.w, inv_j = dj4.x, Pj = dj4.y, cj_snd = dj4.z, pj = vj.w;
-    const float mj = fj ? Cj.mass : Cj.fpmassc * mi;
+    const float mj = SPEC ? (fj ? o.m_free32 : o.fpm_wall32 * mi) : (fj ? Cj.mass : Cj.fpmassc * mi);
     const float v0 = (vi.x - vj.x) + (vil.x - vjl.x), v1 = (vi.y - vj.y) + (vil.y - vjl.y),
                 v2 = (vi.z - vj.z) + (vil.z - vjl.z);
     const float vx = v0 * x0 + v1 * x1 + v2 * x2;
     float PI = 0.f;
-    const float Alpha = 0.5f * (Ci.alpha + Cj.alpha);
-    const float Beta = 0.5f * (Ci.beta + Cj.beta);
+    const float Alpha = SPEC ? o.alpha32 : 0.5f * (Ci.alpha + Cj.alpha);
+    const float Beta = SPEC ? o.beta32 : 0.5f * (Ci.beta + Cj.beta);
     if ((Alpha != 0.f || Beta != 0.f) && vx < 0.f) {
       const float D = r2 + 0.01f * hb * hb;
       const float t = hb * vx;
       PI = __fdividef(t * (-Alpha * 0.5f * (ci_snd + cj_snd) * D + Beta * t), D * D * (0.5f * (di + dj)));
     }
     float TI = 0.f;
-    if ((fi | fjf) & CF_TI) {
+    if (!SPEC && ((fi | fjf) & CF_TI)) {
       float Ri = 0.f, Rj = 0.f;
       if ((pi + pj) < 0.f) {
         if (pi < 0.f) Ri = -pi * inv_i * inv_i;
@@ -426,7 +440,7 @@ __global__ void __maxnreg__(128) forces_fluid32_kernel(DevView v) {
         vab0 = v0; vab1 = v1; vab2 = v2;
         if (uniform_mu) Mu = mu_u;
         else {
-          const float muj = dyn_mu ? v.S.MU32[j] : Cj.mu0;
+          const float muj = dyn_mu ? v.S.MU32[j] : (SPEC ? Ci.mu0 : Cj.mu0);
           Mu = __fdividef(2.f * mui * muj, mui + muj);
         }
       } else {
@@ -492,8 +506,18 @@ __global__ void __maxnreg__(128) forces_fluid32_kernel(DevView v) {
     const int4* __restrict__ nl4 = reinterpret_cast<const int4*>(v.S.nl) + nl_slot(i);
     const size_t N = (size_t)v.nl_stride;
     const int nch = (cnt + 3) >> 2;
+    // the strain-rate flavours load the next chunk one chunk ahead (measured:
+    // it helps there and costs the plain flavour a little)
+    constexpr bool kAhead = FL >= 2;
+    int4 qn = (kAhead && nch > 0) ? nl4[0] : make_int4(0, 0, 0, 0);
     for (int c = 0; c < nch; ++c) {  // one 16-byte chunk of 4 entries per load
-      const int4 q = nl4[(size_t)c * N];
+      int4 q;
+      if (kAhead) {
+        q = qn;
+        if (c + 1 < nch) qn = nl4[(size_t)(c + 1) * N];
+      } else {
+        q = nl4[(size_t)c * N];
+      }
       const int rem = cnt - 4 * c;
       pair(q.x & kIndexMask, entry_code(q.x));
       if (rem > 1) pair(q.y & kIndexMask, entry_code(q.y));
@@ -1461,6 +1485,17 @@ void spec32_dispatch(const DevView& v, int bt, cudaStream_t st) {
   else forces_spec32_kernel<DIM, KT, 3><<<nb, bt, sm, st>>>(v, lg);
 }
 
+template <int DIM, int KT>
+void fluid32_dispatch(const DevView& v, int nb, int bt, cudaStream_t st) {
+  const int fl = !v.o.flavours32 ? 0 : !v.o.need_sr ? 1 : !v.o.closure ? 2 : 3;
+  switch (fl) {
+    case 0: forces_fluid32_kernel<DIM, KT, 0><<<nb, bt, 0, st>>>(v); break;
+    case 1: forces_fluid32_kernel<DIM, KT, 1><<<nb, bt, 0, st>>>(v); break;
+    case 2: forces_fluid32_kernel<DIM, KT, 2><<<nb, bt, 0, st>>>(v); break;
+    default: forces_fluid32_kernel<DIM, KT, 3><<<nb, bt, 0, st>>>(v); break;
+  }
+}
+
 template <int DIM>
 void forces32_dispatch(const DevView& v, cudaStream_t st) {
   const int bt = (v.o.pair_block >= 32 && v.o.pair_block <= kMaxPairBlock) ? v.o.pair_block : kFT32;
@@ -1490,9 +1525,9 @@ void forces32_dispatch(const DevView& v, cudaStream_t st) {
     return;
   }
   switch (v.o.kt) {
-    case 0: forces_fluid32_kernel<DIM, 0><<<nb, bt, 0, st>>>(v); break;
-    case 1: forces_fluid32_kernel<DIM, 1><<<nb, bt, 0, st>>>(v); break;
-    default: forces_fluid32_kernel<DIM, 2><<<nb, bt, 0, st>>>(v); break;
+    case 0: fluid32_dispatch<DIM, 0>(v, nb, bt, st); break;
+    case 1: fluid32_dispatch<DIM, 1>(v, nb, bt, st); break;
+    default: fluid32_dispatch<DIM, 2>(v, nb, bt, st); break;
   }
 }
 
