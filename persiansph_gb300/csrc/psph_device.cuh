@@ -48,7 +48,7 @@ struct Scratch {
   int* nl;           // per-step neighbour lists, entry k of particle i at nl[nl_index(stride, i, k)]:
                      // index | cell-offset code << 26
   int* nl_count;     // list length, or -1 when it exceeded the capacity (scan instead)
-  float4* PX32;      // FP32C form, Options::spec32: (position - cell origin, +-1/density), negative for a fixed one
+  float4* PX32;      // FP32C form, Options::spec32: (position - cell origin, +-|1/density|), negative for a fixed one
   float4* V32;       // FP32C form: (v, pressure)
   float4* D32;       // FP32C form: (1/density, pressure/density^2, sound speed, density)
   float2* RC32;      // FP32C form, Options::spec32, in D32's place: (density, refcell with a skin) of the free ones
@@ -56,7 +56,7 @@ struct Scratch {
   float4* TIR32;     // FP32C solids with TI: symmetric TIR, same layout
   float4* VB32;      // FP32C solids: wall history velocity (MVerlet vb / leapfrog vb)
   float4* V32LO;     // FP32C: v - (float)v, the low-order part of the velocity (fluids: .w = the
-                     // particle's class index and flags as int bits, or the sound speed (spec32))
+                     // particle's class index and flags as int bits, or the sound speed with the density's sign (spec32))
   float* MU32;       // FP32C, per-particle viscosity (LES / Bingham): FP32 copy of Persist::mu
   float4* NSV32;     // FP32C: wall no-slip velocity in FP32
   double4_32a* D4;   // seen by partners: (1/density, pressure/density^2, sound speed, density);

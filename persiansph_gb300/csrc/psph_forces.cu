@@ -182,7 +182,7 @@ PSPH_D void soil_records(const DevView& v, const Persist& P, int w, bool fixed, 
   // body) makes v_i - v_j far smaller than v
   const float vx = d2f_split(vel.x, &lx), vy = d2f_split(vel.y, &ly);
   v.S.PX32[w] = make_float4(x.x, x.y, d2f_rn(sg[0]), d2f_rn(sg[1]));
-  v.S.V32[w] = make_float4(vx, vy, d2f_rn(sg[4]), fixed ? -i32 : i32);
+  v.S.V32[w] = make_float4(vx, vy, d2f_rn(sg[4]), fixed ? __uint_as_float(kFixedMark) : i32);
   v.S.V32LO[w] = make_float4(lx, ly, d2f_rn(vel.z), tens ? 1.f : 0.f);
   if (tens) v.S.TIR32[2 * (size_t)w] = make_float4(d2f_rn(t[0]), d2f_rn(t[1]), 0.f, d2f_rn(t[4]));
 }

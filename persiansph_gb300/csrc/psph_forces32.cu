@@ -276,15 +276,15 @@ PSPH_D void interpolate_wall32(const DevView& v, const Persist& P, int w, int su
     else if (Ce.pres_eq == 1) rw = powf((p - p0) * (7.f / (r0 * cs2)) + 1.f, 1.f / 7.f) * r0;
     else rw = p / cs2;
     const float ratio = rw / r0;
-    cwv = (Ce.pres_eq == 1) ? Ce.cs * ratio * ratio * ratio : Ce.cs;
+    cwv = (Ce.pres_eq == 1) ? fabsf(Ce.cs * ratio * ratio * ratio) : Ce.cs;  // sqrt(cs^2 ratio^6)
   }
   const float inv = 1.f / rw;
   if (o.spec32) {
     // a wall without a free particle in its support has none to meet, but may
     // stand in a list (their margin): its terms are zeros times finite numbers
     const bool odd = sk == 0.f && !(fabsf(inv) <= FLT_MAX);
-    v.S.PX32[w] = make_float4(oi.x, oi.y, oi.z, odd ? -1.f : -inv);
-    v.S.V32LO[w].w = cwv;
+    v.S.PX32[w] = make_float4(oi.x, oi.y, oi.z, odd ? -1.f : with_sign(inv, -1.f));
+    v.S.V32LO[w].w = odd ? 0.f : with_sign(cwv, inv);
   } else {
     v.S.D32[w] = make_float4(inv, p * inv * inv, cwv, rw);
   }
@@ -589,10 +589,10 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
 // rates; 2: with them (LES, Bingham); 3: with the learned closure's sums too.
 //
 // The kernel is bound by instruction issue and the latency of its gathers, so
-//  - a neighbour is three 16-byte records instead of four (PX32: offset and +-1 /
-//    density, negative for a fixed one; V32: velocity and pressure; V32LO: the
-//    velocity's low-order part and the sound speed), what else a pair needs
-//    following from those;
+//  - a neighbour is three 16-byte records instead of four (PX32: offset and the
+//    magnitude of 1 / density, negative for a fixed one; V32: velocity and pressure;
+//    V32LO: the velocity's low-order part and the sound speed, with the density's
+//    sign), what else a pair needs following from those;
 //  - a lane takes two neighbours at a time: six loads in flight, and every
 //    operation that both need in packed FP32x2 arithmetic (one issue slot for
 //    the two values, each rounded as the scalar operation rounds);
@@ -687,8 +687,8 @@ __device__ __noinline__ float2 filter_sums(const DevView& v, const int* __restri
     const float inv_r = (r2 > 0.f) ? rsqrtf(r2) : 0.f;
     const float q = r2 * inv_r * ih;
     const float K = KernF<DIM, KT>::W(q, cwh);
-    const float mj = oj.w > 0.f ? c32.m_free : c32.m_wall;
-    const float inv_j = fabsf(oj.w);
+    const float mj = kind_free(oj.w) ? c32.m_free : c32.m_wall;
+    const float inv_j = with_sign(oj.w, v.S.V32LO[e & kIndexMask].w);
     zw += mj * inv_j * K;
     sd += mj * K;
   };
@@ -697,7 +697,7 @@ __device__ __noinline__ float2 filter_sums(const DevView& v, const int* __restri
     const int code = entry_code(entry(k));
     int mid = k, end = k;  // the cell's free particles, then its fixed ones
     while (end < cnt && entry_code(entry(end)) == code) {
-      if (v.S.PX32[entry(end) & kIndexMask].w > 0.f && mid == end) ++mid;
+      if (kind_free(v.S.PX32[entry(end) & kIndexMask].w) && mid == end) ++mid;
       ++end;
     }
     int a = k, b = mid;
@@ -758,7 +758,7 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
   const float4 xi = v.S.PX32[is];
   const float4 vi = v.S.V32[is];
   const float4 vl = v.S.V32LO[is];
-  const float inv_i = xi.w, Pi = vi.w * inv_i * inv_i, snd_i = vl.w;
+  const float inv_i = with_sign(xi.w, vl.w), Pi = vi.w * inv_i * inv_i, snd_i = fabsf(vl.w);
   const float mui = o.dyn_mu ? v.S.MU32[is] : o.mu_u32;
   const bool shep = (Ci.flags & CF_SHEPARD) && (Is.shepard_counter == o.shepard_step);
   const float3 cs = cell_size_f(g);
@@ -791,7 +791,7 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
     float2 r2 = fma2(x1, x1, x0 * x0);
     if (DIM == 3) r2 = fma2(x2, x2, r2);
     if (!both) r2.y = c32.far2;  // beyond the support: every term of it is zero
-    const bool fa = xa.w > 0.f, fb = xb.w > 0.f;
+    const bool fa = kind_free(xa.w), fb = kind_free(xb.w);
     const bool ia = r2.x <= reach2, ib = r2.y <= reach2;
     npair2 += (ia ? (fa ? 1u : 2u) : 0u) + (ib ? (fb ? 1u : 2u) : 0u);
     if (FL == 3) nnb += (ia ? 1 : 0) + (ib ? 1 : 0);
@@ -799,7 +799,7 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
     const float2 q = r2 * inv_r * dup(o.inv_h32);
     float2 K, GK;
     kern2<DIM, KT>(q, inv_r * dup(c32.h), cwh, cwg, K, GK);
-    const float2 inv_j = f2(fabsf(xa.w), fabsf(xb.w));
+    const float2 inv_j = f2(with_sign(xa.w, la.w), with_sign(xb.w, lb.w));
     // StrainRate += (m_j / rho_j) S with S = -GK [2 v_a x_a, v_a x_b + v_b x_a, ...]
     // (Source/Interaction.cpp:114-117, no 1/2): a = c2 vab, S_rc = a_r x_c + a_c x_r;
     // before the mass is folded in, in the general kernel's roundings: a feature
@@ -833,7 +833,7 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
       const float2 vm = f2(fminf(vx.x, 0.f), fminf(vx.y, 0.f));
       const float2 D = r2 + dup(c32.eps2);
       const float2 ivp = dup(inv_i) * inv_j;
-      const float2 c = (dup(snd_i) + f2(la.w, lb.w)) * ivp;
+      const float2 c = f2(snd_i + fabsf(la.w), snd_i + fabsf(lb.w)) * ivp;
       const float2 den = D * (dup(inv_i) + inv_j);
       float2 num = vm * dup(c32.neg_alpha_h) * c;
       float2 rc = f2(rcp_ftz(den.x), rcp_ftz(den.y));
@@ -1269,7 +1269,7 @@ __global__ void __maxnreg__(128) forces_solid32_kernel(DevView v) {
 // forces_spec32_kernel a lane takes two neighbours at a time in packed FP32x2
 // arithmetic, and a neighbour is three 16-byte records
 // (written by prepare_wall_kernel)
-//   PX32  x, y, Sigma00, Sigma01      V32  vx, vy, Sigma11, +-1/density (- fixed)
+//   PX32  x, y, Sigma00, Sigma01      V32  vx, vy, Sigma11, 1/density (kFixedMark: fixed)
 //   V32LO the low-order parts of vx and vy, vz, whether its TIR is non-zero
 // In 2D the entries with a z index meet a zero separation in the acceleration.
 // The tensile-instability power is evaluated only where one of the two carries a
@@ -1305,7 +1305,7 @@ __global__ void __maxnreg__(112) forces_soil32_kernel(DevView v) {
   const InstState& Is = v.inst[Ci.inst];
   const int is = active ? i : 0;
   const float4 xi = v.S.PX32[is], vi = v.S.V32[is], vl = v.S.V32LO[is];
-  const float inv_i = fabsf(vi.w), mi = Ci.mass, h = Ci.h, ih = 1.f / h, ih2 = ih * ih;
+  const float inv_i = vi.w, mi = Ci.mass, h = Ci.h, ih = 1.f / h, ih2 = ih * ih;
   const float cwh = KernF<2, KT>::cw() * ih2, cwg = cwh * ih2;
   const float ci2 = inv_i * inv_i;
   const float P00 = xi.z * ci2, P01 = xi.w * ci2, P11 = vi.z * ci2;  // the own stress over density squared
@@ -1329,7 +1329,7 @@ __global__ void __maxnreg__(112) forces_soil32_kernel(DevView v) {
     const float2 x1 = fma2(f2(code_back<1>(ca), code_back<1>(cb)), dup(cs.y), f2(xi.y - xa.y, xi.y - xb.y));
     float2 r2 = fma2(x1, x1, x0 * x0);
     if (!both) r2.y = far2;  // beyond the support: every term of it is zero
-    const bool fa = va.w > 0.f, fb = vb.w > 0.f;
+    const bool fa = soil_free(va.w), fb = soil_free(vb.w);
     const bool ia = r2.x <= reach2, ib = r2.y <= reach2;
     npair2 += (ia ? (fa ? 1u : 2u) : 0u) + (ib ? (fb ? 1u : 2u) : 0u);
     const float2 inv_r = f2(rsqrt_ftz(fmaxf(r2.x, 1e-30f)), rsqrt_ftz(fmaxf(r2.y, 1e-30f)));

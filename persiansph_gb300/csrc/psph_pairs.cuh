@@ -28,6 +28,19 @@ PSPH_D float code_back(int code) {
   return __uint_as_float(__byte_perm(0x00003f80u, 0x0000bf80u, (unsigned)sel));
 }
 
+// A neighbour's kind and 1/density in one float of the FP32C records. Both the sign
+// of PX32.w (set: fixed) and the density's own sign count: a wall under strong suction
+// or a fluid blowing up may have a negative one. So PX32.w holds +-|1/density|, and
+// the sound speed (V32LO.w), never negative itself, has the density's sign.
+PSPH_D float with_sign(float magnitude, float sign) {
+  return __uint_as_float((__float_as_uint(magnitude) & 0x7fffffffu) | (__float_as_uint(sign) & 0x80000000u));
+}
+PSPH_D bool kind_free(float px_w) { return __float_as_int(px_w) >= 0; }
+// The 2D soil record: a fixed particle's 1/density is never read (its partner's
+// stands in), so a NaN no computation returns marks it (V32.w).
+constexpr unsigned kFixedMark = 0xffc0f1edu;
+PSPH_D bool soil_free(float v_w) { return __float_as_uint(v_w) != kFixedMark; }
+
 // Neighbour-list layout: chunks of 4 consecutive entries of one particle (16
 // bytes), chunk-major across particles: chunk c of particle i is int4 number
 // c * stride + nl_slot(i), so entry k sits at ((k / 4) * stride + nl_slot(i)) * 4
