@@ -224,13 +224,15 @@ PSPH_D double rcp_refined(double x) {
   const double y = rcp_newton(x);
   return fma(fma(-x, y, 1.0), y, y);
 }
-// (below 2^-1006, where the estimate flushes to zero, a separation is none: 0)
+// Squared separations, x >= 0 or NaN of either sign (which stays NaN): below
+// 2^-1006, where the estimate flushes to zero, a separation is none and both give 0;
+// for an infinite one rsqrt_newton gives NaN, sqrt_newton infinity.
 PSPH_D double rsqrt_newton(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-x * y, y, 1.0);
   const double r = fma(y * e, fma(e, 0.375, 0.5), y);
-  return __double2hiint(x) < 0x01100000 ? 0.0 : r;
+  return (unsigned)__double2hiint(x) < 0x01100000u ? 0.0 : r;
 }
 PSPH_D double sqrt_newton(double x) {
   double y;
@@ -238,17 +240,30 @@ PSPH_D double sqrt_newton(double x) {
   const double t = x * y;
   const double e = fma(-t, y, 1.0);
   const double r = fma(t * e, fma(e, 0.375, 0.5), t);
-  return __double2hiint(x) < 0x01100000 ? 0.0 : r;
+  const unsigned h = (unsigned)__double2hiint(x);
+  return h < 0x01100000u ? 0.0 : (h >= 0x7ff00000u ? x : r);
 }
-// sqrt_newton for any argument (tiny, negative): the library's function there
-__device__ __noinline__ inline double sqrt_small(double x) { return sqrt(x); }
-PSPH_D double sqrt_any(double x) { return __double2hiint(x) < 0x01100000 ? sqrt_small(x) : sqrt_newton(x); }
+// sqrt for any argument: the library's function for those outside [2^-1006, infinity)
+__device__ __noinline__ inline double sqrt_outside(double x) { return sqrt(x); }
+PSPH_D double sqrt_any(double x) {
+  if ((unsigned)__double2hiint(x) - 0x01100000u >= 0x7ff00000u - 0x01100000u) return sqrt_outside(x);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double t = x * y;
+  const double e = fma(-t, y, 1.0);
+  return fma(t * e, fma(e, 0.375, 0.5), t);
+}
 
 // Signs and comparisons of doubles on the integer pipe (an FP64 comparison
-// takes an FP64 issue slot): x < 0 (true for -0.0 too), and a > b for
-// non-negative a and b (true for NaN a).
+// takes an FP64 issue slot): x < 0 (true for -0.0 too, and for a NaN whose sign is
+// set), and a > b for a >= 0 or NaN of either sign (false: it is not outside, and
+// what it enters shows it) and b >= 0.
 PSPH_D bool negative(double x) { return __double2hiint(x) < 0; }
-PSPH_D bool above(double a, double b) { return __double_as_longlong(a) > __double_as_longlong(b); }
+PSPH_D bool above(double a, double b) {
+  const unsigned long long x = (unsigned long long)__double_as_longlong(a),
+                           y = (unsigned long long)__double_as_longlong(b);
+  return x - y - 1ull < 0x7ff0000000000000ull - y;  // y < x <= infinity
+}
 
 // A non-negative integer and a float as doubles, exactly, on the integer pipe (the conversion instructions run on the FP64 pipe).
 PSPH_D double i2d_small(int c) {
