@@ -104,3 +104,30 @@ def test_negative_soil_density(gpu):
         s.set("density", d)
 
     check(dom, dt, change, ("strain_rate", "rotation_rate"))
+
+
+def test_walls_out_of_reach(gpu):
+    """A background pressure under which the inverse Tait equation has no value at
+    p = 0: walls that stand in a list (one with a skin) but in no free particle's
+    support leave its sums alone."""
+    dom, dt, info = tank(2)
+    p = dom.particles
+    p.set("p0", 0.5 * 1000.0 * info["cs"] ** 2)
+    x = p.get("x")
+    x[p.get("is_free") == 0, 1] -= 0.3 * 0.031  # a floor just out of some supports
+    p.set("x", x)
+    cfg = dom.config(dt)
+    o = OracleDomain(cfg, p, initial=True)
+    o.step(1)
+    ref = o.download()
+    cfg.precision = 1
+    for skin in (0, 150):
+        gd = GpuDomain(cfg)
+        gd.upload(p)
+        gd.set_tuning(128, 1, 0, skin)
+        gd.step(1)
+        got = gd.download_fields()
+        a_scale, _ = o.scales()
+        f = ref["is_free"] == 1
+        assert np.max(np.linalg.norm(got["a"] - ref["a"], axis=1)[f] / a_scale[f]) <= 1e-5
+        gd.close()
