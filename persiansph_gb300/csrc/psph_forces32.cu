@@ -662,10 +662,10 @@ PSPH_D void kern2(float2 q, float2 inv_q, float cwh, float cwg, float2& K, float
 
 // On a Shepard step the filter divides SumDen by ZWab: FP32 sums whose rounding
 // goes into the density and, times c^2, into the next step's pressure. They are
-// then taken one neighbour after the other in the order of the cells, a cell's
-// particles by original index, as the general kernel's expressions take them,
-// so that a filtered density depends neither on the pair kernel's lanes nor on
-// the sort's free-first order. (ZWab, SumDen) of particle i, asked for where the
+// then taken one neighbour after the other in the order of the cells and their
+// x-slabs, a slab's particles by original index, as the general kernel's
+// expressions take them, so that a filtered density depends neither on the pair
+// kernel's lanes nor on the sort's free-first order. (ZWab, SumDen) of particle i, asked for where the
 // filter can apply (ZWab above 0.6); a call, so that one step in 41 takes no
 // registers from the others.
 template <int DIM, int KT>
@@ -694,12 +694,16 @@ __device__ __noinline__ float2 filter_sums(const DevView& v, const int* __restri
   };
   auto entry = [&](int k) { return v.S.nl[nl_index(v.nl_stride, i, k)]; };
   for (int k = 0; k < cnt;) {
-    const int code = entry_code(entry(k));
-    int mid = k, end = k;  // the cell's free particles, then its fixed ones
-    while (end < cnt && entry_code(entry(end)) == code) {
-      if (kind_free(v.S.PX32[entry(end) & kIndexMask].w) && mid == end) ++mid;
-      ++end;
-    }
+    // the entries of one slab: its free particles, then its fixed ones, each by original index
+    const int code = entry_code(entry(k)), j0 = entry(k) & kIndexMask, cell = v.S.cellid[j0];
+    int slab = 0;
+    while (slab + 1 < o.xsub && j0 >= v.S.sstart[sort_bin(cell, o.xsub, slab + 1)]) ++slab;
+    const unsigned bin = sort_bin(cell, o.xsub, slab);
+    const int fixed_at = v.S.sstart[bin + 1], slab_end = v.S.sstart[bin + 2];
+    auto below = [&](int e, int at) { return e < cnt && entry_code(entry(e)) == code && (entry(e) & kIndexMask) < at; };
+    int mid = k, end;
+    while (below(mid, fixed_at)) ++mid;
+    for (end = mid; below(end, slab_end);) ++end;
     int a = k, b = mid;
     while (a < mid || b < end) {
       const int ea = a < mid ? entry(a) : 0, eb = b < end ? entry(b) : 0;
