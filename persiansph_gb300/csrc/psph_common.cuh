@@ -210,19 +210,25 @@ __host__ __device__ inline float d2f_rn(double x) { return d2f_split(x, nullptr)
 // Reciprocal, square root and reciprocal square root of a positive normal
 // double by one third-order (Householder) step from the hardware's ~2^-20
 // estimate: with the estimate's relative residual e, the series of 1/(1-e) and
-// 1/sqrt(1-e) to e^2 leave |e|^3 < 2^-57. Within 1 ulp; 3 to 5 FP64 instructions
-// on a part with 2 FP64 lanes per SM. sqrt(0) = 0, and 1/sqrt(0) is returned as
-// 0 (a pair of coincident particles).
+// 1/sqrt(1-e) to e^2 leave |e|^3 < 2^-57. 3 to 5 FP64 instructions on a part with 2
+// FP64 lanes per SM. The reciprocal is within 0.55 ulp, the roots within 1.05 (half
+// an ulp for the last rounding, up to half for that of x y, the series' rest).
+// rcp_newton and rcp_refined: 2^-1022 <= |x| < 2^1022; zero, infinity and what lies
+// outside give NaN, infinity or zero as they come, never a wrong finite number.
 PSPH_D double rcp_newton(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-x, y, 1.0);
   return fma(y, fma(e, e, e), y);
 }
-// rcp_newton with one Newton step more: correctly rounded but for a few in 2^50
+// Correctly rounded: rcp_newton, within an ulp, and one Newton step more (Markstein's
+// theorem). The theorem's one exception is a significand of all ones, whose
+// reciprocal lies 2^-106 above the middle of a power of two and the next double: the latter.
 PSPH_D double rcp_refined(double x) {
   const double y = rcp_newton(x);
-  return fma(fma(-x, y, 1.0), y, y);
+  const double r = fma(fma(-x, y, 1.0), y, y);
+  const unsigned zeros = ~(unsigned)__double2loint(x) | (~(unsigned)__double2hiint(x) & 0xfffffu);  // of the significand
+  return __hiloint2double(__double2hiint(r), __double2loint(r) | (zeros == 0u ? 1 : 0));
 }
 // Squared separations, x >= 0 or NaN of either sign (which stays NaN): below
 // 2^-1006, where the estimate flushes to zero, a separation is none and both give 0;
@@ -265,7 +271,8 @@ PSPH_D bool above(double a, double b) {
   return x - y - 1ull < 0x7ff0000000000000ull - y;  // y < x <= infinity
 }
 
-// A non-negative integer and a float as doubles, exactly, on the integer pipe (the conversion instructions run on the FP64 pipe).
+// A non-negative integer and a float (any) as doubles, exactly, on the integer pipe
+// (the conversion instructions run on the FP64 pipe).
 PSPH_D double i2d_small(int c) {
   const int e = 31 - __clz(c | 1);
   const unsigned long long m = ((unsigned long long)(unsigned)c << (52 - e)) & 0xfffffffffffffull;

@@ -45,17 +45,6 @@ namespace {
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float sigm(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float silu(float z) { return z * sigm(z); }
-// The same sigmoid for the training epilogues, which evaluate 64 a thread in a
-// row: the division's special cases are a branch that keeps them one after the
-// other. The reciprocal here is the hardware's estimate and one Newton step
-// (within 1e-6 ulp of half an ulp); past 8e37 (z < -87) it is zero.
-__device__ __forceinline__ float sigm_row(float z) {
-  const float x = 1.f + expf(-z);
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fminf(x, 8e37f)));
-  r = fmaf(fmaf(-x, r, 1.f), r, r);
-  return x < 8e37f ? r : (x == x ? 0.f : x);
-}
 __device__ __forceinline__ float dsilu_of(float z, float s) { return s * (1.f + z * (1.f - s)); }
 // SiLU of the tensor-core inference epilogues: hardware exp2 and reciprocal
 // approximations (relative error ~1e-6, far below the BF16 rounding of the

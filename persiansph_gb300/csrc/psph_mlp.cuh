@@ -44,6 +44,18 @@ inline __host__ __device__ int sw128_offset(int r, int k) {
   return (r >> 3) * 1024 + (r & 7) * 128 + ((((k >> 3) ^ (r & 7)) & 7) << 4) + (k & 7) * 2;
 }
 
+// The sigmoid of the training epilogues, which evaluate 64 a thread in a
+// row: the division's special cases are a branch that keeps them one after the
+// other. The reciprocal here is the hardware's estimate and one Newton step
+// (within 1e-6 ulp of half an ulp); past 8e37 (z < -87) it is zero.
+__device__ __forceinline__ float sigm_row(float z) {
+  const float x = 1.f + expf(-z);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fminf(x, 8e37f)));
+  r = fmaf(fmaf(-x, r, 1.f), r, r);
+  return x < 8e37f ? r : (x == x ? 0.f : x);
+}
+
 }  // namespace psph
 
 // Device image of a network (for psph_closure_attach).
