@@ -809,7 +809,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
         auto it = index.find(key);
         if (it == index.end()) {
           const int id = (int)c->classes.size();
-          if (id >= 65535) return set_err(c, PSPH_ERR_UNSUPPORTED, "more than 65535 distinct particle parameter sets");
+          if (id >= kMaxClasses) return set_err(c, PSPH_ERR_UNSUPPORTED, "more than 65535 distinct particle parameter sets");
           index.emplace(key, id);
           c->classes.push_back(W.classes[k]);
           remap[k] = id;
@@ -880,7 +880,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
           id = -1;  // closed below
         } else {
           id = (int)c->classes.size();
-          if (id >= 65535) return set_err(c, PSPH_ERR_UNSUPPORTED, "more than 65535 distinct particle parameter sets");
+          if (id >= kMaxClasses) return set_err(c, PSPH_ERR_UNSUPPORTED, "more than 65535 distinct particle parameter sets");
           index.emplace(key, id);
           c->classes.push_back(T);
           depth.push_back(depth[q] + 1);
@@ -1080,7 +1080,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
       return st;
   }
   char* state = nullptr;
-  c->cls_cap = (int)c->classes.size() + (inout ? 256 : 0);  // recycled in-flow particles may need new classes
+  c->cls_cap = (int)c->classes.size() + (inout ? kFlowClasses : 0);  // recycled in-flow particles may need new classes
   if ((st = dalloc(c, &c->d_cls, (size_t)c->cls_cap)) || (st = dalloc(c, &state, kInstAt + sizeof(InstState) * ninst)) ||
       (st = dalloc(c, &c->d_alive, N)) || (st = dalloc(c, &c->d_grids, (size_t)ninst)) ||
       (st = dalloc(c, &c->d_grids_ref, (size_t)ninst)))
@@ -2208,7 +2208,7 @@ psph_status patch_impl(psph_ctx* c, const psph_particles* p) {
         id = it->second;
       } else {
         id = (int)c->classes.size();
-        if (id >= 65535) return set_err(c, PSPH_ERR_UNSUPPORTED, "more than 65535 distinct particle parameter sets");
+        if (id >= kMaxClasses) return set_err(c, PSPH_ERR_UNSUPPORTED, "more than 65535 distinct particle parameter sets");
         c->classes.push_back(C);
         c->class_index.emplace(key, id);
       }

@@ -68,7 +68,7 @@ struct Scratch {
   double* half_zw;
   double* half_sd;       // (on Shepard steps)
   int* half_stamp;       // instance step + 1 when the slot was written this step
-  int* pair_info;        // FP64 form: class | free << 16 | list in use << 17 (kInfo* of psph_forces.cu)
+  int* pair_info;        // FP64 form: class, whether free, whether its list is in use (kInfo* of psph_forces.cu)
   double* zwab;
   double* s_acc;         // SWIType 1: Particle::S, the surface-erosion velocity derivative
   uint8_t* satcheck;     // fluid-soil: Particle::SatCheck of this step
@@ -95,6 +95,10 @@ struct Scratch {
   float* cfeat;          // raw network features, 6 per particle
   double* nut;           // eddy viscosity from the network; -1 = use Smagorinsky
 };
+
+// Distinct parameter sets of an upload, and those an in-flow may add as it recycles
+// particles (FP64 form).
+constexpr int kMaxClasses = 65535, kFlowClasses = 256;
 
 // Pair constants of the FP64 fluid kernel's SPEC form (Options::spec64).
 struct Spec64 {

@@ -156,7 +156,8 @@ PSPH_D double group_sum(double x, int lg) {
 // What the pair loops need to know of a partner, in one word (pair_info, written
 // by prepare_wall_kernel): its class, whether it is free, whether its list is in use,
 // whether its tensile-instability stress is non-zero.
-constexpr int kInfoCls = 0xffff, kInfoFree = 1 << 16, kInfoList = 1 << 17, kInfoTir = 1 << 18;
+constexpr int kInfoCls = 0xffffff, kInfoFree = 1 << 24, kInfoList = 1 << 25, kInfoTir = 1 << 26;
+static_assert(kInfoCls >= kMaxClasses + kFlowClasses, "every class index fits");
 
 // kInfoTir of particle w, from its tensile-instability stress
 PSPH_D int tir_bit(const DevView& v, const Persist& P, int w) {
