@@ -967,7 +967,6 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
   o.swi = k.swi_type;
   o.fp32 = (k.precision == PSPH_FP32C);
   if (ntot >= (1LL << 26)) return set_err(c, PSPH_ERR_UNSUPPORTED, "this build handles fewer than 2^26 particles");
-  o.soil_pairs = (materials & (1 << 3)) != 0;
   o.dyn_mu = dyn_mu;
   o.xsph = k.xsph;
   o.sqrt_h_a = k.sqrt_h_a;

@@ -106,7 +106,6 @@ struct StepScalars {
   int buf;        // which persistent buffer (A=0 / B=1) holds the current sorted state
   unsigned long long pairs_x2;  // 2 x pair-interactions evaluated since upload
   unsigned int work;            // blocks of the update that have finished (Options::fused_tail; zero between steps)
-  int launches;
   unsigned long long closure_eval, closure_fallback;  // closure evaluations / Smagorinsky fallbacks
   int nl_rest;    // particles the neighbour-list scan handles one per lane (set by the sort)
   int n_walls;    // fixed particles (Scratch::walls, set by the sort)

@@ -134,7 +134,6 @@ struct Options {
   int dyn_mu;
   int in_out_flow;    // Domain::BC.InOutFlow (single FP64 fluid domain)
   double out_density; // BC.outDensity (whether out-flow particles keep their density)
-  int soil_pairs;     // Material 3 (soil-soil walls take the partner's density)
   int mixed;          // fluid (Material 1) and a soil or a solid share the domain: each pair
                       // kernel keeps to its material, a coupling kernel adds the pairs of
                       // different materials (FP64 form)
@@ -278,7 +277,6 @@ void launch_prepare32(const DevView& v, cudaStream_t st); // FP32C form: wall in
 void launch_copies32(const DevView& v, cudaStream_t st);
 void launch_forces32(const DevView& v, cudaStream_t st);  // FP32C form: fluid pair forces
 void launch_expand_sr32(const DevView& v, int n, cudaStream_t st);  // sr32 / rates32 -> the FP64 rate tensors
-void launch_wall(const DevView& v, cudaStream_t st);      // wall interpolation
 void launch_forces(const DevView& v, cudaStream_t st);    // pair forces + per-block dt minimum
 void launch_saturation(const DevView& v, cudaStream_t st); // fluid-soil: saturation check and weight switch
 void launch_fsi(const DevView& v, cudaStream_t st);       // fluid-solid: FSI interpolation of the solid
@@ -288,7 +286,6 @@ void launch_update(const DevView& v, cudaStream_t st);    // Move + material upd
 void launch_begin(const DevView& v, cudaStream_t st);     // stop test, first-step counters
 void launch_end(const DevView& v, cudaStream_t st);       // time, counters
 void launch_closure(const DevView& v, cudaStream_t st);   // learned eddy viscosity (tcgen05 MLP)
-int forces_blocks(int ncap);
 void launch_class_constants(PClass* cls, int n, int dim, cudaStream_t st);  // derived class constants, once per upload
 int launches_per_step(const DevView& v);
 void launch_pairs_export(const DevView& v, int which, long long* out, long long cap, unsigned long long* counter,

@@ -1,12 +1,14 @@
-// Gather-form pair kernels of the GB300 hot path.
+// FP64 pair kernels of the GB300 hot path.
 //
 // The reference walks a half stencil of cells, pushes every candidate pair into
 // per-thread lists and then scatters each pair's contribution into both
 // particles under per-particle locks (Source/Domain.cpp:808-945,
-// Source/Interaction.cpp:25-377). Here each particle gathers from the full
-// 3x3(x3) block of cells around its own, so every pair is evaluated twice (once
-// from each side) and each particle's sums are owned by one thread: no atomics,
-// no locks, deterministic results.
+// Source/Interaction.cpp:25-377). Here a group of lanes owns a particle's sums and
+// walks its neighbour list; the lanes' sums join in a fixed order. Fluids without
+// strain rates, XSPH or a second material evaluate each pair of free particles
+// once, from one side, and fold the partner's terms in list order (HALF below);
+// the others evaluate it from both sides. No atomics, no locks, deterministic
+// results.
 //
 //   prepare_wall  free particles: partner-visible density / sound speed, TIR;
 //                 fixed particles: PrimaryComputeAcceleration's wall
@@ -1690,14 +1692,10 @@ void forces_dispatch(const DevView& v, cudaStream_t st) {
 
 }  // namespace
 
-int forces_blocks(int ncap) { return nblk(ncap, kFT); }
-
 void launch_prepare(const DevView& v, cudaStream_t st) {
   if (v.o.dim == 2) prepare_dispatch<2>(v, st);
   else prepare_dispatch<3>(v, st);
 }
-
-void launch_wall(const DevView&, cudaStream_t) {}  // fused into launch_prepare
 
 void launch_saturation(const DevView& v, cudaStream_t st) {
   const int nb = nblk(v.ncap, kFT);

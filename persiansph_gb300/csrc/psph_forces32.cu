@@ -46,11 +46,6 @@ PSPH_D float4 ld_early(const float4* p) {
   asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
   return r;
 }
-PSPH_D int ld_early(const int* p) {
-  int r;
-  asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(r) : "l"(p));
-  return r;
-}
 // the same for an array the kernel itself writes elsewhere (coherent path)
 PSPH_D float4 ld_early_coherent(const float4* p) {
   float4 r;

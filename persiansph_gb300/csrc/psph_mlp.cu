@@ -769,14 +769,14 @@ __device__ __forceinline__ void store_col64(uint8_t* t, int sub_bytes, int c, co
 
 // One CTA of 128 threads per tile of 128 samples (thread t = sample t of the
 // tile), looping over tiles; writes the activations and deltas the CUDA-core
-// gradients need (U, Z1, Z2, layer 3's activations A3, Z4, G4, D1..D3), the loss partial of each tile, and
+// gradients need (U, Z1, Z2, layer 3's activations A3, G4, D1..D3), the loss partial of each tile, and
 // its tensor-core partials of dW3 and dW2 (mma[cta][2][64][64]). A chain of six
 // products and the epilogues between them: 4,096 samples 92 us with scalar row
 // accesses and the division's branches in the sigmoids, 50 without.
 __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
     const TrainImages* __restrict__ img, const float* __restrict__ params, const float* __restrict__ norm,
     const float* __restrict__ X, const float* __restrict__ Y, const float* __restrict__ W, const int* __restrict__ idx,
-    int B, float* U, float* Z1, float* Z2, float* A3, float* Z4, float* G4, float* D1, float* D2, float* D3,
+    int B, float* U, float* Z1, float* Z2, float* A3, float* G4, float* D1, float* D2, float* D3,
     double* loss_part, float* mma, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bars[2];
@@ -898,7 +898,6 @@ __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
       const float e = softplus(o) - y;
       g = 2.f * w * e * sigm(o) / (float)B;
       lp = (double)w * (double)e * (double)e;
-      Z4[b] = o;
       G4[b] = g;
     }
     for (int off = 16; off > 0; off >>= 1) lp += __shfl_down_sync(0xffffffffu, lp, off);
@@ -1053,11 +1052,12 @@ struct psph_mlp {
   int64_t n_data = 0;
   // minibatch scratch
   int cap = 0, nchunk_cap = 0;
-  // training passes: the samples' order (two, the last pass's and the next), the shuffle's lists
+  // training passes: the samples' order (two, the last pass's and the next), the shuffle's
+  // lists; 16 bytes a sample together
   int *d_order[2] = {nullptr, nullptr}, *d_head = nullptr, *d_next = nullptr;
   int64_t order_cap = 0;
   float* d_losses = nullptr;  // kLossRun of them
-  float *d_U = nullptr, *d_Z1 = nullptr, *d_Z2 = nullptr, *d_A3 = nullptr, *d_Z4 = nullptr, *d_G4 = nullptr;
+  float *d_U = nullptr, *d_Z1 = nullptr, *d_Z2 = nullptr, *d_A3 = nullptr, *d_G4 = nullptr;
   float *d_D1 = nullptr, *d_D2 = nullptr, *d_D3 = nullptr, *d_part = nullptr;
   float* d_mma = nullptr;            // per-CTA tensor-core partials of dW3, dW2
   TrainImages* d_timg = nullptr;     // operand images of the current parameters
@@ -1105,7 +1105,7 @@ psph_status ensure_batch(psph_mlp* m, int B) {
     m->mma_cap = nctas;
   }
   if (B <= m->cap && nchunk <= m->nchunk_cap) return PSPH_OK;
-  for (float** p : {&m->d_U, &m->d_Z1, &m->d_Z2, &m->d_A3, &m->d_Z4, &m->d_G4, &m->d_D1, &m->d_D2, &m->d_D3,
+  for (float** p : {&m->d_U, &m->d_Z1, &m->d_Z2, &m->d_A3, &m->d_G4, &m->d_D1, &m->d_D2, &m->d_D3,
                     &m->d_part})
     dfree(*p);
   dfree(m->d_loss);
@@ -1114,7 +1114,6 @@ psph_status ensure_batch(psph_mlp* m, int B) {
   MLP_TRY(m, cudaMemset(m->d_U, 0, 8 * b * sizeof(float)));
   for (float** p : {&m->d_Z1, &m->d_Z2, &m->d_A3, &m->d_D1, &m->d_D2, &m->d_D3})
     MLP_TRY(m, cudaMalloc(p, (size_t)kMlpH * b * sizeof(float)));
-  MLP_TRY(m, cudaMalloc(&m->d_Z4, b * sizeof(float)));
   MLP_TRY(m, cudaMalloc(&m->d_G4, b * sizeof(float)));
   MLP_TRY(m, cudaMalloc(&m->d_part, (size_t)nchunk * kNParams * sizeof(float)));
   MLP_TRY(m, cudaMalloc(&m->d_loss, (size_t)((B + kTrainThreads - 1) / kTrainThreads) * sizeof(double)));
@@ -1152,7 +1151,7 @@ psph_status batch_grad(psph_mlp* m, const float* dX, const float* dY, const floa
   // tensor cores: forward, loss gradient, deltas, dW2 / dW3
   const int nctas = train_ctas(B);
   train_tc_kernel<<<nctas, kTcThreads, kTrSmemBytes>>>(m->d_timg, m->d_params, m->d_norm, dX, dY, dW, d_idx, B,
-                                                       m->d_U, m->d_Z1, m->d_Z2, m->d_A3, m->d_Z4, m->d_G4, m->d_D1,
+                                                       m->d_U, m->d_Z1, m->d_Z2, m->d_A3, m->d_G4, m->d_D1,
                                                        m->d_D2, m->d_D3, m->d_loss, m->d_mma, m->d_status);
   // CUDA cores: W1, the biases and the output layer, per chunk of samples
   const int chunk = 128, nchunk = (B + chunk - 1) / chunk;
@@ -1233,7 +1232,7 @@ void psph_mlp_destroy(psph_mlp* m) {
   if (!m) return;
   cudaDeviceSynchronize();
   for (float** p : {&m->d_params, &m->d_m, &m->d_v, &m->d_grad, &m->d_norm, &m->d_X, &m->d_Y, &m->d_W, &m->d_U, &m->d_Z1,
-                    &m->d_Z2, &m->d_A3, &m->d_Z4, &m->d_G4, &m->d_D1, &m->d_D2, &m->d_D3, &m->d_part})
+                    &m->d_Z2, &m->d_A3, &m->d_G4, &m->d_D1, &m->d_D2, &m->d_D3, &m->d_part})
     dfree(*p);
   dfree(m->d_img);
   dfree(m->d_timg);
