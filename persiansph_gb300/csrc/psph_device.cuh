@@ -263,6 +263,18 @@ PSPH_D void end_step(InstState& I, const Options& o) {
   I.k_initial = 0;
 }
 
+// The device's SMs (152 on a GB300), asked for once.
+inline int sm_count() {
+  static const int n = [] {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      sms = 0;
+    return sms > 0 ? sms : 152;
+  }();
+  return n;
+}
+
 // Launch wrappers (defined in the .cu files).
 void launch_sort(const DevView& v, cudaStream_t st);      // bin + scan + scatter + reorder
 int sort_launches(const DevView& v);

@@ -1658,7 +1658,7 @@ int lanes_log2(int kt) { return kt == PSPH_QUINTIC_SPLINE ? 3 : 2; }
 template <int DIM>
 void prepare_dispatch(const DevView& v, cudaStream_t st) {
   const int lg = lanes_log2(v.o.kt);
-  const int walls = std::min(nblk(v.ncap, kFT >> lg), 32 * 152);  // (how many there are is known on the device)
+  const int walls = std::min(nblk(v.ncap, kFT >> lg), 32 * sm_count());  // (how many there are is known on the device)
   const int nb = walls + nblk(v.ncap, kFT);
   switch (v.o.kt) {
     case 0: prepare_wall_kernel<DIM, 0><<<nb, kFT, 0, st>>>(v, lg, walls); break;

@@ -976,17 +976,6 @@ __global__ void __launch_bounds__(kTcThreads) train_tc_kernel(
 uint64_t splitmix(uint64_t& s) { return splitmix_at(s += kSplitmixStep); }
 double uniform01(uint64_t& s) { return (double)(splitmix(s) >> 11) * (1.0 / 9007199254740992.0); }
 
-int num_sms() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 bool tr_attr_set = false;
 cudaError_t ensure_train_attrs() {
   if (tr_attr_set) return cudaSuccess;
@@ -1020,7 +1009,7 @@ void launch_closure(const DevView& v, cudaStream_t st) {
   const int ntiles = (v.ncap + kMlpTile - 1) / kMlpTile;
   // four CTAs per SM (128 registers x 128 threads, ~52 KB shared memory and 64
   // TMEM columns each): while one waits on its MMAs the others run epilogues
-  const int grid = std::max(1, std::min(ntiles, 4 * num_sms()));
+  const int grid = std::max(1, std::min(ntiles, 4 * sm_count()));
   if (v.o.fp32) {
     if (v.o.dim == 2) closure_kernel<2, true><<<grid, kTcThreads, kTcSmemBytes, st>>>(v);
     else closure_kernel<3, true><<<grid, kTcThreads, kTcSmemBytes, st>>>(v);
@@ -1093,7 +1082,7 @@ void dfree(T*& p) {
 }
 
 // CTAs of train_tc_kernel for a minibatch of B samples
-int train_ctas(int B) { return std::max(1, std::min((B + kMlpTile - 1) / kMlpTile, num_sms())); }
+int train_ctas(int B) { return std::max(1, std::min((B + kMlpTile - 1) / kMlpTile, sm_count())); }
 
 psph_status ensure_batch(psph_mlp* m, int B) {
   const int nchunk = (B + 127) / 128;
@@ -1420,7 +1409,7 @@ psph_status psph_mlp_infer(psph_mlp* m, const float* x, int64_t n, float* c, int
   if (tensor_cores) {
     MLP_TRY(m, ensure_tc_attrs());
     const int ntiles = (int)((n + kMlpTile - 1) / kMlpTile);
-    const int grid = std::max(1, std::min(ntiles, 2 * num_sms()));
+    const int grid = std::max(1, std::min(ntiles, 2 * sm_count()));
     infer_tc_kernel<<<grid, kTcThreads, kTcSmemBytes>>>(m->d_img, dX, (int)n, dC, m->d_status);
   } else {
     infer_cc_kernel<<<(int)((n + 127) / 128), 128>>>(m->d_params, m->d_norm, dX, (int)n, dC);

@@ -620,17 +620,6 @@ __global__ void __launch_bounds__(kNT, 4) nlist_staged_kernel(DevView v, float m
 // 3D dam break).
 constexpr int kStageCapMax = 4096;
 
-int sm_count() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 1;
-  }
-  return n;
-}
-
 }  // namespace
 
 void nlist_configure() {
@@ -658,9 +647,12 @@ void launch_nlist(const DevView& v, cudaStream_t st) {
     return;
   }
   // A lane to a particle while the lanes of two particles would fit the SMs at once
-  // (1,024 an SM): then there are too few of them to cover each other's waits
-  // (86k particles in 2D 18 us against 23, 177k in 3D 87 against 107), where more
-  // take the shared loads and tests of two (1.0M in 3D 390 and 355).
+  // (1,024 an SM, 311k particles on 152): then there are too few of them to cover each
+  // other's waits, where more take the shared loads and tests of two. One lane and two,
+  // us: 3D 177k 86 and 106, 242k 101 and 121, 309k 137 and 146 | 392k 155 and 150, 464k
+  // 182 and 180, 1.0M 388 and 349 (at 564k one is ahead once more, 220 and 233); 2D 86k
+  // 18 and 22, 171k 23 and 27, 265k 32 and 30 | 359k 39 and 41, 515k 51 and 49, 907k 84
+  // and 78. Between 265k and 360k they differ by less than a run does.
   if (v.o.uniform_h && v.o.nlist_stage == 0 && v.ncap <= 2048ll * sm_count()) {
     const int nb = (v.ncap + kNT - 1) / kNT;
     if (v.o.dim == 2) nlist_kernel<2, true><<<nb, kNT, 0, st>>>(v, margin);
