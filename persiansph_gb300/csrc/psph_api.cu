@@ -279,11 +279,15 @@ void record_phase(psph_ctx* c, int k) {
   if (c->timing) cudaEventRecord(c->ev[k], c->stream);
 }
 
-// Most particles of a domain whose update ends the step itself (Options::fused_tail):
-// about one wave of the update's blocks, which then wait for the dt side by side.
-// Two launches less: 920 particles 4 us of a step's 54, 5k soil 2 of 215, 177k 2 of
-// 288; at a million the launches are 0.6 % of the step.
-constexpr int kTailMax = 262144;
+// Whether a domain's update ends the step itself (Options::fused_tail): while its
+// blocks are one wave, which then waits for the dt side by side (155,648 fluid
+// particles on 152 SMs, 77,824 with soil or solids). It saves two launches: 920
+// particles 47.9 -> 45.9 us a step, 6.5k 92.0 -> 91.9, 57k soil 102.5 -> 101.5, 86k even.
+// With more waves each waits again: 269k 303.4 -> 306.6, 359k in 2D 178.1 -> 185.8, soil
+// 112k 713.6 -> 725.5 (FP64), 217k 216.1 -> 219.8, 1.0M 884 -> 903.
+bool tail_fits(int ncap, bool solid) {
+  return ncap <= (long long)update_blocks_per_sm(solid) * kUpdateThreads * sm_count();
+}
 
 DevView view(psph_ctx* c) {
   DevView v{};
@@ -293,7 +297,7 @@ DevView view(psph_ctx* c) {
   v.ninst = c->ninst;
   v.total_cells = c->total_cells;
   v.o = c->opt;
-  v.o.fused_tail = c->ninst == 1 && c->ncap <= kTailMax && !c->in_parts;
+  v.o.fused_tail = c->ninst == 1 && tail_fits(c->ncap, c->opt.has_solid) && !c->in_parts;
   v.PA = c->PA;
   v.PB = c->PB;
   v.S = c->S;

@@ -275,6 +275,10 @@ inline int sm_count() {
   return n;
 }
 
+// Shape of the update kernel: threads of a block and blocks resident on an SM.
+constexpr int kUpdateThreads = 128;
+constexpr int update_blocks_per_sm(bool solid) { return solid ? 4 : 8; }
+
 // Launch wrappers (defined in the .cu files).
 void launch_sort(const DevView& v, cudaStream_t st);      // bin + scan + scatter + reorder
 int sort_launches(const DevView& v);

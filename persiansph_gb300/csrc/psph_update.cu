@@ -10,7 +10,6 @@ namespace psph {
 
 namespace {
 
-constexpr int kUT = 128;
 
 PSPH_D void mat_mult(const double* A, const double* B, double* M) {  // External/matvec.h:814-820
   M[0] = A[2] * B[6] + A[1] * B[3] + A[0] * B[0];
@@ -495,7 +494,7 @@ PSPH_D void update_particle(const DevView& v, const Persist& P, int s, const PCl
 // itself, and the last block to finish stores it and ends the step: two launches
 // of 3 us less, for one more wait in each block, which few blocks do not notice.
 template <int DIM, bool SOLID, bool TAIL>
-__global__ void __launch_bounds__(kUT, SOLID ? 4 : 8) update_kernel(DevView v) {
+__global__ void __launch_bounds__(kUpdateThreads, update_blocks_per_sm(SOLID)) update_kernel(DevView v) {
   StepScalars* sc = v.sc;
   if (sc->all_stop) return;
   const Persist& P = cur_persist(v);
@@ -533,12 +532,12 @@ __global__ void __launch_bounds__(kUT, SOLID ? 4 : 8) update_kernel(DevView v) {
 
 template <int DIM, bool SOLID>
 static void update_launch(const DevView& v, int grid, cudaStream_t st) {
-  if (v.o.fused_tail) update_kernel<DIM, SOLID, true><<<grid, kUT, 0, st>>>(v);
-  else update_kernel<DIM, SOLID, false><<<grid, kUT, 0, st>>>(v);
+  if (v.o.fused_tail) update_kernel<DIM, SOLID, true><<<grid, kUpdateThreads, 0, st>>>(v);
+  else update_kernel<DIM, SOLID, false><<<grid, kUpdateThreads, 0, st>>>(v);
 }
 
 void launch_update(const DevView& v, cudaStream_t st) {
-  const int nb = (v.ncap + kUT - 1) / kUT;
+  const int nb = (v.ncap + kUpdateThreads - 1) / kUpdateThreads;
   const int grid = nb > 0 ? nb : 1;
   if (v.o.has_solid) {
     if (v.o.dim == 2) update_launch<2, true>(v, grid, st);
