@@ -660,11 +660,9 @@ PSPH_D void kern2(float2 q, float2 inv_q, float cwh, float cwg, float2& K, float
 // then taken one neighbour after the other in the order of the cells and their
 // x-slabs, a slab's particles by original index, as the general kernel's
 // expressions take them, so that a filtered density depends neither on the pair
-// kernel's lanes nor on the sort's free-first order. (ZWab, SumDen) of particle i, asked for where the
-// filter can apply (ZWab above 0.6); a call, so that one step in 41 takes no
-// registers from the others.
+// kernel's lanes nor on the sort's free-first order. (ZWab, SumDen) of particle i.
 template <int DIM, int KT>
-__device__ __noinline__ float2 filter_sums(const DevView& v, const int* __restrict__ orig, int i, int cnt, int inst) {
+__device__ __forceinline__ float2 filter_sums(const DevView& v, const int* __restrict__ orig, int i, int cnt, int inst) {
   const Options& o = v.o;
   const Spec32& c32 = o.spec32c;
   const GridDev& g = grid_of(v, inst);
@@ -712,11 +710,17 @@ __device__ __noinline__ float2 filter_sums(const DevView& v, const int* __restri
   return make_float2(zw, sd);
 }
 
-// ZWab of a particle from its lanes' sums
-PSPH_D float group_zw(float2 zw, int L) {
-  float z = zw.x + zw.y;
-  for (int m = 1; m < L; m <<= 1) z += __shfl_xor_sync(0xffffffffu, z, m);
-  return z;
+// On a Shepard step particle i's sums in that order in place of the lanes', where the
+// filter can apply (ZWab above 0.6).
+template <int DIM, int KT>
+__device__ __noinline__ void filter_particle(const DevView& v, int i) {
+  const Persist& P = cur_persist(v);
+  const PClass32& C = v.cls32[P.cls[i]];
+  if (!(C.flags & CF_SHEPARD) || v.inst[C.inst].shepard_counter != v.o.shepard_step) return;
+  if (!(v.S.zwab[i] > 0.599) || v.S.cellid[i] < 0 || v.S.nl_count[i] < 0) return;
+  const float2 f = filter_sums<DIM, KT>(v, P.orig, i, v.S.nl_count[i], C.inst);
+  v.S.zwab[i] = f.x;
+  v.S.sumden[i] = f.y;
 }
 
 constexpr int kSumsMax = 20;  // a particle's sums on their way to its thread
@@ -916,10 +920,6 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
       pairs(e, e, false);
     }
   }
-  float2 filtered = dup(0.f);
-  const float zw_all = group_zw(zw, L);
-  const bool filter = shep && active && cell >= 0 && cnt >= 0 && zw_all > 0.599f;
-  if (filter && sub == 0) filtered = filter_sums<DIM, KT>(v, P.orig, i, cnt, inst_i);
   // even and odd neighbours together, then the lanes of the particle
   float out[kSumsMax];
   {
@@ -940,8 +940,8 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
       out[2 * e] = ss;
       out[2 * e + 1] = cc;
     }
-    out[8] = filter ? filtered.x : zw.x + zw.y;
-    out[9] = filter ? filtered.y : sd.x + sd.y;
+    out[8] = zw.x + zw.y;
+    out[9] = sd.x + sd.y;
     const float mm[9] = {m00, m11, m22, m01, m02, m12, m10, m20, m21};
 #pragma unroll
     for (int e = 0; e < 9; ++e) out[10 + e] = mm[e];
@@ -1016,6 +1016,10 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
     if (cand < dtc) dtc = cand;
   }
   block_dt32_and_pairs(v, inst, active, dtc, (unsigned long long)npair2, cred);
+  // the filter's sums last and in a call of its own, which then takes no registers from
+  // the pair loop (5.6M particles with the closure, which never filter: 2,302 us, 2,331
+  // with the call ahead of the reductions)
+  if (active && o.any_shepard && v.inst[inst].shepard_counter == o.shepard_step) filter_particle<DIM, KT>(v, i);
 }
 
 // ---------------------------------------------------------------------------
