@@ -74,15 +74,15 @@ FORCE32_BYTES_PER_PARTICLE = {False: 104, True: 148}
 # DRAM bytes per particle one launch actually moved: ncu captures of the same
 # kernels on the same tank at dx = 10 mm (1,021,104 particles),
 # dram__bytes per particle (LES + closure flavour with the 5 % list skin the
-# autotuner picks: 340.8 MB; without LES, lists every step: 324.6 MB); the traffic grows
+# autotuner picks: 341.1 MB; without LES, lists every step: 324.9 MB); the traffic grows
 # with the particle count, so a full-size launch moves this x n. Most of the
 # excess over the algorithmic bytes is the neighbour list (~80 entries x 4 B a
 # particle).
-FORCE32_TRAFFIC_BYTES_PER_PARTICLE = {False: 317.9, True: 333.8}
+FORCE32_TRAFFIC_BYTES_PER_PARTICLE = {False: 318.2, True: 334.1}
 # Pipe activity of that launch (LES + closure flavour, list skin) and of the FP64
 # pair kernel (pass A, 177,156 particles; sm__pipe_fp64_cycles_active, % of peak).
-FORCE32_NCU = {"issue_active": 0.609, "l1_wavefronts": 0.557, "fp64_pipe": 0.066, "warps_active": 0.239}
-FORCE64_NCU_FP64_PIPE = 0.785
+FORCE32_NCU = {"issue_active": 0.604, "l1_wavefronts": 0.553, "fp64_pipe": 0.066, "warps_active": 0.241}
+FORCE64_NCU_FP64_PIPE = 0.784
 
 
 def peaks():
