@@ -67,6 +67,7 @@ struct psph_ctx {
   PClass32* d_cls32 = nullptr;
   GridDev* d_grids = nullptr;           // the lists' and the sort's grids (the reference's without a skin)
   GridDev* d_grids_ref = nullptr;       // the reference's grids (CellInitiate)
+  InstForm* d_forms = nullptr;          // ensembles whose instances differ in their parameter sets
   int total_cells_ref = 0;
   InstState* d_inst = nullptr;
   InstState* h_inst = nullptr;  // pinned mirror (behind h_sc, as d_inst behind d_sc: one copy fetches both)
@@ -291,6 +292,7 @@ bool tail_fits(int ncap, bool solid) {
 
 DevView view(psph_ctx* c) {
   DevView v{};
+  v.forms = c->d_forms;
   v.grids = c->d_grids;
   v.grids_ref = c->d_grids_ref;
   v.inst = c->d_inst;
@@ -620,6 +622,8 @@ void derive_class_options(const std::vector<PClass>& classes, bool mixed, bool d
     f.eps2 = (float)o.spec.eps2;
     f.neg_alpha_h = (float)o.spec.neg_alpha_h;
     f.beta_h2 = (float)(C0.beta * C0.h * C0.h);
+    f.inv_h = (float)o.inv_h;
+    f.mu = (float)o.mu_u;
     f.far2 = (float)(100.0 * C0.h * C0.h);
     const int self = ff & (CF_T0 | CF_LES);
     f.sr_free = (self && ((ff & CF_T0) || (ff & CF_LES))) ? -1.f : 0.f;
@@ -628,6 +632,41 @@ void derive_class_options(const std::vector<PClass>& classes, bool mixed, bool d
     f.wall_scaled = o.spec.wall_scaled;
     f.wall_visc = ((ff | fw) & CF_NOSLIP) != 0;
   }
+}
+
+// The instances' own forms (InstForm), and in o whether they are needed: where all
+// instances share the options' form, or none has one, they are not.
+std::vector<InstForm> instance_forms(const std::vector<PClass>& classes, int ninst, bool mixed, bool dyn_mu, Options& o) {
+  o.mix64 = o.mix32 = o.mix_soil = 0;
+  std::vector<std::vector<PClass>> own((size_t)ninst);
+  std::vector<std::vector<int>> index((size_t)ninst);
+  for (size_t q = 0; q < classes.size(); ++q) {
+    own[(size_t)classes[q].inst].push_back(classes[q]);
+    index[(size_t)classes[q].inst].push_back((int)q);
+  }
+  std::vector<InstForm> forms((size_t)ninst);
+  for (int q = 0; q < ninst; ++q) {
+    Options oq = o;
+    derive_class_options(own[(size_t)q], mixed, dyn_mu, oq);
+    InstForm& f = forms[(size_t)q];
+    f.spec64 = oq.spec64 && o.fp64_half;
+    f.spec32 = oq.spec32;
+    f.soil32 = oq.soil32;
+    f.uniform_eos = oq.uniform_eos;
+    f.eos_cls = index[(size_t)q][(size_t)oq.eos_cls];
+    f.soil_noslip = oq.soil_noslip;
+    f.soil_fpm = oq.fpm_wall32;
+    f.spec = oq.spec;
+    f.spec32c = oq.spec32c;
+    o.mix64 |= f.spec64 ? kMixSpec : kMixGeneral;
+    o.mix32 |= f.spec32 ? kMixSpec : kMixGeneral;
+    o.mix_soil |= f.soil32 ? kMixSpec : kMixGeneral;
+  }
+  if (o.spec64 || !(o.mix64 & kMixSpec)) o.mix64 = 0;
+  if (o.spec32 || !(o.mix32 & kMixSpec)) o.mix32 = 0;
+  if (o.soil32 || !(o.mix_soil & kMixSpec)) o.mix_soil = 0;
+  if (!o.mix64 && !o.mix32 && !o.mix_soil && o.uniform_eos) forms.clear();
+  return forms;
 }
 
 psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
@@ -1046,10 +1085,18 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
   if (o.couple_soil && o.swi == 1 && (st = dalloc(c, &S.s_acc, N))) return st;
   if (o.couple_soil && o.swi != 2 && (st = dalloc(c, &S.satcheck, N))) return st;
   if (o.couple_solid && ((st = dalloc(c, &S.fsi_p, N)) || (st = dalloc(c, &S.fsi_nsv, N)))) return st;
-  if ((st = dalloc(c, &S.nl, (size_t)o.nl_cap * nl_stride_of(c->ncap)))) return st;
-  if (!o.fp32 && (st = dalloc(c, &S.pair_info, N))) return st;
   // FP64 fluids without strain-rate sums, XSPH or solids: each pair evaluated once
   o.fp64_half = !o.fp32 && !o.has_solid && !o.need_sr && o.xsph == 0.0;
+  c->d_forms = nullptr;
+  if (ninst > 1 && !mixed) {
+    const std::vector<InstForm> forms = instance_forms(c->classes, ninst, mixed, dyn_mu, o);
+    if (!forms.empty()) {
+      if ((st = dalloc(c, &c->d_forms, forms.size()))) return st;
+      CUDA_TRY(c, cudaMemcpy(c->d_forms, forms.data(), forms.size() * sizeof(InstForm), cudaMemcpyHostToDevice));
+    }
+  }
+  if ((st = dalloc(c, &S.nl, (size_t)o.nl_cap * nl_stride_of(c->ncap)))) return st;
+  if (!o.fp32 && (st = dalloc(c, &S.pair_info, N))) return st;
   if (o.fp64_half) {
     const size_t slots = (size_t)o.nl_cap * nl_stride_of(c->ncap);
     if ((st = dalloc(c, &S.half4, slots)) || (st = dalloc(c, &S.half_zw, slots)) ||
@@ -1064,15 +1111,16 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
     if ((st = dalloc(c, &S.V32, N)) || (st = dalloc(c, &S.D32, N)) || (st = dalloc(c, &S.NSV32, N)) ||
         (st = dalloc(c, &S.V32LO, N)))
       return st;
-    if (o.spec32 && (st = dalloc(c, &S.PX32, N))) return st;
+    if ((o.spec32 || o.mix32) && (st = dalloc(c, &S.PX32, N))) return st;
     if (o.spec32) S.RC32 = reinterpret_cast<float2*>(S.D32);
+    if (o.mix32 && (st = dalloc(c, &S.RC32, N))) return st;  // (some instances write D32)
     if (dyn_mu && (st = dalloc(c, &S.MU32, N))) return st;
     if (o.need_sr && !o.has_solid &&  // FP32 ShearRate and strain-rate sums of the fluid kernel
         ((st = dalloc(c, &S.cshear, N)) || (st = dalloc(c, &S.sr32, 6 * N))))
       return st;
   }
   if (o.fp32 && o.has_solid) {
-    if (o.soil32 && (st = dalloc(c, &S.PX32, N))) return st;
+    if ((o.soil32 || o.mix_soil) && (st = dalloc(c, &S.PX32, N))) return st;
     if ((st = dalloc(c, &S.rates32, 3 * N))) return st;
     if ((st = dalloc(c, &S.SIG32, 2 * N)) || (st = dalloc(c, &S.VB32, N))) return st;
     if (o.any_ti && (st = dalloc(c, &S.TIR32, 2 * N))) return st;

@@ -28,7 +28,7 @@ PSPH_D void fluid_copies32(const DevView& v, const Persist& P, int w, int cls, d
     const float inv = 1.f / rho;
     const float ratio = rho / C.rho0;
     const float c = (C.pres_eq == 1) ? fabsf(C.cs * ratio * ratio * ratio) : C.cs;  // sqrt(cs^2 ratio^6)
-    if (v.o.spec32) {  // the constant-parameter pair kernel's record (the walls' comes with their pressure)
+    if (spec32_of(v, C.inst)) {  // the constant-parameter pair kernel's record (the walls' comes with their pressure)
       v.S.RC32[w] = make_float2(rho, __int_as_float(refcell));
       v.S.PX32[w] = make_float4(x.x, x.y, x.z, with_sign(inv, 1.f));
       lw = with_sign(c, rho);

@@ -121,6 +121,20 @@ struct Spec32 {
   float far2;               // a squared distance outside the support
   float sr_free, sr_wall;   // -1 where a strain rate is summed over free / fixed neighbours, else 0
   int av, wall_scaled, wall_visc;  // wall_visc: a viscous term with walls (one side is no-slip)
+  float inv_h, mu;          // 1/h and the shared viscosity (an instance's own: InstForm)
+};
+
+// What an instance of an ensemble takes from its own parameter sets where the
+// instances differ in them (DevView::forms): the pair kernels' form and its constants,
+// and its walls' equation of state, as in a context of its own, so that it evolves bit
+// for bit as it does alone.
+struct InstForm {
+  int spec64, spec32, soil32;  // Options' fields of the same names
+  int uniform_eos, eos_cls;
+  int soil_noslip;
+  float soil_fpm;              // the walls' FPMassC (soil32)
+  Spec64 spec;
+  Spec32 spec32c;
 };
 
 struct Options {
@@ -181,6 +195,9 @@ struct Options {
   int nclasses;
   int closure;        // learned eddy-viscosity closure attached
   double closure_dx;  // lattice spacing of its h/dx feature
+  // instances that differ in their form (InstForm): kMixSpec some take the
+  // constant-parameter kernel, kMixGeneral some the general one; 0: all take the options'
+  int mix64, mix32, mix_soil;
 };
 
 // Chunk stride of the neighbour lists (nl_slot permutes particles inside
@@ -188,6 +205,7 @@ struct Options {
 inline int nl_stride_of(int ncap) { return (ncap + 63) & ~63; }
 
 // Everything a launch needs, passed by value to the launch wrappers.
+enum : int { kMixSpec = 1, kMixGeneral = 2 };
 struct DevView {
   const GridDev* grids;   // per instance (device array): the cells of the sort and the lists
   const GridDev* grids_ref;  // the reference's grids (CellInitiate); the same as grids without a skin
@@ -205,13 +223,24 @@ struct DevView {
   int ncap;
   int nl_stride;          // neighbour-list chunk stride: ncap rounded up to a multiple of 64 (nl_slot)
   int nclasses;
+  const InstForm* forms;  // per instance; null where the options hold for all of them
 };
 
 PSPH_D const GridDev& grid_of(const DevView& v, int inst) { return v.grids[inst]; }
 
 PSPH_D const Persist& cur_persist(const DevView& v) { return v.sc->buf ? v.PB : v.PA; }
+// Whether an instance takes the FP32C constant-parameter kernels.
+PSPH_D bool spec32_of(const DevView& v, int inst) { return v.o.mix32 ? v.forms[inst].spec32 : v.o.spec32; }
+PSPH_D bool soil32_of(const DevView& v, int inst) { return v.o.mix_soil ? v.forms[inst].soil32 : v.o.soil32; }
+// The EOS class that an instance's walls take their density from, or -1 where its fluid has several.
+PSPH_D int wall_eos(const DevView& v, int inst) {
+  if (v.forms) return v.forms[inst].uniform_eos ? v.forms[inst].eos_cls : -1;
+  return v.o.uniform_eos ? v.o.eos_cls : -1;
+}
 // A free particle's FP32 density (FP32C form).
-PSPH_D float rho32(const DevView& v, int s) { return v.o.spec32 ? v.S.RC32[s].x : v.S.D32[s].w; }
+PSPH_D float rho32(const DevView& v, int s, int inst) {
+  return spec32_of(v, inst) ? v.S.RC32[s].x : v.S.D32[s].w;
+}
 // A particle's row in the tensor arrays.
 PSPH_D size_t tensor_row(const Persist& P, int s) { return 9 * (size_t)P.orig[s]; }
 PSPH_D const Persist& next_persist(const DevView& v) { return v.sc->buf ? v.PA : v.PB; }

@@ -312,7 +312,7 @@ PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int f
   xw = P.X4[w];
   const double* f = sums[threadIdx.x];
   sk = f[0]; p = f[1]; n0 = f[2]; n1 = f[3]; n2 = f[4];
-  const PClass& Ce = CT[o.eos_cls];
+  const int eos_cls = wall_eos(v, Cw.inst);
   if (sk != 0.0) {
     if (mat < 3) p = p / sk;
     if (noslip) { n0 = n0 / sk; n1 = n1 / sk; n2 = n2 / sk; }
@@ -342,12 +342,13 @@ PSPH_D void wall_interpolation(const DevView& v, const Persist& P, int lg, int f
     v.S.pair_info[w] = cls_w | (v.S.cellid[w] >= 0 && v.S.nl_count[w] >= 0 ? kInfoList : 0) | tir_bit(v, P, w);
   // density, 1/density, p/density^2 and sound speed the partners see (Source/Interaction.cpp:41-61)
   double rw = xw.w, cwv = 0.0;
-  if (o.uniform_eos && mat != 3) {
+  if (eos_cls >= 0 && mat != 3) {
+    const PClass& Ce = CT[eos_cls];
     rw = density_solid(Ce.pres_eq, Ce.cs, Ce.p0, p, Ce.rho0);
     cwv = sound_speed(Ce.pres_eq, Ce.cs, rw, Ce.rho0);
   }
   const double inv = rcp_refined(rw);
-  if (DIM == 2 && o.soil32) {
+  if (DIM == 2 && soil32_of(v, Cw.inst)) {
     soil_records(v, P, w, true, vw, inv, sig);
     const double4_32a vb = (o.scheme == PSPH_MVERLET) ? P.H4[w] : P.H4b[w];
     v.S.VB32[w] = make_float4(d2f_rn(vb.x), d2f_rn(vb.y), d2f_rn(vb.z), 0.f);
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(kFT) prepare_wall_kernel(DevView v, int lg, in
   const double4_32a vel = P.V4[q];
   if (o.has_solid && C.material > 1 && C.ti > 0.0)
     tensile_tir<DIM>(P.sigma + tensor_row(P, q), C.ti, rho, P.tir + tensor_row(P, q));
-  if (DIM == 2 && o.soil32) soil_records(v, P, q, false, vel, inv, P.sigma + tensor_row(P, q));
+  if (DIM == 2 && soil32_of(v, C.inst)) soil_records(v, P, q, false, vel, inv, P.sigma + tensor_row(P, q));
   else v.S.D4[q] = make_double4_32a(inv, vel.w * inv * inv, sound_speed(C.pres_eq, C.cs, rho, C.rho0), rho);
   if (v.S.pair_info)
     v.S.pair_info[q] =
@@ -443,18 +444,19 @@ PSPH_D double dt_bound(const DevView& v, const double* a, double h) {
   return (cand < DBL_MAX) ? cand : DBL_MAX;  // NaN never compares less, as in the reference
 }
 
-// SPEC: Morris viscosity, squared-density gradient, one h, one EOS and pair
+// SPEC 1: Morris viscosity, squared-density gradient, one h, one EOS and pair
 // constants (artificial viscosity, masses, viscosity) the same for every class,
 // without tensile instability, strain rates, XSPH or a second material (the dam
 // breaks and the channel): those constants come from the launch parameters and
-// the terms that vanish are not compiled. The FP64 pipe (2 lanes per SM per
+// the terms that vanish are not compiled. SPEC 2: the same with an instance's own
+// constants (InstForm), for ensembles whose instances differ. The FP64 pipe (2 lanes per SM per
 // clock) bounds this kernel, so what counts is FP64 instructions per pair.
 //
 // A particle's list is walked by 2^lg lanes (LaneGroup): each round reads 2^lg
 // entries, drops those the partner evaluates, and queues the rest in shared
 // memory across the group, so that every lane then evaluates the same number of
 // pairs to within one.
-template <int DIM, int KT, bool HALF, bool SPEC>
+template <int DIM, int KT, bool HALF, int SPEC>
 __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v, int lg) {
   __shared__ double red[kFT / 32];
   __shared__ unsigned long long cred[kFT / 32];
@@ -476,7 +478,9 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v, int lg) {
   if (i < n) {
     ci_cls = P.cls[i];
     // a domain of two materials runs this kernel for its fluid particles only
-    const bool run = !v.inst[CT[ci_cls].inst].stop && (!o.mixed || CT[ci_cls].material == 1);
+    const int inst = CT[ci_cls].inst;
+    bool run = !v.inst[inst].stop && (!o.mixed || CT[ci_cls].material == 1);
+    if (o.mix64) run = run && (SPEC != 0) == (v.forms[inst].spec64 != 0);  // the other kernel takes the others
     active = run && CT[ci_cls].is_free;
     cell = v.S.cellid[i];
     if (run && !active && G.sub == 0) {
@@ -489,6 +493,7 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v, int lg) {
   const PClass& Ci = CT[ci_cls];
   const GridDev& g = grid_of(v, Ci.inst);
   const InstState& Is = v.inst[Ci.inst];
+  const Spec64& sp = SPEC == 2 ? v.forms[Ci.inst].spec : o.spec;
   const double4_32a xi = active ? P.X4[i] : make_double4_32a(0, 0, 0, 1);
   const double4_32a vi = active ? P.V4[i] : make_double4_32a(0, 0, 0, 0);
   const double4_32a di4 = active ? v.S.D4[i] : make_double4_32a(1, 0, 0, 1);
@@ -564,11 +569,11 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v, int lg) {
       const bool fj = infoj & kInfoFree;
       const PClass& Cj = CT[SPEC ? 0 : (infoj & kInfoCls)];
       if (!HALF && !SPEC && o.mixed && Cj.material != 1) continue;  // soil or solid partners: the coupling kernel
-      const double hb = SPEC ? o.spec.h : (hi + Cj.h) / 2;
+      const double hb = SPEC ? sp.h : (hi + Cj.h) / 2;
       double x0 = xi.x - xj.x, x1 = xi.y - xj.y, x2 = xi.z - xj.z;
       if (any_periodic) periodic_fix(g, x0, x1, x2, hb, cci, decode(g, v.S.cellid[j]));
       const double r2 = x0 * x0 + x1 * x1 + x2 * x2;
-      const double inv_hb = SPEC ? o.spec.inv_h : (o.uniform_h ? o.inv_h : 1.0 / hb);
+      const double inv_hb = SPEC ? sp.inv_h : (o.uniform_h ? o.inv_h : 1.0 / hb);
       double rij, inv_r = 0.0;
       if (KT == 1 && (SPEC || o.vis_eq <= 1)) {
         rij = sqrt_newton(r2);
@@ -585,35 +590,35 @@ __global__ void __launch_bounds__(kFT) forces_fluid_kernel(DevView v, int lg) {
       const double vx = v0 * x0 + v1 * x1 + v2 * x2;
       if (SPEC) {
         // kernel and gradient times a free partner's mass
-        double GKm = Kern<DIM, KT>::GK(q, hb * inv_r, o.spec.cwg_m);
-        double Km = Kern<DIM, KT>::W(q, o.spec.cwh_m);
+        double GKm = Kern<DIM, KT>::GK(q, hb * inv_r, sp.cwg_m);
+        double Km = Kern<DIM, KT>::W(q, sp.cwh_m);
         const double inv_j = dj4.x;
         double PI = 0.0;
-        if (o.spec.av && negative(vx)) {
+        if (sp.av && negative(vx)) {
           // (-a c MU + b MU^2) / rho_ij with MU = h v.x / D; without b one factor D less
-          const double D = r2 + o.spec.eps2, c2 = ci_snd + dj4.z, d2 = di + dj4.w;
-          if (!o.spec.av_beta) {
-            PI = (vx * o.spec.neg_alpha_h) * c2 * rcp_newton(D * d2);
+          const double D = r2 + sp.eps2, c2 = ci_snd + dj4.z, d2 = di + dj4.w;
+          if (!sp.av_beta) {
+            PI = (vx * sp.neg_alpha_h) * c2 * rcp_newton(D * d2);
           } else {
-            const double t = o.spec.h * vx;
-            PI = vx * (0.5 * (o.spec.neg_alpha_h * c2) * D + o.spec.beta_h * t) * rcp_newton(D * D * (0.5 * d2));
+            const double t = sp.h * vx;
+            PI = vx * (0.5 * (sp.neg_alpha_h * c2) * D + sp.beta_h * t) * rcp_newton(D * D * (0.5 * d2));
           }
         }
         double vab0 = v0, vab1 = v1, vab2 = v2;
         double c = 0.0;
         if (fj) {
-          c = o.spec.mu2 * inv_i;
+          c = sp.mu2 * inv_i;
         } else {  // a wall: its mass, and its no-slip velocity, or no viscous term between two that slip
-          if (o.spec.wall_scaled) {
-            GKm *= o.spec.wall_scale;
-            Km *= o.spec.wall_scale;
+          if (sp.wall_scaled) {
+            GKm *= sp.wall_scale;
+            Km *= sp.wall_scale;
           }
           if (Ci.no_slip || CT[infoj & kInfoCls].no_slip) {
             const double4_32a ns = v.S.nsv4[j];
             vab0 = vi.x - (2.0 * vj.x - ns.x);
             vab1 = vi.y - (2.0 * vj.y - ns.y);
             vab2 = vi.z - (2.0 * vj.z - ns.z);
-            c = o.spec.mu2 * inv_i;
+            c = sp.mu2 * inv_i;
           }
         }
         c = c * inv_j * GKm;
@@ -1672,11 +1677,13 @@ void fluid_forces(const DevView& v, cudaStream_t st) {
   const int lg = lanes_log2(v.o.kt);
   const int nb = nblk(v.ncap, kFT >> lg);
   if (v.o.fp64_half) {  // each pair once: pass A, then the partners' terms
-    if (v.o.spec64) forces_fluid_kernel<DIM, KT, true, true><<<nb, kFT, 0, st>>>(v, lg);
-    else forces_fluid_kernel<DIM, KT, true, false><<<nb, kFT, 0, st>>>(v, lg);
+    if (v.o.mix64 & kMixSpec) forces_fluid_kernel<DIM, KT, true, 2><<<nb, kFT, 0, st>>>(v, lg);
+    else if (v.o.spec64) forces_fluid_kernel<DIM, KT, true, 1><<<nb, kFT, 0, st>>>(v, lg);
+    if (v.o.mix64 ? (v.o.mix64 & kMixGeneral) : !v.o.spec64)
+      forces_fluid_kernel<DIM, KT, true, 0><<<nb, kFT, 0, st>>>(v, lg);
     forces_fluid_fold_kernel<<<nb, kFT, 0, st>>>(v, lg);
   } else {
-    forces_fluid_kernel<DIM, KT, false, false><<<nb, kFT, 0, st>>>(v, lg);
+    forces_fluid_kernel<DIM, KT, false, 0><<<nb, kFT, 0, st>>>(v, lg);
   }
 }
 

@@ -177,8 +177,9 @@ PSPH_D void interpolate_wall32(const DevView& v, const Persist& P, int w, int su
   float sk = 0.f, p = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
   const float hw = fabsf(oi.w), ihw = 1.f / hw;
   // a free neighbour's density and, with a skin, its cell in the reference's grid
+  const bool spec = spec32_of(v, C.inst);
   auto density_and_cell = [&](int f) {
-    return o.spec32 ? ld_early_coherent(v.S.RC32 + f)
+    return spec ? ld_early_coherent(v.S.RC32 + f)
                     : make_float2(ld_early_coherent(&v.S.D32[f].w),
                                   skin && need_orient ? __int_as_float(v.S.refcell[f]) : 0.f);
   };
@@ -262,9 +263,10 @@ PSPH_D void interpolate_wall32(const DevView& v, const Persist& P, int w, int su
   v.S.nsv4[w] = make_double4_32a(n0, n1, n2, 0.0);
   v.S.NSV32[w] = make_float4(n0, n1, n2, 0.f);
   v.S.V32[w] = make_float4(d2f_rn(vw.x), d2f_rn(vw.y), d2f_rn(vw.z), p);
-  const PClass32& Ce = CT[o.eos_cls];
+  const int eos_cls = wall_eos(v, C.inst);
   float rw = d2f_rn(P.X4[w].w), cwv = 0.f;
-  if (o.uniform_eos) {
+  if (eos_cls >= 0) {
+    const PClass32& Ce = CT[eos_cls];
     // DensitySolid / SoundSpeed of the fluid's EOS (Source/Functions.cpp:214-264), FP32
     const float cs2 = Ce.cs * Ce.cs, r0 = Ce.rho0, p0 = Ce.p0;
     if (Ce.pres_eq == 0) rw = (p - p0) / cs2 + r0;
@@ -274,7 +276,7 @@ PSPH_D void interpolate_wall32(const DevView& v, const Persist& P, int w, int su
     cwv = (Ce.pres_eq == 1) ? fabsf(Ce.cs * ratio * ratio * ratio) : Ce.cs;  // sqrt(cs^2 ratio^6)
   }
   const float inv = 1.f / rw;
-  if (o.spec32) {
+  if (spec) {
     // a wall without a free particle in its support has none to meet, but may
     // stand in a list (their margin): its terms are zeros times finite numbers
     const bool odd = sk == 0.f && !(fabsf(inv) <= FLT_MAX);
@@ -334,7 +336,8 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
   int cell = -1, ci_cls = 0;
   if (i < n) {
     ci_cls = P.cls[i];
-    const bool run = !v.inst[CT[ci_cls].inst].stop;
+    bool run = !v.inst[CT[ci_cls].inst].stop;
+    if (o.mix32) run = run && !v.forms[CT[ci_cls].inst].spec32;  // (forces_spec32_kernel takes those)
     active = run && (CT[ci_cls].flags & CF_FREE);
     cell = v.S.cellid[i];
     if (run && !active) {
@@ -661,14 +664,14 @@ PSPH_D void kern2(float2 q, float2 inv_q, float cwh, float cwg, float2& K, float
 // x-slabs, a slab's particles by original index, as the general kernel's
 // expressions take them, so that a filtered density depends neither on the pair
 // kernel's lanes nor on the sort's free-first order. (ZWab, SumDen) of particle i.
-template <int DIM, int KT>
+template <int DIM, int KT, bool OWN>
 __device__ __forceinline__ float2 filter_sums(const DevView& v, const int* __restrict__ orig, int i, int cnt, int inst) {
   const Options& o = v.o;
-  const Spec32& c32 = o.spec32c;
+  const Spec32& c32 = OWN ? v.forms[inst].spec32c : o.spec32c;
   const GridDev& g = grid_of(v, inst);
   const float3 cs = cell_size_f(g);
   const float4 xi = v.S.PX32[i];
-  const float hi = c32.h, ih = o.inv_h32, ih2 = ih * ih;
+  const float hi = c32.h, ih = OWN ? c32.inv_h : o.inv_h32, ih2 = ih * ih;
   const float cwh = KernF<DIM, KT>::cw() * (DIM == 2 ? ih2 : ih2 * ih);
   float zw = 0.f, sd = 0.f;
   auto one = [&](const int e) {
@@ -712,20 +715,21 @@ __device__ __forceinline__ float2 filter_sums(const DevView& v, const int* __res
 
 // On a Shepard step particle i's sums in that order in place of the lanes', where the
 // filter can apply (ZWab above 0.6).
-template <int DIM, int KT>
+template <int DIM, int KT, bool OWN>
 __device__ __noinline__ void filter_particle(const DevView& v, int i) {
   const Persist& P = cur_persist(v);
   const PClass32& C = v.cls32[P.cls[i]];
   if (!(C.flags & CF_SHEPARD) || v.inst[C.inst].shepard_counter != v.o.shepard_step) return;
   if (!(v.S.zwab[i] > 0.599) || v.S.cellid[i] < 0 || v.S.nl_count[i] < 0) return;
-  const float2 f = filter_sums<DIM, KT>(v, P.orig, i, v.S.nl_count[i], C.inst);
+  const float2 f = filter_sums<DIM, KT, OWN>(v, P.orig, i, v.S.nl_count[i], C.inst);
   v.S.zwab[i] = f.x;
   v.S.sumden[i] = f.y;
 }
 
 constexpr int kSumsMax = 20;  // a particle's sums on their way to its thread
 
-template <int DIM, int KT, int FL>
+// OWN: an instance's own constants (InstForm), for ensembles whose instances differ.
+template <int DIM, int KT, int FL, bool OWN>
 __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32_kernel(DevView v, int lg) {
   // in 3D the partner's mass is folded into the kernel's constants (the closure
   // flavour does not fit its registers otherwise: 3204 us against 2740)
@@ -745,7 +749,8 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
   int cell = -1, ci_cls = 0;
   if (i < n) {
     ci_cls = P.cls[i];
-    const bool run = !v.inst[CT[ci_cls].inst].stop;
+    bool run = !v.inst[CT[ci_cls].inst].stop;
+    if (OWN) run = run && v.forms[CT[ci_cls].inst].spec32;
     active = run && (CT[ci_cls].flags & CF_FREE);
     cell = v.S.cellid[i];
     if (run && !active && sub == 0) {
@@ -762,13 +767,14 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
   const float4 vi = v.S.V32[is];
   const float4 vl = v.S.V32LO[is];
   const float inv_i = with_sign(xi.w, vl.w), Pi = vi.w * inv_i * inv_i, snd_i = fabsf(vl.w);
-  const float mui = o.dyn_mu ? v.S.MU32[is] : o.mu_u32;
+  const Spec32& c32 = OWN ? v.forms[inst_i].spec32c : o.spec32c;
+  const float inv_h = OWN ? c32.inv_h : o.inv_h32;
+  const float mui = o.dyn_mu ? v.S.MU32[is] : (OWN ? c32.mu : o.mu_u32);
   const bool shep = (Ci.flags & CF_SHEPARD) && (Is.shepard_counter == o.shepard_step);
   const float3 cs = cell_size_f(g);
-  const Spec32& c32 = o.spec32c;
   const float reach2 = g.cellfac2_32 * c32.h * c32.h;
-  const float ih2 = o.inv_h32 * o.inv_h32;
-  float cwh = KernF<DIM, KT>::cw() * (DIM == 2 ? ih2 : ih2 * o.inv_h32), cwg = cwh * ih2;
+  const float ih2 = inv_h * inv_h;
+  float cwh = KernF<DIM, KT>::cw() * (DIM == 2 ? ih2 : ih2 * inv_h), cwg = cwh * ih2;
   if (FOLD) {
     cwh *= c32.m_free;
     if (FL == 1) cwg *= c32.m_free;
@@ -799,7 +805,7 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
     npair2 += (ia ? (fa ? 1u : 2u) : 0u) + (ib ? (fb ? 1u : 2u) : 0u);
     if (FL == 3) nnb += (ia ? 1 : 0) + (ib ? 1 : 0);
     const float2 inv_r = f2(rsqrt_ftz(fmaxf(r2.x, 1e-30f)), rsqrt_ftz(fmaxf(r2.y, 1e-30f)));
-    const float2 q = r2 * inv_r * dup(o.inv_h32);
+    const float2 q = r2 * inv_r * dup(inv_h);
     float2 K, GK;
     kern2<DIM, KT>(q, inv_r * dup(c32.h), cwh, cwg, K, GK);
     const float2 inv_j = f2(with_sign(xa.w, la.w), with_sign(xb.w, lb.w));
@@ -966,6 +972,7 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
           if (e < last) out[e] = staged[e * np + threadIdx.x];
         ci_cls = P.cls[i];
         active = !v.inst[CT[ci_cls].inst].stop && (CT[ci_cls].flags & CF_FREE);
+        if (OWN) active = active && v.forms[CT[ci_cls].inst].spec32;
       }
     }
   }
@@ -1012,14 +1019,15 @@ __global__ void __maxnreg__(DIM == 3 ? 128 : (FL == 1 ? 96 : 112)) forces_spec32
     // minimum over particles (FP32 within a warp) and AdaptiveTimeStep stay FP64
     const float ax32 = d2f_rn(axd), ay32 = d2f_rn(ayd), az32 = d2f_rn(azd);
     const float an = sqrtf(ax32 * ax32 + ay32 * ay32 + az32 * az32);
-    const float cand = o.sqrt_h_a32 * sqrtf(c32.h / an);
+    const float h = OWN ? CT[ci_cls].h : c32.h;  // (with lanes this thread's particle may be another instance's)
+    const float cand = o.sqrt_h_a32 * sqrtf(h / an);
     if (cand < dtc) dtc = cand;
   }
   block_dt32_and_pairs(v, inst, active, dtc, (unsigned long long)npair2, cred);
   // the filter's sums last and in a call of its own, which then takes no registers from
   // the pair loop (5.6M particles with the closure, which never filter: 2,299 us, 2,331
   // with the call ahead of the reductions)
-  if (active && o.any_shepard && v.inst[inst].shepard_counter == o.shepard_step) filter_particle<DIM, KT>(v, i);
+  if (active && o.any_shepard && v.inst[inst].shepard_counter == o.shepard_step) filter_particle<DIM, KT, OWN>(v, i);
 }
 
 // ---------------------------------------------------------------------------
@@ -1046,7 +1054,7 @@ __global__ void __launch_bounds__(kFT32) solid_copies32_kernel(DevView v) {
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= sc->n) return;
   const PClass32& C = v.cls32[P.cls[w]];
-  if (v.inst[C.inst].stop) return;
+  if (v.inst[C.inst].stop || (v.o.mix_soil && v.forms[C.inst].soil32)) return;  // (soil_records)
   const double4_32a vv = P.V4[w];
   float lx, ly, lz;
   const float vx = d2f_split(vv.x, &lx), vy = d2f_split(vv.y, &ly), vz = d2f_split(vv.z, &lz);
@@ -1096,7 +1104,8 @@ __global__ void __maxnreg__(128) forces_solid32_kernel(DevView v) {
   int cell = -1, ci_cls = 0;
   if (i < n) {
     ci_cls = P.cls[i];
-    const bool run = !v.inst[CT[ci_cls].inst].stop;
+    bool run = !v.inst[CT[ci_cls].inst].stop;
+    if (o.mix_soil) run = run && !v.forms[CT[ci_cls].inst].soil32;  // (forces_soil32_kernel takes those)
     active = run && (CT[ci_cls].flags & CF_FREE);
     cell = v.S.cellid[i];
     if (run && !active) {
@@ -1279,7 +1288,8 @@ __global__ void __maxnreg__(128) forces_solid32_kernel(DevView v) {
 // tensile stress (elsewhere it multiplies a zero).
 // 1.0M particles in ten columns: 513 us before (nine loads a neighbour and the
 // power for every pair), 197 us now.
-template <int KT>
+// OWN: for ensembles whose instances differ (InstForm).
+template <int KT, bool OWN>
 __global__ void __maxnreg__(112) forces_soil32_kernel(DevView v) {
   __shared__ unsigned long long cred[32];
   const StepScalars* sc = v.sc;
@@ -1295,7 +1305,8 @@ __global__ void __maxnreg__(112) forces_soil32_kernel(DevView v) {
   int cell = -1, ci_cls = 0;
   if (i < n) {
     ci_cls = P.cls[i];
-    const bool run = !v.inst[CT[ci_cls].inst].stop;
+    bool run = !v.inst[CT[ci_cls].inst].stop;
+    if (OWN) run = run && v.forms[CT[ci_cls].inst].soil32;
     active = run && (CT[ci_cls].flags & CF_FREE);
     cell = v.S.cellid[i];
     if (run && !active) {
@@ -1313,12 +1324,12 @@ __global__ void __maxnreg__(112) forces_soil32_kernel(DevView v) {
   const float ci2 = inv_i * inv_i;
   const float P00 = xi.z * ci2, P01 = xi.w * ci2, P11 = vi.z * ci2;  // the own stress over density squared
   const bool shep = (Ci.flags & CF_SHEPARD) && (Is.shepard_counter == o.shepard_step);
-  const float fpm = o.fpm_wall32;
+  const float fpm = OWN ? v.forms[Ci.inst].soil_fpm : o.fpm_wall32;
   const bool wall_scaled = fpm != 1.f, av = Ci.alpha != 0.f || Ci.beta != 0.f;
   const float ac = Ci.alpha * Ci.cs;
   const float3 cs = cell_size_f(g);
   const float reach2 = g.cellfac2_32 * h * h, far2 = 100.f * h * h, eps2 = 0.01f * h * h;
-  const bool noslip = o.soil_noslip;
+  const bool noslip = OWN ? v.forms[Ci.inst].soil_noslip : o.soil_noslip;
   Kahan2 ax, ay, dr;
   float2 zw = dup(0.f), sd = dup(0.f);
   float2 s00 = dup(0.f), s01 = dup(0.f), s11 = dup(0.f), r01 = dup(0.f), s02 = dup(0.f), s12 = dup(0.f);
@@ -1483,9 +1494,15 @@ void spec32_dispatch(const DevView& v, int bt, cudaStream_t st) {
   const int nb = v.ncap <= 0 ? 1 : (v.ncap + per - 1) / per;
   const size_t sm = lg > 0 ? sizeof(float) * kSumsMax * per : 0;
   const Options& o = v.o;
-  if (!o.need_sr) forces_spec32_kernel<DIM, KT, 1><<<nb, bt, sm, st>>>(v, lg);
-  else if (!o.closure) forces_spec32_kernel<DIM, KT, 2><<<nb, bt, sm, st>>>(v, lg);
-  else forces_spec32_kernel<DIM, KT, 3><<<nb, bt, sm, st>>>(v, lg);
+  if (o.mix32) {
+    if (!o.need_sr) forces_spec32_kernel<DIM, KT, 1, true><<<nb, bt, sm, st>>>(v, lg);
+    else if (!o.closure) forces_spec32_kernel<DIM, KT, 2, true><<<nb, bt, sm, st>>>(v, lg);
+    else forces_spec32_kernel<DIM, KT, 3, true><<<nb, bt, sm, st>>>(v, lg);
+    return;
+  }
+  if (!o.need_sr) forces_spec32_kernel<DIM, KT, 1, false><<<nb, bt, sm, st>>>(v, lg);
+  else if (!o.closure) forces_spec32_kernel<DIM, KT, 2, false><<<nb, bt, sm, st>>>(v, lg);
+  else forces_spec32_kernel<DIM, KT, 3, false><<<nb, bt, sm, st>>>(v, lg);
 }
 
 template <int DIM, int KT>
@@ -1499,17 +1516,23 @@ void fluid32_dispatch(const DevView& v, int nb, int bt, cudaStream_t st) {
   }
 }
 
+template <int KT>
+void soil32_dispatch(const DevView& v, int nb, int bt, cudaStream_t st) {
+  if (v.o.mix_soil) forces_soil32_kernel<KT, true><<<nb, bt, 0, st>>>(v);
+  else forces_soil32_kernel<KT, false><<<nb, bt, 0, st>>>(v);
+}
+
 template <int DIM>
 void forces32_dispatch(const DevView& v, cudaStream_t st) {
   const int bt = (v.o.pair_block >= 32 && v.o.pair_block <= kMaxPairBlock) ? v.o.pair_block : kFT32;
   const int nb = v.ncap <= 0 ? 1 : (v.ncap + bt - 1) / bt;
-  if (DIM == 2 && v.o.soil32) {
+  if (DIM == 2 && (v.o.soil32 || (v.o.mix_soil & kMixSpec))) {
     switch (v.o.kt) {
-      case 0: forces_soil32_kernel<0><<<nb, bt, 0, st>>>(v); break;
-      case 1: forces_soil32_kernel<1><<<nb, bt, 0, st>>>(v); break;
-      default: forces_soil32_kernel<2><<<nb, bt, 0, st>>>(v); break;
+      case 0: soil32_dispatch<0>(v, nb, bt, st); break;
+      case 1: soil32_dispatch<1>(v, nb, bt, st); break;
+      default: soil32_dispatch<2>(v, nb, bt, st); break;
     }
-    return;
+    if (!(v.o.mix_soil & kMixGeneral)) return;
   }
   if (v.o.has_solid) {
     switch (v.o.kt) {
@@ -1519,13 +1542,13 @@ void forces32_dispatch(const DevView& v, cudaStream_t st) {
     }
     return;
   }
-  if (v.o.spec32) {
+  if (v.o.spec32 || (v.o.mix32 & kMixSpec)) {
     switch (v.o.kt) {
       case 0: spec32_dispatch<DIM, 0>(v, bt, st); break;
       case 1: spec32_dispatch<DIM, 1>(v, bt, st); break;
       default: spec32_dispatch<DIM, 2>(v, bt, st); break;
     }
-    return;
+    if (!(v.o.mix32 & kMixGeneral)) return;
   }
   switch (v.o.kt) {
     case 0: fluid32_dispatch<DIM, 0>(v, nb, bt, st); break;
@@ -1543,7 +1566,7 @@ void launch_copies32(const DevView& v, cudaStream_t st) {
 void launch_prepare32(const DevView& v, cudaStream_t st) {
   if (v.o.has_solid) {  // FP64 wall stress interpolation and TIR, then the FP32 copies
     launch_prepare(v, st);
-    if (v.o.soil32) return;  // which wrote the pair kernel's records too
+    if (v.o.soil32 || v.o.mix_soil == kMixSpec) return;  // which wrote the pair kernel's records too
     const int nb = nblk32(v.ncap);
     if (v.o.dim == 2) solid_copies32_kernel<2><<<nb, kFT32, 0, st>>>(v);
     else solid_copies32_kernel<3><<<nb, kFT32, 0, st>>>(v);

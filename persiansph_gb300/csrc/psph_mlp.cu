@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kTcThreads) closure_kernel(DevView v) {
         f[0] = logf(fmaxf(sh32 * tscale, 1e-12f));
         f[1] = v.S.cr3[s];
         f[2] = logf(fmaxf(v.S.cvort[s] * tscale, 1e-12f));
-        f[3] = rho32(v, s) / C.rho0;
+        f[3] = rho32(v, s, C.inst) / C.rho0;
         f[4] = C.h_over_dx;
         f[5] = v.S.cnnb[s];
       }

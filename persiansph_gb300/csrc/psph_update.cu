@@ -595,7 +595,8 @@ void launch_upload_pack(const double* sx, const double* sd, const double* sp, co
 
 int launches_per_step(const DevView& v) {
   // begin, sort, neighbour lists, prepare, forces, dt, update, end (the last three in one with few particles)
-  return 7 - (v.o.fused_tail ? 2 : 0) + sort_launches(v) + (v.o.fp32 && v.o.has_solid && !v.o.soil32 ? 1 : 0) + (v.o.closure ? 1 : 0) +
+  return 7 - (v.o.fused_tail ? 2 : 0) + sort_launches(v) + (v.o.fp32 && v.o.has_solid && !v.o.soil32 && v.o.mix_soil != kMixSpec ? 1 : 0) +
+         (v.o.mix64 == 3 || v.o.mix32 == 3 || v.o.mix_soil == 3 ? 1 : 0) + (v.o.closure ? 1 : 0) +
          (v.o.fp64_half ? 1 : 0) + (v.o.mixed ? 2 : 0) + (v.o.couple_soil && v.o.swi != 2 ? 2 : 0) +
          (v.o.fsi ? 1 : 0) + (v.o.skin > 0.f ? 1 : 0);
 }
