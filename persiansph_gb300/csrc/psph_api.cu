@@ -591,8 +591,8 @@ void derive_class_options(const std::vector<PClass>& classes, bool mixed, bool d
     if (ff < 0) ff = 0;
     if (fw < 0) fw = 0;
     o.flavours32 = o.fp32 && o.vis_eq == PSPH_MORRIS && o.grad_type == PSPH_SQUARED_DENSITY && o.uniform_h &&
-                   o.uniform_av && o.uniform_mass && (o.uniform_mu || dyn_mu) && !o.any_ti && o.xsph == 0.0 &&
-                   !o.has_solid;
+                   o.uniform_av && o.uniform_mass && (o.uniform_mu || dyn_mu) && o.uniform_eos && !o.any_ti &&
+                   o.xsph == 0.0 && !o.has_solid;
     o.spec32 = o.flavours32 && one;
     // the FP32C 2D soil kernel's: also one sound speed and tensile instability, and
     // one free mass per instance
@@ -645,6 +645,7 @@ std::vector<InstForm> instance_forms(const std::vector<PClass>& classes, int nin
     index[(size_t)classes[q].inst].push_back((int)q);
   }
   std::vector<InstForm> forms((size_t)ninst);
+  bool several = false;
   for (int q = 0; q < ninst; ++q) {
     Options oq = o;
     derive_class_options(own[(size_t)q], mixed, dyn_mu, oq);
@@ -661,7 +662,9 @@ std::vector<InstForm> instance_forms(const std::vector<PClass>& classes, int nin
     o.mix64 |= f.spec64 ? kMixSpec : kMixGeneral;
     o.mix32 |= f.spec32 ? kMixSpec : kMixGeneral;
     o.mix_soil |= f.soil32 ? kMixSpec : kMixGeneral;
+    several = several || !f.uniform_eos;
   }
+  o.several_eos = several;
   if (o.spec64 || !(o.mix64 & kMixSpec)) o.mix64 = 0;
   if (o.spec32 || !(o.mix32 & kMixSpec)) o.mix32 = 0;
   if (o.soil32 || !(o.mix_soil & kMixSpec)) o.mix_soil = 0;
@@ -1088,6 +1091,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
   // FP64 fluids without strain-rate sums, XSPH or solids: each pair evaluated once
   o.fp64_half = !o.fp32 && !o.has_solid && !o.need_sr && o.xsph == 0.0;
   c->d_forms = nullptr;
+  o.several_eos = !o.uniform_eos;
   if (ninst > 1 && !mixed) {
     const std::vector<InstForm> forms = instance_forms(c->classes, ninst, mixed, dyn_mu, o);
     if (!forms.empty()) {

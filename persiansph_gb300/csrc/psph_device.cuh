@@ -198,6 +198,7 @@ struct Options {
   // instances that differ in their form (InstForm): kMixSpec some take the
   // constant-parameter kernel, kMixGeneral some the general one; 0: all take the options'
   int mix64, mix32, mix_soil;
+  int several_eos;    // some instance's fluid has more than one equation of state
 };
 
 // Chunk stride of the neighbour lists (nl_slot permutes particles inside

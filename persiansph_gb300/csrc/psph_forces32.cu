@@ -159,6 +159,16 @@ __global__ void __launch_bounds__(kFT32) copies32_kernel(DevView v) {
 template <int DIM>
 constexpr int kWallLanesLog2 = DIM == 2 ? 2 : 0;
 
+// DensitySolid / SoundSpeed of a fluid's EOS at a wall's pressure (Source/Functions.cpp:214-264), FP32
+PSPH_D void wall_state32(const PClass32& Ce, float p, float* rw, float* cw) {
+  const float cs2 = Ce.cs * Ce.cs, r0 = Ce.rho0, p0 = Ce.p0;
+  if (Ce.pres_eq == 0) *rw = (p - p0) / cs2 + r0;
+  else if (Ce.pres_eq == 1) *rw = powf((p - p0) * (7.f / (r0 * cs2)) + 1.f, 1.f / 7.f) * r0;
+  else *rw = p / cs2;
+  const float ratio = *rw / r0;
+  *cw = (Ce.pres_eq == 1) ? fabsf(Ce.cs * ratio * ratio * ratio) : Ce.cs;  // sqrt(cs^2 ratio^6)
+}
+
 template <int DIM, int KT>
 PSPH_D void interpolate_wall32(const DevView& v, const Persist& P, int w, int sub) {
   const Options& o = v.o;
@@ -265,16 +275,7 @@ PSPH_D void interpolate_wall32(const DevView& v, const Persist& P, int w, int su
   v.S.V32[w] = make_float4(d2f_rn(vw.x), d2f_rn(vw.y), d2f_rn(vw.z), p);
   const int eos_cls = wall_eos(v, C.inst);
   float rw = d2f_rn(P.X4[w].w), cwv = 0.f;
-  if (eos_cls >= 0) {
-    const PClass32& Ce = CT[eos_cls];
-    // DensitySolid / SoundSpeed of the fluid's EOS (Source/Functions.cpp:214-264), FP32
-    const float cs2 = Ce.cs * Ce.cs, r0 = Ce.rho0, p0 = Ce.p0;
-    if (Ce.pres_eq == 0) rw = (p - p0) / cs2 + r0;
-    else if (Ce.pres_eq == 1) rw = powf((p - p0) * (7.f / (r0 * cs2)) + 1.f, 1.f / 7.f) * r0;
-    else rw = p / cs2;
-    const float ratio = rw / r0;
-    cwv = (Ce.pres_eq == 1) ? fabsf(Ce.cs * ratio * ratio * ratio) : Ce.cs;  // sqrt(cs^2 ratio^6)
-  }
+  if (eos_cls >= 0) wall_state32(CT[eos_cls], p, &rw, &cwv);
   const float inv = 1.f / rw;
   if (spec) {
     // a wall without a free particle in its support has none to meet, but may
@@ -303,8 +304,10 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
 // ---------------------------------------------------------------------------
 // Fluid pair force, FP32 with compensated sums, over the neighbour lists
 // ---------------------------------------------------------------------------
-// FL 0: every option read at run time. FL 1, 2 and 3: Morris viscosity,
-// squared-density gradient, no tensile instability or XSPH, one h, and pair
+// FL 0: every option read at run time. FL 4: the same where some fluid has several
+// EOS (Options::several_eos), a wall's state then from its partner's (86k particles in
+// 2D with tensile instability 55 us; with this in FL 0 58). FL 1, 2 and 3: Morris viscosity,
+// squared-density gradient, no tensile instability or XSPH, one h, one EOS, and pair
 // constants (artificial viscosity, masses) the same for every class, taken from
 // the launch (Options::flavours32), without (1) or with (2) the strain-rate sums
 // of LES and Bingham, or with the learned closure's vorticity too (3); the
@@ -319,8 +322,8 @@ __global__ void __launch_bounds__(kFT32) prepare32_kernel(DevView v) {
 // flavour: 916 and 495 us without rates, 1049 and 606 with LES, 1012 and 606 with
 // the closure; 86k in 2D 44 and 25.
 template <int DIM, int KT, int FL>
-__global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_kernel(DevView v) {
-  constexpr bool SPEC = FL != 0;
+__global__ void __maxnreg__(FL == 0 || FL == 4 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_kernel(DevView v) {
+  constexpr bool SPEC = FL >= 1 && FL <= 3;
   constexpr bool CLOSURE = FL == 3;
   __shared__ unsigned long long cred[32];
   const StepScalars* sc = v.sc;
@@ -377,6 +380,7 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
   const bool closure = SPEC ? (CLOSURE && (fi & CF_LES)) : (o.closure && (fi & CF_LES));
   // the closure flavour always keeps the antisymmetric sums apart
   const bool split_sr = SPEC ? CLOSURE : closure;
+  const bool own_eos = FL == 4 && wall_eos(v, Ci.inst) < 0;
   const float cf2 = g.cellfac2_32;
   const bool uniform_h = o.uniform_h;
   const float ih_u = o.inv_h32;
@@ -408,7 +412,13 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
     const float cwg = cwh * ih2;
     const float GK = KernF<DIM, KT>::GK(q, inv_q, cwg);
     const float K = KernF<DIM, KT>::W(q, cwh);
-    const float dj = dj4.w, inv_j = dj4.x, Pj = dj4.y, cj_snd = dj4.z, pj = vj.w;
+    float dj = dj4.w, inv_j = dj4.x, Pj = dj4.y, cj_snd = dj4.z;
+    const float pj = vj.w;
+    if (own_eos && !fj) {  // wall density from this particle's EOS (Source/Interaction.cpp:53-57)
+      wall_state32(Ci, pj, &dj, &cj_snd);
+      inv_j = 1.f / dj;
+      Pj = pj * inv_j * inv_j;
+    }
     const float mj = SPEC ? (fj ? o.m_free32 : o.fpm_wall32 * mi) : (fj ? Cj.mass : Cj.fpmassc * mi);
     const float v0 = (vi.x - vj.x) + (vil.x - vjl.x), v1 = (vi.y - vj.y) + (vil.y - vjl.y),
                 v2 = (vi.z - vj.z) + (vil.z - vjl.z);
@@ -506,7 +516,7 @@ __global__ void __maxnreg__(FL == 0 ? 128 : (FL == 1 ? 80 : 96)) forces_fluid32_
     const int nch = (cnt + 3) >> 2;
     // the strain-rate flavours load the next chunk one chunk ahead (measured:
     // it helps there and costs the plain flavour a little)
-    constexpr bool kAhead = FL >= 2;
+    constexpr bool kAhead = SPEC && FL >= 2;
     int4 qn = (kAhead && nch > 0) ? nl4[0] : make_int4(0, 0, 0, 0);
     for (int c = 0; c < nch; ++c) {  // one 16-byte chunk of 4 entries per load
       int4 q;
@@ -1507,8 +1517,9 @@ void spec32_dispatch(const DevView& v, int bt, cudaStream_t st) {
 
 template <int DIM, int KT>
 void fluid32_dispatch(const DevView& v, int nb, int bt, cudaStream_t st) {
-  const int fl = !v.o.flavours32 ? 0 : !v.o.need_sr ? 1 : !v.o.closure ? 2 : 3;
+  const int fl = v.o.several_eos ? 4 : !v.o.flavours32 ? 0 : !v.o.need_sr ? 1 : !v.o.closure ? 2 : 3;
   switch (fl) {
+    case 4: forces_fluid32_kernel<DIM, KT, 4><<<nb, bt, 0, st>>>(v); break;
     case 0: forces_fluid32_kernel<DIM, KT, 0><<<nb, bt, 0, st>>>(v); break;
     case 1: forces_fluid32_kernel<DIM, KT, 1><<<nb, bt, 0, st>>>(v); break;
     case 2: forces_fluid32_kernel<DIM, KT, 2><<<nb, bt, 0, st>>>(v); break;

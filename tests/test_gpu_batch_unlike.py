@@ -29,6 +29,10 @@ def stirred(dom, dt, dx, params):
             slip = p.get("no_slip")
             slip[~free & (p.get("x")[:, 1] > a)] = 0
             p.set("no_slip", slip)
+        elif k == "right_cs":  # two equations of state within the instance
+            cs = p.get("cs")
+            cs[p.get("x")[:, 0] > 0.2] = a
+            p.set("cs", cs)
         else:
             p.set(k, a)
     return dom, 0.2 * dt
@@ -62,6 +66,7 @@ CASES = {
     "slip": lambda: [dam2(), dam2(no_slip=0)],
     "lid": lambda: [dam2(), dam2(lid=0.3)],  # one instance in each form
     "tension": lambda: [dam2(), dam2(ti=0.3, ti_init_dist=0.04), dam2(alpha=0.3)],
+    "several_eos": lambda: [dam2(ti=0.3, ti_init_dist=0.04), dam2(right_cs=60.0), dam2(lid=0.3), dam2()],
     "soil_lattice": lambda: [column(), column(0.03)],
     "soil_modulus": lambda: [column(), column(E=1.5e6)],
     "soil_tension": lambda: [column(), column(ti=0.0), column(tin=3.0)],
