@@ -135,14 +135,25 @@ psph_status set_err(psph_ctx* c, psph_status code, const char* fmt, ...) {
                      "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__);        \
   } while (0)
 
+// Device memory of a context, zeroed in its stream's order. Nothing of a context goes
+// through the default stream: its own stream does not wait for that one, so a memset
+// or a copy there, which returns before it is done, could land behind the kernels and
+// copies that follow here.
 template <class T>
 psph_status dalloc(psph_ctx* c, T** p, size_t count) {
   void* ptr = nullptr;
   if (count == 0) count = 1;
   CUDA_TRY(c, cudaMalloc(&ptr, count * sizeof(T)));
-  CUDA_TRY(c, cudaMemset(ptr, 0, count * sizeof(T)));
   c->allocs.push_back(ptr);
+  CUDA_TRY(c, cudaMemsetAsync(ptr, 0, count * sizeof(T), c->stream));
   *p = (T*)ptr;
+  return PSPH_OK;
+}
+
+// Device data to the host, in the stream's order, and waited for.
+psph_status fetch(psph_ctx* c, void* dst, const void* src, size_t bytes) {
+  CUDA_TRY(c, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream));
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   return PSPH_OK;
 }
 
@@ -1096,7 +1107,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
     const std::vector<InstForm> forms = instance_forms(c->classes, ninst, mixed, dyn_mu, o);
     if (!forms.empty()) {
       if ((st = dalloc(c, &c->d_forms, forms.size()))) return st;
-      CUDA_TRY(c, cudaMemcpy(c->d_forms, forms.data(), forms.size() * sizeof(InstForm), cudaMemcpyHostToDevice));
+      CUDA_TRY(c, cudaMemcpyAsync(c->d_forms, forms.data(), forms.size() * sizeof(InstForm), cudaMemcpyHostToDevice, c->stream));
     }
   }
   if ((st = dalloc(c, &S.nl, (size_t)o.nl_cap * nl_stride_of(c->ncap)))) return st;
@@ -1160,7 +1171,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
       F.h_over_dx = c->opt.closure ? (float)(C.h / c->opt.closure_dx) : 0.f;
     }
     if ((st = dalloc(c, &c->d_cls32, c32.size()))) return st;
-    CUDA_TRY(c, cudaMemcpy(c->d_cls32, c32.data(), c32.size() * sizeof(PClass32), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_cls32, c32.data(), c32.size() * sizeof(PClass32), cudaMemcpyHostToDevice, c->stream));
   }
 
   // ---- pack and copy --------------------------------------------------------------
@@ -1212,15 +1223,15 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
         const size_t off = 9 * (size_t)c->inst_off[q];
         for (int a = 0; a < 7; ++a)
           if (srcs[a])
-            CUDA_TRY(c, cudaMemcpy(dsts[a] + off, srcs[a], 9 * (size_t)p->n * sizeof(double), cudaMemcpyHostToDevice));
+            CUDA_TRY(c, cudaMemcpyAsync(dsts[a] + off, srcs[a], 9 * (size_t)p->n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
       }
     }
-    CUDA_TRY(c, cudaMemcpy(c->d_cls, c->classes.data(), c->classes.size() * sizeof(PClass), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_cls, c->classes.data(), c->classes.size() * sizeof(PClass), cudaMemcpyHostToDevice, c->stream));
     launch_class_constants(c->d_cls, (int)c->classes.size(), o.dim, c->stream);
     CUDA_TRY(c, cudaGetLastError());
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    CUDA_TRY(c, cudaMemcpy(c->d_grids, c->gdevs.data(), ninst * sizeof(GridDev), cudaMemcpyHostToDevice));
-    CUDA_TRY(c, cudaMemcpy(c->d_grids_ref, c->gdevs.data(), ninst * sizeof(GridDev), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_grids, c->gdevs.data(), ninst * sizeof(GridDev), cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_grids_ref, c->gdevs.data(), ninst * sizeof(GridDev), cudaMemcpyHostToDevice, c->stream));
     std::vector<InstState> is(ninst);
     for (int q = 0; q < ninst; ++q) {
       InstState& I = is[q];
@@ -1237,7 +1248,7 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
       I.shepard_counter = it.shepard_counter;
       I.t_stop = 1e300;
     }
-    CUDA_TRY(c, cudaMemcpy(c->d_inst, is.data(), ninst * sizeof(InstState), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_inst, is.data(), ninst * sizeof(InstState), cudaMemcpyHostToDevice, c->stream));
     StepScalars sc;
     std::memset(&sc, 0, sizeof sc);
     sc.n = (int)ntot;
@@ -1245,7 +1256,8 @@ psph_status upload_impl(psph_ctx* c, const psph_particles* parts, int initial) {
     sc.buf = 0;
     sc.rebuild = 1;
     sc.force_rebuild = 1;
-    CUDA_TRY(c, cudaMemcpy(c->d_sc, &sc, sizeof sc, cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_sc, &sc, sizeof sc, cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   }
   c->inout = inout;
   c->inoutcounter = 0;
@@ -1402,7 +1414,7 @@ psph_status inout_fresh(psph_ctx* c) {
     CUDA_TRY(c, cudaStreamSynchronize(s));
     cand.resize((size_t)m);
     if (m > 0)
-      CUDA_TRY(c, cudaMemcpy(cand.data(), c->d_flow_buf, (size_t)m * sizeof(FlowCand), cudaMemcpyDeviceToHost));
+      if ((st = fetch(c, cand.data(), c->d_flow_buf, (size_t)m * sizeof(FlowCand)))) return st;
     std::sort(cand.begin(), cand.end(), [](const FlowCand& a, const FlowCand& b) {
       if (a.cy != b.cy) return a.cy < b.cy;
       if (a.cz != b.cz) return a.cz < b.cz;
@@ -1469,7 +1481,7 @@ psph_status inout_fresh(psph_ctx* c) {
       CUDA_TRY(c, cudaStreamSynchronize(s));
       parts.resize((size_t)std::min(m, n_out));
       if (!parts.empty())
-        CUDA_TRY(c, cudaMemcpy(parts.data(), c->d_flow_buf, parts.size() * sizeof(FlowSlot), cudaMemcpyDeviceToHost));
+        if ((st = fetch(c, parts.data(), c->d_flow_buf, parts.size() * sizeof(FlowSlot)))) return st;
       std::sort(parts.begin(), parts.end(), [](const FlowSlot& a, const FlowSlot& b) { return a.orig < b.orig; });
       if ((st = flow_profile_apply(c, PSPH_FLOW_OUT, parts, temp11, set_v, set_d))) return st;
     } else {
@@ -1496,7 +1508,7 @@ psph_status inout_leave(psph_ctx* c) {
   CUDA_TRY(c, cudaMemcpyAsync(&ndel, c->d_flow_count, sizeof(int), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(c, cudaStreamSynchronize(s));
   std::vector<FlowSlot> del((size_t)ndel);
-  if (ndel > 0) CUDA_TRY(c, cudaMemcpy(del.data(), c->d_flow_buf, (size_t)ndel * sizeof(FlowSlot), cudaMemcpyDeviceToHost));
+  if (ndel > 0 && (st = fetch(c, del.data(), c->d_flow_buf, (size_t)ndel * sizeof(FlowSlot)))) return st;
   std::sort(del.begin(), del.end(), [](const FlowSlot& a, const FlowSlot& b) { return a.orig < b.orig; });
   // AddPart: in-flow particles past InFlowLoc1, in BC.InPart order
   std::vector<FlowSlot> add;
@@ -1796,11 +1808,11 @@ psph_status alive_of(psph_ctx* c, int q, std::vector<std::pair<int, int>>& order
   const Persist& P = sc.buf ? c->PB : c->PA;
   std::vector<uint8_t> alive(n);
   std::vector<int> orig(n);
-  CUDA_TRY(c, cudaMemcpy(alive.data(), c->d_alive, n, cudaMemcpyDeviceToHost));
-  CUDA_TRY(c, cudaMemcpy(orig.data(), P.orig, n * sizeof(int), cudaMemcpyDeviceToHost));
+  if ((st = fetch(c, alive.data(), c->d_alive, n))) return st;
+  if ((st = fetch(c, orig.data(), P.orig, n * sizeof(int)))) return st;
   if (cls_out) {
     cls_out->resize(n);
-    CUDA_TRY(c, cudaMemcpy(cls_out->data(), P.cls, n * sizeof(int), cudaMemcpyDeviceToHost));
+    if ((st = fetch(c, cls_out->data(), P.cls, n * sizeof(int)))) return st;
   }
   // original indices are unique: place each alive slot at its original index
   // (a counting sort, linear in n) instead of sorting the pairs
@@ -2497,7 +2509,8 @@ psph_status psph_pairs_export(psph_ctx* c, int which, int64_t* pairs, int64_t ca
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   if (dcap > 0) {
     const long long k = std::min<long long>((long long)total, dcap);
-    CUDA_TRY(c, cudaMemcpy(pairs, d_out, (size_t)k * 2 * sizeof(long long), cudaMemcpyDeviceToHost));
+    const psph_status st = fetch(c, pairs, d_out, (size_t)k * 2 * sizeof(long long));
+    if (st) return st;
   }
   cudaFreeAsync(d_out, c->stream);
   cudaFreeAsync(d_counter, c->stream);
@@ -2749,19 +2762,20 @@ psph_status psph_closure_attach(psph_ctx* c, const psph_mlp* mlp, double dx) {
         (st = dalloc(c, &c->S.cfeat, 6 * N)) || (st = dalloc(c, &c->S.nut, N)))
       return st;
   }
-  CUDA_TRY(c, cudaMemcpy(c->d_mlp, img, sizeof(MlpImage), cudaMemcpyDeviceToDevice));
+  CUDA_TRY(c, cudaMemcpyAsync(c->d_mlp, img, sizeof(MlpImage), cudaMemcpyDeviceToDevice, c->stream));
   c->opt.closure = 1;
   c->opt.closure_dx = dx;
   {  // the h/dx feature per class, as the FP64 form rounds it
     std::vector<PClass32> c32(c->classes.size());
-    CUDA_TRY(c, cudaMemcpy(c32.data(), c->d_cls32, c32.size() * sizeof(PClass32), cudaMemcpyDeviceToHost));
+    if ((st = fetch(c, c32.data(), c->d_cls32, c32.size() * sizeof(PClass32)))) return st;
     for (size_t q = 0; q < c32.size(); ++q) c32[q].h_over_dx = (float)(c->classes[q].h / dx);
-    CUDA_TRY(c, cudaMemcpy(c->d_cls32, c32.data(), c32.size() * sizeof(PClass32), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpyAsync(c->d_cls32, c32.data(), c32.size() * sizeof(PClass32), cudaMemcpyHostToDevice, c->stream));
   }
   if ((st = sync_scalars(c))) return st;
   c->h_sc->closure_eval = 0;
   c->h_sc->closure_fallback = 0;
-  CUDA_TRY(c, cudaMemcpy(c->d_sc, c->h_sc, sizeof(StepScalars), cudaMemcpyHostToDevice));
+  CUDA_TRY(c, cudaMemcpyAsync(c->d_sc, c->h_sc, sizeof(StepScalars), cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   if (c->graph) {  // the step sequence changes: capture it again
     cudaGraphExecDestroy(c->graph);
     c->graph = nullptr;
@@ -2787,7 +2801,7 @@ psph_status psph_closure_features(psph_ctx* c, float* out) {
   if (st) return st;
   const size_t n = (size_t)c->h_sc->n;
   std::vector<float> f(6 * n);
-  CUDA_TRY(c, cudaMemcpy(f.data(), c->S.cfeat, 6 * n * sizeof(float), cudaMemcpyDeviceToHost));
+  if ((st = fetch(c, f.data(), c->S.cfeat, 6 * n * sizeof(float)))) return st;
   for (size_t r = 0; r < order.size(); ++r)
     for (int k = 0; k < 6; ++k) out[6 * r + k] = f[6 * (size_t)order[r].second + k];
   return PSPH_OK;
