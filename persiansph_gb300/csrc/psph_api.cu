@@ -1874,6 +1874,14 @@ __global__ void dl_gather_kernel(DlBatch b, const int* __restrict__ row, int n) 
     for (int e = 0; e < f.width; ++e) f.dst[(size_t)r * f.width + e] = f.src[at + e];
   }
 }
+// In a domain of two materials the rates are kept for the soil or solid particles, by
+// sorted place: a fluid particle's (strain rates aside, where it sums them) are zero, not
+// what the place's last owner left.
+__global__ void dl_fluid_rates_kernel(DevView v, double* __restrict__ dst, const int* __restrict__ row, int n) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n || row[s] < 0 || v.cls[cur_persist(v).cls[s]].material != 1) return;
+  for (int e = 0; e < 9; ++e) dst[(size_t)row[s] * 9 + e] = 0.0;
+}
 // psph_patch: the caller's row r = row[s] back into slot s (dl_gather_kernel's reverse)
 __global__ void patch_scatter_kernel(double* __restrict__ dst, int stride, int off, int width,
                                      const double* __restrict__ src, const int* __restrict__ row, int n,
@@ -2030,6 +2038,9 @@ psph_status download_impl(psph_ctx* c, int q, psph_particles* out) {
                         f.stride, f.off, f.width};
     }
     if (g.count) dl_gather_kernel<<<nb, 256, 0, s>>>(g, c->dl_row, n);
+    for (int k = 0; k < g.count && o.mixed; ++k)
+      if (g.f[k].src == c->S.rotation_rate || (g.f[k].src == c->S.strain_rate && !o.need_sr))
+        dl_fluid_rates_kernel<<<nb, 256, 0, s>>>(view(c), g.f[k].dst, c->dl_row, n);
   };
   static_assert(kStageWidth <= kDlFields, "a batch's fields");
   size_t values = 0;
