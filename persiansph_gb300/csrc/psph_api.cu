@@ -665,6 +665,7 @@ std::vector<InstForm> instance_forms(const std::vector<PClass>& classes, int nin
     f.spec32 = oq.spec32;
     f.soil32 = oq.soil32;
     f.uniform_eos = oq.uniform_eos;
+    f.uniform_h = oq.uniform_h;
     f.eos_cls = index[(size_t)q][(size_t)oq.eos_cls];
     f.soil_noslip = oq.soil_noslip;
     f.soil_fpm = oq.fpm_wall32;
@@ -679,7 +680,7 @@ std::vector<InstForm> instance_forms(const std::vector<PClass>& classes, int nin
   if (o.spec64 || !(o.mix64 & kMixSpec)) o.mix64 = 0;
   if (o.spec32 || !(o.mix32 & kMixSpec)) o.mix32 = 0;
   if (o.soil32 || !(o.mix_soil & kMixSpec)) o.mix_soil = 0;
-  if (!o.mix64 && !o.mix32 && !o.mix_soil && o.uniform_eos) forms.clear();
+  if (!o.mix64 && !o.mix32 && !o.mix_soil && o.uniform_eos && o.uniform_h) forms.clear();
   return forms;
 }
 

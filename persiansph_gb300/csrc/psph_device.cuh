@@ -130,7 +130,7 @@ struct Spec32 {
 // for bit as it does alone.
 struct InstForm {
   int spec64, spec32, soil32;  // Options' fields of the same names
-  int uniform_eos, eos_cls;
+  int uniform_eos, eos_cls, uniform_h;
   int soil_noslip;
   float soil_fpm;              // the walls' FPMassC (soil32)
   Spec64 spec;

@@ -382,8 +382,9 @@ __global__ void __maxnreg__(FL == 0 || FL == 4 ? 128 : (FL == 1 ? 80 : 96)) forc
   const bool split_sr = SPEC ? CLOSURE : closure;
   const bool own_eos = FL == 4 && wall_eos(v, Ci.inst) < 0;
   const float cf2 = g.cellfac2_32;
-  const bool uniform_h = o.uniform_h;
-  const float ih_u = o.inv_h32;
+  const bool own_h = !SPEC && v.forms;
+  const bool uniform_h = own_h ? v.forms[Ci.inst].uniform_h : o.uniform_h;
+  const float ih_u = own_h ? v.forms[Ci.inst].spec32c.inv_h : o.inv_h32;
   auto pair = [&](const int j, const int code) {
     const float4 oj = v.S.OFF32[j];
     const float4 vjl = ld_early(v.S.V32LO + j);

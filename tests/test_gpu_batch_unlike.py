@@ -59,6 +59,7 @@ CASES = {
     "lattice": lambda: [dam2(), dam2(0.05)],
     "lattice_quintic": lambda: [dam2(kernel=2), dam2(0.05, kernel=2), dam2(alpha=0.2, kernel=2)],
     "lattice_3d": lambda: [dam3(), dam3(0.06)],
+    "lattice_general": lambda: [dam3(lid=0.1), dam3(0.06, lid=0.1), dam3(ti=0.3, ti_init_dist=0.05)],
     "viscosity": lambda: [dam2(), dam2(mu=0.1, mu_ref=0.1)],
     "wall_mass": lambda: [dam2(), dam2(fpmassc=0.8)],
     "sound_speed": lambda: [dam2(), dam2(cs=60.0)],
