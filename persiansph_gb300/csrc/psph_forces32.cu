@@ -612,8 +612,8 @@ __global__ void __maxnreg__(FL == 0 || FL == 4 ? 128 : (FL == 1 ? 80 : 96)) forc
 //    joined at the end by an exact two-sum;
 //  - 2^lg lanes share a particle's list.
 // Measured per step (pair kernel alone, before -> now): 6.7M particles with the
-// closure 4330 -> 2740 us, 1.0M without strain rates 485 -> 320 us, 86k in 2D
-// 24.6 -> 20.4 us, the 920-particle channel 34.8 -> 15.4 us. Register caps: 3D
+// closure 4330 -> 2700 us, 1.0M without strain rates 485 -> 320 us, 86k in 2D
+// 24.6 -> 19.5 us, the 920-particle channel 34.8 -> 14.3 us. Register caps: 3D
 // 128 (136, 144: 3276; the first form of this kernel at 112: 3173, at 96: 3438).
 // ---------------------------------------------------------------------------
 PSPH_D float2 f2(float a, float b) { return make_float2(a, b); }
